@@ -1,4 +1,8 @@
-"""ctypes front end of libportdnn_b200.so working on torch CUDA tensors.
+"""Python front end of libportdnn_b200.so working on torch CUDA tensors.
+
+The operators go through a small extension module (csrc/front.cpp) that checks the tensors and calls the C
+ABI: a call costs the host 4-5 us, most of it the kernel launch, where the same checks in Python and ctypes
+took 14; queries and set-up calls use ctypes.
 
 Function names and argument meaning follow the reference's launch functions
 (include/portdnn/<op>/launch.h); the parameter structs have the reference's field order.
@@ -10,6 +14,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB = None
+_F = None  # the native half of this module (csrc/front.cpp), loaded with the library
 
 FORWARD, INPUT_BACKPROP, FILTER_BACKPROP = 0, 1, 2
 F32, F16, BF16 = 0, 1, 2
@@ -70,16 +75,6 @@ class BatchNormParams(ctypes.Structure):
         [("epsilon", ctypes.c_float), ("momentum", ctypes.c_float), ("input_format", ctypes.c_int)]
 
 
-class _BackpropFusion(ctypes.Structure):
-    _fields_ = [("relu_forward_output", ctypes.c_void_p), ("output_f32", ctypes.c_int), ("accumulate", ctypes.c_int),
-                ("relu_bitmask", ctypes.c_void_p), ("constant_filter", ctypes.c_int)]
-
-
-class _Epilogue(ctypes.Structure):
-    _fields_ = [("bias", ctypes.c_void_p), ("activation", ctypes.c_int), ("alpha", ctypes.c_float),
-                ("beta", ctypes.c_float), ("relu_bitmask", ctypes.c_void_p), ("constant_filter", ctypes.c_int)]
-
-
 def library_path():
     return os.path.join(_HERE, "libportdnn_b200.so")
 
@@ -98,6 +93,23 @@ def lib():
         L.pdnn_noalloc_scratch_bytes.restype = ctypes.c_size_t
         _LIB = L
     return _LIB
+
+
+def _front():
+    """Loads the extension module behind the operators (it links against the library beside it)."""
+    global _F
+    if _F is None:
+        lib()
+        _torch()  # its libraries must be in the process before the extension is
+        path = os.path.join(_HERE, "_front.so")
+        if not os.path.exists(path):
+            raise ImportError("%s is missing: build it with `python -m portdnn_b200.build`" % path)
+        from importlib import machinery, util
+        loader = machinery.ExtensionFileLoader("portdnn_b200._front", path)
+        module = util.module_from_spec(util.spec_from_file_location("portdnn_b200._front", path, loader=loader))
+        loader.exec_module(module)
+        _F = module
+    return _F
 
 
 def _check(status):
@@ -200,74 +212,13 @@ def conv2d(pass_, inp, fil, params, algorithm=ALGO_IM2COL, out=None, workspace=N
     the forward pass beside its output, read by the input backprop in place of relu_forward_output.
     constant_filter (Forward, InputBackprop): filter and bias were not written by the kernel that precedes this
     call in the stream, so the kernel may fetch them while that kernel is still finishing."""
-    torch = _torch()
-    _require_cuda(inp, fil, out, workspace, bias)
-    n_in, n_fil, n_out = conv_sizes(pass_, params)
-    if inp.numel() != n_in or fil.numel() != n_fil:
-        raise ValueError("tensor sizes do not match the parameters: %d/%d, %d/%d" % (inp.numel(), n_in, fil.numel(), n_fil))
-    _require_cuda(relu_bitmask)
-    if relu_bitmask is not None:
-        if pass_ == FILTER_BACKPROP:
-            raise ValueError("relu_bitmask belongs to the forward pass (output) and the input backprop (input)")
-        n_bits = n_out  # forward: the output's mask; input backprop: the mask of dx
-        if relu_bitmask.dtype != torch.uint8 or relu_bitmask.numel() * 8 != n_bits:
-            raise ValueError("relu_bitmask must be a uint8 tensor of one bit per element")
-    backprop_fused = (relu_forward_output is not None or output_f32 or accumulate or
-                      (relu_bitmask is not None and pass_ != FORWARD) or (constant_filter and pass_ == INPUT_BACKPROP))
-    if backprop_fused and (pass_ == FORWARD or (relu_forward_output is not None and pass_ != INPUT_BACKPROP) or
-                           (output_f32 and pass_ != FILTER_BACKPROP)):
-        raise ValueError("relu_forward_output belongs to the input backprop, output_f32 to the filter backprop")
-    if accumulate and out is None:
-        raise ValueError("accumulate needs the tensor to add to as out")
-    _require_cuda(relu_forward_output)
-    if out is None:
-        out = torch.empty(n_out, dtype=torch.float32 if output_f32 else inp.dtype, device=inp.device)
-    if out.numel() != n_out or out.dtype != (torch.float32 if output_f32 else inp.dtype):
-        raise ValueError("output tensor does not match the parameters")
-    ws_elems = workspace.numel() * workspace.element_size() // inp.element_size() if workspace is not None else 0
-    if backprop_fused:
-        if relu_forward_output is not None and relu_forward_output.numel() != n_out:
-            raise ValueError("relu_forward_output must have the shape of the input gradient")
-        fus = _BackpropFusion(relu_forward_output.data_ptr() if relu_forward_output is not None else None, int(output_f32),
-                              int(accumulate),  # accumulate: False / True, or 2 (dx already carries the mask)
-                              relu_bitmask.data_ptr() if relu_bitmask is not None else None, int(bool(constant_filter)))
-        _check(lib().pdnn_conv2d_backprop_fused(pass_, _dtype_code(inp), _ptr(inp), _ptr(fil), _ptr(out),
-                                                ctypes.byref(params), algorithm, ctypes.byref(fus), _ptr(workspace),
-                                                ctypes.c_size_t(ws_elems), _stream()))
-        return out
-    fused = (bias is not None or activation != ACT_NONE or alpha != 1.0 or beta != 0.0 or relu_bitmask is not None or
-             (constant_filter and pass_ == FORWARD))
-    if fused:
-        if pass_ != FORWARD:
-            raise ValueError("the fused epilogue exists for the forward pass only")
-        epi = _Epilogue(bias.data_ptr() if bias is not None else None, activation, alpha, beta,
-                        relu_bitmask.data_ptr() if relu_bitmask is not None else None, int(bool(constant_filter)))
-        st = lib().pdnn_conv2d_fused(_dtype_code(inp), _ptr(inp), _ptr(fil), _ptr(out), ctypes.byref(params), algorithm,
-                                     ctypes.byref(epi), _ptr(workspace), ctypes.c_size_t(ws_elems), _stream())
-    else:
-        st = lib().pdnn_conv2d(pass_, _dtype_code(inp), _ptr(inp), _ptr(fil), _ptr(out), ctypes.byref(params), algorithm,
-                               _ptr(workspace), ctypes.c_size_t(ws_elems), _stream())
-    _check(st)
-    return out
+    return (_F or _front()).conv2d(pass_, inp, fil, params, algorithm, out, workspace, bias, activation, alpha, beta,
+                                   relu_forward_output, output_f32, accumulate, relu_bitmask, constant_filter)
 
 
 def depthwise_conv2d(pass_, inp, fil, params, out=None, workspace=None):
     """depthwise_conv2d::launch<T, ConvType> (include/portdnn/depthwise_conv2d/launch.h:54-91)."""
-    torch = _torch()
-    _require_cuda(inp, fil, out, workspace)
-    p = params
-    x = p.batch * p.in_rows * p.in_cols * p.channels
-    w = p.window_rows * p.window_cols * p.channels * p.channel_multiplier
-    y = p.batch * p.out_rows * p.out_cols * p.channels * p.channel_multiplier
-    n_in, n_fil, n_out = {FORWARD: (x, w, y), INPUT_BACKPROP: (y, w, x), FILTER_BACKPROP: (x, y, w)}[pass_]
-    if inp.numel() != n_in or fil.numel() != n_fil:
-        raise ValueError("tensor sizes do not match the parameters")
-    if out is None:
-        out = torch.empty(n_out, dtype=inp.dtype, device=inp.device)
-    ws_bytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    _check(lib().pdnn_depthwise_conv2d(pass_, _dtype_code(inp), _ptr(inp), _ptr(fil), _ptr(out), ctypes.byref(p),
-                                       _ptr(workspace), ctypes.c_size_t(ws_bytes), _stream()))
-    return out
+    return (_F or _front()).depthwise_conv2d(pass_, inp, fil, params, out, workspace)
 
 
 def depthwise_filter_backprop_noalloc(inp, output_grad, params, out):
@@ -291,107 +242,46 @@ def depthwise_workspace_bytes(pass_, dtype, params):
 def pooling(op, direction, inp, params, out=None):
     """pooling::launch<T, Op, Direction>, two-pointer form (include/portdnn/pooling/launch.h:112-180):
     direction 0 = Forward (x -> y); direction 1 = Backpropagate, Average only (dy -> dx)."""
-    torch = _torch()
-    _require_cuda(inp, out)
-    p = params
-    n_out = (p.batch * p.out_rows * p.out_cols if direction == 0 else p.batch * p.in_rows * p.in_cols) * p.channels
-    if out is None:
-        out = torch.empty(n_out, dtype=inp.dtype, device=inp.device)
-    _check(lib().pdnn_pooling(op, direction, _dtype_code(inp), _ptr(inp), _ptr(out), ctypes.byref(p), _stream()))
-    return out
+    return (_F or _front()).pooling(op, direction, inp, params, out)
 
 
 def pooling_max_grad(op, input_data, output_data, input_backprop, params, out=None, relu_input=False):
     """pooling::launch<T, Max|MaxWithNan, Backpropagate>, four-pointer form
     (include/portdnn/pooling/launch.h:182-257): (x, y, dy) -> dx.  relu_input: x is a ReLU's output and
     dx is to be the gradient with respect to that ReLU's input (pdnn_pooling_max_grad_relu)."""
-    torch = _torch()
-    _require_cuda(input_data, output_data, input_backprop, out)
-    if out is None:
-        out = torch.empty(input_data.numel(), dtype=input_data.dtype, device=input_data.device)
-    fn = lib().pdnn_pooling_max_grad_relu if relu_input else lib().pdnn_pooling_max_grad
-    _check(fn(op, _dtype_code(input_data), _ptr(input_data), _ptr(output_data),
-                                       _ptr(input_backprop), _ptr(out), ctypes.byref(params), _stream()))
-    return out
+    return (_F or _front()).pooling_max_grad(op, input_data, output_data, input_backprop, params, out, relu_input)
 
 
 def pointwise(op, inp, out=None):
     """pointwise::launch<T, Op, Forward> (include/portdnn/pointwise/launch.h:61-100)."""
-    torch = _torch()
-    _require_cuda(inp, out)
-    if out is None:
-        out = torch.empty_like(inp)
-    _check(lib().pdnn_pointwise(op, _dtype_code(inp), _ptr(inp), _ptr(out), ctypes.c_size_t(inp.numel()), _stream()))
-    return out
+    return (_F or _front()).pointwise(op, inp, out)
 
 
 def pointwise_grad(op, output_forward, input_backprop, out=None):
     """pointwise::launch<T, Op, Gradient> (include/portdnn/pointwise/launch.h:133-179)."""
-    torch = _torch()
-    _require_cuda(output_forward, input_backprop, out)
-    if out is None:
-        out = torch.empty_like(output_forward)
-    _check(lib().pdnn_pointwise_grad(op, _dtype_code(output_forward), _ptr(output_forward), _ptr(input_backprop),
-                                     _ptr(out), ctypes.c_size_t(output_forward.numel()), _stream()))
-    return out
+    return (_F or _front()).pointwise_grad(op, output_forward, input_backprop, out)
 
 
 def bias_add(inp, bias, channels, activation=ACT_NONE, out=None):
     """binaryop::launch<T, Add> with lhs_dims={rows, C}, rhs_dims={1, C} (test/bias/bias_fixture.h:78-85)."""
-    torch = _torch()
-    _require_cuda(inp, bias, out)
-    if out is None:
-        out = torch.empty_like(inp)
-    _check(lib().pdnn_bias_add(_dtype_code(inp), _ptr(inp), _ptr(bias), _ptr(out),
-                               ctypes.c_size_t(inp.numel() // channels), int(channels), int(activation), _stream()))
-    return out
+    return (_F or _front()).bias_add(inp, bias, channels, activation, out)
 
 
 def binaryop(op, lhs, lhs_dims, rhs, rhs_dims, out=None):
     """binaryop::launch<T, Op> (include/portdnn/binaryop/launch.h:58-97): lhs (op) rhs with numpy-style
     broadcasting of at most four extents per operand; `op` is one of BINARY_ADD / SUB / MUL / DIV."""
-    torch = _torch()
-    _require_cuda(lhs, rhs, out)
-    lhs_dims, rhs_dims = [int(d) for d in lhs_dims], [int(d) for d in rhs_dims]
-    if out is None:
-        n = max(len(lhs_dims), len(rhs_dims))
-        pad = lambda d: [1] * (n - len(d)) + d
-        numel = 1
-        for x, y in zip(pad(lhs_dims), pad(rhs_dims)):
-            numel *= max(x, y, 0)
-        out = torch.empty(numel, dtype=lhs.dtype, device=lhs.device)
-    ld = (ctypes.c_int * max(len(lhs_dims), 1))(*lhs_dims)
-    rd = (ctypes.c_int * max(len(rhs_dims), 1))(*rhs_dims)
-    _check(lib().pdnn_binaryop(int(op), _dtype_code(lhs), _ptr(lhs), ld, len(lhs_dims), _ptr(rhs), rd, len(rhs_dims),
-                               _ptr(out), _stream()))
-    return out
+    return (_F or _front()).binaryop(op, lhs, lhs_dims, rhs, rhs_dims, out)
 
 
 def scale_blend(a, alpha, b=None, beta=0.0, out=None):
     """out = alpha*a + beta*b, the compat layer's blend (include/portdnn/compat/scaling.hpp:202-281)."""
-    torch = _torch()
-    _require_cuda(a, b, out)
-    if out is None:
-        out = torch.empty_like(a)
-    _check(lib().pdnn_scale_blend(_dtype_code(a), _ptr(a), ctypes.c_float(alpha), _ptr(b), ctypes.c_float(beta),
-                                  _ptr(out), ctypes.c_size_t(a.numel()), _stream()))
-    return out
+    return (_F or _front()).scale_blend(a, alpha, b, beta, out)
 
 
 def matmul(lhs, rhs, batches, m, k, n, transpose_lhs=False, transpose_rhs=False, beta=0.0, out=None):
     """matmul::launch<T, TransposeLHS, TransposeRHS> (include/portdnn/matmul/launch.h:37-90):
     out[b] = beta*out[b] + op(lhs[b]) @ op(rhs[b]), row-major, strided batches."""
-    torch = _torch()
-    _require_cuda(lhs, rhs, out)
-    if lhs.numel() != batches * m * k or rhs.numel() != batches * k * n:
-        raise ValueError("tensor sizes do not match the parameters")
-    if out is None:
-        if beta != 0.0:
-            raise ValueError("beta != 0 needs an output tensor to accumulate into")
-        out = torch.empty(batches * m * n, dtype=lhs.dtype, device=lhs.device)
-    _check(lib().pdnn_matmul(_dtype_code(lhs), int(transpose_lhs), int(transpose_rhs), _ptr(lhs), _ptr(rhs), _ptr(out),
-                             int(batches), int(m), int(k), int(n), ctypes.c_float(beta), _stream()))
-    return out
+    return (_F or _front()).matmul(lhs, rhs, batches, m, k, n, transpose_lhs, transpose_rhs, beta, out)
 
 
 def transpose(inp, dims, permutation, out=None):
@@ -414,16 +304,7 @@ def transpose(inp, dims, permutation, out=None):
 def softmax(inp, batch, rows, cols, channels, gradient=None, out=None):
     """softmax::launch<T, Forward> (gradient None) or <T, Gradient> (inp = the forward output, gradient = dy),
     include/portdnn/softmax/launch.h:64-165."""
-    torch = _torch()
-    _require_cuda(inp, gradient, out)
-    if inp.numel() != batch * rows * cols * channels:
-        raise ValueError("tensor size does not match the parameters")
-    if out is None:
-        out = torch.empty_like(inp)
-    p = SoftmaxParams(channels, batch, rows, cols, 0)
-    _check(lib().pdnn_softmax(0 if gradient is None else 1, _dtype_code(inp), _ptr(inp), _ptr(gradient), _ptr(out),
-                              ctypes.byref(p), _stream()))
-    return out
+    return (_F or _front()).softmax(inp, batch, rows, cols, channels, gradient, out)
 
 
 def batchnorm_params(batch, rows, cols, channels, training, epsilon=1e-3, momentum=0.9):
@@ -433,30 +314,13 @@ def batchnorm_params(batch, rows, cols, channels, training, epsilon=1e-3, moment
 def batchnorm_forward(inp, beta, gamma, mean, variance, params, out=None):
     """batchnorm::launch<T, Backend, Forward> (include/portdnn/batchnorm/launch.h:222-330)
     -> (output, running_mean, running_variance); the last two are None for frozen parameters."""
-    torch = _torch()
-    _require_cuda(inp, beta, gamma, mean, variance, out)
-    if out is None:
-        out = torch.empty_like(inp)
-    rm = rv = None
-    if params.is_training:
-        rm, rv = torch.empty_like(mean), torch.empty_like(variance)
-    _check(lib().pdnn_batchnorm_forward(_dtype_code(inp), _ptr(inp), _ptr(beta), _ptr(gamma), _ptr(mean), _ptr(variance),
-                                        _ptr(rm), _ptr(rv), _ptr(out), ctypes.byref(params), _stream()))
-    return out, rm, rv
+    return (_F or _front()).batchnorm_forward(inp, beta, gamma, mean, variance, params, out)
 
 
 def batchnorm_gradient(inp, gradient, gamma, params, pop_mean=None, pop_variance=None, out=None):
     """batchnorm::launch<T, Backend, Gradient> (include/portdnn/batchnorm/launch.h:332-444)
     -> (input gradient, beta gradient, gamma gradient)."""
-    torch = _torch()
-    _require_cuda(inp, gradient, gamma, pop_mean, pop_variance, out)
-    if out is None:
-        out = torch.empty_like(inp)
-    bg, gg = torch.empty_like(gamma), torch.empty_like(gamma)
-    _check(lib().pdnn_batchnorm_gradient(_dtype_code(inp), _ptr(inp), _ptr(gradient), _ptr(gamma), _ptr(pop_mean),
-                                         _ptr(pop_variance), _ptr(bg), _ptr(gg), _ptr(out), ctypes.byref(params),
-                                         _stream()))
-    return out, bg, gg
+    return (_F or _front()).batchnorm_gradient(inp, gradient, gamma, params, pop_mean, pop_variance, out)
 
 
 def device_error_record(clear=True):

@@ -179,8 +179,10 @@ class ConvStackRunner:
             self.grads = [None] * len(layers)
             conv_ids = [i for i, l in enumerate(layers) if isinstance(l, ConvLayer)]
             self.conv_ids = conv_ids
+            self.conv_index = {i: k for k, i in enumerate(conv_ids)}
             self.bucket = pdist.FilterGradientBucket([self.weights[i].numel() for i in conv_ids], device,
                                                      pad_to=25_500_000)
+            self.grad_views = [self.bucket.view(k) for k in range(len(conv_ids))]
             self.scratch = torch.empty(max(sizes), dtype=self.dtype, device=device)
             last = conv_ids[-1]
             self.dy_last = torch.randn(sizes[last], device=device, generator=g).to(self.dtype)
@@ -198,6 +200,8 @@ class ConvStackRunner:
             for l, n in zip(layers, sizes):
                 names[l.dst] = max(names.get(l.dst, 0), n)
             self.buffers = {k: torch.empty(v, dtype=self.dtype, device=device) for k, v in names.items()}
+            # what each layer writes of its buffer, sliced once (a slice costs the host 1-2 us)
+            self.out_views = [self.buffers[l.dst][:n] for l, n in zip(layers, sizes)]
         self.chunk, self.chunk_layers = None, 0
         if chunk and chunk_layers and not training and first.batch % chunk == 0 and chunk < first.batch:
             self.chunk, self.chunk_layers, batch = chunk, chunk_layers, first.batch
@@ -227,7 +231,7 @@ class ConvStackRunner:
 
     # ---- forward -------------------------------------------------------------------------------
     def _out(self, i):
-        return self.acts[i] if self.training else self.buffers[self.layers[i].dst][:self.sizes[i]]
+        return self.acts[i] if self.training else self.out_views[i]
 
     def _in(self, i):
         j = self.src_idx[i]
@@ -304,7 +308,7 @@ class ConvStackRunner:
                 self.segments.append({"tag": tag, "layers": []})
             self.segments[-1]["layers"].append(i)
         for seg in self.segments:
-            ks = [self.conv_ids.index(i) for i in seg["layers"] if i in self.weights]
+            ks = [self.conv_index[i] for i in seg["layers"] if i in self.weights]
             seg["bucket"] = self.bucket.span(min(ks), max(ks)) if ks else None
 
     def _add_grad(self, j, producer):
@@ -354,10 +358,10 @@ class ConvStackRunner:
                 if l.name.endswith("_1x1b"):
                     # the block's output gradient after its ReLU: what the shortcut branch receives too
                     self._block_grad[l.name[:-5]] = g
-                k = self.conv_ids.index(i)
+                k = self.conv_index[i]
                 f32_out = self.dtype != self.torch.float32
                 add = self.fuse_accumulate and f32_out
-                api.conv2d(api.FILTER_BACKPROP, self._in(i), g, p, algorithm=api.ALGO_IM2COL, out=self.bucket.view(k),
+                api.conv2d(api.FILTER_BACKPROP, self._in(i), g, p, algorithm=api.ALGO_IM2COL, out=self.grad_views[k],
                            output_f32=f32_out, accumulate=add,
                            workspace=self.fbp_workspace if i in self.fbp_ws else None)
                 if j >= 0:
