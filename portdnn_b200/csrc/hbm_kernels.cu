@@ -7,6 +7,7 @@
 //
 // Semantics follow portDNN: src/pooling/kernels.h, src/pooling/operators_impl.h,
 // src/depthwise_conv2d/kernels.h, src/pointwise/kernels.h, src/binaryop/kernels.h.
+#include "column_sums.cuh"
 #include "common.cuh"
 
 #include <cfloat>
@@ -1061,16 +1062,7 @@ __global__ void __launch_bounds__(kFbpRowsWarps * 32, kFbpRowsBlocks)
   }
 }
 
-// Stage 2: dW[i] = sum over slices of partial[slice][i], in slice order (deterministic).
-template <typename T>
-__global__ void __launch_bounds__(kBlock)
-    reduce_slices_kernel(const float* __restrict__ partial, T* __restrict__ out, int slices, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (size_t)gridDim.x * kBlock) {
-    float sum = 0.f;
-    for (int sl = 0; sl < slices; ++sl) sum += partial[(size_t)sl * n + i];
-    out[i] = from_f32<T>(sum);
-  }
-}
+// Stage 2: dW[i] = sum over slices of partial[slice][i], in a fixed order (column_sums.cuh).
 
 // ------------------------------------------------------------------------------------------
 // Pointwise, bias, blend
@@ -2017,7 +2009,7 @@ int launch_depthwise(int pass, int dtype, const void* in, const void* fil, void*
       const int written = launch_fbp_partials<T>(vec, static_cast<const T*>(in), static_cast<const T*>(fil), partial, p, slices, s);
       int st = check_launch("depthwise filter backprop (partial sums)");
       if (st == PDNN_OK) {
-        reduce_slices_kernel<T><<<grid_for(n_out, kBlock, sms), kBlock, 0, s>>>(partial, static_cast<T*>(out), written, n_out);
+        launch_column_sums(partial, written, n_out, sms, s, StoreSum<T>{static_cast<T*>(out), false});
         st = check_launch("depthwise filter backprop (slice reduction)");
       }
       if (own) cudaFreeAsync(partial, s);
@@ -2360,7 +2352,7 @@ int launch_depthwise_filter_backprop_static(int dtype, const void* in, const voi
     const int written = launch_fbp_partials<T>(vec, static_cast<const T*>(in), static_cast<const T*>(dy), partial, p, slices, s);
     int st = check_launch("depthwise filter backprop, fixed scratch (partial sums)");
     if (st != PDNN_OK) return st;
-    reduce_slices_kernel<T><<<grid_for(n_out, kBlock, sms), kBlock, 0, s>>>(partial, static_cast<T*>(dw), written, n_out);
+    launch_column_sums(partial, written, n_out, sms, s, StoreSum<T>{static_cast<T*>(dw), false});
     return check_launch("depthwise filter backprop, fixed scratch (slice reduction)");
   });
 }

@@ -3,6 +3,7 @@
 // store.  The reference composes both from reduce / binaryop / pointwise launches
 // (include/portdnn/internal/softmax/launch_internal.h:45-275,
 // include/portdnn/internal/batchnorm/launch_internal.h:95-640); here each is one to three kernels.
+#include "column_sums.cuh"
 #include "common.cuh"
 
 namespace pdnn {
@@ -382,17 +383,15 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// totals[k][c] = sum over slices of partial[slice][k][c], optionally divided by `divide_by`.
-__global__ void __launch_bounds__(kBlock)
-    batchnorm_totals_kernel(const float* __restrict__ partial, float* __restrict__ totals, int slices, int C,
-                            float divide0, float divide1) {
-  const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= 2 * C) return;
-  const int k = i / C, c = i % C;
-  float sum = 0.f;
-  for (int s = 0; s < slices; ++s) sum += partial[((size_t)s * 2 + k) * C + c];
-  totals[i] = sum / (k == 0 ? divide0 : divide1);
-}
+// totals[k][c] = sum over slices of partial[slice][k][c], divided by divide0 (k = 0) or divide1.
+struct StoreTotals {
+  float* totals;
+  int C;
+  float divide0, divide1;
+  __device__ __forceinline__ void operator()(size_t i, float sum) const {
+    totals[i] = sum / (i < (size_t)C ? divide0 : divide1);
+  }
+};
 
 // Training forward, last step: running = batch * (1 - m) + given * m.
 template <typename T>
@@ -581,21 +580,20 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
     st = get_scratch(&sc, slices, C, s);
     if (st != PDNN_OK) return st;
     const dim3 grid(slices, (C + 31) / 32), vgrid(slices, (C / VN + 31) / 32);
-    const unsigned cgrid = (2 * C + kBlock - 1) / kBlock;
     if (vec)
       batchnorm_sums_vec_kernel<T, VN, 0><<<vgrid, kBlock, 0, s>>>(static_cast<const T*>(input), nullptr, nullptr,
                                                                   nullptr, sc.partial, rows, C, per_slice);
     else
       batchnorm_sums_kernel<T, 0><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), nullptr, nullptr, nullptr,
                                                          sc.partial, rows, C, per_slice);
-    batchnorm_totals_kernel<<<cgrid, kBlock, 0, s>>>(sc.partial, sc.stats0, slices, C, (float)rows, (float)rows);
+    launch_column_sums(sc.partial, slices, 2 * (size_t)C, sms, s, StoreTotals{sc.stats0, C, (float)rows, (float)rows});
     if (vec)
       batchnorm_sums_vec_kernel<T, VN, 1><<<vgrid, kBlock, 0, s>>>(static_cast<const T*>(input), nullptr, sc.stats0,
                                                                   nullptr, sc.partial, rows, C, per_slice);
     else
       batchnorm_sums_kernel<T, 1><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), nullptr, sc.stats0, nullptr,
                                                          sc.partial, rows, C, per_slice);
-    batchnorm_totals_kernel<<<cgrid, kBlock, 0, s>>>(sc.partial, sc.stats1, slices, C, (float)rows, 1.f);
+    launch_column_sums(sc.partial, slices, 2 * (size_t)C, sms, s, StoreTotals{sc.stats1, C, (float)rows, 1.f});
     batchnorm_running_kernel<T><<<(C + kBlock - 1) / kBlock, kBlock, 0, s>>>(
         sc.stats0, sc.stats1, static_cast<const T*>(mean), static_cast<const T*>(variance),
         static_cast<T*>(running_mean), static_cast<T*>(running_variance), C, p.momentum);
@@ -631,15 +629,15 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
     int st = get_scratch(&sc, slices, C, s);
     if (st != PDNN_OK) return st;
     const dim3 grid(slices, (C + 31) / 32), vgrid(slices, (C / VN + 31) / 32);
-    const unsigned cgrid = (2 * C + kBlock - 1) / kBlock, c1grid = (C + kBlock - 1) / kBlock;
+    const unsigned c1grid = (C + kBlock - 1) / kBlock;
     const T *x = static_cast<const T*>(input), *dy = static_cast<const T*>(gradient), *g = static_cast<const T*>(gamma);
     if (p.is_training) {
       if (vec) batchnorm_sums_vec_kernel<T, VN, 0><<<vgrid, kBlock, 0, s>>>(x, dy, nullptr, nullptr, sc.partial, rows, C, per_slice);
       else batchnorm_sums_kernel<T, 0><<<grid, kBlock, 0, s>>>(x, dy, nullptr, nullptr, sc.partial, rows, C, per_slice);
-      batchnorm_totals_kernel<<<cgrid, kBlock, 0, s>>>(sc.partial, sc.stats0, slices, C, (float)rows, (float)rows);
+      launch_column_sums(sc.partial, slices, 2 * (size_t)C, sms, s, StoreTotals{sc.stats0, C, (float)rows, (float)rows});
       if (vec) batchnorm_sums_vec_kernel<T, VN, 1><<<vgrid, kBlock, 0, s>>>(x, dy, sc.stats0, nullptr, sc.partial, rows, C, per_slice);
       else batchnorm_sums_kernel<T, 1><<<grid, kBlock, 0, s>>>(x, dy, sc.stats0, nullptr, sc.partial, rows, C, per_slice);
-      batchnorm_totals_kernel<<<cgrid, kBlock, 0, s>>>(sc.partial, sc.stats1, slices, C, (float)rows, 1.f);
+      launch_column_sums(sc.partial, slices, 2 * (size_t)C, sms, s, StoreTotals{sc.stats1, C, (float)rows, 1.f});
       if (vec)
         batchnorm_grad_training_vec_kernel<T, VN><<<channel_stable_grid(n / VN, C / VN, sms), kBlock, 0, s>>>(
             x, dy, g, sc.stats0, sc.stats1, static_cast<T*>(output), n / VN, C, (float)rows, p.epsilon);
@@ -653,7 +651,7 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
                                                                  C, p.epsilon);
       if (vec) batchnorm_sums_vec_kernel<T, VN, 2><<<vgrid, kBlock, 0, s>>>(x, dy, sc.shift, sc.scale, sc.partial, rows, C, per_slice);
       else batchnorm_sums_kernel<T, 2><<<grid, kBlock, 0, s>>>(x, dy, sc.shift, sc.scale, sc.partial, rows, C, per_slice);
-      batchnorm_totals_kernel<<<cgrid, kBlock, 0, s>>>(sc.partial, sc.stats0, slices, C, 1.f, 1.f);
+      launch_column_sums(sc.partial, slices, 2 * (size_t)C, sms, s, StoreTotals{sc.stats0, C, 1.f, 1.f});
       if (vec)
         batchnorm_grad_frozen_vec_kernel<T, VN><<<channel_stable_grid(n / VN, C / VN, sms), kBlock, 0, s>>>(
             dy, g, static_cast<const T*>(pop_variance), static_cast<T*>(output), n / VN, C, p.epsilon);

@@ -18,6 +18,7 @@
 //
 // Warp roles (192 threads; 320 with the split): warp 0 TMA producer, warp 1 MMA issuer and TMEM
 // owner, warps 2-5 epilogue, warps 6-9 hi/lo split.
+#include "column_sums.cuh"
 #include "tc_gemm.cuh"
 #include "umma.cuh"
 
@@ -2788,16 +2789,6 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms) {
   return f;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, T* __restrict__ out,
-                                                            int splits, size_t n, bool accumulate) {
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
-    float sum = accumulate ? to_f32(out[i]) : 0.f;
-    for (int sp = 0; sp < splits; ++sp) sum += partial[(size_t)sp * n + i];
-    out[i] = from_f32<T>(sum);
-  }
-}
-
 // ---- filter backprop for very few input channels (network stems) ---------------------------------
 // Mirror image of conv_forward_small_c: with the input packed to CP channels per pixel and
 // padded, the gradient of filter row r is one GEMM  dWp[r][64][K] = Xr^T * dy, where a row of
@@ -3084,10 +3075,9 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
   }
   int st = launch_gemm(g, dtype, s);
   if (st == PDNN_OK && use_partial) {
-    const unsigned grid = grid_for(n_out, 256, sms);
-    if (dtype == PDNN_F32 || out_f32) reduce_splits_kernel<float><<<grid, 256, 0, s>>>(partial, static_cast<float*>(dw), f.splits, n_out, accumulate);
-    else if (dtype == PDNN_F16) reduce_splits_kernel<__half><<<grid, 256, 0, s>>>(partial, static_cast<__half*>(dw), f.splits, n_out, accumulate);
-    else reduce_splits_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(partial, static_cast<__nv_bfloat16*>(dw), f.splits, n_out, accumulate);
+    if (dtype == PDNN_F32 || out_f32) launch_column_sums(partial, f.splits, n_out, sms, s, StoreSum<float>{static_cast<float*>(dw), accumulate});
+    else if (dtype == PDNN_F16) launch_column_sums(partial, f.splits, n_out, sms, s, StoreSum<__half>{static_cast<__half*>(dw), accumulate});
+    else launch_column_sums(partial, f.splits, n_out, sms, s, StoreSum<__nv_bfloat16>{static_cast<__nv_bfloat16*>(dw), accumulate});
     st = check_launch("filter backprop split reduction");
   }
   if (own) cudaFreeAsync(partial, s);

@@ -1,0 +1,49 @@
+"""The fixed-order second stage of the split reductions (column_sums.cuh), through operators that end in it:
+few rows of partial sums (one thread per column), row counts around the 32 lanes and the four loads each
+lane has in flight, and column counts that leave the last block ragged."""
+import numpy as np
+import pytest
+
+import portdnn_b200 as pd
+from gpu_util import to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+
+# A sum of n fp32 terms in lanes of at most n / 256 and trees of at most 10 levels, against float64.  The
+# terms are of order 1 and of both signs, so errors are measured against the sum of their magnitudes.
+BOUND = 2.0 ** -23
+
+
+@pytest.mark.parametrize("rows,channels", [(64, 1), (64 * 8, 33), (64 * 9 + 1, 31), (64 * 33 - 5, 40), (64 * 130, 12), (64 * 700 + 3, 64)])
+def test_batchnorm_sums(rows, channels):
+    rng = np.random.default_rng(rows)
+    x = rng.standard_normal((rows, channels)).astype(np.float32)
+    dy = rng.standard_normal((rows, channels)).astype(np.float32)
+    one, zero = np.ones(channels, np.float32), np.zeros(channels, np.float32)
+    p = pd.batchnorm_params(1, 1, rows, channels, True, 1e-3, 0.0)
+    _, mean, var = pd.batchnorm_forward(to_dev(x, "f32"), *(to_dev(t, "f32") for t in (zero, one, zero, one)), p)
+    _, dbeta, dgamma = pd.batchnorm_gradient(to_dev(x, "f32"), to_dev(dy, "f32"), to_dev(one, "f32"), p)
+    x64, dy64 = x.astype(np.float64), dy.astype(np.float64)
+    xc = x64 - x64.mean(0)
+    steps = rows / 256 + 12
+    assert np.all(np.abs(to_host(mean) - x64.mean(0)) <= BOUND * steps * np.abs(x64).mean(0))
+    assert np.all(np.abs(to_host(var) - (xc ** 2).mean(0)) <= BOUND * (steps + 4) * (xc ** 2).mean(0))
+    assert np.all(np.abs(to_host(dbeta) - dy64.sum(0)) <= BOUND * (steps + 2) * np.abs(dy64).sum(0))
+    ref = (dy64 * xc).sum(0) / np.sqrt((xc ** 2).mean(0) + 1e-3)
+    assert np.all(np.abs(to_host(dgamma) - ref) <= BOUND * (steps + 8) * np.abs(dy64 * xc).sum(0))
+
+
+@pytest.mark.parametrize("batch,rows,channels", [(1, 5, 3), (2, 33, 40), (40, 28, 72)])
+def test_depthwise_filter_gradient(batch, rows, channels):
+    rng = np.random.default_rng(channels)
+    p = pd.depthwise_params(batch, rows, rows, channels, 1, 3, 1)
+    x = rng.standard_normal((batch, rows, rows, channels)).astype(np.float32)
+    dy = rng.standard_normal((batch, rows, rows, channels)).astype(np.float32)
+    dw = to_host(pd.depthwise_conv2d(pd.FILTER_BACKPROP, to_dev(x.ravel(), "f32"), to_dev(dy.ravel(), "f32"), p))
+    xp = np.pad(x.astype(np.float64), ((0, 0), (1, 1), (1, 1), (0, 0)))
+    for r in range(3):
+        for c in range(3):
+            terms = xp[:, r:r + rows, c:c + rows] * dy
+            got = dw.reshape(3, 3, channels)[r, c]
+            bound = BOUND * (batch * rows * rows / 256 + 30) * np.abs(terms).sum((0, 1, 2))
+            assert np.all(np.abs(got - terms.sum((0, 1, 2))) <= bound)
