@@ -1,5 +1,6 @@
 // extern "C" entry points declared in include/portdnn_b200.h.
 #include "common.cuh"
+#include "padded_conv.cuh"
 #include "tc_gemm.cuh"
 
 #include <mutex>
@@ -224,6 +225,9 @@ int dispatch_conv(int pass, int dtype, const void* in, const void* fil, void* ou
   if (algorithm != PDNN_ALGO_DIRECT && tc_conv_supported(pass, dtype, in, fil, out, *p)) {
     const int st2 = tc_conv2d(pass, dtype, in, fil, out, *p, epi, fusion, ws, ws_elems, s);
     if (st2 != kNeedsDirect) return st2;
+  } else if (algorithm != PDNN_ALGO_DIRECT && padded_conv_applicable(pass, dtype, *p, epi)) {
+    const int st2 = padded_conv(pass, dtype, in, fil, out, *p, epi, fusion, ws, ws_elems, s);
+    if (st2 != kNeedsDirect) return st2;
   }
   if (pass != PDNN_FORWARD) return run_direct_backprop(pass, dtype, in, fil, out, *p, fusion, s);
   return launch_direct_conv(pass, dtype, in, fil, out, *p, epi, s);
@@ -291,6 +295,7 @@ int pdnn_conv2d_workspace_size(int pass, int dtype, const PdnnConv2DParams* para
   // The implicit-GEMM kernels read the tensors in place; only the filter backprop's split
   // reduction wants scratch, and it can do without (it then allocates for the call).
   size_t elems = tc_conv_workspace_elems(pass, dtype, *params);
+  if (elems == 0) elems = padded_conv_workspace_elems(pass, dtype, *params);
   // Winograd: 16 * (C*K + tiles*C + tiles*K), include/portdnn/conv2d/workspace_size.h:53-73.  It is
   // reported as recommended, not required: without it the layer still runs (on the implicit GEMM).
   if ((algorithm == PDNN_ALGO_WINOGRAD || algorithm == PDNN_ALGO_WINOGRAD_LARGE) &&
