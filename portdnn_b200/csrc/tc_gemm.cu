@@ -1439,6 +1439,253 @@ __global__ void __launch_bounds__(192, 1) umma_gemm_pair2_kernel(const __grid_co
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512u);
 }
 
+// ------------------------------------------------------------------------------------------------
+// Forward-style GEMMs of few tiles (one image through a network, small matrices): a cluster of `splits`
+// CTAs works on one tile, each on its share of the reduction steps, and the partial tiles are added through
+// distributed shared memory in the order of the ranks, so that the result does not vary from run to run.
+// What bounds these layers is latency - of one launch after another, and of the reduction steps of a tile,
+// which the persistent kernel works off on as few as eight CTAs - so a CTA does one tile and leaves, and
+// takes less than half of an SM's shared memory and tensor memory: the set-up of the next launch, and
+// under constant_filter its first filter tiles, run beside the end of this one.
+//   warp 0  TMA producer; warp 1  MMA issuer, owns the TMEM allocation; warps 2..5  accumulator -> shared memory
+//   all     rows [rank, rank + 1) * 128 / splits of the sum, in 16-byte packets: bias, activation, mask, store
+// ------------------------------------------------------------------------------------------------
+constexpr int kClusterThreads = 192;
+constexpr int kClusterBars = 2 * kMaxStages + 1;  // full, empty per stage; accumulator full
+constexpr int kClusterSmem = 111 * 1024;          // two launches share an SM
+
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// Eight columns of a row, summed over the CTAs of the cluster.
+template <int SPLITS>
+__device__ __forceinline__ void sum_ranks(uint32_t addr, float (&v)[8]) {
+  float4 lo[SPLITS], hi[SPLITS];
+#pragma unroll
+  for (int r = 0; r < SPLITS; ++r) {
+    const uint32_t at = cluster_map_shared(addr, (uint32_t)r);
+    lo[r] = ld_cluster_v4(at);
+    hi[r] = ld_cluster_v4(at + 16u);
+  }
+  v[0] = lo[0].x, v[1] = lo[0].y, v[2] = lo[0].z, v[3] = lo[0].w;
+  v[4] = hi[0].x, v[5] = hi[0].y, v[6] = hi[0].z, v[7] = hi[0].w;
+#pragma unroll
+  for (int r = 1; r < SPLITS; ++r) {
+    v[0] += lo[r].x, v[1] += lo[r].y, v[2] += lo[r].z, v[3] += lo[r].w;
+    v[4] += hi[r].x, v[5] += hi[r].y, v[6] += hi[r].z, v[7] += hi[r].w;
+  }
+}
+
+// One 16-byte packet of the result (add: the packet's bias), with the arithmetic of the packed epilogue: rounded to the output type
+// first, then bias (or the earlier contents), activation and mask in that type.
+template <typename OutT>
+__device__ __forceinline__ void finish_packet(const GemmArgs& a, const float (&v)[8], uint4 add, long long off, int col) {
+  using P2 = typename Pair<OutT>::type;
+  const P2 zero2 = Pair<OutT>::splat(0.f), six2 = Pair<OutT>::splat(6.f);
+  OutT* out = static_cast<OutT*>(a.out) + off + col;
+  const bool has_add = a.accumulate != 0 || a.bias != nullptr;
+  if (a.accumulate != 0) add = ld_global_v4(out);
+  const uint32_t aw[4] = {add.x, add.y, add.z, add.w};
+  uint32_t keep[4] = {~0u, ~0u, ~0u, ~0u};
+  if (a.mask_bits != nullptr) {
+    const uint32_t b = static_cast<const uint8_t*>(a.mask_bits)[(off + col) >> 3];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) keep[i] = ((b >> (2 * i)) & 1u ? 0xFFFFu : 0u) | ((b >> (2 * i + 1)) & 1u ? 0xFFFF0000u : 0u);
+  } else if (a.relu_mask != nullptr) {
+    const uint4 m = ld_global_v4(static_cast<const OutT*>(a.relu_mask) + off + col);
+    const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) keep[i] = __hgt2_mask(bits_pair<P2>(mw[i]), zero2);
+  }
+  uint32_t o[4], bits = 0u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    P2 r = Pair<OutT>::pack(v[2 * i], v[2 * i + 1]);
+    if (has_add) r = __hadd2(r, bits_pair<P2>(aw[i]));
+    if (a.act != PDNN_ACT_NONE) r = __hmax2(r, zero2);
+    if (a.act == PDNN_ACT_RELU6) r = __hmin2(r, six2);
+    o[i] = pair_bits(r) & keep[i];
+    const uint32_t pos = __hgt2_mask(r, zero2);
+    bits |= ((pos & 1u) | ((pos >> 15) & 2u)) << (2 * i);
+  }
+  *reinterpret_cast<uint4*>(out) = make_uint4(o[0], o[1], o[2], o[3]);
+  if (a.bitmask_out != nullptr) static_cast<uint8_t*>(a.bitmask_out)[(off + col) >> 3] = (uint8_t)bits;
+}
+
+template <typename OutT>
+__global__ void __launch_bounds__(kClusterThreads, 1) umma_gemm_cluster_kernel(const __grid_constant__ GemmArgs args) {
+  extern __shared__ uint8_t smem_raw[];
+  const GemmArgs& a = args;
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - raw);
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = (int)(threadIdx.x & 31);
+  const int splits = a.splits, rank = (int)blockIdx.x % splits;
+  const int S = a.stages;
+  const uint32_t b_bytes = a.b_step_bytes, stage_bytes = (uint32_t)kABytes + b_bytes;
+  // the barriers come first, the ring after them; the partial tile takes the ring's place at the end
+  const uint32_t ring = base + 1024u;
+  auto full_bar = [&](int s) { return base + 8u * (uint32_t)s; };
+  auto empty_bar = [&](int s) { return base + 8u * (uint32_t)(kMaxStages + s); };
+  const uint32_t acc_bar = base + 8u * (uint32_t)(2 * kMaxStages);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 8 * kClusterBars);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 8 * kClusterBars + 4);
+  if ((int)threadIdx.x < kClusterBars) {
+    mbar_init(base + 8u * threadIdx.x, 1u);
+    if (threadIdx.x == 0) *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), (uint32_t)a.tmem_cols);
+    tmem_relinquish();
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&a.a_map[0]);
+    prefetch_tensormap(&a.b_map);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  TileWalker walker;
+  walker.init(a, (int)blockIdx.x / splits, 1);
+  const TileCoord t = walker.coord(a);
+  const int k0 = rank * a.slabs_per_split, k1 = min(k0 + a.slabs_per_split, a.num_taps * a.cblocks);
+
+  if (warp == 0) {
+    // ------------------------------- producer ------------------------------------------------
+    auto load_a = [&](int s, int tap, int cb) {
+      const TapEntry e = a.taps[tap];
+      warp_tma_load_4d(ring + (uint32_t)s * stage_bytes, &a.a_map[e.a_map], full_bar(s), cb * a.epr, t.w0 + e.dw, t.h0 + e.dh, t.n0);
+    };
+    auto load_b = [&](int s, int tap, int cb) {
+      const uint32_t sb = ring + (uint32_t)s * stage_bytes + (uint32_t)kABytes, fb = full_bar(s);
+      const int kc = cb * a.epr, btap = a.taps[tap].b_tap + t.n0 * a.b_batch_mul;
+      switch (a.b_mode) {
+        case B_MN_3X: warp_tma_load_4d(sb, &a.b_map, fb, 0, kc, t.nf0 / a.epr, btap); break;
+        case B_K_3: warp_tma_load_4d(sb, &a.b_map, fb, kc, t.nf0, btap, 0); break;
+        case B_K_FHWC: warp_tma_load_4d(sb, &a.b_map, fb, kc, btap, t.nf0, 0); break;
+        default:  // B_MN_3, B_MN_FHWC: one copy per 64 columns
+#pragma unroll 1
+          for (int j = 0; j < a.b_boxes; ++j) {
+            const uint32_t to = sb + (uint32_t)j * a.b_box_bytes;
+            if (a.b_mode == B_MN_3) warp_tma_load_4d(to, &a.b_map, fb, t.nf0 + j * a.epr, kc, btap, 0);
+            else warp_tma_load_4d(to, &a.b_map, fb, t.nf0 + j * a.epr, btap, kc, 0);
+          }
+      }
+    };
+    const int cblocks = a.cblocks, tap0 = k0 / cblocks, cb0 = k0 - tap0 * cblocks;
+    const int early = a.early_b != 0 ? min(S, k1 - k0) : 0;  // filter tiles requested before the preceding kernel has ended
+    for (int i = 0, tap = tap0, cb = cb0; i < early; ++i) {
+      warp_arrive_expect_tx(full_bar(i), stage_bytes);
+      load_b(i, tap, cb);
+      if (++cb == cblocks) cb = 0, ++tap;
+    }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    int s = 0;
+    uint32_t ph = 0;
+#pragma unroll 1
+    for (int k = k0, tap = tap0, cb = cb0; k < k1; ++k) {
+      if (k - k0 >= early) {
+        if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g_error_record, a.wait_limit_ns, 0xD00u + (unsigned)s)) break;
+        warp_arrive_expect_tx(full_bar(s), stage_bytes);
+        load_b(s, tap, cb);
+      }
+      load_a(s, tap, cb);
+      if (++cb == cblocks) cb = 0, ++tap;
+      if (++s == S) {
+        s = 0;
+        ph ^= 1u;
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------- MMA issuer -----------------------------------------------
+    const uint64_t a_desc0 = make_smem_desc(0, a.a_lbo, a.a_sbo, a.a_layout);
+    const uint64_t b_desc0 = make_smem_desc(0, a.b_lbo, a.b_sbo, a.b_layout);
+    const uint32_t a_kadv = a.a_kadv >> 4, b_kadv = a.b_kadv >> 4, idesc = a.idesc;
+    int s = 0;
+    uint32_t ph = 0, accumulate = 0u;
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+      if (!mbar_wait(full_bar(s), ph, abort_flag, g_error_record, a.wait_limit_ns, 0xE00u + (unsigned)s)) break;
+      // (a shared-memory address of a cluster carries the CTA's rank above bit 24; a descriptor takes the offset)
+      const uint32_t sa = (ring + (uint32_t)s * stage_bytes) & 0x3FFFFu;
+      const uint64_t da = a_desc0 + (uint64_t)(sa >> 4), db = b_desc0 + (uint64_t)((sa + (uint32_t)kABytes) >> 4);
+      warp_mma_f16(tmem_base, da, db, idesc, accumulate);
+      warp_mma_f16(tmem_base, da + a_kadv, db + b_kadv, idesc, 1u);
+      warp_mma_f16(tmem_base, da + 2 * a_kadv, db + 2 * b_kadv, idesc, 1u);
+      warp_mma_f16(tmem_base, da + 3 * a_kadv, db + 3 * b_kadv, idesc, 1u);
+      accumulate = 1u;
+      warp_commit(empty_bar(s));
+      if (++s == S) {
+        s = 0;
+        ph ^= 1u;
+      }
+    }
+    warp_commit(acc_bar);
+  }
+  // ------------------------------- partial tile -> shared memory ------------------------------
+  // rows of bn floats and 16 bytes more, so that neither the row-wise stores nor the packets below conflict
+  const uint32_t row_bytes = (uint32_t)a.bn * 4u + 16u;
+  if (warp >= 2) {
+    if (mbar_wait(acc_bar, 0u, abort_flag, g_error_record, a.wait_limit_ns, 0xF00u)) {
+      // every copy into the ring has landed and every MMA has read it
+      tc_fence_after_sync();
+      const int q = warp & 3;
+      uint8_t* row = smem + 1024 + (size_t)(q * 32 + lane) * row_bytes;
+#pragma unroll 1
+      for (int c0 = 0; c0 < a.bn; c0 += 32) {
+        uint32_t acc[32];
+        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, acc);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<uint4*>(row + (size_t)(c0 + 4 * j) * 4) = make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+      }
+    }
+    tc_fence_before_sync();
+  }
+  if (warp != 0) grid_dependency_wait();  // the stores below, and what they add or mask with
+  // a thread's packets all lie in the same columns: kClusterThreads is a multiple of the packets of a row
+  const int packets = a.bn >> 3, pk = (int)threadIdx.x % packets, col = t.nf0 + pk * 8;
+  uint4 bias = make_uint4(0u, 0u, 0u, 0u);
+  if (a.bias != nullptr && col < a.ext_cols) bias = ld_global_v4(static_cast<const OutT*>(a.bias) + col);
+  __syncwarp();
+  cluster_sync_all();
+  // ------------------------------- the CTA's rows of the sum ----------------------------------
+  if (!*abort_flag) {
+    const int rows = kTileM / splits, items = rows * packets;
+    const int sh_w = __ffs(a.etw) - 1, sh_h = __ffs(a.eth) - 1;
+#pragma unroll 2
+    for (int i = (int)threadIdx.x; i < items; i += kClusterThreads) {
+      const int row = rank * rows + i / packets;
+      const int w = t.w0 + (row & (a.etw - 1)), h = t.h0 + ((row >> sh_w) & (a.eth - 1)), n = t.n0 + (row >> (sh_w + sh_h));
+      if (!(w < a.ext_w && h < a.ext_h && n < a.ext_n && col < a.ext_cols)) continue;
+      const uint32_t addr = base + 1024u + (uint32_t)row * row_bytes + (uint32_t)pk * 32u;
+      float v[8];
+      if (splits == 8) sum_ranks<8>(addr, v);
+      else if (splits == 4) sum_ranks<4>(addr, v);
+      else sum_ranks<2>(addr, v);
+      finish_packet<OutT>(a, v, bias, (long long)n * a.stride_n + (long long)h * a.stride_h + (long long)w * a.stride_w, col);
+    }
+  } else {
+    const uint64_t t0 = global_timer_ns();  // loads already issued may still be landing in shared memory
+    while (global_timer_ns() - t0 < 200000ull) {
+    }
+  }
+  // no CTA leaves while another may still read its partial tile
+  __syncwarp();
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, (uint32_t)a.tmem_cols);
+  }
+}
+
 // ================================================================================================
 // Host side: tensor maps and launch plans
 // ================================================================================================
@@ -2054,6 +2301,82 @@ int launch_gemm_multi(const GemmArgs* list, int count, cudaStream_t s) {
   return check_launch("tensor-core gemm (several GEMMs)");
 }
 
+// ---- GEMMs of few tiles on clusters (umma_gemm_cluster_kernel) -------------------------------------
+// Number of CTAs to a tile for a GEMM of `row_tiles` row tiles and `ksteps` reduction steps, or 0 where the
+// persistent kernel is the better one.  The tiles are 64 columns wide: a step pulls its bytes through one SM's
+// port to L2 (0.3 us for A and B of 64 columns, hardly more for 128), so what helps is more CTAs, not
+// wider tiles.  Measured (f16, one image, us a launch in a chain of launches; persistent / 1, 2, 4, 8 CTAs):
+//   7x7   512 -> 512   3x3, 72 steps: 27.7 / 24.9  13.9  8.6  6.5    14x14 256 -> 256  3x3, 36: 16.2 / 15.3  9.0  6.9  6.2
+//   7x7   2048 -> 512  1x1, 32 steps: 14.0 / 13.2   7.9  5.6  4.7    28x28 128 -> 128  3x3, 18: 10.7 /  9.8  6.5  5.7
+//   14x14 1024 -> 256  1x1, 16 steps:  8.9 /  9.3   6.1  5.2  5.4    28x28 512 -> 128  1x1,  8:  5.4 /  6.8  4.9  5.1  5.9
+// One CTA to a tile gains nothing over the persistent kernel, nor do fewer than four steps to a CTA; more
+// CTAs than SMs lose (8 images, 14x14 256 -> 256 3x3: 2 CTAs 9.6, 4 CTAs 10.2, 8 CTAs 20.0).
+constexpr int kClusterColumns = 64;
+int cluster_splits(int dtype, long long row_tiles, int cols, int ksteps, int sms) {
+  if (dtype == PDNN_F32 || cols % 8 != 0) return 0;
+  const long long tiles = row_tiles * ceil_div(cols, kClusterColumns);
+  for (int splits : {8, 4, 2})
+    if (tiles * splits <= sms && 4 * splits <= ksteps && (splits - 1) * ceil_div(ksteps, splits) < ksteps) return splits;
+  return 0;
+}
+
+// The packed epilogue's conditions; out and strides of `g` are set.
+bool cluster_epilogue_ok(const GemmArgs& g) {
+  return g.alpha == 1.f && g.beta == 0.f && g.out_dtype != PDNN_F32 && aligned16(g.out) && (g.bias == nullptr || aligned16(g.bias)) &&
+         (g.relu_mask == nullptr || g.mask_bits != nullptr || aligned16(g.relu_mask)) &&
+         (g.act == PDNN_ACT_NONE || g.act == PDNN_ACT_RELU || g.act == PDNN_ACT_RELU6);
+}
+
+int launch_gemm_cluster(const GemmArgs& g, int splits, cudaStream_t s) {
+  GemmKernel kernel = g.out_dtype == PDNN_F16 ? umma_gemm_cluster_kernel<__half> : umma_gemm_cluster_kernel<__nv_bfloat16>;
+  {
+    static std::mutex mu;
+    static bool opted_in[kMaxDevices] = {};
+    const int dev = current_device();
+    if (dev < 0 || dev >= kMaxDevices) return fail(PDNN_ALLOCATION_PROBLEM, "tensor-core gemm: no usable current device");
+    std::lock_guard<std::mutex> lock(mu);
+    if (!opted_in[dev]) {
+      if (cudaFuncSetAttribute(umma_gemm_cluster_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem) != cudaSuccess ||
+          cudaFuncSetAttribute(umma_gemm_cluster_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(PDNN_ALLOCATION_PROBLEM, "cannot opt in to %d bytes of shared memory", kClusterSmem);
+      }
+      opted_in[dev] = true;
+    }
+  }
+  const int steps = g.num_taps * g.cblocks;
+  const long long tiles = (long long)g.n_tiles * g.tiles_w * g.tiles_h * g.tiles_n;
+  GemmArgs args = g;
+  args.tap_pack = 1;
+  args.wait_limit_ns = kWaitLimitNs;
+  args.splits = splits;
+  args.slabs_per_split = ceil_div(steps, splits);
+  args.tmem_cols = kClusterColumns;
+  const int stage = kABytes + g.bn * 128, head = 2048;  // alignment and barriers
+  args.stages = std::min(std::min(kMaxStages, args.slabs_per_split), (kClusterSmem - head) / stage);
+  const size_t partial = (size_t)kTileM * (g.bn * 4 + 16);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * splits));
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = head + std::max((size_t)args.stages * stage, partial);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)splits;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, args);
+  if (le != cudaSuccess) {
+    cudaGetLastError();
+    return fail(PDNN_ALLOCATION_PROBLEM, "tensor-core gemm (clusters): launch failed: %s", cudaGetErrorString(le));
+  }
+  if (g.bitmask_out != nullptr) bitmask_written_flag() = true;
+  return check_launch("tensor-core gemm (clusters)");
+}
+
 void set_epilogue(GemmArgs& g, const PdnnConvEpilogue* epi) {
   g.bitmask_out = nullptr;
   g.bias = nullptr;
@@ -2110,7 +2433,7 @@ bool make_parity_maps(GemmArgs& g, int dtype, bool mn_major, const void* x, cons
 // Output side of a forward convolution: y is [N, Ho, Wo, K].
 // plan_out (may be null): the finished plan is stored there instead of being launched.
 int finish_forward(GemmArgs& g, int dtype, void* y, const PdnnConv2DParams& p, const PdnnConvEpilogue* epi,
-                   cudaStream_t s, int y_ld = 0, GemmArgs* plan_out = nullptr) {
+                   cudaStream_t s, int y_ld = 0, GemmArgs* plan_out = nullptr, int cluster = 0) {
   const size_t es = dtype_size(dtype);
   const long long ld = y_ld > 0 ? y_ld : p.features;
   set_epilogue(g, epi);
@@ -2124,6 +2447,7 @@ int finish_forward(GemmArgs& g, int dtype, void* y, const PdnnConv2DParams& p, c
   g.stride_h = (long long)p.out_cols * ld;
   g.stride_n = (long long)p.out_rows * p.out_cols * ld;
   g.vec_ok = 1;
+  if (cluster != 0) return cluster_epilogue_ok(g) ? launch_gemm_cluster(g, cluster, s) : kPlanAgain;
   const uint64_t od[4] = {(uint64_t)p.features, (uint64_t)p.out_cols, (uint64_t)p.out_rows, (uint64_t)p.batch};
   const uint64_t os[3] = {(uint64_t)ld * es, (uint64_t)p.out_cols * ld * es, (uint64_t)p.out_rows * p.out_cols * ld * es};
   if (!setup_store(g, dtype, od, os)) return (g.halo || g.pair) ? kPlanAgain : PDNN_INVALID_PARAMETER;
@@ -2364,7 +2688,7 @@ __global__ void __launch_bounds__(256) split_lo_kernel(const float* __restrict__
 
 int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnConv2DParams& p,
                  const PdnnConvEpilogue* epi, cudaStream_t s, bool try_halo = true, bool try_cta_pair = true,
-                 const ConvLd* ld = nullptr, GemmArgs* plan_out = nullptr) {
+                 const ConvLd* ld = nullptr, GemmArgs* plan_out = nullptr, bool try_cluster = true) {
   if (plan_out != nullptr && dtype == PDNN_F32) return PDNN_INVALID_PARAMETER;  // (the fp32 plan owns scratch)
   const int x_ld = ld != nullptr ? ld->x : 0, y_ld = ld != nullptr ? ld->y : 0;
   const uint64_t w_ld = ld != nullptr && ld->w > 0 ? (uint64_t)ld->w : (uint64_t)p.features;
@@ -2399,6 +2723,10 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   g.tiles_n = ceil_div(p.batch, g.tn);
   const long long row_tiles = (long long)g.tiles_w * g.tiles_h * g.tiles_n;
   const int ksteps_all = p.window_rows * p.window_cols * ceil_div(p.channels, epr);
+  // One image, few tiles and a long reduction: clusters that share a tile's steps.  From two images on every
+  // plan adds the terms of a sum in the same order, so that an image's result does not depend on how many
+  // others are in its batch (running the first layers in slices of the batch relies on it).
+  const int cluster = (try_cluster && !halo && plan_out == nullptr && p.batch == 1) ? cluster_splits(dtype, row_tiles, p.features, ksteps_all, sms) : 0;
   // Long reductions over filters too large to keep in shared memory are bound by the bytes that
   // pass through an SM's shared memory per MMA (the operand reads of the tensor core and the TMA
   // fills share its 128 bytes per cycle): the two pipelines then share one B tile per stage (pair
@@ -2410,7 +2738,7 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   const int pair_bn_auto = (p.features % 256 == 0 && p.features >= 512) ? 256 : 128;
   const bool pair_auto = ksteps_all >= (p.features >= 256 ? 32 : 16) &&
                          (row_tiles / 2) * ceil_div(p.features, pair_bn_auto) >= sms;
-  const bool pairing = try_halo && !halo && dtype != PDNN_F32 && hwcf && p.features % 128 == 0 && pair_auto &&
+  const bool pairing = try_halo && !halo && cluster == 0 && dtype != PDNN_F32 && hwcf && p.features % 128 == 0 && pair_auto &&
                        row_tiles >= 2 && (!epi || epi->beta == 0.f);
   // Pairs of row tiles with 256 columns go to clusters of two CTAs (umma_gemm_pair2_kernel) when the
   // epilogue is the plain packed one: half the B operand reads per SM, double-buffered accumulators.
@@ -2433,6 +2761,8 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
       g.pair_dim = 3;  // an odd count leaves the last pair half empty: loads read zeros, stores are clipped
       g.tiles_n = ceil_div(g.tiles_n, 2);
     }
+  } else if (cluster != 0) {
+    g.bn = kClusterColumns;
   } else {
     g.bn = pick_bn(row_tiles, p.features, hwcf ? epr : 16, dtype == PDNN_F32 ? 128 : 256, sms, ksteps_all);
     // A single tap with a long reduction into exactly 256 features: one 256-column tile per row tile
@@ -2528,11 +2858,12 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
     if (w_split != nullptr) cudaFreeAsync(w_split, s);
     return PDNN_INVALID_PARAMETER;
   }
-  const int status = finish_forward(g, dtype, y, p, epi, s, y_ld, plan_out);
+  const int status = finish_forward(g, dtype, y, p, epi, s, y_ld, plan_out, cluster);
   if (w_split != nullptr) cudaFreeAsync(w_split, s);
+  if (status == kPlanAgain && cluster != 0) return conv_forward(dtype, x, w, y, p, epi, s, try_halo, try_cta_pair, ld, plan_out, false);
   if (status == kPlanAgain)  // first without the CTA pairs, then without halo / pair mode
-    return g.cta_pair ? conv_forward(dtype, x, w, y, p, epi, s, try_halo, false, ld, plan_out)
-                      : conv_forward(dtype, x, w, y, p, epi, s, false, false, ld, plan_out);
+    return g.cta_pair ? conv_forward(dtype, x, w, y, p, epi, s, try_halo, false, ld, plan_out, try_cluster)
+                      : conv_forward(dtype, x, w, y, p, epi, s, false, false, ld, plan_out, try_cluster);
   return status;
 }
 
@@ -2544,7 +2875,7 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
 // tap) are left as they are.
 int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, const PdnnConv2DParams& p,
                         const void* relu_mask, const void* mask_bits, int accumulate, bool constant_filter, cudaStream_t s,
-                        bool try_halo = true) {
+                        bool try_halo = true, bool try_cluster = true) {
   bool mask_pending = false;  // some parity class could not apply the mask in its epilogue
   const size_t es = dtype_size(dtype);
   const int sms = device_sm_count();
@@ -2610,13 +2941,16 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
           if (pos_mod(qh + p.pad_rows - r, p.stride_rows) == 0 && pos_mod(qw + p.pad_cols - c, p.stride_cols) == 0) ++class_taps;
       if (class_taps == 0 && accumulate == 2) continue;  // nothing to add, and what is there is masked already
       const int ksteps_all = class_taps * ceil_div(p.features, epr);
+      // few tiles: clusters, as in the forward pass (the classes of a strided layer run side by side instead)
+      const int cluster = (try_cluster && !halo && p.stride_rows == 1 && p.stride_cols == 1)
+                              ? cluster_splits(dtype, row_tiles, p.channels, ksteps_all, sms) : 0;
       // Pair mode as in the forward pass (two row tiles share the filter tile of a stage); the output
       // columns are the channels here.
       // 128-column tiles throughout (the epilogue of this pass is the longer one when it applies the
       // ReLU mask, and two accumulator buffers hide it), pairs from 16 reduction steps on.
       const int pair_bn_auto = 128;
       const bool pair_auto = ksteps_all >= 16 && (row_tiles / 2) * ceil_div(p.channels, pair_bn_auto) >= sms;
-      const bool pairing = try_halo && !halo && dtype != PDNN_F32 && hwcf && p.channels % 128 == 0 && row_tiles >= 2 &&
+      const bool pairing = try_halo && !halo && cluster == 0 && dtype != PDNN_F32 && hwcf && p.channels % 128 == 0 && row_tiles >= 2 &&
                            pair_auto;
       if (pairing) {
         g.pair = 1;
@@ -2631,6 +2965,8 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
           g.pair_dim = 3;
           g.tiles_n = ceil_div(g.tiles_n, 2);
         }
+      } else if (cluster != 0) {
+        g.bn = kClusterColumns;
       } else {
         g.bn = pick_bn(row_tiles, p.channels, hwcf ? 16 : epr, 128, sms, ksteps_all);
       }
@@ -2698,7 +3034,7 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
       g.relu_mask = (relu_mask != nullptr && !mask_pending && aligned16(relu_mask))
                         ? static_cast<const char*>(relu_mask) + ((size_t)qh * p.in_cols + qw) * p.channels * es
                         : nullptr;
-      if (mask_bits != nullptr && !mask_pending && p.channels % 64 == 0 && ((uintptr_t)mask_bits & 7u) == 0) {
+      if (mask_bits != nullptr && !mask_pending && (p.channels % 64 == 0 || cluster != 0) && ((uintptr_t)mask_bits & 7u) == 0) {
         // the mask as one bit per element: the class's first pixel starts ((qh * W + qw) * C) / 8 bytes in
         g.mask_bits = static_cast<const char*>(mask_bits) + ((size_t)qh * p.in_cols + qw) * p.channels / 8;
         g.relu_mask = g.mask_bits;  // "a mask is applied in the epilogue"
@@ -2713,6 +3049,12 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
       g.stride_h = (long long)p.stride_rows * p.in_cols * p.channels;
       g.stride_n = (long long)p.in_rows * p.in_cols * p.channels;
       g.vec_ok = 1;
+      if (cluster != 0) {
+        g.accumulate = accumulate ? 1 : 0;
+        if (!cluster_epilogue_ok(g) || ((relu_mask != nullptr || mask_bits != nullptr) && g.relu_mask == nullptr))
+          return conv_input_backprop(dtype, dy, w, dx, p, relu_mask, mask_bits, accumulate, constant_filter, s, try_halo, false);
+        return launch_gemm_cluster(g, cluster, s);  // (stride 1: the only class)
+      }
       {
         const uint64_t od[4] = {(uint64_t)p.channels, (uint64_t)Wq, (uint64_t)Hq, (uint64_t)p.batch};
         const uint64_t os[3] = {(uint64_t)p.stride_cols * p.channels * es,
@@ -2728,7 +3070,7 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
           planned = setup_store(g, dtype, od, os);
         }
         if (!planned) {
-          if (g.halo || g.pair) return conv_input_backprop(dtype, dy, w, dx, p, relu_mask, mask_bits, accumulate, constant_filter, s, false);  // plan again without the halo / pairing
+          if (g.halo || g.pair) return conv_input_backprop(dtype, dy, w, dx, p, relu_mask, mask_bits, accumulate, constant_filter, s, false, try_cluster);  // plan again without the halo / pairing
           return PDNN_INVALID_PARAMETER;
         }
       }
@@ -3260,7 +3602,10 @@ int tc_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, void*
   g.a_mn = tl ? 1 : 0;
   const int m_tiles = ceil_div(m, kTileM);
   const int b_mn = tr ? 0 : 1;
-  g.bn = pick_bn((long long)m_tiles * batches, n, b_mn ? epr : 16, dtype == PDNN_F32 ? 128 : 256, sms, ceil_div(k, epr));
+  const int cluster =
+      (!tl && beta == 0.f && !out_f32) ? cluster_splits(dtype, (long long)m_tiles * batches, n, ceil_div(k, epr), sms) : 0;
+  g.bn = cluster != 0 ? kClusterColumns
+                 : pick_bn((long long)m_tiles * batches, n, b_mn ? epr : 16, dtype == PDNN_F32 ? 128 : 256, sms, ceil_div(k, epr));
   g.n_tiles = ceil_div(n, g.bn);
   set_operand_layout(g, dtype, b_mn);
   g.taps[0] = TapEntry{0, 0, 0, 0};
@@ -3338,6 +3683,7 @@ int tc_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, void*
   g.out_dtype = out_f32 ? PDNN_F32 : dtype;
   g.ext_cols = n;
   g.vec_ok = 1;
+  if (cluster != 0 && cluster_epilogue_ok(g)) return launch_gemm_cluster(g, cluster, s);
   {
     const uint64_t eo = dtype_size(g.out_dtype);
     const uint64_t od[4] = {(uint64_t)n, (uint64_t)m, 1, (uint64_t)batches};
