@@ -180,11 +180,13 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// Max-pool gradient when the windows tile the input exactly (stride == window, no padding,
-// in == out * stride: the 2x2/2 pools of VGG).  Every input element belongs to exactly one window,
-// so one thread per output packet reads its window once, finds per channel the first element equal
-// to y (the same rule as above) and writes dy there and zero elsewhere: x, y and dy are read once
-// and dx is written once.
+// Max-pool gradient when the windows do not overlap (stride == window, no padding: the 2x2/2 pools of VGG,
+// on images of any size).  Every input element belongs to one window at most, so one thread per output
+// packet reads its window once, finds per channel the first element equal to y (the same rule as above)
+// and writes dy there and zero elsewhere: x, y and dy are read once and dx is written once.  Windows that
+// reach over the edge are cut; rows and columns that no window covers get their zeros from the threads
+// of the last window row and column.  Bound by HBM.  16 x 113x151x64, 2x2/2, fp32 (262 MB): with both kernels
+// of the general path (winner map and gather) 85 us, here 33.
 template <typename T, int OP, int V, typename Index>
 __global__ void __launch_bounds__(kBlock)
     pool_max_grad_tiled_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ dy,
@@ -204,8 +206,10 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
     for (int i = 0; i < V; ++i) open[i] = true;
     const size_t base = ((size_t)n * p.in_rows + (size_t)oh * p.stride_rows) * p.in_cols + (size_t)ow * p.stride_cols;
-    for (int r = 0; r < p.window_rows; ++r)
-      for (int c = 0; c < p.window_cols; ++c) {
+    const int rows_left = p.in_rows - oh * p.stride_rows, cols_left = p.in_cols - ow * p.stride_cols;
+    const int rows = min(p.window_rows, rows_left), cols = min(p.window_cols, cols_left);
+    for (int r = 0; r < rows; ++r)
+      for (int c = 0; c < cols; ++c) {
         const size_t off = ((base + (size_t)r * p.in_cols + c) * p.channels) + (size_t)cv * V;
         float xv[V], g[V];
         load_vec<T, V>(x + off, xv);
@@ -217,6 +221,15 @@ __global__ void __launch_bounds__(kBlock)
         }
         store_vec<T, V>(dx + off, g);
       }
+    const bool below = oh == p.out_rows - 1 && rows_left > rows, right = ow == p.out_cols - 1 && cols_left > cols;
+    if (below || right) {
+      // the rest of the window's rows to the right, and of its columns below
+      const float zeros[V] = {};
+      const int all_rows = below ? rows_left : rows, all_cols = right ? cols_left : cols;
+      for (int r = 0; r < all_rows; ++r)
+        for (int c = r < rows ? cols : 0; c < all_cols; ++c)
+          store_vec<T, V>(dx + ((base + (size_t)r * p.in_cols + c) * p.channels) + (size_t)cv * V, zeros);
+    }
   }
 }
 
@@ -1787,9 +1800,10 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
     const T *xt = static_cast<const T*>(x), *yt = static_cast<const T*>(y), *dyt = static_cast<const T*>(dy);
     T* dxt = static_cast<T*>(dx);
     if (vec && small && p.pad_rows == 0 && p.pad_cols == 0 && p.stride_rows == p.window_rows &&
-        p.stride_cols == p.window_cols && p.in_rows == p.out_rows * p.stride_rows &&
-        p.in_cols == p.out_cols * p.stride_cols) {
-      // the windows tile the input: one pass
+        p.stride_cols == p.window_cols && (p.out_rows - 1) * p.stride_rows < p.in_rows &&
+        (p.out_cols - 1) * p.stride_cols < p.in_cols && p.in_rows < (p.out_rows + 1) * p.stride_rows &&
+        p.in_cols < (p.out_cols + 1) * p.stride_cols) {
+      // no window overlaps another, and less than a window is left over at the edges: one pass
       const unsigned g1 = grid_for(out_items, kBlock, sms);
       if (op == PDNN_POOL_MAX)
         pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX, VN, unsigned><<<g1, kBlock, 0, s>>>(xt, yt, dyt, dxt, p, (unsigned)out_items);
