@@ -541,19 +541,53 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// The same when one window covers the whole image (global pooling): every pixel of an image
-// receives dy / (rows * cols); one division by a runtime value per thread instead of the window walk.
-template <typename T, int V>
+// Global average pooling (one window that is the whole image): a thread owns one 32-bit word of channels and
+// adds the image's pixels in order, eight loads in flight.  The general kernel's packet of 16 bytes per thread
+// leaves too few threads (one block for one image of 2048 channels), and its window loop waits for one load
+// after another.  7x7x2048 f16, 250 images (51 MB): 22.7 -> 11.4 us;
+// one image: 10 us less.
+template <typename T>
 __global__ void __launch_bounds__(kBlock)
-    pool_avg_grad_global_kernel(const T* __restrict__ dy, T* __restrict__ dx, unsigned cvecs, unsigned per_image,
-                                float count, unsigned n_items) {
+    pool_avg_global_kernel(const T* __restrict__ x, T* __restrict__ y, unsigned words, unsigned pixels, unsigned n_items) {
+  constexpr int E = 4 / (int)sizeof(T);
   for (unsigned idx = blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += gridDim.x * kBlock) {
-    const unsigned n = idx / per_image, cv = idx % cvecs;  // per_image is a multiple of cvecs
+    const unsigned n = idx / words, wd = idx - n * words;
+    const unsigned* xp = reinterpret_cast<const unsigned*>(x) + (size_t)n * pixels * words + wd;
+    float acc[E] = {};
+#pragma unroll 8
+    for (unsigned i = 0; i < pixels; ++i) {
+      const unsigned raw = __ldg(xp + (size_t)i * words);
+      const T* v = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+      for (int k = 0; k < E; ++k) acc[k] += to_f32(v[k]);
+    }
+    unsigned out;
+#pragma unroll
+    for (int k = 0; k < E; ++k) reinterpret_cast<T*>(&out)[k] = from_f32<T>(acc[k] / (float)pixels);
+    reinterpret_cast<unsigned*>(y)[idx] = out;
+  }
+}
+
+// Threads and tiles of the gradient: a block takes 32 packets of channels of one image, eight threads to a
+// packet, each with every eighth pixel.
+constexpr int kGlobalPoolLanes = 8;
+
+// Its gradient: every pixel of an image receives dy / pixels.  250 x 7x7x2048 f16 (51 MB written): 21.2 -> 9.5 us.
+template <typename T, int V>
+__global__ void __launch_bounds__(32 * kGlobalPoolLanes)
+    pool_avg_grad_global_kernel(const T* __restrict__ dy, T* __restrict__ dx, unsigned cvecs, unsigned tiles, unsigned pixels,
+                                unsigned n_blocks) {
+  const unsigned tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
+  for (unsigned block = blockIdx.x; block < n_blocks; block += gridDim.x) {
+    const unsigned n = block / tiles, cv = (block - n * tiles) * 32u + tx;
+    if (cv >= cvecs) continue;
     float dv[V];
     load_vec<T, V>(dy + ((size_t)n * cvecs + cv) * V, dv);
 #pragma unroll
-    for (int i = 0; i < V; ++i) dv[i] = dv[i] / count;  // the division of the general kernel, for equal results
-    store_vec<T, V>(dx + (size_t)idx * V, dv);
+    for (int k = 0; k < V; ++k) dv[k] = dv[k] / (float)pixels;  // the division of the general kernel, for equal results
+    T* to = dx + ((size_t)n * pixels * cvecs + cv) * V;
+#pragma unroll 4
+    for (unsigned i = ty; i < pixels; i += kGlobalPoolLanes) store_vec<T, V>(to + (size_t)i * cvecs * V, dv);
   }
 }
 
@@ -1728,13 +1762,20 @@ int launch_pooling(int op, int direction, int dtype, const void* in, void* out, 
     const size_t pixels = direction == 0 ? (size_t)p.batch * p.out_rows * p.out_cols
                                          : (size_t)p.batch * p.in_rows * p.in_cols;
     const size_t items = pixels * (p.channels / (vec ? VN : 1));
-    if (direction == 1 && vec && p.out_rows == 1 && p.out_cols == 1 && p.pad_rows == 0 && p.pad_cols == 0 &&
-        p.window_rows == p.in_rows && p.window_cols == p.in_cols && items < 0xFFFF0000ull) {
-      const unsigned cvecs = (unsigned)(p.channels / VN);
-      pool_avg_grad_global_kernel<T, VN><<<grid_for(items, kBlock, sms), kBlock, 0, s>>>(
-          static_cast<const T*>(in), static_cast<T*>(out), cvecs, (unsigned)(p.in_rows * p.in_cols) * cvecs,
-          (float)(p.in_rows * p.in_cols), (unsigned)items);
-      return check_launch("pooling average gradient (global)");
+    if (op == PDNN_POOL_AVERAGE && vec && p.out_rows == 1 && p.out_cols == 1 && p.pad_rows == 0 && p.pad_cols == 0 &&
+        p.window_rows == p.in_rows && p.window_cols == p.in_cols &&
+        (size_t)p.batch * p.in_rows * p.in_cols * p.channels < 0xFF000000ull) {
+      const unsigned cvecs = (unsigned)(p.channels / VN), tiles = (cvecs + 31u) / 32u, px = (unsigned)(p.in_rows * p.in_cols);
+      const unsigned n_blocks = (unsigned)p.batch * tiles, most = (unsigned)sms * 32u;
+      const unsigned blocks = n_blocks < most ? n_blocks : most;
+      const T* from = static_cast<const T*>(in);
+      constexpr unsigned E = 4 / (unsigned)sizeof(T);
+      const unsigned words = (unsigned)p.channels / E, items0 = (unsigned)p.batch * words;
+      if (direction == 0)
+        pool_avg_global_kernel<T><<<grid_for(items0, kBlock, sms), kBlock, 0, s>>>(from, static_cast<T*>(out), words, px, items0);
+      else
+        pool_avg_grad_global_kernel<T, VN><<<blocks, 32 * kGlobalPoolLanes, 0, s>>>(from, static_cast<T*>(out), cvecs, tiles, px, n_blocks);
+      return check_launch(direction == 0 ? "pooling average (global)" : "pooling average gradient (global)");
     }
     const unsigned grid = grid_for(items, kBlock, sms);
     const bool wide = items >= 0xFFFFFFFFull - (size_t)grid * kBlock;

@@ -1,5 +1,6 @@
-"""Pooling forms with kernels of their own - max-pool gradients of windows that do not overlap - at the sizes
-where they can go wrong: windows cut by the edge, rows and columns that no window covers, ties, NaN."""
+"""Pooling forms with kernels of their own - max-pool gradients of windows that do not overlap, and global
+average pools - at the sizes where they can go wrong: windows cut by the edge, rows and columns that no window
+covers, ties, NaN; fewer pixels than threads to a packet, a last tile of few packets."""
 import numpy as np
 import pytest
 import torch
@@ -38,3 +39,21 @@ def test_max_grad_of_disjoint_windows(rows, cols, window, same, with_nan, dtype)
                     hits = np.argwhere((win == top) | (np.isnan(win) & np.isnan(top)))
                     ref[i, r * window + hits[0][0], s * window + hits[0][1], k] = dy[i, r, s, k]
     assert np.array_equal(to_host(dx).reshape(ref.shape), ref)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("n,rows,cols,c", [(1, 1, 1, 8), (2, 1, 5, 264), (3, 7, 7, 256), (1, 9, 8, 1288), (150, 2, 3, 2048)])
+def test_global_average(n, rows, cols, c, dtype):
+    rng = np.random.default_rng(c)
+    p = pd.pool_params(n, rows, cols, c, 1, 1, False)
+    p.window_rows, p.window_cols, p.out_rows, p.out_cols = rows, cols, 1, 1
+    x = to_dev(rng.standard_normal((n, rows * cols, c)).astype(np.float32), dtype)
+    dy = to_dev(rng.standard_normal((n, 1, c)).astype(np.float32), dtype)
+    y, dx = pd.pooling(pd.POOL_AVERAGE, 0, x.reshape(-1), p), pd.pooling(pd.POOL_AVERAGE, 1, dy.reshape(-1), p)
+    unit = {"f32": 2.0 ** -24, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[dtype]
+    # one rounding to the type, and fp32 sums of at most 72 terms and one division
+    ref = x.double().mean(1)
+    bound = unit * (ref.abs() + 2.0 ** -13) * 1.01 + 73 * 2.0 ** -24 * x.double().abs().mean(1)
+    assert ((y.view(n, c).double() - ref).abs() <= bound).all()
+    share = (dy.float() / torch.full_like(dy, rows * cols, dtype=torch.float32)).to(dy.dtype)
+    assert torch.equal(dx.view(n, rows * cols, c), share.expand(n, rows * cols, c))
