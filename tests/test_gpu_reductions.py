@@ -47,3 +47,21 @@ def test_depthwise_filter_gradient(batch, rows, channels):
             got = dw.reshape(3, 3, channels)[r, c]
             bound = BOUND * (batch * rows * rows / 256 + 30) * np.abs(terms).sum((0, 1, 2))
             assert np.all(np.abs(got - terms.sum((0, 1, 2))) <= bound)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("rows,channels", [(1, 8), (37, 128), (9, 256), (250, 1000), (3, 1032)])
+def test_softmax_gradient(rows, channels, dtype):
+    """Packets of a lane from one to the four it holds, and the widths before and behind them."""
+    rng = np.random.default_rng(channels)
+    y = np.exp(rng.standard_normal((rows, channels)))
+    y = to_dev((y / y.sum(1, keepdims=True)).astype(np.float32), dtype)
+    dy = to_dev(rng.standard_normal((rows, channels)).astype(np.float32), dtype)
+    dx = pd.softmax(y.reshape(-1), rows, 1, 1, channels, gradient=dy.reshape(-1)).view(rows, channels).double()
+    y64, dy64 = y.double(), dy.double()
+    terms = y64 * dy64
+    ref = (dy64 - terms.sum(1, keepdim=True)) * y64
+    unit = 2.0 ** -24 if dtype == "f32" else 2.0 ** -11
+    # one rounding to the type (smallest f16 numbers: 2^-25), fp32 sums of at most channels / 32 + 5 additions in a row
+    slack = BOUND * (channels / 32 + 8) * (terms.abs().sum(1, keepdim=True) + dy64.abs()) * y64
+    assert ((dx - ref).abs() <= unit * ref.abs() * 1.01 + slack + (2.0 ** -25 if dtype == "f16" else 0.0)).all()
