@@ -65,3 +65,37 @@ def test_softmax_gradient(rows, channels, dtype):
     # one rounding to the type (smallest f16 numbers: 2^-25), fp32 sums of at most channels / 32 + 5 additions in a row
     slack = BOUND * (channels / 32 + 8) * (terms.abs().sum(1, keepdim=True) + dy64.abs()) * y64
     assert ((dx - ref).abs() <= unit * ref.abs() * 1.01 + slack + (2.0 ** -25 if dtype == "f16" else 0.0)).all()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("rows,channels", [(1, 8), (31, 8), (64, 136), (97, 128), (5000, 264), (40000, 8)])
+def test_batchnorm_moments_far_from_zero(rows, channels, dtype):
+    """The one-pass moments where the mean is large against the deviations: fewer rows than row lanes, slices
+    that end inside a batch, channel tiles with idle lanes."""
+    rng = np.random.default_rng(rows)
+    x = to_dev((32.0 + rng.standard_normal((rows, channels))).astype(np.float32), dtype)
+    dy = to_dev((8.0 + rng.standard_normal((rows, channels))).astype(np.float32), dtype)
+    one, zero = (to_dev(np.full(channels, v, np.float32), dtype) for v in (1.0, 0.0))
+    p = pd.batchnorm_params(1, 1, rows, channels, True, 1e-3, 0.0)
+    out, mean, var = (t.double().view(-1, channels) for t in pd.batchnorm_forward(x.reshape(-1), zero, one, zero, one, p))
+    dx, dbeta, dgamma = (t.double().view(-1, channels) for t in pd.batchnorm_gradient(x.reshape(-1), dy.reshape(-1), one, p))
+    x64, dy64 = x.double(), dy.double()
+    m, xc = x64.mean(0), x64 - x64.mean(0)
+    v, dc = (xc ** 2).mean(0), dy64 - dy64.mean(0)
+    # one rounding to the type, and fp32 means with an error of a few units of 32 (or 8), which enters the sums
+    # around them twice
+    unit = 2.0 ** -24 if dtype == "f32" else 2.0 ** -8
+    near = lambda got, ref, slack: bool(((got - ref).abs() <= 1.01 * unit * ref.abs() + slack).all())
+    e = 2.0 ** -24 * (rows / 256 + 12)
+    assert near(out, x64 / (1 + 1e-3) ** 0.5, 2.0 ** -20 * x64.abs())
+    assert near(mean[0], m, 33 * e)
+    assert near(var[0], v, 2 * 33 * e * xc.abs().mean(0) + 4 * e * v)
+    assert near(dbeta[0], dy64.sum(0), 9 * e * rows)
+    sd = (v + 1e-3).sqrt()
+    cov = (xc * dc).sum(0)
+    cov_slack = 33 * e * dc.abs().sum(0) + 9 * e * xc.abs().sum(0) + 4 * e * (xc * dc).abs().sum(0)
+    assert near(dgamma[0], cov / sd, cov_slack / sd * 1.01 + 33 * e * (cov / sd).abs() / sd ** 2)
+    ref = (dc - xc * (cov / rows / (v + 1e-3))) / sd
+    share = cov.abs() / rows / (v + 1e-3)
+    slack = (9 * e + 2.0 ** -20 * dy64.abs() + (33 * e + 2.0 ** -20 * x64.abs()) * share + xc.abs() * (cov_slack / rows + 66 * e * share) / (v + 1e-3)) / sd
+    assert near(dx, ref, 2 * slack)
