@@ -1475,6 +1475,199 @@ __global__ void __launch_bounds__(192, 1) umma_gemm_pair2_kernel(const __grid_co
 }
 
 // ------------------------------------------------------------------------------------------------
+// CTA-pair variant of the filter gradient: dW[tap] = x^T dy on tiles of 256 channels x 256 features, both
+// operands MN-major.  A stage is 64 pixels; each CTA of the cluster loads its own 128 channels of x and 128
+// of the 256 features of dy, rank 0 issues the MMAs of 256 x 256 x 16, and each CTA adds its own 128 rows of the
+// accumulator to the gradient (or to the split's partial sums) through the staged fp32 epilogue while the other
+// accumulator buffer takes the next tile.
+// What bounds the tiles of 128 x 128 in one CTA is shared memory: per 64-pixel step TMA writes 32 KB and the MMAs
+// read 32 KB of it again, 512 cycles at 128 bytes a cycle for 256 cycles of math.  Here the same bytes carry
+// twice the math.  256 images, f16, added to an fp32 gradient: 3x3 256 -> 256 at 14x14 48.3 -> 40.4 us (1.47
+// PFLOP/s), 1x1 1024 -> 512 at 14x14 51.3 -> 42.1 us, 1x1 512 -> 2048 at 7x7 30.5 -> 26.7 us.
+// The roles and barriers are those of umma_gemm_pair2_kernel.
+// ------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(192, 1) umma_gemm_filter_pair_kernel(const __grid_constant__ GemmArgs args) {
+  extern __shared__ uint8_t smem_raw[];
+  const GemmArgs& a = args;
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - raw);
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = (int)(threadIdx.x & 31);
+  const uint32_t rank = cluster_cta_rank();
+  const bool leader = rank == 0;
+  const int S = a.stages;
+  constexpr uint32_t kStage = 2u * kABytes;  // 64 pixels of 128 channels and of 128 features
+  const uint32_t staging_off = (uint32_t)S * kStage;
+  const uint32_t bar_off = staging_off + (uint32_t)a.nsw * 4u * 4096u;
+  uint8_t* bar_mem = smem + bar_off;
+  const uint32_t bar_base = base + bar_off;
+  auto full_bar = [&](int s) { return bar_base + 8u * (uint32_t)s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (uint32_t)(kMaxStages + s); };
+  auto acc_full_bar = [&](int b) { return bar_base + 8u * (uint32_t)(2 * kMaxStages + b); };
+  auto acc_empty_bar = [&](int b) { return bar_base + 8u * (uint32_t)(2 * kMaxStages + 2 + b); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_mem + 8 * (2 * kMaxStages + 4));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * (2 * kMaxStages + 4) + 4);
+
+  if ((int)threadIdx.x < 2 * kMaxStages + 4) {  // one barrier per thread
+    const int j = (int)threadIdx.x;
+    mbar_init(bar_base + 8u * (uint32_t)j, j >= 2 * kMaxStages + 2 ? 8u : 1u);
+    if (j == 0) *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&a.a_map[0]);
+    prefetch_tensormap(&a.b_map);
+    prefetch_tensormap(&a.out_map);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(smem_u32(tmem_slot), 512u);
+    tmem_relinquish_pair();
+  }
+  // the peer's barriers are initialised before anything of this CTA signals them
+  tc_fence_before_sync();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait();
+  grid_launch_dependents();
+
+  const int total_tiles = a.n_tiles * a.tiles_w * a.num_taps * a.splits;
+  const int first_tile = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
+  TileWalker walker;
+  walker.init(a, first_tile, tile_step);
+  // the CTA's part of a tile: 128 of its 256 channels
+  auto coord = [&] {
+    TileCoord t = walker.coord(a);
+    t.w0 = walker.d1 * 256 + (int)rank * kTileM;
+    return t;
+  };
+
+  if (warp == 0) {
+    // ------------------------------- producer ------------------------------------------------
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
+      const TileCoord t = coord();
+      const TapEntry e = a.taps[t.tap];
+      const CUtensorMap* amap = &a.a_map[e.a_map];
+      const int f0 = t.nf0 + (int)rank * 128;
+      int iw = t.ks_begin % a.slabs_w, ih = (t.ks_begin / a.slabs_w) % a.slabs_h, in = t.ks_begin / (a.slabs_w * a.slabs_h);
+#pragma unroll 1
+      for (int ks = t.ks_begin; ks < t.ks_end; ++ks) {
+        if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g_error_record, a.wait_limit_ns, 0x1100u + (unsigned)s)) {
+          ok = false;
+          break;
+        }
+        const uint32_t fb = full_bar(s);
+        if (leader) warp_arrive_expect_tx(fb, 2u * kStage);  // the bytes of both CTAs
+        const uint32_t sa = base + (uint32_t)s * kStage;
+        const int kw = iw * a.tw, kh = ih * a.th, kn = in * a.tn;
+        warp_tma_load_4d_pair(sa, amap, fb, t.w0, kw + e.dw, kh + e.dh, kn);
+        warp_tma_load_4d_pair(sa + kABytes / 2, amap, fb, t.w0 + 64, kw + e.dw, kh + e.dh, kn);
+        warp_tma_load_4d_pair(sa + kABytes, &a.b_map, fb, f0, kw, kh, kn);
+        warp_tma_load_4d_pair(sa + kABytes + kABytes / 2, &a.b_map, fb, f0 + 64, kw, kh, kn);
+        if (++iw == a.slabs_w) {
+          iw = 0;
+          if (++ih == a.slabs_h) {
+            ih = 0;
+            ++in;
+          }
+        }
+        if (++s == S) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------- MMA issuer (rank 0) --------------------------------------
+    if (leader) {
+      const uint64_t a_desc0 = make_smem_desc(0, a.a_lbo, a.a_sbo, a.a_layout);
+      const uint64_t b_desc0 = make_smem_desc(0, a.b_lbo, a.b_sbo, a.b_layout);
+      const uint32_t a_kadv = a.a_kadv >> 4, b_kadv = a.b_kadv >> 4, idesc = a.idesc;
+      int s = 0;
+      uint32_t ph = 0, buf = 0, aph = 0;
+      bool ok = true;
+#pragma unroll 1
+      for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
+        const TileCoord t = coord();
+        if (!mbar_wait(acc_empty_bar((int)buf), aph ^ 1u, abort_flag, g_error_record, a.wait_limit_ns, 0x1200u + buf)) break;
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + buf * 256u;
+        uint32_t accumulate = 0u;
+#pragma unroll 1
+        for (int ks = t.ks_begin; ks < t.ks_end; ++ks) {
+          if (!mbar_wait(full_bar(s), ph, abort_flag, g_error_record, a.wait_limit_ns, 0x1300u + (unsigned)s)) {
+            ok = false;
+            break;
+          }
+          const uint32_t sa = (base + (uint32_t)s * kStage) & 0x3FFFFu;  // offset inside the CTA's shared memory
+          const uint64_t da = a_desc0 + (uint64_t)(sa >> 4), db = b_desc0 + (uint64_t)((sa + kABytes) >> 4);
+          warp_mma_f16_pair(d_tmem, da, db, idesc, accumulate);
+          warp_mma_f16_pair(d_tmem, da + a_kadv, db + b_kadv, idesc, 1u);
+          warp_mma_f16_pair(d_tmem, da + 2 * a_kadv, db + 2 * b_kadv, idesc, 1u);
+          warp_mma_f16_pair(d_tmem, da + 3 * a_kadv, db + 3 * b_kadv, idesc, 1u);
+          accumulate = 1u;
+          warp_commit_pair(empty_bar(s), cluster_map_shared(empty_bar(s), 1u));  // both CTAs may refill the stage
+          if (++s == S) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+        if (!ok) break;
+        warp_commit_pair(acc_full_bar((int)buf), cluster_map_shared(acc_full_bar((int)buf), 1u));
+        if (++buf == 2u) {
+          buf = 0;
+          aph ^= 1u;
+        }
+      }
+    }
+  } else {
+    // ------------------------------- epilogue (own 128 channels) ------------------------------
+    const int q = warp & 3;  // TMEM lanes [32q, 32q+32)
+    uint32_t store_count = 0;
+    WarpStore ws;
+    ws.nsw = a.nsw;
+    const uint32_t my_staging = staging_off + (uint32_t)(warp - 2) * (uint32_t)a.nsw * 4096u;
+    ws.buf = smem + my_staging;
+    ws.buf_addr = base + my_staging;
+    ws.qw = q * 32;
+    ws.qh = ws.qn = 0;
+    uint32_t buf = 0, aph = 0;
+#pragma unroll 1
+    for (int tile = first_tile; tile < total_tiles; tile += tile_step, walker.advance()) {
+      const TileCoord t = coord();
+      if (!mbar_wait(acc_full_bar((int)buf), aph, abort_flag, g_error_record, a.wait_limit_ns, 0x1400u + buf)) break;
+      tc_fence_after_sync();
+      epilogue_tile_tma<float>(a, t, tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256u, lane, false, ws, store_count);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(acc_empty_bar((int)buf) & kPeerBitMask);  // rank 0 collects both CTAs
+      if (++buf == 2u) {
+        buf = 0;
+        aph ^= 1u;
+      }
+    }
+    if (lane == 0) bulk_wait_group<0>();
+  }
+
+  // ------------------------------- teardown ---------------------------------------------------
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) {
+    }
+    __syncthreads();
+  }
+  // neither CTA leaves (and frees its shared and tensor memory) while the other may still use them
+  cluster_sync_all();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, 512u);
+}
+
+// ------------------------------------------------------------------------------------------------
 // Forward-style GEMMs of few tiles (one image through a network, small matrices): a cluster of `splits`
 // CTAs works on one tile, each on its share of the reduction steps, and the partial tiles are added through
 // distributed shared memory in the order of the ranks, so that the result does not vary from run to run.
@@ -1970,7 +2163,7 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
   // the filter tiles are the part of the L2 -> SM traffic that never changes.
   if (g.cta_pair) {
     // one pipeline per CTA: a stage is the CTA's A tile and its half of the B tile
-    if (split || !g.tma_store || !g.epi_fast || g.relu_mask != nullptr || g.bn != 256) return false;
+    if (split || !g.tma_store || g.epi_fast == g.a_mn || g.relu_mask != nullptr || g.bn != 256) return false;
     g.groups = 1;
     g.acc_bufs = 2;
     g.acc_stride = 256;
@@ -2073,7 +2266,8 @@ GemmKernel select_grouped_kernel(int epi, int out_dtype) {
 // Launch of the CTA-pair kernel: clusters of two CTAs, one cluster per pair of SMs.
 int launch_gemm_pair2(const GemmArgs& g, long long total_pairs, cudaStream_t s) {
   const bool bits = g.bitmask_out != nullptr;
-  GemmKernel kernel = g.out_dtype == PDNN_F16 ? (bits ? umma_gemm_pair2_kernel<__half, true> : umma_gemm_pair2_kernel<__half, false>)
+  GemmKernel kernel = g.a_mn ? umma_gemm_filter_pair_kernel
+                      : g.out_dtype == PDNN_F16 ? (bits ? umma_gemm_pair2_kernel<__half, true> : umma_gemm_pair2_kernel<__half, false>)
                                               : (bits ? umma_gemm_pair2_kernel<__nv_bfloat16, true>
                                                       : umma_gemm_pair2_kernel<__nv_bfloat16, false>);
   const size_t smem = 1024 + (size_t)g.stages * 2 * kABytes + (size_t)g.nsw * 4 * 4096 + kBarBlockBytes + (size_t)g.bias_smem_bytes;
@@ -2088,7 +2282,7 @@ int launch_gemm_pair2(const GemmArgs& g, long long total_pairs, cudaStream_t s) 
       bool ok = true;
       for (GemmKernel k : {GemmKernel(umma_gemm_pair2_kernel<__half, false>), GemmKernel(umma_gemm_pair2_kernel<__half, true>),
                            GemmKernel(umma_gemm_pair2_kernel<__nv_bfloat16, false>),
-                           GemmKernel(umma_gemm_pair2_kernel<__nv_bfloat16, true>)})
+                           GemmKernel(umma_gemm_pair2_kernel<__nv_bfloat16, true>), GemmKernel(umma_gemm_filter_pair_kernel)})
         ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) == cudaSuccess;
       if (!ok) {
         cudaGetLastError();
@@ -3258,7 +3452,10 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
 
 struct FbpPlan {
   int tw, th, tn, slabs_w, slabs_h, slabs_n, splits, slabs_per_split, m_tiles, n_tiles, bn, tap_pack;
+  bool pair;  // tiles of 256 x 256 on clusters of two CTAs (m_tiles counts those)
 };
+
+constexpr long long kMinPairSlabs = 16;
 
 FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms) {
   FbpPlan f;
@@ -3267,6 +3464,26 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms) {
   f.slabs_w = ceil_div(p.out_cols, f.tw);
   f.slabs_h = ceil_div(p.out_rows, f.th);
   f.slabs_n = ceil_div(p.batch, f.tn);
+  f.pair = false;
+  // Whole tiles of 256 channels x 256 features: CTA pairs, as many splits as fill the device once, if each is long
+  // enough to pay for adding its 256 KB tile.  From eight slabs down there is nothing left of the gain (24
+  // images: 13.4 -> 13.2 us, through partial sums 16.9 -> 17.4), and a single tile means a partial sum per cluster
+  // (28x28 256 -> 256 1x1, 256 images: 39.4 -> 39.3 us, through partial sums 47 -> 50).
+  if (dtype != PDNN_F32 && p.channels % 256 == 0 && p.features % 256 == 0 && sms % 2 == 0) {
+    const long long tiles = (long long)(p.channels / 256) * (p.features / 256) * p.window_rows * p.window_cols;
+    const long long slabs = (long long)f.slabs_w * f.slabs_h * f.slabs_n, want = std::max<long long>(1, (sms / 2) / tiles);
+    const long long per = (slabs + want - 1) / want;
+    if (per >= kMinPairSlabs && tiles >= 2) {
+      f.pair = true;
+      f.m_tiles = p.channels / 256;
+      f.n_tiles = p.features / 256;
+      f.bn = 256;
+      f.tap_pack = 1;
+      f.slabs_per_split = (int)per;
+      f.splits = (int)((slabs + per - 1) / per);
+      return f;
+    }
+  }
   f.m_tiles = ceil_div(p.channels, kTileM);
   const int max_bn = dtype == PDNN_F32 ? 128 : 256;
   // 128-column tiles: two accumulator buffers per pipeline, so the fp32 epilogue of one tile overlaps the
@@ -3499,6 +3716,10 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
   g.slabs_per_split = f.slabs_per_split;
   g.split_is_batch = 0;
   set_operand_layout(g, dtype, 1);
+  if (f.pair) {
+    g.cta_pair = 1;
+    g.idesc = make_idesc(dtype == PDNN_BF16 ? 1 : 0, 1, 1, 256, 256);
+  }
   const uint32_t box[4] = {(uint32_t)epr, (uint32_t)f.tw, (uint32_t)f.th, (uint32_t)f.tn};
   if (!make_parity_maps(g, dtype, true, x, p, box)) return PDNN_INVALID_PARAMETER;
   {
@@ -3525,7 +3746,8 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
   float* partial = nullptr;
   bool own = false;
   const bool reduce = try_reduce && accumulate && (out_f32 || dtype == PDNN_F32) && aligned16(dw);
-  const bool use_partial = !reduce && (f.splits > 1 || accumulate);
+  // (the CTA pairs' epilogue writes fp32 only)
+  const bool use_partial = !reduce && (f.splits > 1 || accumulate || (f.pair && !out_f32));
   if (use_partial) {
     const size_t need_bytes = (size_t)f.splits * n_out * sizeof(float);
     if (ws != nullptr && ws_elems * es >= need_bytes && aligned16(ws)) {
@@ -3706,7 +3928,7 @@ size_t tc_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p) {
   int sms = device_sm_count();
   if (sms <= 0) sms = 148;
   const FbpPlan f = plan_filter_backprop(dtype, p, sms);
-  if (f.splits <= 1) return 0;
+  if (f.splits <= 1 && !f.pair) return 0;
   const size_t bytes = (size_t)f.splits * p.window_rows * p.window_cols * p.channels * p.features * sizeof(float);
   return (bytes + dtype_size(dtype) - 1) / dtype_size(dtype);
 }
