@@ -18,6 +18,7 @@ constexpr int kSumFlat = 256;  // threads of a block without row lanes
 template <int LANES, typename Finish>
 __global__ void __launch_bounds__(32 * LANES)
     column_sums_kernel(const float* __restrict__ m, int rows, size_t n, Finish finish) {
+  overlap_wait();
   __shared__ float red[LANES][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (size_t first = (size_t)blockIdx.x * 32; first < n; first += (size_t)gridDim.x * 32) {
@@ -48,6 +49,7 @@ __global__ void __launch_bounds__(32 * LANES)
 template <typename Finish>
 __global__ void __launch_bounds__(kSumFlat)
     column_sums_flat_kernel(const float* __restrict__ m, int rows, size_t n, Finish finish) {
+  overlap_wait();
   for (size_t i = (size_t)blockIdx.x * kSumFlat + threadIdx.x; i < n; i += (size_t)gridDim.x * kSumFlat) {
     float sum = 0.f;
 #pragma unroll 8
@@ -62,11 +64,11 @@ __global__ void __launch_bounds__(kSumFlat)
 template <typename Finish>
 void launch_column_sums(const float* m, int rows, size_t n, int sms, cudaStream_t s, Finish finish) {
   if (rows <= 8 || n >= (size_t)sms * 1024)
-    column_sums_flat_kernel<<<grid_for(n, kSumFlat, sms), kSumFlat, 0, s>>>(m, rows, n, finish);
+    launch_overlapped(column_sums_flat_kernel<Finish>, grid_for(n, kSumFlat, sms), kSumFlat, s, m, rows, n, finish);
   else if (rows >= 256 || n < 4096)
-    column_sums_kernel<32><<<grid_for(n, 32, sms), 32 * 32, 0, s>>>(m, rows, n, finish);
+    launch_overlapped(column_sums_kernel<32, Finish>, grid_for(n, 32, sms), 32 * 32, s, m, rows, n, finish);
   else
-    column_sums_kernel<8><<<grid_for(n, 32, sms), 32 * 8, 0, s>>>(m, rows, n, finish);
+    launch_overlapped(column_sums_kernel<8, Finish>, grid_for(n, 32, sms), 32 * 8, s, m, rows, n, finish);
 }
 
 // The plain finish: out[i] = sum, or out[i] += sum.

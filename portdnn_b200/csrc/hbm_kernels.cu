@@ -60,6 +60,7 @@ __device__ __forceinline__ void store_vec(T* p, const float (&v)[V]) {
 template <typename T, int OP, int V, typename Index>
 __global__ void __launch_bounds__(kBlock) pool_forward_kernel(const T* __restrict__ x, T* __restrict__ y,
                                                               PdnnPoolingParams p, Index n_items) {
+  overlap_wait();
   const Index cvecs = (Index)(p.channels / V);
   for (Index idx = (Index)blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += (Index)gridDim.x * kBlock) {
     const Index cv = idx % cvecs;
@@ -191,6 +192,7 @@ template <typename T, int OP, int V, typename Index>
 __global__ void __launch_bounds__(kBlock)
     pool_max_grad_tiled_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ dy,
                                T* __restrict__ dx, PdnnPoolingParams p, Index n_items) {
+  overlap_wait();
   const Index cvecs = (Index)(p.channels / V);
   for (Index idx = (Index)blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += (Index)gridDim.x * kBlock) {
     const Index cv = idx % cvecs;
@@ -408,6 +410,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(kBlock)
     pool_max_grad_s2_kernel(const unsigned char* __restrict__ winner, const T* __restrict__ dy, T* __restrict__ dx,
                             PoolS2Geometry g, unsigned n_items) {
+  overlap_wait();
   const unsigned cvecs = (unsigned)(g.C / V);
   for (unsigned idx = blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += gridDim.x * kBlock) {
     const unsigned cv = idx % cvecs;
@@ -549,6 +552,7 @@ __global__ void __launch_bounds__(kBlock)
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
     pool_avg_global_kernel(const T* __restrict__ x, T* __restrict__ y, unsigned words, unsigned pixels, unsigned n_items) {
+  overlap_wait();
   constexpr int E = 4 / (int)sizeof(T);
   for (unsigned idx = blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += gridDim.x * kBlock) {
     const unsigned n = idx / words, wd = idx - n * words;
@@ -577,6 +581,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(32 * kGlobalPoolLanes)
     pool_avg_grad_global_kernel(const T* __restrict__ dy, T* __restrict__ dx, unsigned cvecs, unsigned tiles, unsigned pixels,
                                 unsigned n_blocks) {
+  overlap_wait();
   const unsigned tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
   for (unsigned block = blockIdx.x; block < n_blocks; block += gridDim.x) {
     const unsigned n = block / tiles, cv = (block - n * tiles) * 32u + tx;
@@ -697,6 +702,7 @@ struct IbpS2Geometry {
 template <typename T, int V>
 __global__ void __launch_bounds__(kBlock) depthwise_ibp_s2_kernel(const T* __restrict__ dy, const T* __restrict__ w,
                                                                   T* __restrict__ dx, IbpS2Geometry g, unsigned n_items) {
+  overlap_wait();
   const unsigned cvecs = (unsigned)(g.C / V);
   for (unsigned idx = blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += gridDim.x * kBlock) {
     const unsigned cv = idx % cvecs;
@@ -965,6 +971,7 @@ template <typename T, int ST>
 __global__ void __launch_bounds__(kFbpRowsWarps * 32, kFbpRowsBlocks)
     depthwise_filter_backprop_rows_kernel(const T* __restrict__ x, const T* __restrict__ dy, float* __restrict__ partial,
                                           PdnnDepthwiseConv2DParams p, int segs, int seg_cols, int per_full, int per_tail) {
+  overlap_wait();
   constexpr int E = WordOf<T>::E;
   // U output columns per trip: their ST * U new input columns and U dy words are requested together
   // (a warp has to keep a dozen lines in flight to cover the latency), the CARRY columns the next
@@ -1140,6 +1147,7 @@ __device__ __forceinline__ float pointwise_grad_value(float v, float e, int op) 
 template <typename T, int V, int MODE>  // MODE 0: forward, 1: gradient
 __global__ void __launch_bounds__(kBlock)
     pointwise_kernel(int op, const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, size_t n_packets) {
+  overlap_wait();
   for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n_packets; i += (size_t)gridDim.x * kBlock) {
     float av[V], res[V];
     load_vec<T, V>(a + i * V, av);
@@ -1159,6 +1167,7 @@ __global__ void __launch_bounds__(kBlock)
 template <typename T, int V>
 __global__ void __launch_bounds__(kBlock) bias_add_kernel(const T* __restrict__ in, const T* __restrict__ bias,
                                                           T* __restrict__ out, size_t n_packets, int cvecs, int act) {
+  overlap_wait();
   for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n_packets; i += (size_t)gridDim.x * kBlock) {
     float v[V], b[V];
     load_vec<T, V>(in + i * V, v);
@@ -1402,6 +1411,7 @@ template <typename T, int ST, int MODE>
 __global__ void __launch_bounds__(kStripBlock)
     window3_strip_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, StripGeometry g,
                          size_t n_threads) {
+  overlap_wait();
   using P = Packet<T>;
   constexpr int V = 16 / sizeof(T);
   constexpr int kStripW = StripWidth<ST>::value;
@@ -1712,9 +1722,9 @@ int launch_window3_strip(const T* x, const T* w, T* y, int stride, StripGeometry
       return 0;
   }
   if (stride == 1)
-    window3_strip_kernel<T, 1, MODE><<<(unsigned)blocks, kStripBlock, 0, s>>>(x, w, y, g, n_threads);
+    launch_overlapped(window3_strip_kernel<T, 1, MODE>, (unsigned)blocks, kStripBlock, s, x, w, y, g, n_threads);
   else
-    window3_strip_kernel<T, 2, MODE><<<(unsigned)blocks, kStripBlock, 0, s>>>(x, w, y, g, n_threads);
+    launch_overlapped(window3_strip_kernel<T, 2, MODE>, (unsigned)blocks, kStripBlock, s, x, w, y, g, n_threads);
   return 0;
 }
 
@@ -1772,9 +1782,11 @@ int launch_pooling(int op, int direction, int dtype, const void* in, void* out, 
       constexpr unsigned E = 4 / (unsigned)sizeof(T);
       const unsigned words = (unsigned)p.channels / E, items0 = (unsigned)p.batch * words;
       if (direction == 0)
-        pool_avg_global_kernel<T><<<grid_for(items0, kBlock, sms), kBlock, 0, s>>>(from, static_cast<T*>(out), words, px, items0);
+        launch_overlapped(pool_avg_global_kernel<T>, grid_for(items0, kBlock, sms), kBlock, s, from, static_cast<T*>(out),
+            words, px, items0);
       else
-        pool_avg_grad_global_kernel<T, VN><<<blocks, 32 * kGlobalPoolLanes, 0, s>>>(from, static_cast<T*>(out), cvecs, tiles, px, n_blocks);
+        launch_overlapped(pool_avg_grad_global_kernel<T, VN>, blocks, 32 * kGlobalPoolLanes, s, from, static_cast<T*>(out),
+            cvecs, tiles, px, n_blocks);
       return check_launch(direction == 0 ? "pooling average (global)" : "pooling average gradient (global)");
     }
     const unsigned grid = grid_for(items, kBlock, sms);
@@ -1787,11 +1799,11 @@ int launch_pooling(int op, int direction, int dtype, const void* in, void* out, 
       if (direction == 1) {
         pool_avg_grad_kernel<T, V, Index><<<grid, kBlock, 0, s>>>(x, y, p, (Index)items);
       } else if (op == PDNN_POOL_MAX) {
-        pool_forward_kernel<T, PDNN_POOL_MAX, V, Index><<<grid, kBlock, 0, s>>>(x, y, p, (Index)items);
+        launch_overlapped(pool_forward_kernel<T, PDNN_POOL_MAX, V, Index>, grid, kBlock, s, x, y, p, (Index)items);
       } else if (op == PDNN_POOL_MAX_WITH_NAN) {
-        pool_forward_kernel<T, PDNN_POOL_MAX_WITH_NAN, V, Index><<<grid, kBlock, 0, s>>>(x, y, p, (Index)items);
+        launch_overlapped(pool_forward_kernel<T, PDNN_POOL_MAX_WITH_NAN, V, Index>, grid, kBlock, s, x, y, p, (Index)items);
       } else {
-        pool_forward_kernel<T, PDNN_POOL_AVERAGE, V, Index><<<grid, kBlock, 0, s>>>(x, y, p, (Index)items);
+        launch_overlapped(pool_forward_kernel<T, PDNN_POOL_AVERAGE, V, Index>, grid, kBlock, s, x, y, p, (Index)items);
       }
     };
     if (vec) {
@@ -1847,9 +1859,11 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
       // no window overlaps another, and less than a window is left over at the edges: one pass
       const unsigned g1 = grid_for(out_items, kBlock, sms);
       if (op == PDNN_POOL_MAX)
-        pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX, VN, unsigned><<<g1, kBlock, 0, s>>>(xt, yt, dyt, dxt, p, (unsigned)out_items);
+        launch_overlapped(pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX, VN, unsigned>, g1, kBlock, s, xt, yt, dyt, dxt, p,
+            (unsigned)out_items);
       else
-        pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX_WITH_NAN, VN, unsigned><<<g1, kBlock, 0, s>>>(xt, yt, dyt, dxt, p, (unsigned)out_items);
+        launch_overlapped(pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX_WITH_NAN, VN, unsigned>, g1, kBlock, s, xt, yt, dyt, dxt,
+            p, (unsigned)out_items);
       return check_launch("pooling max gradient (tiling windows)");
     }
     if (vec && small && p.window_rows * p.window_cols < 255) {
@@ -1884,7 +1898,7 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
           while (g.rows > 4 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 2048) g.rows = (g.rows + 1) / 2;
           g.strips = (g.M + g.rows - 1) / g.rows;
           const size_t n_items = columns * g.strips;
-          pool_max_grad_s2_kernel<T, VN><<<grid_for(n_items, kBlock, sms), kBlock, 0, s>>>(winner, dyt, dxt, g,
+          launch_overlapped(pool_max_grad_s2_kernel<T, VN>, grid_for(n_items, kBlock, sms), kBlock, s, winner, dyt, dxt, g,
                                                                                          (unsigned)n_items);
           st = check_launch("pooling max gradient (3x3 / 2 gather)");
         } else if (st == PDNN_OK) {
@@ -2005,8 +2019,10 @@ int launch_fbp_partials(bool vec, const T* in, const T* dy, float* partial, cons
     while (segs < 4 && units * segs < (long long)gx * kFbpRowsWarps * 12 && (p.out_cols + 2 * segs - 1) / (2 * segs) >= 2 * trip) segs *= 2;
     const int seg_cols = ((p.out_cols + segs - 1) / segs + trip - 1) / trip * trip;
     segs = (p.out_cols + seg_cols - 1) / seg_cols;
-    if (p.stride_rows == 1) depthwise_filter_backprop_rows_kernel<T, 1><<<grid, kFbpRowsWarps * 32, 0, s>>>(in, dy, partial, p, segs, seg_cols, (int)gx, (int)g_tail);
-    else depthwise_filter_backprop_rows_kernel<T, 2><<<grid, kFbpRowsWarps * 32, 0, s>>>(in, dy, partial, p, segs, seg_cols, (int)gx, (int)g_tail);
+    if (p.stride_rows == 1) launch_overlapped(depthwise_filter_backprop_rows_kernel<T, 1>, grid, kFbpRowsWarps * 32, s, in, dy,
+        partial, p, segs, seg_cols, (int)gx, (int)g_tail);
+    else launch_overlapped(depthwise_filter_backprop_rows_kernel<T, 2>, grid, kFbpRowsWarps * 32, s, in, dy, partial, p, segs,
+        seg_cols, (int)gx, (int)g_tail);
     return (int)gx;
   }
   if (fbp_all_taps(p, V)) {
@@ -2100,8 +2116,8 @@ int launch_depthwise(int pass, int dtype, const void* in, const void* fil, void*
       g.strips = (g.M + g.rows - 1) / g.rows;
       const size_t n_items = columns * g.strips;
       if (n_items < 0xFFFF0000ull) {
-        depthwise_ibp_s2_kernel<T, VN><<<grid_for(n_items, kBlock, sms), kBlock, 0, s>>>(
-            static_cast<const T*>(in), static_cast<const T*>(fil), static_cast<T*>(out), g, (unsigned)n_items);
+        launch_overlapped(depthwise_ibp_s2_kernel<T, VN>, grid_for(n_items, kBlock, sms), kBlock, s, static_cast<const T*>(in),
+            static_cast<const T*>(fil), static_cast<T*>(out), g, (unsigned)n_items);
         return check_launch("depthwise input backprop (3x3, stride 2)");
       }
     }
@@ -2141,10 +2157,10 @@ int launch_pointwise(int op, int dtype, const void* in, void* out, size_t n, cud
     constexpr int VN = Vec16<T>::N;
     // the reference picks the widest vector that divides n (src/pointwise/launch_pointwise_forward.cc:32-70)
     if (n % VN == 0 && aligned16(in) && aligned16(out))
-      pointwise_kernel<T, VN, 0><<<grid_for(n / VN, kBlock, sms), kBlock, 0, s>>>(
-          op, static_cast<const T*>(in), nullptr, static_cast<T*>(out), n / VN);
+      launch_overlapped(pointwise_kernel<T, VN, 0>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(in),
+          nullptr, static_cast<T*>(out), n / VN);
     else
-      pointwise_kernel<T, 1, 0><<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(op, static_cast<const T*>(in), nullptr,
+      launch_overlapped(pointwise_kernel<T, 1, 0>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(in), nullptr,
                                                                             static_cast<T*>(out), n);
     return check_launch("pointwise");
   });
@@ -2160,11 +2176,11 @@ int launch_pointwise_grad(int op, int dtype, const void* fwd, const void* err, v
     using T = decltype(tag);
     constexpr int VN = Vec16<T>::N;
     if (n % VN == 0 && aligned16(fwd) && aligned16(err) && aligned16(out))
-      pointwise_kernel<T, VN, 1><<<grid_for(n / VN, kBlock, sms), kBlock, 0, s>>>(
-          op, static_cast<const T*>(fwd), static_cast<const T*>(err), static_cast<T*>(out), n / VN);
+      launch_overlapped(pointwise_kernel<T, VN, 1>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(fwd),
+          static_cast<const T*>(err), static_cast<T*>(out), n / VN);
     else
-      pointwise_kernel<T, 1, 1><<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(
-          op, static_cast<const T*>(fwd), static_cast<const T*>(err), static_cast<T*>(out), n);
+      launch_overlapped(pointwise_kernel<T, 1, 1>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(fwd),
+          static_cast<const T*>(err), static_cast<T*>(out), n);
     return check_launch("pointwise gradient");
   });
 }
@@ -2181,11 +2197,11 @@ int launch_bias_add(int dtype, const void* in, const void* bias, void* out, size
     constexpr int VN = Vec16<T>::N;
     const size_t n = rows * (size_t)channels;
     if (channels % VN == 0 && aligned16(in) && aligned16(bias) && aligned16(out))
-      bias_add_kernel<T, VN><<<grid_for(n / VN, kBlock, sms), kBlock, 0, s>>>(
-          static_cast<const T*>(in), static_cast<const T*>(bias), static_cast<T*>(out), n / VN, channels / VN, act);
+      launch_overlapped(bias_add_kernel<T, VN>, grid_for(n / VN, kBlock, sms), kBlock, s, static_cast<const T*>(in),
+          static_cast<const T*>(bias), static_cast<T*>(out), n / VN, channels / VN, act);
     else
-      bias_add_kernel<T, 1><<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(
-          static_cast<const T*>(in), static_cast<const T*>(bias), static_cast<T*>(out), n, channels, act);
+      launch_overlapped(bias_add_kernel<T, 1>, grid_for(n, kBlock, sms), kBlock, s, static_cast<const T*>(in),
+          static_cast<const T*>(bias), static_cast<T*>(out), n, channels, act);
     return check_launch("bias add");
   });
 }
@@ -2224,6 +2240,7 @@ struct BinaryGeometry {
 template <typename T, int V>
 __global__ void __launch_bounds__(kBlock) binaryop_kernel(int op, const T* __restrict__ lhs, const T* __restrict__ rhs,
                                                           T* __restrict__ out, BinaryGeometry g, size_t n_packets) {
+  overlap_wait();
   const unsigned inner_packets = g.od[3] / V;
   for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n_packets; i += (size_t)gridDim.x * kBlock) {
     // the output has fewer than 2^32 elements (checked by the host): 32-bit divisions
@@ -2318,11 +2335,11 @@ int launch_binaryop(int op, int dtype, const void* lhs, const int* lhs_dims, int
     const bool vec = g.od[3] % VN == 0 && aligned16(lhs) && aligned16(rhs) && aligned16(out);
     const size_t n = (size_t)total;
     if (vec)
-      binaryop_kernel<T, VN><<<grid_for(n / VN, kBlock, sms), kBlock, 0, s>>>(
-          op, static_cast<const T*>(lhs), static_cast<const T*>(rhs), static_cast<T*>(out), g, n / VN);
+      launch_overlapped(binaryop_kernel<T, VN>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(lhs),
+          static_cast<const T*>(rhs), static_cast<T*>(out), g, n / VN);
     else
-      binaryop_kernel<T, 1><<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(
-          op, static_cast<const T*>(lhs), static_cast<const T*>(rhs), static_cast<T*>(out), g, n);
+      launch_overlapped(binaryop_kernel<T, 1>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(lhs),
+          static_cast<const T*>(rhs), static_cast<T*>(out), g, n);
     return check_launch("binaryop");
   });
 }

@@ -60,6 +60,7 @@ __device__ __forceinline__ void store_v(T* p, const float (&v)[V]) {
 template <typename T, int V, int R>
 __global__ void __launch_bounds__(kBlock) softmax_forward_vec_kernel(const T* __restrict__ x, T* __restrict__ y,
                                                                      size_t rows, int C) {
+  overlap_wait();
   const int lane = threadIdx.x & 31, packets = C / V;
   const size_t warps = (size_t)gridDim.x * (kBlock / 32);
   for (size_t row = (size_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); row < rows; row += warps) {
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kBlock) softmax_forward_kernel(const T* __rest
 template <typename T, int V, int R>
 __global__ void __launch_bounds__(kBlock) softmax_grad_vec_kernel(const T* __restrict__ y, const T* __restrict__ dy,
                                                                   T* __restrict__ dx, size_t rows, int C) {
+  overlap_wait();
   const int lane = threadIdx.x & 31, packets = C / V;
   const size_t warps = (size_t)gridDim.x * (kBlock / 32);
   for (size_t row = (size_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); row < rows; row += warps) {
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(kBlock)
     batchnorm_apply_vec_kernel(const T* __restrict__ x, const T* __restrict__ beta, const T* __restrict__ gamma,
                                const T* __restrict__ mean, const T* __restrict__ var, T* __restrict__ out, size_t n,
                                int C, float eps) {
+  overlap_wait();
   const size_t cvecs = (size_t)(C / V);
   const size_t step = (size_t)gridDim.x * kBlock;
   size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x;
@@ -222,6 +225,7 @@ __global__ void __launch_bounds__(kBlock)
     batchnorm_grad_training_vec_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ gamma,
                                        const float* __restrict__ stats0, const float* __restrict__ stats1,
                                        T* __restrict__ out, size_t n, int C, float rows, float eps) {
+  overlap_wait();
   const size_t cvecs = (size_t)(C / V);
   const size_t step = (size_t)gridDim.x * kBlock;
   size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x;
@@ -541,6 +545,7 @@ __global__ void __launch_bounds__(kBlock, 3)
     batchnorm_moments_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ beta,
                              const T* __restrict__ gamma, const T* __restrict__ mean, const T* __restrict__ var,
                              T* __restrict__ out, float* __restrict__ partial, size_t rows, int C, size_t rows_per_slice, float eps) {
+  overlap_wait();
   constexpr int NC = kMomentChannels, NS = DY ? 4 : 2;
   __shared__ float red[8][NS][NC][32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -658,6 +663,7 @@ __global__ void __launch_bounds__(kBlock, 3)
 template <bool DY, typename Finish>
 __global__ void __launch_bounds__(1024)
     batchnorm_merge_kernel(const float* __restrict__ partial, int slices, int C, size_t rows, size_t rows_per_slice, Finish finish) {
+  overlap_wait();
   constexpr int NS = DY ? 4 : 2;
   __shared__ float red[32][NS + 1][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
@@ -832,19 +838,21 @@ int launch_softmax(int direction, int dtype, const void* input, const void* grad
     constexpr int VN = Vec16<T>::N;
     const bool vec = p.channels % VN == 0 && aligned16(input) && aligned16(output);
     if (direction == 0 && vec && p.channels <= 32 * VN)
-      softmax_forward_vec_kernel<T, VN, 1><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input),
+      launch_overlapped(softmax_forward_vec_kernel<T, VN, 1>, grid, kBlock, s, static_cast<const T*>(input),
                                                                   static_cast<T*>(output), rows, p.channels);
     else if (direction == 0 && vec && p.channels <= 128 * VN)
-      softmax_forward_vec_kernel<T, VN, 4><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input),
+      launch_overlapped(softmax_forward_vec_kernel<T, VN, 4>, grid, kBlock, s, static_cast<const T*>(input),
                                                                   static_cast<T*>(output), rows, p.channels);
     else if (direction == 0)
       softmax_forward_kernel<T><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), static_cast<T*>(output), rows,
                                                         p.channels);
     else if (vec && aligned16(gradient) && p.channels <= 32 * VN)
-      softmax_grad_vec_kernel<T, VN, 1><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), static_cast<const T*>(gradient),
+      launch_overlapped(softmax_grad_vec_kernel<T, VN, 1>, grid, kBlock, s, static_cast<const T*>(input),
+          static_cast<const T*>(gradient),
                                                                 static_cast<T*>(output), rows, p.channels);
     else if (vec && aligned16(gradient) && p.channels <= 128 * VN)
-      softmax_grad_vec_kernel<T, VN, 4><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), static_cast<const T*>(gradient),
+      launch_overlapped(softmax_grad_vec_kernel<T, VN, 4>, grid, kBlock, s, static_cast<const T*>(input),
+          static_cast<const T*>(gradient),
                                                                 static_cast<T*>(output), rows, p.channels);
     else
       softmax_grad_kernel<T><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), static_cast<const T*>(gradient),
@@ -881,18 +889,17 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
       if (st != PDNN_OK) return st;
       const dim3 grid((unsigned)slices, (unsigned)((C / kMomentChannels + 31) / 32));
       const T *mt = static_cast<const T*>(mean), *vt = static_cast<const T*>(variance);
-      batchnorm_moments_kernel<T, false, true><<<grid, kBlock, 0, s>>>(
-          static_cast<const T*>(input), nullptr, static_cast<const T*>(beta), static_cast<const T*>(gamma), mt, vt,
+      launch_overlapped(batchnorm_moments_kernel<T, false, true>, grid, kBlock, s, static_cast<const T*>(input), nullptr,
+          static_cast<const T*>(beta), static_cast<const T*>(gamma), mt, vt,
           static_cast<T*>(output), sc.partial, rows, C, per, p.epsilon);
-      batchnorm_merge_kernel<false><<<(C + 31) / 32, 1024, 0, s>>>(
-          sc.partial, slices, C, rows, per,
+      launch_overlapped(batchnorm_merge_kernel<false, StoreRunning<T>>, (C + 31) / 32, 1024, s, sc.partial, slices, C, rows, per,
           StoreRunning<T>{mt, vt, static_cast<T*>(running_mean), static_cast<T*>(running_variance), (float)rows, p.momentum});
       count_launch();
       cudaFreeAsync(sc.base, s);
       return check_launch("batchnorm forward (training)");
     }
     if (vec)
-      batchnorm_apply_vec_kernel<T, VN><<<channel_stable_grid(n / VN, C / VN, sms), kBlock, 0, s>>>(
+      launch_overlapped(batchnorm_apply_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s,
           static_cast<const T*>(input), static_cast<const T*>(beta), static_cast<const T*>(gamma),
           static_cast<const T*>(mean), static_cast<const T*>(variance), static_cast<T*>(output), n / VN, C, p.epsilon);
     else
@@ -955,13 +962,14 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
     const T *x = static_cast<const T*>(input), *dy = static_cast<const T*>(gradient), *g = static_cast<const T*>(gamma);
     if (one_pass) {
       const dim3 mgrid((unsigned)slices, (unsigned)((C / kMomentChannels + 31) / 32));
-      batchnorm_moments_kernel<T, true, false><<<mgrid, kBlock, 0, s>>>(x, dy, nullptr, nullptr, nullptr, nullptr, nullptr, sc.partial,
+      launch_overlapped(batchnorm_moments_kernel<T, true, false>, mgrid, kBlock, s, x, dy, nullptr, nullptr, nullptr, nullptr,
+          nullptr, sc.partial,
                                                                        rows, C, per_slice, 0.f);
-      batchnorm_merge_kernel<true><<<(C + 31) / 32, 1024, 0, s>>>(
-          sc.partial, slices, C, rows, per_slice,
+      launch_overlapped(batchnorm_merge_kernel<true, StoreGradStats<T>>, (C + 31) / 32, 1024, s, sc.partial, slices, C, rows,
+          per_slice,
           StoreGradStats<T>{sc.stats0, sc.stats1, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), C, (float)rows, p.epsilon});
-      batchnorm_grad_training_vec_kernel<T, VN><<<channel_stable_grid(n / VN, C / VN, sms), kBlock, 0, s>>>(
-          x, dy, g, sc.stats0, sc.stats1, static_cast<T*>(output), n / VN, C, (float)rows, p.epsilon);
+      launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s, x, dy,
+          g, sc.stats0, sc.stats1, static_cast<T*>(output), n / VN, C, (float)rows, p.epsilon);
       count_launch(2);
       cudaFreeAsync(sc.base, s);
       return check_launch("batchnorm gradient (training)");

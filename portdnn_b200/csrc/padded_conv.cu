@@ -9,6 +9,8 @@
 #include "padded_conv.cuh"
 #include "tc_gemm.cuh"
 
+#include <type_traits>
+
 namespace pdnn {
 namespace {
 
@@ -69,6 +71,7 @@ __device__ __forceinline__ void repitch(const RepitchJob& j, unsigned first, uns
 
 // Up to three copies (activations, filter, bias) side by side in one launch.
 __global__ void __launch_bounds__(kBlock) repitch_kernel(const RepitchJobs jobs) {
+  overlap_wait();
   int n = 0;
   while (n + 1 < jobs.count && blockIdx.x >= jobs.job[n + 1].first_block) ++n;
   const RepitchJob& j = jobs.job[n];
@@ -94,7 +97,7 @@ void add_job(RepitchJobs& jobs, const void* in, void* out, size_t matrices, int 
 
 int run_jobs(const RepitchJobs& jobs, cudaStream_t s) {
   if (jobs.count == 0) return PDNN_OK;
-  repitch_kernel<<<jobs.blocks, kBlock, 0, s>>>(jobs);
+  launch_overlapped(repitch_kernel, jobs.blocks, kBlock, s, jobs);
   return check_launch("conv2d padding");
 }
 
@@ -102,6 +105,7 @@ int run_jobs(const RepitchJobs& jobs, cudaStream_t s) {
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(kBlock)
     cut_kernel(const InT* __restrict__ in, OutT* __restrict__ out, unsigned n, int bo, int bi, int co, int ci, bool accumulate) {
+  overlap_wait();
   for (unsigned i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
     const unsigned row = i / (unsigned)co, c = i - row * (unsigned)co, a = row / (unsigned)bo, b = row - a * (unsigned)bo;
     float v = to_f32(in[((size_t)a * bi + b) * ci + c]);
@@ -266,10 +270,12 @@ int padded_conv(int pass, int dtype, const void* in, const void* fil, void* out,
       const unsigned n = (unsigned)plan.real_x;
       if (fusion != nullptr && fusion->accumulate) {
         if (dtype == PDNN_F16)
-          cut_kernel<<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(static_cast<const __half*>(dx), static_cast<__half*>(out), n, px_in,
+          launch_overlapped(cut_kernel<__half, __half>, grid_for(n, kBlock, sms), kBlock, s, static_cast<const __half*>(dx),
+              static_cast<__half*>(out), n, px_in,
                                                                  px_in, p.channels, q.channels, true);
         else
-          cut_kernel<<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(static_cast<const __nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(out),
+          launch_overlapped(cut_kernel<__nv_bfloat16, __nv_bfloat16>, grid_for(n, kBlock, sms), kBlock, s,
+              static_cast<const __nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(out),
                                                                  n, px_in, px_in, p.channels, q.channels, true);
         st = check_launch("conv2d input gradient");
       } else {
@@ -295,7 +301,8 @@ int padded_conv(int pass, int dtype, const void* in, const void* fil, void* out,
       const unsigned n = (unsigned)plan.real_w, grid = grid_for(n, kBlock, sms);
       const bool add = fusion != nullptr && fusion->accumulate;
       auto cut = [&](auto* to) {
-        cut_kernel<<<grid, kBlock, 0, s>>>(dw, to, n, p.channels, q.channels, p.features, q.features, add);
+        launch_overlapped(cut_kernel<float, std::remove_pointer_t<decltype(to)>>, grid, kBlock, s, dw, to, n, p.channels,
+            q.channels, p.features, q.features, add);
       };
       if (fusion != nullptr && fusion->output_f32) cut(static_cast<float*>(out));
       else if (dtype == PDNN_F16) cut(static_cast<__half*>(out));

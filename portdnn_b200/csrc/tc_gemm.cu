@@ -2716,6 +2716,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) pack_small_c_input_kernel(const T* __restrict__ x, uint4* __restrict__ xp, int N,
                                                                 int H, int W, int C, int Hp, int Wp, int pad_top,
                                                                 int pad_left) {
+  overlap_wait();
   constexpr int CP = 16 / sizeof(T);
   const int wp = (int)(blockIdx.x * 256u + threadIdx.x), hp = (int)blockIdx.y, n = (int)blockIdx.z;
   if (wp >= Wp) return;
@@ -2734,6 +2735,7 @@ __global__ void __launch_bounds__(256) pack_small_c_input_narrow_kernel(const un
                                                                        uint2* __restrict__ xp, int N, int H, int W,
                                                                        int C, int Hp, int Wp, int pad_top,
                                                                        int pad_left) {
+  overlap_wait();
   const int wp = (int)(blockIdx.x * 256u + threadIdx.x), hp = (int)blockIdx.y, n = (int)blockIdx.z;
   if (wp >= Wp) return;
   const int h = hp - pad_top, w = wp - pad_left;
@@ -2749,6 +2751,7 @@ __global__ void __launch_bounds__(256) pack_small_c_input_narrow_kernel(const un
 template <typename T>
 __global__ void __launch_bounds__(256) pack_small_c_filter_kernel(const T* __restrict__ w, T* __restrict__ wp, int R,
                                                                  int S, int C, int K, int CP) {
+  overlap_wait();
   const size_t total = (size_t)R * 8 * CP * K;
   for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (size_t)gridDim.x * 256) {
     const int k = (int)(idx % K);
@@ -2895,23 +2898,21 @@ int conv_forward_small_c(int dtype, const void* x, const void* w, void* y, const
   }
   const size_t n_fil = (size_t)p.window_rows * krows * p.features;
   if (dtype == PDNN_F32) {
-    pack_small_c_input_kernel<float><<<dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, 0, s>>>(
-        static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, sp.Hp,
+    launch_overlapped(pack_small_c_input_kernel<float>, dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, s, static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, sp.Hp,
         sp.Wp, p.pad_rows, p.pad_cols);
-    pack_small_c_filter_kernel<float><<<grid_for(n_fil, 256, sms), 256, 0, s>>>(
-        static_cast<const float*>(w), reinterpret_cast<float*>(wpk), p.window_rows, p.window_cols, p.channels, p.features, 4);
+    launch_overlapped(pack_small_c_filter_kernel<float>, grid_for(n_fil, 256, sms), 256, s, static_cast<const float*>(w),
+        reinterpret_cast<float*>(wpk), p.window_rows, p.window_cols, p.channels, p.features, 4);
   } else {
     // fp16 and bf16 are both moved as 16-bit words
     if (narrow)
-      pack_small_c_input_narrow_kernel<<<dim3((unsigned)ceil_div(Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, 0, s>>>(
-          static_cast<const unsigned short*>(x), reinterpret_cast<uint2*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
+      launch_overlapped(pack_small_c_input_narrow_kernel, dim3((unsigned)ceil_div(Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch),
+          256, s, static_cast<const unsigned short*>(x), reinterpret_cast<uint2*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
           sp.Hp, Wp, p.pad_rows, p.pad_cols);
     else
-      pack_small_c_input_kernel<__half><<<dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, 0, s>>>(
-          static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, sp.Hp,
+      launch_overlapped(pack_small_c_input_kernel<__half>, dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, s, static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, sp.Hp,
           sp.Wp, p.pad_rows, p.pad_cols);
-    pack_small_c_filter_kernel<__half><<<grid_for(n_fil, 256, sms), 256, 0, s>>>(
-        static_cast<const __half*>(w), reinterpret_cast<__half*>(wpk), p.window_rows, p.window_cols, p.channels, p.features,
+    launch_overlapped(pack_small_c_filter_kernel<__half>, grid_for(n_fil, 256, sms), 256, s, static_cast<const __half*>(w),
+        reinterpret_cast<__half*>(wpk), p.window_rows, p.window_cols, p.channels, p.features,
         narrow ? 4 : 8);
   }
   int st = check_launch("conv2d small-channel packing");
@@ -2925,6 +2926,7 @@ int conv_forward_small_c(int dtype, const void* x, const void* w, void* y, const
 // The lo part of a 3xTF32 operand: the tensor core reads the 19 leading bits of an fp32 word (hi, which
 // therefore needs no copy); lo = x - hi is exact in fp32.
 __global__ void __launch_bounds__(256) split_lo_kernel(const float* __restrict__ x, float* __restrict__ lo, size_t n) {
+  overlap_wait();
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
     const float v = x[i];
     lo[i] = v - __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
@@ -3065,7 +3067,8 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   if (dtype == PDNN_F32 && (size_t)p.batch * p.out_rows * p.out_cols >= 2048 && aligned16(w) &&
       (!hwcf || w_ld == (uint64_t)p.features)) {  // (a column slice of a wider filter is not one contiguous run)
     if (cudaMallocAsync(reinterpret_cast<void**>(&w_split), filter_elems * sizeof(float), s) == cudaSuccess) {
-      split_lo_kernel<<<grid_for(filter_elems, 256, sms), 256, 0, s>>>(static_cast<const float*>(w), w_split, filter_elems);
+      launch_overlapped(split_lo_kernel, grid_for(filter_elems, 256, sms), 256, s, static_cast<const float*>(w), w_split,
+          filter_elems);
       count_launch();
       g.b_presplit = 1;
     } else {
@@ -3118,6 +3121,7 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
 __global__ void __launch_bounds__(256)
     pack_grouped_filter_kernel(const unsigned short* __restrict__ w, unsigned short* __restrict__ packed, int taps, int Cg, int Kg, int groups,
                                int per_tile, int rows, bool fhwc) {
+  overlap_wait();
   const unsigned total = (unsigned)taps * (unsigned)rows * 64u, K = (unsigned)(groups * Kg);
   for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
     const unsigned slot = i & 63u, row = (i >> 6) % (unsigned)rows, tap = (i >> 6) / (unsigned)rows;
@@ -3205,8 +3209,9 @@ int conv_forward_grouped(int dtype, const void* x, const void* w, void* y, const
                                                                        : PDNN_INVALID_PARAMETER;
   if (status == PDNN_OK && !plan.tma_store) status = PDNN_INVALID_PARAMETER;
   if (status == PDNN_OK) {
-    pack_grouped_filter_kernel<<<grid_for(packed_bytes / 2, 256, sms), 256, 0, s>>>(
-        static_cast<const unsigned short*>(w), static_cast<unsigned short*>(packed), taps, Cg, Kg, p.groups, per_tile, rows, p.filter_format == 2);
+    launch_overlapped(pack_grouped_filter_kernel, grid_for(packed_bytes / 2, 256, sms), 256, s,
+        static_cast<const unsigned short*>(w), static_cast<unsigned short*>(packed), taps, Cg, Kg, p.groups, per_tile, rows,
+        p.filter_format == 2);
     status = check_launch("conv2d grouped filter packing");
     if (status == PDNN_OK) status = launch_gemm(plan, dtype, s);
     cudaFreeAsync(packed, s);
@@ -3235,7 +3240,8 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
   float* w_split = nullptr;
   if (dtype == PDNN_F32 && (size_t)p.batch * p.in_rows * p.in_cols >= 2048 && aligned16(w) &&
       cudaMallocAsync(reinterpret_cast<void**>(&w_split), filter_elems * sizeof(float), s) == cudaSuccess) {
-    split_lo_kernel<<<grid_for(filter_elems, 256, sms), 256, 0, s>>>(static_cast<const float*>(w), w_split, filter_elems);
+    launch_overlapped(split_lo_kernel, grid_for(filter_elems, 256, sms), 256, s, static_cast<const float*>(w), w_split,
+        filter_elems);
     count_launch();
   } else if (dtype == PDNN_F32) {
     cudaGetLastError();
@@ -3513,6 +3519,7 @@ template <typename T, typename OutT = T>
 __global__ void __launch_bounds__(256)
     unpack_small_c_filter_grad_kernel(const float* __restrict__ partial, OutT* __restrict__ dw, int splits, int R, int S,
                                       int C, int K, int rows_per_tap, bool accumulate) {
+  overlap_wait();
   constexpr int CP = 16 / sizeof(T);
   const size_t total = (size_t)R * S * C * K;
   const size_t split_stride = (size_t)R * rows_per_tap * K;
@@ -3655,12 +3662,10 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
     }
   }
   if (dtype == PDNN_F32)
-    pack_small_c_input_kernel<float><<<dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, 0, s>>>(
-        static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, q.sp.Hp,
+    launch_overlapped(pack_small_c_input_kernel<float>, dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, s, static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, q.sp.Hp,
         q.sp.Wp, p.pad_rows, p.pad_cols);
   else
-    pack_small_c_input_kernel<__half><<<dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, 0, s>>>(
-        static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
+    launch_overlapped(pack_small_c_input_kernel<__half>, dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, s, static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
         q.sp.Hp, q.sp.Wp, p.pad_rows, p.pad_cols);
   int st = check_launch("conv2d small-channel packing");
   if (st == PDNN_OK) st = launch_gemm(g, dtype, s);
@@ -3668,17 +3673,17 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
     const size_t n_out = (size_t)p.window_rows * p.window_cols * p.channels * p.features;
     const unsigned grid = grid_for(n_out, 256, sms);
     if (dtype == PDNN_F32)
-      unpack_small_c_filter_grad_kernel<float><<<grid, 256, 0, s>>>(partial, static_cast<float*>(dw), f.splits,
+      launch_overlapped(unpack_small_c_filter_grad_kernel<float>, grid, 256, s, partial, static_cast<float*>(dw), f.splits,
                                                                     p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
     else if (out_f32)  // 16-bit tensors (8 channels per packed pixel), fp32 gradient
-      unpack_small_c_filter_grad_kernel<__half, float><<<grid, 256, 0, s>>>(
-          partial, static_cast<float*>(dw), f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
+      launch_overlapped(unpack_small_c_filter_grad_kernel<__half, float>, grid, 256, s, partial, static_cast<float*>(dw),
+          f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
     else if (dtype == PDNN_F16)
-      unpack_small_c_filter_grad_kernel<__half><<<grid, 256, 0, s>>>(partial, static_cast<__half*>(dw), f.splits,
+      launch_overlapped(unpack_small_c_filter_grad_kernel<__half>, grid, 256, s, partial, static_cast<__half*>(dw), f.splits,
                                                                      p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
     else
-      unpack_small_c_filter_grad_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(
-          partial, static_cast<__nv_bfloat16*>(dw), f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
+      launch_overlapped(unpack_small_c_filter_grad_kernel<__nv_bfloat16>, grid, 256, s, partial,
+          static_cast<__nv_bfloat16*>(dw), f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
     st = check_launch("conv2d small-channel filter gradient unpack");
   }
   release();
