@@ -112,7 +112,7 @@ int device_sm_count();   // SM count of the current device; -1 if it is not an s
 // nothing under an ordinary launch.)  Grids of fewer than four waves only: beside a kernel of that length
 // the gap is nothing, and long ones chained this way cost the kernels around them.  All launches ordinary /
 // grids below four waves / all overlapped, us: MobileNet-v2 forward at 64 images (80 launches) 824 / 785 / 782,
-// 7x45x61 100 -> 150 3x3 with gradients 152 / 135 / 135, two max pools with gradients 121 / 111 / 111, one
+// 7x45x61 100 -> 150 3x3 with gradients 152 / 135 / 135, two max pools with gradients 121 / 114 / 114, one
 // image through ResNet-50 325 / 318 / 318, VGG-16 training step in fp32 6899 / 6897 / 7190.
 __device__ __forceinline__ void overlap_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");

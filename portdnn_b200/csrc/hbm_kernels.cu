@@ -1721,10 +1721,13 @@ int launch_window3_strip(const T* x, const T* w, T* y, int stride, StripGeometry
                     : launch_depthwise3_async<T, 2, 1>(x, w, y, g, n_threads, (unsigned)blocks, s))
       return 0;
   }
+  // An ordinary launch: blocks placed beside the end of a GEMM share the SM with its shared memory and keep
+  // what is left of the L1 cache, in which the rows of neighbouring strips meet (ResNet-50 forward, 256 images:
+  // 3160 us, overlapped 3220).
   if (stride == 1)
-    launch_overlapped(window3_strip_kernel<T, 1, MODE>, (unsigned)blocks, kStripBlock, s, x, w, y, g, n_threads);
+    window3_strip_kernel<T, 1, MODE><<<(unsigned)blocks, kStripBlock, 0, s>>>(x, w, y, g, n_threads);
   else
-    launch_overlapped(window3_strip_kernel<T, 2, MODE>, (unsigned)blocks, kStripBlock, s, x, w, y, g, n_threads);
+    window3_strip_kernel<T, 2, MODE><<<(unsigned)blocks, kStripBlock, 0, s>>>(x, w, y, g, n_threads);
   return 0;
 }
 
