@@ -492,35 +492,40 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // ---- batch statistics in one pass -------------------------------------------------------------------
-// Per-channel moments of the rows, without a first pass for the mean: a thread takes kBatch rows of four
-// channels at a time, forms their means and the sums around them exactly as a two-pass computation would,
-// and merges them into its running moments (Chan, Golub and LeVeque's pairwise update: the sums of two sets
-// around their own means, plus the product of the means' differences weighted n_a n_b / (n_a + n_b)).
-// Threads, then slices of rows are merged the same way, in a fixed order.  Bound by HBM: one pass over
-// the tensors where sums around a mean that is known beforehand take two, and in the forward pass the one that
-// writes the output.  64 x 28x28x256 f16: forward 64 -> 26 us (five launches to two), statistics of the
-// gradient 46 -> 28 us.
+// Per-channel moments of the rows, without a first pass for the mean.  A thread subtracts a value of its own,
+// the mean of its first kBatch rows, from the rows it reads, so that what it adds up is of the size of the
+// deviations however far the channel lies from zero; sets of rows are then merged pairwise (Chan, Golub and
+// LeVeque: the sums of two sets around their own means, plus the product of the means' differences weighted
+// n_a n_b / (n_a + n_b)), the difference of two means being that of the subtracted values plus that of what is
+// left.  So a large mean enters no sum: in fp32 the variance is off by 6e-8 of itself at a mean of 1000 deviations
+// (two passes 5e-8 to 1.5e-7, growing with the rows).  Threads, then slices of rows are merged in a fixed order.
+// Bound by HBM: one pass over the tensors where sums around a mean that is known beforehand take two, and in
+// the forward pass the one that writes the output.  Convolution, normalisation and ReLU in training, 64 x 28x28,
+// 128 -> 256, f16: 218 us with two passes, 123 here.
 constexpr int kBatch = 4;          // rows a thread has in flight
 constexpr int kMomentChannels = 4; // channels per thread: 8 or 16 bytes
 
-// Sum of x, sum (x - mean x)^2, sum of dy, sum (x - mean x)(dy - mean dy).  (Sums and not means are kept: an
-// infinity then stays one in the statistics it reaches.)
+// A set of rows: its means as hx + lx and hy + ly, sum (x - mean x)^2, sum (x - mean x)(dy - mean dy), and the
+// sums as they are.  (The means of the results come from those: an infinity then stays one.)
 template <bool DY>
 struct Moments {
-  float sx, sxx, sy, sxy;
+  static constexpr int N = DY ? 8 : 4;
+  float v[N];  // hx, lx, sxx, sx, then hy, ly, sxy, sy
   // Adds a set of nb rows to one of na.
-  __device__ __forceinline__ void merge(const Moments& b, float inv_na, float inv_nb, float weight) {
-    const float dx = b.sx * inv_nb - sx * inv_na;
-    sx += b.sx;
-    sxx += b.sxx + dx * dx * weight;
-    if (DY) {
-      const float dy = b.sy * inv_nb - sy * inv_na;
-      sy += b.sy;
-      sxy += b.sxy + dx * dy * weight;
-    }
-  }
   __device__ __forceinline__ void merge(const Moments& b, float na, float nb) {
-    merge(b, na > 0.f ? 1.f / na : 0.f, 1.f / nb, na * nb / (na + nb));
+    if (na == 0.f) *this = b;
+    if (na == 0.f || nb == 0.f) return;
+    const float share = nb / (na + nb), weight = na * share;
+    const float dx = (b.v[0] - v[0]) + (b.v[1] - v[1]);
+    v[1] += dx * share;
+    v[2] += b.v[2] + dx * dx * weight;
+    v[3] += b.v[3];
+    if constexpr (DY) {
+      const float dy = (b.v[4] - v[4]) + (b.v[5] - v[5]);
+      v[5] += dy * share;
+      v[6] += b.v[6] + dx * dy * weight;
+      v[7] += b.v[7];
+    }
   }
 };
 
@@ -538,7 +543,7 @@ __device__ __forceinline__ void load_four(const T* p, float (&v)[kMomentChannels
 }
 
 // Block: 32 lanes x 4 channels, 8 row lanes; blockIdx.x the slice of rows, blockIdx.y the channel tile.
-// partial[slice][sx, sxx (, sy, sxy)][c].  APPLY: the forward output is written on the way,
+// partial[slice][value of the set][c].  APPLY: the forward output is written on the way,
 // out = (x - mean) / sqrt(var + eps) * gamma + beta with the given mean and variance.
 template <typename T, bool DY, bool APPLY>
 __global__ void __launch_bounds__(kBlock, 3)
@@ -546,13 +551,15 @@ __global__ void __launch_bounds__(kBlock, 3)
                              const T* __restrict__ gamma, const T* __restrict__ mean, const T* __restrict__ var,
                              T* __restrict__ out, float* __restrict__ partial, size_t rows, int C, size_t rows_per_slice, float eps) {
   overlap_wait();
-  constexpr int NC = kMomentChannels, NS = DY ? 4 : 2;
+  constexpr int NC = kMomentChannels, NS = Moments<DY>::N;
   __shared__ float red[8][NS][NC][32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = (blockIdx.y * 32 + tx) * NC;
   const size_t begin = (size_t)blockIdx.x * rows_per_slice;
   const size_t end = begin + rows_per_slice < rows ? begin + rows_per_slice : rows;
-  Moments<DY> m[NC] = {};
+  // the subtracted values, and sums of d, d^2 and x (h, d h and dy), d = x - hx, h = dy - hy
+  float hx[NC] = {}, s1[NC] = {}, s2[NC] = {}, sx[NC] = {}, hy[NC] = {}, t1[NC] = {}, sxy[NC] = {}, sy[NC] = {};
+  float n = 0.f;
   if (c < C) {
     float am[NC], as[NC], ag[NC], ab[NC];
     if (APPLY) {
@@ -576,7 +583,18 @@ __global__ void __launch_bounds__(kBlock, 3)
         *reinterpret_cast<uint2*>(to) = q;
       }
     };
-    float n = 0.f;
+    auto add = [&](int k, float xv, float gv) {
+      const float d = xv - hx[k];
+      s1[k] += d;
+      s2[k] = fmaf(d, d, s2[k]);
+      sx[k] += xv;
+      if (DY) {
+        const float h = gv - hy[k];
+        t1[k] += h;
+        sxy[k] = fmaf(d, h, sxy[k]);
+        sy[k] += gv;
+      }
+    };
     // one offset moves through the tensors; eight rows further down is the row lane's next one
     size_t at = (begin + ty) * C + c;
     const unsigned next = 8u * (unsigned)C;
@@ -592,23 +610,18 @@ __global__ void __launch_bounds__(kBlock, 3)
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) apply(xv[i], out + at + (size_t)i * next);
       }
-      constexpr float inv_batch = 1.f / (float)kBatch;
-      const float inv_n = n > 0.f ? 1.f / n : 0.f, weight = n * (float)kBatch / (n + (float)kBatch);
+      if (n == 0.f) {
+        constexpr float inv_batch = 1.f / (float)kBatch;
 #pragma unroll
-      for (int k = 0; k < NC; ++k) {
-        Moments<DY> b;
-        b.sx = (xv[0][k] + xv[1][k]) + (xv[2][k] + xv[3][k]);
-        b.sy = DY ? (gv[0][k] + gv[1][k]) + (gv[2][k] + gv[3][k]) : 0.f;
-        b.sxx = b.sxy = 0.f;
-        const float mx = b.sx * inv_batch, my = b.sy * inv_batch;
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-          const float d = xv[i][k] - mx;
-          b.sxx += d * d;
-          if (DY) b.sxy += d * (gv[i][k] - my);
+        for (int k = 0; k < NC; ++k) {
+          hx[k] = ((xv[0][k] + xv[1][k]) + (xv[2][k] + xv[3][k])) * inv_batch;
+          if (DY) hy[k] = ((gv[0][k] + gv[1][k]) + (gv[2][k] + gv[3][k])) * inv_batch;
         }
-        m[k].merge(b, inv_n, inv_batch, weight);
       }
+#pragma unroll
+      for (int k = 0; k < NC; ++k)
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) add(k, xv[i][k], DY ? gv[i][k] : 0.f);
       n += (float)kBatch;
     }
     for (; left > 0; left -= 8, at += next) {
@@ -616,72 +629,81 @@ __global__ void __launch_bounds__(kBlock, 3)
       load_four(x + at, xv);
       if (DY) load_four(dy + at, gv);
       if (APPLY) apply(xv, out + at);
-      const float inv_n = n > 0.f ? 1.f / n : 0.f, weight = n / (n + 1.f);
 #pragma unroll
       for (int k = 0; k < NC; ++k) {
-        const Moments<DY> b{xv[k], 0.f, DY ? gv[k] : 0.f, 0.f};
-        m[k].merge(b, inv_n, 1.f, weight);
+        if (n == 0.f) {
+          hx[k] = xv[k];
+          if (DY) hy[k] = gv[k];
+        }
+        add(k, xv[k], DY ? gv[k] : 0.f);
       }
       n += 1.f;
     }
   }
+  const float inv_n = n > 0.f ? 1.f / n : 0.f;
 #pragma unroll
   for (int k = 0; k < NC; ++k) {
-    red[ty][0][k][tx] = m[k].sx;
-    red[ty][1][k][tx] = m[k].sxx;
-    if (DY) {
-      red[ty][2][k][tx] = m[k].sy;
-      red[ty][3][k][tx] = m[k].sxy;
+    const float lx = s1[k] * inv_n, sxx = fmaf(-s1[k], lx, s2[k]);
+    red[ty][0][k][tx] = hx[k];
+    red[ty][1][k][tx] = lx;
+    red[ty][2][k][tx] = sxx < 0.f ? 0.f : sxx;  // (a NaN stays)
+    red[ty][3][k][tx] = sx[k];
+    if constexpr (DY) {
+      const float ly = t1[k] * inv_n;
+      red[ty][4][k][tx] = hy[k];
+      red[ty][5][k][tx] = ly;
+      red[ty][6][k][tx] = fmaf(-s1[k], ly, sxy[k]);
+      red[ty][7][k][tx] = sy[k];
     }
   }
   __syncthreads();
   // thread (tx, k): channel c + k, its eight row lanes one after another
   if (ty < NC && c < C && begin < end) {
     const size_t here = end - begin;
-    Moments<DY> t{red[0][0][ty][tx], red[0][1][ty][tx], DY ? red[0][NS - 2][ty][tx] : 0.f, DY ? red[0][NS - 1][ty][tx] : 0.f};
-    float n = (float)((here + 7) / 8);
+    Moments<DY> t;
+    float nt = 0.f;
 #pragma unroll
-    for (int l = 1; l < 8; ++l) {
+    for (int l = 0; l < 8; ++l) {
       if ((size_t)l >= here) break;
       const float nb = (float)((here - l + 7) / 8);
-      const Moments<DY> b{red[l][0][ty][tx], red[l][1][ty][tx], DY ? red[l][NS - 2][ty][tx] : 0.f, DY ? red[l][NS - 1][ty][tx] : 0.f};
-      t.merge(b, n, nb);
-      n += nb;
+      Moments<DY> b;
+#pragma unroll
+      for (int i = 0; i < NS; ++i) b.v[i] = red[l][i][ty][tx];
+      t.merge(b, nt, nb);
+      nt += nb;
     }
     float* to = partial + (size_t)blockIdx.x * NS * C + c + ty;
-    to[0] = t.sx;
-    to[C] = t.sxx;
-    if (DY) {
-      to[2 * (size_t)C] = t.sy;
-      to[3 * (size_t)C] = t.sxy;
-    }
+#pragma unroll
+    for (int i = 0; i < NS; ++i) to[(size_t)i * C] = t.v[i];
   }
 }
 
-// Merges the slices of a channel: 32 channels to a block, 32 threads to a channel.
+// Merges the slices of a channel: 8 channels to a block, 64 threads to a channel.  Bound by latency: with four
+// slices' values requested together, and a few slices to a thread, the block waits for L2 twice.
 // finish(c, moments): what becomes of channel c.
+constexpr int kMergeChannels = 8, kMergeLanes = 64, kMergeWarps = kMergeChannels * kMergeLanes / 32;
 template <bool DY, typename Finish>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(kMergeChannels * kMergeLanes)
     batchnorm_merge_kernel(const float* __restrict__ partial, int slices, int C, size_t rows, size_t rows_per_slice, Finish finish) {
   overlap_wait();
-  constexpr int NS = DY ? 4 : 2;
-  __shared__ float red[32][NS + 1][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  constexpr int NS = Moments<DY>::N;
+  __shared__ float red[kMergeWarps][NS + 1][kMergeChannels];
+  const int tx = threadIdx.x % kMergeChannels, ty = threadIdx.x / kMergeChannels, c = blockIdx.x * kMergeChannels + tx;
   Moments<DY> t{};
   float n = 0.f;
   if (c < C) {
-    // four slices' sums requested together: the chain of merges would wait for each of them in turn
 #pragma unroll 1
-    for (int s0 = ty; s0 < slices; s0 += 4 * 32) {
+    for (int s0 = ty; s0 < slices; s0 += 4 * kMergeLanes) {
       Moments<DY> b[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float* at = partial + (size_t)min(s0 + 32 * i, slices - 1) * NS * C + c;
-        b[i] = Moments<DY>{__ldg(at), __ldg(at + C), DY ? __ldg(at + 2 * (size_t)C) : 0.f, DY ? __ldg(at + 3 * (size_t)C) : 0.f};
+        const float* at = partial + (size_t)min(s0 + kMergeLanes * i, slices - 1) * NS * C + c;
+#pragma unroll
+        for (int j = 0; j < NS; ++j) b[i].v[j] = __ldg(at + (size_t)j * C);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int s = s0 + 32 * i;
+        const int s = s0 + kMergeLanes * i;
         if (s >= slices) break;
         const size_t left = rows - (size_t)s * rows_per_slice;
         const float nb = (float)(left < rows_per_slice ? left : rows_per_slice);
@@ -690,39 +712,36 @@ __global__ void __launch_bounds__(1024)
       }
     }
   }
-  red[ty][0][tx] = t.sx;
-  red[ty][1][tx] = t.sxx;
-  if (DY) {
-    red[ty][2][tx] = t.sy;
-    red[ty][NS - 1][tx] = t.sxy;
-  }
-  red[ty][NS][tx] = n;
-  __syncthreads();
-  // warp ty merges the 32 sets of channel ty: neighbours first, the lower lane's set before the upper one's
-  t.sx = red[tx][0][ty];
-  t.sxx = red[tx][1][ty];
-  if (DY) {
-    t.sy = red[tx][2][ty];
-    t.sxy = red[tx][NS - 1][ty];
-  }
-  n = red[tx][NS][ty];
+  // neighbours first, the lower lane's set before the upper one's: the lanes of a warp that share a channel,
+  // then the warps
+  auto merge_down = [&](int o, bool here) {
+    Moments<DY> b;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    Moments<DY> b{};
-    b.sx = __shfl_down_sync(0xFFFFFFFFu, t.sx, o);
-    b.sxx = __shfl_down_sync(0xFFFFFFFFu, t.sxx, o);
-    if (DY) {
-      b.sy = __shfl_down_sync(0xFFFFFFFFu, t.sy, o);
-      b.sxy = __shfl_down_sync(0xFFFFFFFFu, t.sxy, o);
-    }
+    for (int j = 0; j < NS; ++j) b.v[j] = __shfl_down_sync(0xFFFFFFFFu, t.v[j], o);
     const float nb = __shfl_down_sync(0xFFFFFFFFu, n, o);
-    if ((tx & (2 * o - 1)) == 0 && nb > 0.f) {
+    if (here) {
       t.merge(b, n, nb);
       n += nb;
     }
+  };
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = kMergeChannels; o < 32; o <<= 1) merge_down(o, (lane & (2 * o - kMergeChannels)) == 0);
+  if (lane < kMergeChannels) {
+#pragma unroll
+    for (int j = 0; j < NS; ++j) red[warp][j][lane] = t.v[j];
+    red[warp][NS][lane] = n;
   }
-  const int mine = blockIdx.x * 32 + ty;
-  if (tx == 0 && mine < C) finish(mine, t);
+  __syncthreads();
+  if (warp >= kMergeChannels) return;
+  const int set = min(lane, kMergeWarps - 1);  // a lane takes a warp's set
+#pragma unroll
+  for (int j = 0; j < NS; ++j) t.v[j] = red[set][j][warp];
+  n = red[set][NS][warp];
+#pragma unroll
+  for (int o = 1; o < kMergeWarps; o <<= 1) merge_down(o, (lane & (2 * o - 1)) == 0);
+  const int mine = blockIdx.x * kMergeChannels + warp;
+  if (lane == 0 && mine < C) finish(mine, t);
 }
 
 // Training forward: running = batch * (1 - m) + given * m.
@@ -732,8 +751,8 @@ struct StoreRunning {
   T *run_mean, *run_var;
   float rows, momentum;
   __device__ __forceinline__ void operator()(int c, const Moments<false>& t) const {
-    run_mean[c] = from_f32<T>(t.sx / rows * (1.f - momentum) + to_f32(mean[c]) * momentum);
-    run_var[c] = from_f32<T>(t.sxx / rows * (1.f - momentum) + to_f32(var[c]) * momentum);
+    run_mean[c] = from_f32<T>(t.v[3] / rows * (1.f - momentum) + to_f32(mean[c]) * momentum);
+    run_var[c] = from_f32<T>(t.v[2] / rows * (1.f - momentum) + to_f32(var[c]) * momentum);
   }
 };
 
@@ -745,13 +764,13 @@ struct StoreGradStats {
   int C;
   float rows, eps;
   __device__ __forceinline__ void operator()(int c, const Moments<true>& t) const {
-    const float variance = t.sxx / rows;
-    stats0[c] = t.sx / rows;
-    stats0[C + c] = t.sy / rows;
+    const float variance = t.v[2] / rows;
+    stats0[c] = t.v[3] / rows;
+    stats0[C + c] = t.v[7] / rows;
     stats1[c] = variance;
-    stats1[C + c] = t.sxy;
-    beta_grad[c] = from_f32<T>(t.sy);
-    gamma_grad[c] = from_f32<T>(t.sxy / sqrtf(variance + eps));
+    stats1[C + c] = t.v[6];
+    beta_grad[c] = from_f32<T>(t.v[7]);
+    gamma_grad[c] = from_f32<T>(t.v[6] / sqrtf(variance + eps));
   }
 };
 
@@ -885,14 +904,15 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
       size_t per = 0;
       const int slices = moment_slices(rows, C, sms, &per);
       Scratch sc;
-      const int st = get_scratch(&sc, slices, C, s);
+      const int st = get_scratch(&sc, Moments<false>::N / 2 * slices, C, s);
       if (st != PDNN_OK) return st;
       const dim3 grid((unsigned)slices, (unsigned)((C / kMomentChannels + 31) / 32));
       const T *mt = static_cast<const T*>(mean), *vt = static_cast<const T*>(variance);
       launch_overlapped(batchnorm_moments_kernel<T, false, true>, grid, kBlock, s, static_cast<const T*>(input), nullptr,
           static_cast<const T*>(beta), static_cast<const T*>(gamma), mt, vt,
           static_cast<T*>(output), sc.partial, rows, C, per, p.epsilon);
-      launch_overlapped(batchnorm_merge_kernel<false, StoreRunning<T>>, (C + 31) / 32, 1024, s, sc.partial, slices, C, rows, per,
+      launch_overlapped(batchnorm_merge_kernel<false, StoreRunning<T>>, (C + kMergeChannels - 1) / kMergeChannels, kMergeChannels * kMergeLanes, s,
+          sc.partial, slices, C, rows, per,
           StoreRunning<T>{mt, vt, static_cast<T*>(running_mean), static_cast<T*>(running_variance), (float)rows, p.momentum});
       count_launch();
       cudaFreeAsync(sc.base, s);
@@ -955,7 +975,7 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
     const int slices = one_pass ? moment_slices(rows, C, sms, &per_slice) : slices_for(rows, C, sms, vec ? 32 * VN : 32);
     if (!one_pass) per_slice = (rows + slices - 1) / slices;
     Scratch sc;
-    int st = get_scratch(&sc, one_pass ? 2 * slices : slices, C, s);
+    int st = get_scratch(&sc, one_pass ? Moments<true>::N / 2 * slices : slices, C, s);
     if (st != PDNN_OK) return st;
     const dim3 grid(slices, (C + 31) / 32), vgrid(slices, (C / VN + 31) / 32);
     const unsigned c1grid = (C + kBlock - 1) / kBlock;
@@ -965,8 +985,8 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
       launch_overlapped(batchnorm_moments_kernel<T, true, false>, mgrid, kBlock, s, x, dy, nullptr, nullptr, nullptr, nullptr,
           nullptr, sc.partial,
                                                                        rows, C, per_slice, 0.f);
-      launch_overlapped(batchnorm_merge_kernel<true, StoreGradStats<T>>, (C + 31) / 32, 1024, s, sc.partial, slices, C, rows,
-          per_slice,
+      launch_overlapped(batchnorm_merge_kernel<true, StoreGradStats<T>>, (C + kMergeChannels - 1) / kMergeChannels, kMergeChannels * kMergeLanes,
+          s, sc.partial, slices, C, rows, per_slice,
           StoreGradStats<T>{sc.stats0, sc.stats1, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), C, (float)rows, p.epsilon});
       launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s, x, dy,
           g, sc.stats0, sc.stats1, static_cast<T*>(output), n / VN, C, (float)rows, p.epsilon);

@@ -99,3 +99,52 @@ def test_batchnorm_moments_far_from_zero(rows, channels, dtype):
     share = cov.abs() / rows / (v + 1e-3)
     slack = (9 * e + 2.0 ** -20 * dy64.abs() + (33 * e + 2.0 ** -20 * x64.abs()) * share + xc.abs() * (cov_slack / rows + 66 * e * share) / (v + 1e-3)) / sd
     assert near(dx, ref, 2 * slack)
+
+
+def _batch_statistics(x, dy):
+    """Batch mean and variance, and the gradients, of fp32 rows x channels; the same in float64."""
+    rows, channels = x.shape
+    one, zero = np.ones(channels, np.float32), np.zeros(channels, np.float32)
+    p = pd.batchnorm_params(1, 1, rows, channels, True, 1e-3, 0.0)
+    _, mean, var = pd.batchnorm_forward(to_dev(x, "f32"), *(to_dev(t, "f32") for t in (zero, one, zero, one)), p)
+    dx, dbeta, dgamma = pd.batchnorm_gradient(to_dev(x, "f32"), to_dev(dy, "f32"), to_dev(one, "f32"), p)
+    got = [to_host(t).astype(np.float64) for t in (mean, var, dgamma, dbeta)] + [to_host(dx).astype(np.float64).reshape(x.shape)]
+    with np.errstate(all="ignore"):
+        x64, dy64 = x.astype(np.float64), dy.astype(np.float64)
+        xc = x64 - x64.mean(0)
+        v = (xc ** 2).mean(0)
+        cov = ((dy64 - dy64.mean(0)) * xc).sum(0)
+        dx64 = (dy64 - dy64.mean(0) - xc * cov / rows / (v + 1e-3)) / np.sqrt(v + 1e-3)
+    return got, [x64.mean(0), v, cov / np.sqrt(v + 1e-3), dy64.sum(0), dx64]
+
+
+@pytest.mark.parametrize("rows,channels", [(40, 8), (1000, 24), (6001, 136)])
+@pytest.mark.parametrize("mean,deviation,dy_mean", [(1e3, 1.0, 0.0), (1e3, 1.0, 8.0), (2e19, 1e17, 1.0), (-3e19, 1e16, 0.0)])
+def test_batchnorm_moments_ignore_the_mean(rows, channels, mean, deviation, dy_mean):
+    """The variance and the sums with the gradient are as exact far from zero as near it, and finite where
+    the square of the mean is not (a mean is known to 2^-24 of itself, which enters neither)."""
+    rng = np.random.default_rng(rows)
+    x = (mean + deviation * rng.standard_normal((rows, channels))).astype(np.float32)
+    dy = (dy_mean + rng.standard_normal((rows, channels))).astype(np.float32)
+    got, ref = _batch_statistics(x, dy)
+    # a lane's sums of at most 4 + rows / 64 rows lose 2^-24 of themselves with each, and the terms are up to twice
+    # the squared deviations (the subtracted value is not the mean); then three levels of merging
+    u = 2.0 ** -24 * (2 * (4 + rows / 256) + 8)
+    magnitude = np.abs((x - ref[0]) * (dy - dy.astype(np.float64).mean(0))).sum(0) / np.sqrt(ref[1] + 1e-3)
+    assert np.all(np.abs(got[1] - ref[1]) <= u * ref[1])
+    assert np.all(np.abs(got[2] - ref[2]) <= 2 * u * (magnitude + np.abs(ref[2])))
+    assert np.all(np.isfinite(got[4]))
+
+
+@pytest.mark.parametrize("rows", [64, 1000, 6001])
+@pytest.mark.parametrize("at", [0, 3, 63])
+def test_batchnorm_moments_of_one_row(rows, at):
+    """A channel that is the same everywhere but in one row, which a lane may have subtracted from the others."""
+    x = np.full((rows, 8), 5.0, np.float32)
+    x[at] = 1000.0 + np.arange(8)
+    dy = np.random.default_rng(at).standard_normal((rows, 8)).astype(np.float32)
+    got, ref = _batch_statistics(x, dy)
+    # the lane of that row adds up to 4 + rows / 256 terms that are together up to 1 + rows / 256 / 4 times their
+    # squared deviations
+    u = 2.0 ** -24 * (8 + rows / 64) * (1 + rows / 1024)
+    assert np.all(np.abs(got[1] - ref[1]) <= u * ref[1])
