@@ -115,7 +115,7 @@ def _batch_statistics(x, dy):
         v = (xc ** 2).mean(0)
         cov = ((dy64 - dy64.mean(0)) * xc).sum(0)
         dx64 = (dy64 - dy64.mean(0) - xc * cov / rows / (v + 1e-3)) / np.sqrt(v + 1e-3)
-    return got, [x64.mean(0), v, cov / np.sqrt(v + 1e-3), dy64.sum(0), dx64]
+        return got, [x64.mean(0), v, cov / np.sqrt(v + 1e-3), dy64.sum(0), dx64]
 
 
 @pytest.mark.parametrize("rows,channels", [(40, 8), (1000, 24), (6001, 136)])
@@ -148,3 +148,29 @@ def test_batchnorm_moments_of_one_row(rows, at):
     # squared deviations
     u = 2.0 ** -24 * (8 + rows / 64) * (1 + rows / 1024)
     assert np.all(np.abs(got[1] - ref[1]) <= u * ref[1])
+
+
+@pytest.mark.parametrize("rows,channels", [(40, 8), (1000, 24)])
+def test_batchnorm_infinities(rows, channels):
+    """What an infinity or a NaN makes of the results: what the formulas make of it, in the channel it is in."""
+    rng = np.random.default_rng(rows)
+    x, dy = (rng.standard_normal((rows, channels)).astype(np.float32) for _ in range(2))
+    inf, last = np.float32(np.inf), rows - 1
+    x[last, 0] = 3.0
+    x[2, 1] = -3.0
+    dy[last, 0] = inf              # dgamma = inf * (3 - mean) / deviation
+    dy[2, 1] = inf                 # the same with -3
+    dy[1, 2], dy[last, 2] = inf, -inf  # dbeta = NaN
+    x[5, 3] = inf                  # mean = inf, variance = NaN
+    dy[7, 4] = np.nan
+    x[0, 5], x[1, 5] = 3e38, -3e38  # the variance overflows
+    got, ref = _batch_statistics(x, dy)
+    mean, var, dgamma, dbeta, dx = got
+    assert dgamma[0] == np.inf and dgamma[1] == -np.inf and dbeta[0] == dbeta[1] == np.inf
+    assert np.isnan(dbeta[2])
+    assert mean[3] == np.inf and np.isnan(var[3]) and np.isnan(dgamma[3]) and np.isfinite(dbeta[3])
+    assert np.isfinite(mean[4]) and np.isfinite(var[4]) and np.isnan(dgamma[4]) and np.isnan(dbeta[4])
+    assert np.isfinite(mean[5]) and var[5] == np.inf
+    for t, r in zip(got[:4], ref):
+        assert np.allclose(t[6:], r[6:], rtol=1e-4, atol=1e-4)
+    assert np.all(np.isfinite(dx[:, 6:])) and not np.any(np.isfinite(dx[:, :2]))
