@@ -63,23 +63,26 @@ int dtype_code(const at::Tensor& t) {
   }
 }
 
+// A whole number.  (A text or a fraction is a mistake in the call: neither is turned into one.)
 long integer(PyObject* o) {
-  if (PyLong_CheckExact(o)) {
-    const long v = PyLong_AsLong(o);
-    if (v == -1 && PyErr_Occurred()) throw PyFailure();
-    return v;
-  }
-  PyObject* n = PyNumber_Long(o);  // whatever int() takes
+  const long v = PyLong_AsLong(o);
+  if (v == -1 && PyErr_Occurred()) throw PyFailure();
+  return v;
+}
+// Whatever int() takes.
+long to_integer(PyObject* o) {
+  if (PyLong_CheckExact(o)) return integer(o);
+  PyObject* n = PyNumber_Long(o);
   if (n == nullptr) throw PyFailure();
   const long v = PyLong_AsLong(n);
   Py_DECREF(n);
   if (v == -1 && PyErr_Occurred()) throw PyFailure();
   return v;
 }
-float real(PyObject* o) {
+double real(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
   if (v == -1.0 && PyErr_Occurred()) throw PyFailure();
-  return (float)v;
+  return v;
 }
 bool truth(PyObject* o) {
   const int v = PyObject_IsTrue(o);
@@ -132,7 +135,7 @@ PyObject* conv2d(PyObject* const* a) {
   at::Tensor out = tensor(a[5]);
   const at::Tensor &workspace = tensor(a[6]), &bias = tensor(a[7]);
   const int activation = (int)integer(a[8]);
-  const float alpha = real(a[9]), beta = real(a[10]);
+  const double alpha = real(a[9]), beta = real(a[10]);
   const at::Tensor& relu_out = tensor(a[11]);
   const bool output_f32 = truth(a[12]);
   const bool accumulate = truth(a[13]);
@@ -175,7 +178,7 @@ PyObject* conv2d(PyObject* const* a) {
     PdnnBackpropFusion f = {};
     f.relu_forward_output = ptr(relu_out);
     f.output_f32 = output_f32;
-    f.accumulate = (int)integer(a[13]);  // False / True, or 2 (dx already carries the mask)
+    f.accumulate = (int)to_integer(a[13]);  // False / True, or 2 (dx already carries the mask)
     f.relu_bitmask = ptr(bits);
     f.constant_filter = constant_filter;
     call([&] {
@@ -184,15 +187,15 @@ PyObject* conv2d(PyObject* const* a) {
     });
     return THPVariable_Wrap(out);
   }
-  const bool fused = bias.defined() || activation != PDNN_ACT_NONE || alpha != 1.f || beta != 0.f || bits.defined() ||
+  const bool fused = bias.defined() || activation != PDNN_ACT_NONE || alpha != 1.0 || beta != 0.0 || bits.defined() ||
                      (constant_filter && pass == PDNN_FORWARD);
   if (fused) {
     if (pass != PDNN_FORWARD) raise(PyExc_ValueError, "the fused epilogue exists for the forward pass only");
     PdnnConvEpilogue e = {};
     e.bias = ptr(bias);
     e.activation = activation;
-    e.alpha = alpha;
-    e.beta = beta;
+    e.alpha = (float)alpha;
+    e.beta = (float)beta;
     e.relu_bitmask = ptr(bits);
     e.constant_filter = constant_filter;
     call([&] {
@@ -286,7 +289,7 @@ PyObject* bias_add(PyObject* const* a) {
   require_cuda(inp, bias, tensor(a[4]));
   if (channels == 0) raise(PyExc_ZeroDivisionError, "integer division or modulo by zero");
   const at::Tensor out = out_or_like(tensor(a[4]), inp);
-  const int dtype = dtype_code(inp), activation = (int)integer(a[3]);
+  const int dtype = dtype_code(inp), activation = (int)to_integer(a[3]);
   call([&] {
     return pdnn_bias_add(dtype, ptr(inp), ptr(bias), ptr(out), (size_t)(inp.numel() / channels), (int)channels, activation,
                          stream());
@@ -299,32 +302,30 @@ PyObject* scale_blend(PyObject* const* a) {
   require_cuda(x, b, tensor(a[4]));
   const at::Tensor out = out_or_like(tensor(a[4]), x);
   const int dtype = dtype_code(x);
-  const float alpha = real(a[1]), beta = real(a[3]);
+  const float alpha = (float)real(a[1]), beta = (float)real(a[3]);
   call([&] { return pdnn_scale_blend(dtype, ptr(x), alpha, ptr(b), beta, ptr(out), (size_t)x.numel(), stream()); });
   return THPVariable_Wrap(out);
 }
 
-// A sequence of extents; at most `most` of them are kept, all are counted.
+// A sequence of extents: all are counted, the first kMostDims kept (the library takes no more than four).
 constexpr int kMostDims = 16;
 int extents(PyObject* o, int (&d)[kMostDims]) {
   PyObject* seq = PySequence_Fast(o, "expected a sequence of extents");
   if (seq == nullptr) throw PyFailure();
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
-  bool ok = n <= kMostDims;
-  for (Py_ssize_t i = 0; ok && i < n; ++i) {
+  for (Py_ssize_t i = 0; i < n && !PyErr_Occurred(); ++i) {
     PyObject* v = PyNumber_Long(PySequence_Fast_GET_ITEM(seq, i));
-    d[i] = v != nullptr ? (int)PyLong_AsLong(v) : 0;
+    const int extent = v != nullptr ? (int)PyLong_AsLong(v) : 0;
     Py_XDECREF(v);
-    ok = !PyErr_Occurred();
+    if (i < kMostDims) d[i] = extent;
   }
   Py_DECREF(seq);
   if (PyErr_Occurred()) throw PyFailure();
-  if (!ok) raise(PyExc_ValueError, "too many extents");
   return (int)n;
 }
 
 PyObject* binaryop(PyObject* const* a) {
-  const int op = (int)integer(a[0]);
+  const int op = (int)to_integer(a[0]);
   const at::Tensor &lhs = tensor(a[1]), &rhs = tensor(a[3]);
   int ld[kMostDims] = {}, rd[kMostDims] = {};
   require_cuda(lhs, rhs, tensor(a[5]));
@@ -332,8 +333,8 @@ PyObject* binaryop(PyObject* const* a) {
   at::Tensor out = tensor(a[5]);
   if (!out.defined()) {
     const int n = nl > nr ? nl : nr;
-    int64_t numel = 1;
-    for (int i = 0; i < n; ++i) {
+    int64_t numel = n <= kMostDims ? 1 : 0;  // (more than the library takes)
+    for (int i = 0; i < n && numel != 0; ++i) {
       const int l = i < n - nl ? 1 : ld[i - (n - nl)], r = i < n - nr ? 1 : rd[i - (n - nr)];
       const int m = l > r ? l : r;
       numel *= m > 0 ? m : 0;
@@ -347,20 +348,23 @@ PyObject* binaryop(PyObject* const* a) {
 
 PyObject* matmul(PyObject* const* a) {
   const at::Tensor &lhs = tensor(a[0]), &rhs = tensor(a[1]);
-  const long batches = integer(a[2]), m = integer(a[3]), k = integer(a[4]), n = integer(a[5]);
+  auto extent = [](PyObject* o) {  // 8.0 is one, 8.5 is not
+    return PyFloat_Check(o) && PyFloat_AS_DOUBLE(o) == (double)(int)PyFloat_AS_DOUBLE(o) ? to_integer(o) : integer(o);
+  };
+  const long batches = extent(a[2]), m = extent(a[3]), k = extent(a[4]), n = extent(a[5]);
   const bool tl = truth(a[6]), tr = truth(a[7]);
-  const float beta = real(a[8]);
+  const double beta = real(a[8]);
   at::Tensor out = tensor(a[9]);
   require_cuda(lhs, rhs, out);
   if (lhs.numel() != (int64_t)batches * m * k || rhs.numel() != (int64_t)batches * k * n)
     raise(PyExc_ValueError, "tensor sizes do not match the parameters");
   if (!out.defined()) {
-    if (beta != 0.f) raise(PyExc_ValueError, "beta != 0 needs an output tensor to accumulate into");
+    if (beta != 0.0) raise(PyExc_ValueError, "beta != 0 needs an output tensor to accumulate into");
     out = flat((int64_t)batches * m * n, lhs.options());
   }
   const int dtype = dtype_code(lhs);
   call([&] {
-    return pdnn_matmul(dtype, tl, tr, ptr(lhs), ptr(rhs), ptr(out), (int)batches, (int)m, (int)k, (int)n, beta, stream());
+    return pdnn_matmul(dtype, tl, tr, ptr(lhs), ptr(rhs), ptr(out), (int)batches, (int)m, (int)k, (int)n, (float)beta, stream());
   });
   return THPVariable_Wrap(out);
 }

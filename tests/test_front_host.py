@@ -22,3 +22,23 @@ X = torch.zeros(512)
 def test_wrong_calls_raise(call, error):
     with pytest.raises(error):
         call()
+
+
+@pytest.mark.parametrize("call", [
+    lambda: pd.conv2d("0", X, X, P),
+    lambda: pd.conv2d(0.5, X, X, P),
+    lambda: pd.conv2d(pd.FORWARD, X, X, P, algorithm="4"),
+    lambda: pd.depthwise_conv2d(0.5, X, X, pd.depthwise_params(1, 8, 8, 8, 1, 3, 1)),
+    lambda: pd.pooling("0", 0, X, pd.pool_params(1, 8, 8, 8, 2, 2)),
+    lambda: pd.pooling(pd.POOL_MAX, 0.5, X, pd.pool_params(1, 8, 8, 8, 2, 2)),
+    lambda: pd.pointwise("1", X),
+    lambda: pd.pointwise_grad(1.5, X, X),
+    lambda: pd.bias_add(X, X, "8"),
+    lambda: pd.bias_add(X, X, 8.5),
+    lambda: pd.softmax(X, 1.0, 8, 8, 8),
+    lambda: pd.matmul(X, X, 1, 8.5, 8, 8),
+])
+def test_texts_and_fractions_are_no_integers(call):
+    """Before anything else is looked at, an argument that has to be a whole number is one."""
+    with pytest.raises(TypeError):
+        call()
