@@ -11,6 +11,7 @@ torch is used for device memory and streams only.
 import ctypes
 import enum
 import os
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB = None
@@ -95,13 +96,20 @@ def lib():
     return _LIB
 
 
+def front_path():
+    """The extension module behind the operators.  It is compiled against one Python and one torch, which its name
+    carries: under another it is missing, not loaded."""
+    torch = _torch()
+    return os.path.join(_HERE, "_front.%s-torch%s-abi%d.so" % (
+        sysconfig.get_config_var("SOABI"), torch.__version__, int(torch._C._GLIBCXX_USE_CXX11_ABI)))
+
+
 def _front():
     """Loads the extension module behind the operators (it links against the library beside it)."""
     global _F
     if _F is None:
         lib()
-        _torch()  # its libraries must be in the process before the extension is
-        path = os.path.join(_HERE, "_front.so")
+        path = front_path()  # (and torch's libraries are in the process before the extension is)
         if not os.path.exists(path):
             raise ImportError("%s is missing: build it with `python -m portdnn_b200.build`" % path)
         from importlib import machinery, util

@@ -1,21 +1,24 @@
 """Builds libportdnn_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and
-_front.so, the native half of api.py, with the host compiler against torch's headers.
+the extension module behind api.py (api.front_path()), with the host compiler against torch's headers.
 
 Each source is compiled to its own object (in parallel, only when it or a header changed) and
 the objects are linked into the shared library.
 
 Usage: python -m portdnn_b200.build [--force] [--verbose]
 """
+import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
+
+from .api import front_path
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_obj")
 LIB = os.path.join(HERE, "libportdnn_b200.so")
-FRONT = os.path.join(HERE, "_front.so")
 FRONT_SOURCE = os.path.join(CSRC, "front.cpp")
 SOURCES = ["c_api.cu", "hbm_kernels.cu", "direct_conv.cu", "tc_gemm.cu", "winograd.cu", "norm_kernels.cu",
            "layout_kernels.cu", "padded_conv.cu", "collective.cu"]
@@ -43,7 +46,7 @@ def _stale(target, deps):
 
 
 def needs_build():
-    return _stale(LIB, [os.path.join(CSRC, s) for s in SOURCES] + _headers()) or _stale(FRONT, _front_deps())
+    return _stale(LIB, [os.path.join(CSRC, s) for s in SOURCES] + _headers()) or _stale(front_path(), _front_deps())
 
 
 def _front_deps():
@@ -52,7 +55,6 @@ def _front_deps():
 
 def _front_command():
     """The extension finds libportdnn_b200.so beside itself and torch's libraries in the running process."""
-    import sysconfig
     import torch
     from torch.utils import cpp_extension
     includes = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(os.path.dirname(_nvcc()), "..", "include")]
@@ -60,7 +62,7 @@ def _front_command():
     return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
             "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] + \
         [f for i in includes for f in ("-isystem", i)] + \
-        [FRONT_SOURCE, "-o", FRONT, "-L" + HERE, "-lportdnn_b200", "-L" + libdir, "-lc10", "-lc10_cuda", "-ltorch_cpu",
+        [FRONT_SOURCE, "-o", front_path(), "-L" + HERE, "-lportdnn_b200", "-L" + libdir, "-lc10", "-lc10_cuda", "-ltorch_cpu",
          "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
 
 
@@ -87,8 +89,11 @@ def build(force=False, verbose=False):
     objs = [os.path.join(OBJ, s[:-3] + ".o") for s in SOURCES]
     if jobs or _stale(LIB, objs):
         _run([nvcc, "-shared", "-cudart", "shared", "-Xcompiler", "-fPIC"] + objs + ["-ldl", "-o", LIB], verbose)
-    if force or _stale(FRONT, _front_deps()):
+    if force or _stale(front_path(), _front_deps()):
         _run(_front_command(), verbose)
+        for other in glob.glob(os.path.join(HERE, "_front.*so")):  # of another Python or torch
+            if other != front_path():
+                os.remove(other)
     return LIB
 
 

@@ -1,8 +1,11 @@
 """Argument checks of the native front end that need no GPU: what a wrong call raises."""
+import os
+
 import pytest
 import torch
 
 import portdnn_b200 as pd
+from portdnn_b200 import api, build
 
 P = pd.conv_params(1, 8, 8, 8, 8, 3, 1)
 X = torch.zeros(512)
@@ -42,3 +45,14 @@ def test_texts_and_fractions_are_no_integers(call):
     """Before anything else is looked at, an argument that has to be a whole number is one."""
     with pytest.raises(TypeError):
         call()
+
+
+def test_the_extension_of_another_torch_is_not_loaded(monkeypatch):
+    """It is compiled against torch's headers: under another torch it counts as not built, and says so."""
+    built = api.front_path()
+    assert os.path.exists(built)
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    monkeypatch.setattr(api, "_F", None)
+    assert api.front_path() != built and build.needs_build()
+    with pytest.raises(ImportError, match="portdnn_b200.build"):
+        pd.pointwise(pd.ACT_RELU, X)
