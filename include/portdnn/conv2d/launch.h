@@ -44,6 +44,7 @@ struct FusedEpilogue {
   float beta = 0.f;
   void* relu_bitmask = nullptr;  // PdnnConvEpilogue::relu_bitmask
   bool constant_filter = false;  // PdnnConvEpilogue::constant_filter
+  bool any_order = false;        // PdnnConvEpilogue::any_order
 };
 
 template <typename T, typename ConvType, typename Backend>
@@ -72,7 +73,7 @@ SNNStatus launch_fused(T const* input, T const* filter, T* output, Conv2DParams 
                        Backend& backend, FusedEpilogue const& epilogue, T* workspace = nullptr, size_t workspace_size = 0) {
   const Algorithm algo = selector.select<conv_type::Forward>(params);
   const PdnnConvEpilogue e{epilogue.bias,         epilogue.activation, epilogue.alpha, epilogue.beta,
-                           epilogue.relu_bitmask, epilogue.constant_filter ? 1 : 0};
+                           epilogue.relu_bitmask, epilogue.constant_filter ? 1 : 0, epilogue.any_order ? 1 : 0};
   const int st = pdnn_conv2d_fused(backend::dtype_of<T>::value, input, filter, output,
                                    reinterpret_cast<const PdnnConv2DParams*>(&params), int(algo), &e, workspace,
                                    workspace_size, backend.get_queue());

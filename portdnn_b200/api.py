@@ -210,7 +210,7 @@ def conv2d_workspace_size(pass_, dtype, params, algorithm):
 
 def conv2d(pass_, inp, fil, params, algorithm=ALGO_IM2COL, out=None, workspace=None, bias=None, activation=ACT_NONE,
            alpha=1.0, beta=0.0, relu_forward_output=None, output_f32=False, accumulate=False, relu_bitmask=None,
-           constant_filter=False):
+           constant_filter=False, any_order=False):
     """conv2d::launch<T, ConvType>(input, filter, output, params, selector, backend, workspace, size)
     (include/portdnn/conv2d/launch.h:59-72) with the selector's answer passed as ``algorithm``.
     Slots: Forward (x, w) -> y; InputBackprop (dy, w) -> dx; FilterBackprop (x, dy) -> dW.
@@ -219,9 +219,12 @@ def conv2d(pass_, inp, fil, params, algorithm=ALGO_IM2COL, out=None, workspace=N
     PdnnBackpropFusion.  relu_bitmask: a uint8 tensor of one bit per element (numel / 8 bytes) - written by
     the forward pass beside its output, read by the input backprop in place of relu_forward_output.
     constant_filter (Forward, InputBackprop): filter and bias were not written by the kernel that precedes this
-    call in the stream, so the kernel may fetch them while that kernel is still finishing."""
+    call in the stream, so the kernel may fetch them while that kernel is still finishing.
+    any_order (Forward): the order in which the products of an output are added may depend on the batch, which
+    lets a single image take a faster kernel; without it an image's result is the same, bit by bit, alone and
+    beside others."""
     return (_F or _front()).conv2d(pass_, inp, fil, params, algorithm, out, workspace, bias, activation, alpha, beta,
-                                   relu_forward_output, output_f32, accumulate, relu_bitmask, constant_filter)
+                                   relu_forward_output, output_f32, accumulate, relu_bitmask, constant_filter, any_order)
 
 
 def depthwise_conv2d(pass_, inp, fil, params, out=None, workspace=None):
@@ -288,7 +291,8 @@ def scale_blend(a, alpha, b=None, beta=0.0, out=None):
 
 def matmul(lhs, rhs, batches, m, k, n, transpose_lhs=False, transpose_rhs=False, beta=0.0, out=None):
     """matmul::launch<T, TransposeLHS, TransposeRHS> (include/portdnn/matmul/launch.h:37-90):
-    out[b] = beta*out[b] + op(lhs[b]) @ op(rhs[b]), row-major, strided batches."""
+    out[b] = beta*out[b] + op(lhs[b]) @ op(rhs[b]), row-major, strided batches.  The order in which the products
+    of an output are added depends on the sizes, the number of rows among them."""
     return (_F or _front()).matmul(lhs, rhs, batches, m, k, n, transpose_lhs, transpose_rhs, beta, out)
 
 

@@ -140,7 +140,7 @@ PyObject* conv2d(PyObject* const* a) {
   const bool output_f32 = truth(a[12]);
   const bool accumulate = truth(a[13]);
   const at::Tensor& bits = tensor(a[14]);
-  const bool constant_filter = truth(a[15]);
+  const bool constant_filter = truth(a[15]), any_order = truth(a[16]);
 
   require_cuda(inp, fil, out, workspace, bias);
   const int64_t x = (int64_t)p.batch * p.in_rows * p.in_cols * p.channels;
@@ -188,7 +188,7 @@ PyObject* conv2d(PyObject* const* a) {
     return THPVariable_Wrap(out);
   }
   const bool fused = bias.defined() || activation != PDNN_ACT_NONE || alpha != 1.0 || beta != 0.0 || bits.defined() ||
-                     (constant_filter && pass == PDNN_FORWARD);
+                     (constant_filter && pass == PDNN_FORWARD) || any_order;
   if (fused) {
     if (pass != PDNN_FORWARD) raise(PyExc_ValueError, "the fused epilogue exists for the forward pass only");
     PdnnConvEpilogue e = {};
@@ -198,6 +198,7 @@ PyObject* conv2d(PyObject* const* a) {
     e.beta = (float)beta;
     e.relu_bitmask = ptr(bits);
     e.constant_filter = constant_filter;
+    e.any_order = any_order;
     call([&] {
       return pdnn_conv2d_fused(dtype, ptr(inp), ptr(fil), ptr(out), &p, algorithm, &e, ptr(workspace), ws_elems, stream());
     });
@@ -452,7 +453,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 #define ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<name, n>)), METH_FASTCALL, nullptr}
-PyMethodDef kMethods[] = {ENTRY(conv2d, 16),
+PyMethodDef kMethods[] = {ENTRY(conv2d, 17),
                           ENTRY(depthwise_conv2d, 6),
                           ENTRY(pooling, 5),
                           ENTRY(pooling_max_grad, 7),

@@ -2970,10 +2970,13 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   g.tiles_n = ceil_div(p.batch, g.tn);
   const long long row_tiles = (long long)g.tiles_w * g.tiles_h * g.tiles_n;
   const int ksteps_all = p.window_rows * p.window_cols * ceil_div(p.channels, epr);
-  // One image, few tiles and a long reduction: clusters that share a tile's steps.  From two images on every
-  // plan adds the terms of a sum in the same order, so that an image's result does not depend on how many
-  // others are in its batch (running the first layers in slices of the batch relies on it).
-  const int cluster = (try_cluster && !halo && plan_out == nullptr && p.batch == 1) ? cluster_splits(dtype, row_tiles, p.features, ksteps_all, sms) : 0;
+  // One image, few tiles and a long reduction: clusters that share a tile's steps, if the caller leaves the order
+  // of the sums open.  All other plans add the terms of a sum in the same order, so that an image's result
+  // does not depend on how many others are in its batch (running the first layers in slices of the batch,
+  // of one image or more, relies on it).
+  const bool any_order = epi != nullptr && epi->any_order != 0;
+  const int cluster = (try_cluster && any_order && !halo && plan_out == nullptr && p.batch == 1)
+                          ? cluster_splits(dtype, row_tiles, p.features, ksteps_all, sms) : 0;
   // Long reductions over filters too large to keep in shared memory are bound by the bytes that
   // pass through an SM's shared memory per MMA (the operand reads of the tensor core and the TMA
   // fills share its 128 bytes per cycle): the two pipelines then share one B tile per stage (pair

@@ -249,7 +249,8 @@ class ConvStackRunner:
             api.conv2d(api.FORWARD, self._in(i), self.weights[i], p, algorithm=api.ALGO_IM2COL, out=self._out(i),
                        bias=self.biases[i], activation=l.activation, workspace=self.workspaces.get(i),
                        relu_bitmask=self.bits.get(i) if self.training else None,
-                       constant_filter=True)  # the weights are not written inside a step
+                       constant_filter=True,  # the weights are not written inside a step
+                       any_order=True)  # (a single image is a network of its own here: no slices of it to agree with)
         else:
             api.pooling(l.op, 0, self._in(i), p, out=self._out(i))
 

@@ -41,7 +41,8 @@ SHAPES = [
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("fhwc", [False, True])
-def test_conv(shape, dtype, fhwc):
+@pytest.mark.parametrize("any_order", [False, True])
+def test_conv(shape, dtype, fhwc, any_order):
     n, h, w, c, k, win, st = shape
     dt, g = TORCH_DTYPES[dtype], torch.Generator(device="cuda").manual_seed(h * c + k)
     p = pd.conv_params(n, h, w, c, k, win, st, filter_format=2 if fhwc else 0)
@@ -52,14 +53,31 @@ def test_conv(shape, dtype, fhwc):
     w64 = wt.double().permute(3, 2, 0, 1)
     ref = torch.nn.functional.conv2d(xp, w64, stride=st).permute(0, 2, 3, 1)
     mag = torch.nn.functional.conv2d(xp.abs(), w64.abs(), stride=st).permute(0, 2, 3, 1)
-    y = pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p).view(ref.shape)
+    y = pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, any_order=any_order).view(ref.shape)
     _check(y, ref, mag, dtype)
-    assert torch.equal(y, pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, constant_filter=True).view(ref.shape))
+    assert torch.equal(y, pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, constant_filter=True,
+                                    any_order=any_order).view(ref.shape))
     bits = torch.zeros(y.numel() // 8, dtype=torch.uint8, device="cuda")
-    yb = pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, bias=b, activation=pd.ACT_RELU, relu_bitmask=bits).view(ref.shape)
+    yb = pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, bias=b, activation=pd.ACT_RELU, relu_bitmask=bits,
+                   any_order=any_order).view(ref.shape)
     _check(yb, (ref + b.double()).relu(), mag + b.double().abs(), dtype, before_bias=ref)
     unpacked = (bits[:, None] >> torch.arange(8, device="cuda", dtype=torch.uint8)) & 1
     assert torch.equal(unpacked.view(ref.shape).bool(), yb > 0)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_an_image_alone_and_in_a_batch(shape, dtype):
+    """Without any_order an image's result has the same bits whatever is beside it."""
+    _, h, w, c, k, win, st = shape
+    dt, g = TORCH_DTYPES[dtype], torch.Generator(device="cuda").manual_seed(h * c + k)
+    x, wt, b = _rand(g, 5, h, w, c).to(dt), (_rand(g, win, win, c, k) / (win * win * c) ** 0.5).to(dt), _rand(g, k).to(dt)
+    call = lambda xs: pd.conv2d(pd.FORWARD, xs.reshape(-1), wt.reshape(-1), pd.conv_params(len(xs), h, w, c, k, win, st),
+                                bias=b, activation=pd.ACT_RELU, constant_filter=True).view(len(xs), -1)
+    for many in (2, 3, 5):
+        together = call(x[:many])
+        assert all(torch.equal(together[i], call(x[i:i + 1])[0]) for i in range(many))
+    assert_no_device_error()
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])

@@ -87,9 +87,11 @@ def test_resnet50_forward_every_layer_and_end_to_end(orc):
 def test_resnet50_depth_first_slices_equal_layer_by_layer():
     dev = torch.device("cuda", 0)
     a = workloads.ConvStackRunner(workloads.resnet50_v15(8), dev, seed=5)
-    b = workloads.ConvStackRunner(workloads.resnet50_v15(8), dev, seed=5, chunk=2, chunk_layers=25)
-    assert b.chunk == 2
-    assert torch.equal(a.forward(), b.forward())
+    want = a.forward()
+    for chunk in (2, 1):
+        b = workloads.ConvStackRunner(workloads.resnet50_v15(8), dev, seed=5, chunk=chunk, chunk_layers=25)
+        assert b.chunk == chunk
+        assert torch.equal(want, b.forward())
     assert_no_device_error()
 
 
