@@ -65,7 +65,7 @@ def test_conv(shape, dtype, fhwc, any_order):
     assert torch.equal(unpacked.view(ref.shape).bool(), yb > 0)
 
 
-@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_an_image_alone_and_in_a_batch(shape, dtype):
     """Without any_order an image's result has the same bits whatever is beside it."""
