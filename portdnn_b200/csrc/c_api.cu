@@ -221,7 +221,7 @@ int dispatch_conv(int pass, int dtype, const void* in, const void* fil, void* ou
     return launch_winograd(pass, dtype, in, fil, out, *p, epi, ws, ws_elems, s);
   if (pass == PDNN_FORWARD && p->groups > 1 && tc_grouped_conv_supported(dtype, in, fil, out, *p) &&
       (epi == nullptr || epi->relu_bitmask == nullptr))
-    return tc_grouped_conv_forward(dtype, in, fil, out, *p, epi, s);
+    return tc_grouped_conv_forward(dtype, in, fil, out, *p, epi, ws, ws_elems, s);
   if (algorithm != PDNN_ALGO_DIRECT && tc_conv_supported(pass, dtype, in, fil, out, *p)) {
     const int st2 = tc_conv2d(pass, dtype, in, fil, out, *p, epi, fusion, ws, ws_elems, s);
     if (st2 != kNeedsDirect) return st2;
@@ -292,8 +292,8 @@ int pdnn_conv2d_workspace_size(int pass, int dtype, const PdnnConv2DParams* para
   int st = validate_conv(pass, params, algorithm);
   if (st != PDNN_OK) return st;
   if (algorithm == PDNN_ALGO_DIRECT) return PDNN_OK;
-  // The implicit-GEMM kernels read the tensors in place; only the filter backprop's split
-  // reduction wants scratch, and it can do without (it then allocates for the call).
+  // The implicit-GEMM kernels read the tensors in place.  What is copied - partial sums of a filter backprop,
+  // packed and padded operands - goes to scratch that the call allocates where the caller brings none.
   size_t elems = tc_conv_workspace_elems(pass, dtype, *params);
   if (elems == 0) elems = padded_conv_workspace_elems(pass, dtype, *params);
   // Winograd: 16 * (C*K + tiles*C + tiles*K), include/portdnn/conv2d/workspace_size.h:53-73.  It is

@@ -196,7 +196,7 @@ int padded_conv(int pass, int dtype, const void* in, const void* fil, void* out,
   const bool own = base == nullptr || ws_elems * 2 < need;
   if (own && cudaMallocAsync(reinterpret_cast<void**>(&base), need, s) != cudaSuccess) {
     cudaGetLastError();
-    return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for padded tensors", need);
+    return kNeedsDirect;  // (the direct kernel reads the tensors where they are)
   }
   char* at = reinterpret_cast<char*>(round_up(reinterpret_cast<uintptr_t>(base), 256));
   auto take = [&](size_t bytes) {

@@ -9,7 +9,9 @@ namespace pdnn {
 // tc_conv_supported asks, and enough work to pay for the copies.
 bool padded_conv_applicable(int pass, int dtype, const PdnnConv2DParams& p, const PdnnConvEpilogue* epi);
 
-// Scratch elements (of dtype) of the copies; without them the call allocates.
+// Scratch elements (of dtype) of the copies; without them the call allocates, and where there is no memory
+// either padded_conv asks for the direct kernel.  (Tensors off a 16-byte boundary are not known to the query:
+// their copies are not counted for a layer whose channel and feature counts need none.)
 size_t padded_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p);
 
 // May return kNeedsDirect (tc_gemm.cuh).

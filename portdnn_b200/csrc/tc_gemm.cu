@@ -3139,15 +3139,25 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// All groups in one launch of umma_gemm_grouped_kernel, or kNeedsDirect where the layer does not fit it: 16-bit
-// tensors, groups of 16, 32, 48 or 64 channels, tiles of 64, 128 or 256 features; and more groups than one
-// launch of the multi-GEMM kernel takes, since with the packing of the filter this one is two launches.
-int conv_forward_grouped(int dtype, const void* x, const void* w, void* y, const PdnnConv2DParams& p,
-                         const PdnnConvEpilogue* epi, cudaStream_t s, bool try_halo = true) {
+// Bytes of the packed filter of a layer that fits umma_gemm_grouped_kernel, else 0: 16-bit tensors, groups of 16,
+// 32, 48 or 64 channels, tiles of 64, 128 or 256 features; and more groups than one launch of the multi-GEMM
+// kernel takes, since with the packing of the filter this one is two launches.
+size_t grouped_filter_bytes(int dtype, const PdnnConv2DParams& p) {
   const int Cg = p.channels / p.groups, Kg = p.features / p.groups;
-  if (dtype == PDNN_F32 || p.groups <= kMaxMulti || Cg % 16 != 0 || Cg > 64 || Kg % 16 != 0) return kNeedsDirect;
+  if (dtype == PDNN_F32 || p.groups <= kMaxMulti || Cg % 16 != 0 || Cg > 64 || Kg % 16 != 0) return 0;
+  const int bn = 64 / Cg * Kg;
+  if (bn != 64 && bn != 128 && bn != 256) return 0;
+  return (size_t)p.window_rows * p.window_cols * ceil_div(p.features, bn) * Kg * 128;
+}
+
+// All groups in one launch, or kNeedsDirect where the layer does not fit or its packed filter finds no memory:
+// neither in ws nor, for the duration of the call, on the device.
+int conv_forward_grouped(int dtype, const void* x, const void* w, void* y, const PdnnConv2DParams& p,
+                         const PdnnConvEpilogue* epi, void* ws, size_t ws_bytes, cudaStream_t s, bool try_halo = true) {
+  const size_t packed_bytes = grouped_filter_bytes(dtype, p);
+  if (packed_bytes == 0 || (epi != nullptr && epi->beta != 0.f)) return kNeedsDirect;
+  const int Cg = p.channels / p.groups, Kg = p.features / p.groups;
   const int per_tile = 64 / Cg, bn = per_tile * Kg, sms = device_sm_count();
-  if ((bn != 64 && bn != 128 && bn != 256) || (epi != nullptr && epi->beta != 0.f)) return kNeedsDirect;
   GemmArgs g;
   std::memset(&g, 0, sizeof(g));
   g.bn = bn;
@@ -3197,11 +3207,11 @@ int conv_forward_grouped(int dtype, const void* x, const void* w, void* y, const
   g.num_taps = nt;
   g.cblocks = 1;
   const int taps = p.window_rows * p.window_cols, rows = g.n_tiles * Kg;
-  const size_t packed_bytes = (size_t)taps * rows * 128;
-  void* packed = nullptr;
-  if (cudaMallocAsync(&packed, packed_bytes, s) != cudaSuccess) {
+  void* packed = ws;
+  const bool own = ws == nullptr || ws_bytes < packed_bytes || !aligned16(ws);
+  if (own && cudaMallocAsync(&packed, packed_bytes, s) != cudaSuccess) {
     cudaGetLastError();
-    return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for the packed filter", packed_bytes);
+    return kNeedsDirect;
   }
   g.b_mode = B_K_3;
   const uint64_t dims[4] = {64, (uint64_t)rows, (uint64_t)taps, 1};
@@ -3217,11 +3227,11 @@ int conv_forward_grouped(int dtype, const void* x, const void* w, void* y, const
         p.filter_format == 2);
     status = check_launch("conv2d grouped filter packing");
     if (status == PDNN_OK) status = launch_gemm(plan, dtype, s);
-    cudaFreeAsync(packed, s);
+    if (own) cudaFreeAsync(packed, s);
     return status;
   }
-  cudaFreeAsync(packed, s);
-  return halo ? conv_forward_grouped(dtype, x, w, y, p, epi, s, false) : kNeedsDirect;
+  if (own) cudaFreeAsync(packed, s);
+  return halo ? conv_forward_grouped(dtype, x, w, y, p, epi, ws, ws_bytes, s, false) : kNeedsDirect;
 }
 
 // relu_mask (may be null): the forward output of the layer that produced the tensor dx is the gradient
@@ -3466,7 +3476,7 @@ struct FbpPlan {
 
 constexpr long long kMinPairSlabs = 16;
 
-FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms) {
+FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool try_pair = true) {
   FbpPlan f;
   const int epr = dtype == PDNN_F32 ? 32 : 64;
   choose_box(epr, p.out_cols, p.out_rows, p.batch, &f.tw, &f.th, &f.tn);
@@ -3478,7 +3488,7 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms) {
   // enough to pay for adding its 256 KB tile.  From eight slabs down there is nothing left of the gain (24
   // images: 13.4 -> 13.2 us, through partial sums 16.9 -> 17.4), and a single tile means a partial sum per cluster
   // (28x28 256 -> 256 1x1, 256 images: 39.4 -> 39.3 us, through partial sums 47 -> 50).
-  if (dtype != PDNN_F32 && p.channels % 256 == 0 && p.features % 256 == 0 && sms % 2 == 0) {
+  if (try_pair && dtype != PDNN_F32 && p.channels % 256 == 0 && p.features % 256 == 0 && sms % 2 == 0) {
     const long long tiles = (long long)(p.channels / 256) * (p.features / 256) * p.window_rows * p.window_cols;
     const long long slabs = (long long)f.slabs_w * f.slabs_h * f.slabs_n, want = std::max<long long>(1, (sms / 2) / tiles);
     const long long per = (slabs + want - 1) / want;
@@ -3699,11 +3709,12 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
 // reduction (no partial sums, no second kernel; the order of the float additions is then not fixed);
 // otherwise the split reduction adds to what dW held.
 int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, const PdnnConv2DParams& p, bool out_f32,
-                         bool accumulate, void* ws, size_t ws_elems, cudaStream_t s, bool try_reduce = true) {
+                         bool accumulate, void* ws, size_t ws_elems, cudaStream_t s, bool try_reduce = true,
+                         bool try_pair = true) {
   const size_t es = dtype_size(dtype);
   const int sms = device_sm_count();
   const int epr = dtype == PDNN_F32 ? 32 : 64;
-  const FbpPlan f = plan_filter_backprop(dtype, p, sms);
+  const FbpPlan f = plan_filter_backprop(dtype, p, sms, try_pair);
   GemmArgs g;
   std::memset(&g, 0, sizeof(g));
   g.a_mn = 1;
@@ -3763,6 +3774,8 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
     } else {
       if (cudaMallocAsync(reinterpret_cast<void**>(&partial), need_bytes, s) != cudaSuccess) {
         cudaGetLastError();
+        // (whole tiles of the tensors' own type need no partial sums outside the CTA pairs)
+        if (f.pair) return conv_filter_backprop(dtype, x, dy, dw, p, out_f32, accumulate, ws, ws_elems, s, try_reduce, false);
         return fail(PDNN_ALLOCATION_PROBLEM, "filter backprop: cannot allocate %zu bytes of scratch", need_bytes);
       }
       own = true;
@@ -3798,7 +3811,7 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
       return PDNN_INVALID_PARAMETER;
     }
     // only the staged TMA epilogue can add; anything else goes through partial sums
-    if (reduce && !g.tma_store) return conv_filter_backprop(dtype, x, dy, dw, p, out_f32, accumulate, ws, ws_elems, s, false);
+    if (reduce && !g.tma_store) return conv_filter_backprop(dtype, x, dy, dw, p, out_f32, accumulate, ws, ws_elems, s, false, try_pair);
   }
   int st = launch_gemm(g, dtype, s);
   if (st == PDNN_OK && use_partial) {
@@ -3874,8 +3887,8 @@ bool tc_grouped_conv_supported(int dtype, const void* in, const void* fil, const
 }
 
 int tc_grouped_conv_forward(int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
-                            const PdnnConvEpilogue* epi, cudaStream_t s) {
-  const int together = conv_forward_grouped(dtype, in, fil, out, p, epi, s);
+                            const PdnnConvEpilogue* epi, void* ws, size_t ws_elems, cudaStream_t s) {
+  const int together = conv_forward_grouped(dtype, in, fil, out, p, epi, ws, ws_elems * dtype_size(dtype), s);
   if (together != kNeedsDirect) return together;
   const size_t es = dtype_size(dtype);
   PdnnConv2DParams q = p;
@@ -3922,6 +3935,10 @@ int tc_grouped_conv_forward(int dtype, const void* in, const void* fil, void* ou
 }
 
 size_t tc_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p) {
+  if (pass == PDNN_FORWARD && p.groups > 1) {
+    const void* aligned = reinterpret_cast<const void*>(uintptr_t(256));
+    return tc_grouped_conv_supported(dtype, aligned, aligned, aligned, p) ? grouped_filter_bytes(dtype, p) / dtype_size(dtype) : 0;
+  }
   if (pass == PDNN_FORWARD && small_c_applicable(dtype, p)) {
     const SmallCPlan sp = plan_small_c(dtype, p);
     return (sp.xp_bytes + sp.wp_bytes) / dtype_size(dtype);

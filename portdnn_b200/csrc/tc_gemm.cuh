@@ -10,7 +10,8 @@ namespace pdnn {
 bool tc_conv_supported(int pass, int dtype, const void* in, const void* fil, const void* out,
                        const PdnnConv2DParams& p);
 
-// Scratch elements (of dtype) the pass needs: only the filter backprop's split reduction uses any.
+// Scratch elements (of dtype) the pass can use: the filter backprop's partial sums, the packed copies of a layer
+// of few channels, the packed filter of a grouped layer.
 size_t tc_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p);
 
 // Returned by tc_conv2d when the tensor maps of a few-channel layer could not be encoded: the caller
@@ -21,10 +22,11 @@ int tc_conv2d(int pass, int dtype, const void* in, const void* fil, void* out, c
               const PdnnConvEpilogue* epi, const PdnnBackpropFusion* fusion, void* ws, size_t ws_elems, cudaStream_t s);
 
 // Grouped forward convolution with STRIDED groups whose per-group channel and feature counts meet
-// tc_conv_supported's alignment rules: one implicit GEMM per group on channel slices of the tensors.
+// tc_conv_supported's alignment rules: all groups in one launch on a packed filter (in ws, or allocated for the
+// call), or one implicit GEMM per group on channel slices of the tensors.
 bool tc_grouped_conv_supported(int dtype, const void* in, const void* fil, const void* out, const PdnnConv2DParams& p);
 int tc_grouped_conv_forward(int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
-                            const PdnnConvEpilogue* epi, cudaStream_t s);
+                            const PdnnConvEpilogue* epi, void* ws, size_t ws_elems, cudaStream_t s);
 
 bool tc_matmul_supported(int dtype, int tl, int tr, const void* lhs, const void* rhs, const void* out, int batches,
                          int m, int k, int n);
