@@ -17,7 +17,7 @@ constexpr int kSumFlat = 256;  // threads of a block without row lanes
 // finish(i, sum): what becomes of column i.
 template <int LANES, typename Finish>
 __global__ void __launch_bounds__(32 * LANES)
-    column_sums_kernel(const float* __restrict__ m, int rows, size_t n, Finish finish) {
+    column_sums_kernel(const float* m, int rows, size_t n, Finish finish) {
   overlap_wait();
   __shared__ float red[LANES][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -27,11 +27,11 @@ __global__ void __launch_bounds__(32 * LANES)
     if (i < n) {
       int r = ty;
       for (; r + 3 * LANES < rows; r += 4 * LANES) {
-        const float a = __ldg(m + (size_t)r * n + i), b = __ldg(m + (size_t)(r + LANES) * n + i);
-        const float c = __ldg(m + (size_t)(r + 2 * LANES) * n + i), d = __ldg(m + (size_t)(r + 3 * LANES) * n + i);
+        const float a = m[(size_t)r * n + i], b = m[(size_t)(r + LANES) * n + i];
+        const float c = m[(size_t)(r + 2 * LANES) * n + i], d = m[(size_t)(r + 3 * LANES) * n + i];
         sum += (a + b) + (c + d);
       }
-      for (; r < rows; r += LANES) sum += __ldg(m + (size_t)r * n + i);
+      for (; r < rows; r += LANES) sum += m[(size_t)r * n + i];
     }
     red[ty][tx] = sum;
     __syncthreads();
@@ -48,12 +48,12 @@ __global__ void __launch_bounds__(32 * LANES)
 // One thread per column, for matrices of few rows or so many columns that they fill the device.
 template <typename Finish>
 __global__ void __launch_bounds__(kSumFlat)
-    column_sums_flat_kernel(const float* __restrict__ m, int rows, size_t n, Finish finish) {
+    column_sums_flat_kernel(const float* m, int rows, size_t n, Finish finish) {
   overlap_wait();
   for (size_t i = (size_t)blockIdx.x * kSumFlat + threadIdx.x; i < n; i += (size_t)gridDim.x * kSumFlat) {
     float sum = 0.f;
 #pragma unroll 8
-    for (int r = 0; r < rows; ++r) sum += __ldg(m + (size_t)r * n + i);
+    for (int r = 0; r < rows; ++r) sum += m[(size_t)r * n + i];
     finish(i, sum);
   }
 }

@@ -70,7 +70,7 @@ struct Vec16 {
 template <typename T>
 __device__ __forceinline__ Vec16<T> load16(const T* p) {
   Vec16<T> v;
-  v.raw = __ldg(reinterpret_cast<const uint4*>(p));
+  v.raw = *reinterpret_cast<const uint4*>(p);
   return v;
 }
 template <typename T>
@@ -109,7 +109,10 @@ int device_sm_count();   // SM count of the current device; -1 if it is not an s
 // last ones of its predecessor still run, and overlap_wait(), the first statement of every kernel launched this
 // way, holds them until the predecessor has ended and what it wrote is visible.  The successor may be placed
 // once all blocks have got past that wait, so that two kernels at most are in flight.  (Both instructions do
-// nothing under an ordinary launch.)  Grids of fewer than four waves only: beside a kernel of that length
+// nothing under an ordinary launch.)  The life of such a kernel begins while its predecessor still writes what it
+// will read, so the read-only path is not open to it, which asks for data that nobody writes meanwhile and
+// promises nothing else: its inputs are plain pointers (const without __restrict__, from which the compiler would
+// infer read-only loads) and plain loads, which stay behind the wait.  Grids of fewer than four waves only: beside a kernel of that length
 // the gap is nothing, and long ones chained this way cost the kernels around them.  All launches ordinary /
 // grids below four waves / all overlapped, us: MobileNet-v2 forward at 64 images (80 launches) 824 / 785 / 782,
 // 7x45x61 100 -> 150 3x3 with gradients 152 / 135 / 135, two max pools with gradients 121 / 114 / 114, one

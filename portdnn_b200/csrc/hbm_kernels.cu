@@ -33,7 +33,7 @@ __device__ __forceinline__ float lowest_of<__nv_bfloat16>() { return -3.38953138
 template <typename T, int V>
 __device__ __forceinline__ void load_vec(const T* p, float (&v)[V]) {
   if constexpr (V == 1) {
-    v[0] = to_f32(__ldg(p));
+    v[0] = to_f32(*p);
   } else {
     Vec16<T> pk = load16(p);
 #pragma unroll
@@ -58,7 +58,7 @@ __device__ __forceinline__ void store_vec(T* p, const float (&v)[V]) {
 // NaN never wins; MaxWithNan takes a NaN and then keeps it (src/pooling/operators_impl.h:27-65).
 // ------------------------------------------------------------------------------------------
 template <typename T, int OP, int V, typename Index>
-__global__ void __launch_bounds__(kBlock) pool_forward_kernel(const T* __restrict__ x, T* __restrict__ y,
+__global__ void __launch_bounds__(kBlock) pool_forward_kernel(const T* x, T* __restrict__ y,
                                                               PdnnPoolingParams p, Index n_items) {
   overlap_wait();
   const Index cvecs = (Index)(p.channels / V);
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kBlock)
 // of the general path (winner map and gather) 85 us, here 33.
 template <typename T, int OP, int V, typename Index>
 __global__ void __launch_bounds__(kBlock)
-    pool_max_grad_tiled_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ dy,
+    pool_max_grad_tiled_kernel(const T* x, const T* y, const T* dy,
                                T* __restrict__ dx, PdnnPoolingParams p, Index n_items) {
   overlap_wait();
   const Index cvecs = (Index)(p.channels / V);
@@ -210,19 +210,29 @@ __global__ void __launch_bounds__(kBlock)
     const size_t base = ((size_t)n * p.in_rows + (size_t)oh * p.stride_rows) * p.in_cols + (size_t)ow * p.stride_cols;
     const int rows_left = p.in_rows - oh * p.stride_rows, cols_left = p.in_cols - ow * p.stride_cols;
     const int rows = min(p.window_rows, rows_left), cols = min(p.window_cols, cols_left);
-    for (int r = 0; r < rows; ++r)
-      for (int c = 0; c < cols; ++c) {
-        const size_t off = ((base + (size_t)r * p.in_cols + c) * p.channels) + (size_t)cv * V;
-        float xv[V], g[V];
-        load_vec<T, V>(x + off, xv);
+    // the window in order, four elements requested together
+    for (int at = 0, r = 0, c = 0; at < rows * cols; at += 4) {
+      const int left = rows * cols - at;
+      size_t off[4];
+      float xv[4][V], g[V];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        off[u] = ((base + (size_t)r * p.in_cols + c) * p.channels) + (size_t)cv * V;
+        if (u < left) load_vec<T, V>(x + off[u], xv[u]);
+        if (++c == cols) c = 0, ++r;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (u >= left) break;
 #pragma unroll
         for (int i = 0; i < V; ++i) {
-          const bool hit = open[i] && pool_equal<OP>(xv[i], yv[i]);
+          const bool hit = open[i] && pool_equal<OP>(xv[u][i], yv[i]);
           g[i] = hit ? dv[i] : 0.f;
           open[i] = open[i] && !hit;
         }
-        store_vec<T, V>(dx + off, g);
+        store_vec<T, V>(dx + off[u], g);
       }
+    }
     const bool below = oh == p.out_rows - 1 && rows_left > rows, right = ow == p.out_cols - 1 && cols_left > cols;
     if (below || right) {
       // the rest of the window's rows to the right, and of its columns below
@@ -252,11 +262,11 @@ __device__ __forceinline__ void load_bytes(const unsigned char* p, unsigned (&v)
   static_assert(V == 4 || V == 8, "packet of 4 or 8 channels");
   unsigned lo, hi = 0u;
   if constexpr (V == 8) {
-    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
     lo = raw.x;
     hi = raw.y;
   } else {
-    lo = __ldg(reinterpret_cast<const unsigned*>(p));
+    lo = *reinterpret_cast<const unsigned*>(p);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) v[i] = (lo >> (8 * i)) & 0xFFu;
@@ -408,7 +418,7 @@ struct PoolS2Geometry {
 
 template <typename T, int V>
 __global__ void __launch_bounds__(kBlock)
-    pool_max_grad_s2_kernel(const unsigned char* __restrict__ winner, const T* __restrict__ dy, T* __restrict__ dx,
+    pool_max_grad_s2_kernel(const unsigned char* winner, const T* dy, T* __restrict__ dx,
                             PoolS2Geometry g, unsigned n_items) {
   overlap_wait();
   const unsigned cvecs = (unsigned)(g.C / V);
@@ -551,7 +561,7 @@ __global__ void __launch_bounds__(kBlock)
 // one image: 10 us less.
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
-    pool_avg_global_kernel(const T* __restrict__ x, T* __restrict__ y, unsigned words, unsigned pixels, unsigned n_items) {
+    pool_avg_global_kernel(const T* x, T* __restrict__ y, unsigned words, unsigned pixels, unsigned n_items) {
   overlap_wait();
   constexpr int E = 4 / (int)sizeof(T);
   for (unsigned idx = blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += gridDim.x * kBlock) {
@@ -560,7 +570,7 @@ __global__ void __launch_bounds__(kBlock)
     float acc[E] = {};
 #pragma unroll 8
     for (unsigned i = 0; i < pixels; ++i) {
-      const unsigned raw = __ldg(xp + (size_t)i * words);
+      const unsigned raw = xp[(size_t)i * words];
       const T* v = reinterpret_cast<const T*>(&raw);
 #pragma unroll
       for (int k = 0; k < E; ++k) acc[k] += to_f32(v[k]);
@@ -579,7 +589,7 @@ constexpr int kGlobalPoolLanes = 8;
 // Its gradient: every pixel of an image receives dy / pixels.  250 x 7x7x2048 f16 (51 MB written): 21.2 -> 9.5 us.
 template <typename T, int V>
 __global__ void __launch_bounds__(32 * kGlobalPoolLanes)
-    pool_avg_grad_global_kernel(const T* __restrict__ dy, T* __restrict__ dx, unsigned cvecs, unsigned tiles, unsigned pixels,
+    pool_avg_grad_global_kernel(const T* dy, T* __restrict__ dx, unsigned cvecs, unsigned tiles, unsigned pixels,
                                 unsigned n_blocks) {
   overlap_wait();
   const unsigned tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
@@ -668,7 +678,7 @@ __global__ void __launch_bounds__(kBlock)
         const T* dp = dyn + ((size_t)oh * p.out_cols + ow) * F;
         const T* wp = w + ((size_t)r * p.window_cols + s) * F + (size_t)c * M;
         if constexpr (V == 1) {
-          for (int m = 0; m < M; ++m) acc[0] = fmaf(to_f32(__ldg(dp + m)), to_f32(__ldg(wp + m)), acc[0]);
+          for (int m = 0; m < M; ++m) acc[0] = fmaf(to_f32(dp[m]), to_f32(wp[m]), acc[0]);
         } else {
           float dv[V], wv[V];
           load_vec<T, V>(dp, dv);
@@ -700,7 +710,7 @@ struct IbpS2Geometry {
 };
 
 template <typename T, int V>
-__global__ void __launch_bounds__(kBlock) depthwise_ibp_s2_kernel(const T* __restrict__ dy, const T* __restrict__ w,
+__global__ void __launch_bounds__(kBlock) depthwise_ibp_s2_kernel(const T* dy, const T* w,
                                                                   T* __restrict__ dx, IbpS2Geometry g, unsigned n_items) {
   overlap_wait();
   const unsigned cvecs = (unsigned)(g.C / V);
@@ -969,7 +979,7 @@ struct WordOf<__nv_bfloat16> {
 constexpr int kFbpRowsWarps = 8, kFbpRowsBlocks = 3;  // 80 registers per thread, 24 warps per SM
 template <typename T, int ST>
 __global__ void __launch_bounds__(kFbpRowsWarps * 32, kFbpRowsBlocks)
-    depthwise_filter_backprop_rows_kernel(const T* __restrict__ x, const T* __restrict__ dy, float* __restrict__ partial,
+    depthwise_filter_backprop_rows_kernel(const T* x, const T* dy, float* __restrict__ partial,
                                           PdnnDepthwiseConv2DParams p, int segs, int seg_cols, int per_full, int per_tail) {
   overlap_wait();
   constexpr int E = WordOf<T>::E;
@@ -1030,7 +1040,7 @@ __global__ void __launch_bounds__(kFbpRowsWarps * 32, kFbpRowsBlocks)
     auto fetch_col = [&](int iw, unsigned (&col)[3]) {
       const unsigned off = (unsigned)min(max(iw, 0), p.in_cols - 1) * wstride;
 #pragma unroll
-      for (int r = 0; r < 3; ++r) col[r] = __ldg(xw + xrow[r] + off);
+      for (int r = 0; r < 3; ++r) col[r] = xw[xrow[r] + off];
     };
     auto zero_outside = [&](int iw, unsigned (&col)[3]) {
       const bool cok = iw >= 0 && iw < p.in_cols;
@@ -1057,15 +1067,15 @@ __global__ void __launch_bounds__(kFbpRowsWarps * 32, kFbpRowsBlocks)
 #pragma unroll
         for (int j = 0; j < NEW; ++j, off += wstride)
 #pragma unroll
-          for (int r = 0; r < 3; ++r) nx[j][r] = __ldg(xw + xrow[r] + off);
+          for (int r = 0; r < 3; ++r) nx[j][r] = xw[xrow[r] + off];
         unsigned doff = drow + (unsigned)ow * wstride;
 #pragma unroll
-        for (int uu = 0; uu < U; ++uu, doff += wstride) nd[uu] = __ldg(dw + doff);
+        for (int uu = 0; uu < U; ++uu, doff += wstride) nd[uu] = dw[doff];
       } else {
 #pragma unroll
         for (int j = 0; j < NEW; ++j) fetch_col(iw_new + j, nx[j]);
 #pragma unroll
-        for (int uu = 0; uu < U; ++uu) nd[uu] = __ldg(dw + drow + (unsigned)min(ow + uu, p.out_cols - 1) * wstride);
+        for (int uu = 0; uu < U; ++uu) nd[uu] = dw[drow + (unsigned)min(ow + uu, p.out_cols - 1) * wstride];
       }
     };
     fetch(ow_begin);
@@ -1146,26 +1156,32 @@ __device__ __forceinline__ float pointwise_grad_value(float v, float e, int op) 
 
 template <typename T, int V, int MODE>  // MODE 0: forward, 1: gradient
 __global__ void __launch_bounds__(kBlock)
-    pointwise_kernel(int op, const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, size_t n_packets) {
+    pointwise_kernel(int op, const T* a, const T* b, T* __restrict__ out, size_t n_packets) {
   overlap_wait();
-  for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n_packets; i += (size_t)gridDim.x * kBlock) {
-    float av[V], res[V];
-    load_vec<T, V>(a + i * V, av);
-    if (MODE == 0) {
+  const size_t step = (size_t)gridDim.x * kBlock;
+  for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n_packets; i += 2 * step) {
+    // two packets requested together
+    const int count = i + step < n_packets ? 2 : 1;
+    float av[2][V], bv[2][V], res[V];
 #pragma unroll
-      for (int j = 0; j < V; ++j) res[j] = pointwise_forward_value(av[j], op);
-    } else {
-      float bv[V];
-      load_vec<T, V>(b + i * V, bv);
-#pragma unroll
-      for (int j = 0; j < V; ++j) res[j] = pointwise_grad_value(av[j], bv[j], op);
+    for (int u = 0; u < 2; ++u) {
+      if (u >= count) break;
+      load_vec<T, V>(a + (i + u * step) * V, av[u]);
+      if (MODE == 1) load_vec<T, V>(b + (i + u * step) * V, bv[u]);
     }
-    store_vec<T, V>(out + i * V, res);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u >= count) break;
+#pragma unroll
+      for (int j = 0; j < V; ++j)
+        res[j] = MODE == 0 ? pointwise_forward_value(av[u][j], op) : pointwise_grad_value(av[u][j], bv[u][j], op);
+      store_vec<T, V>(out + (i + u * step) * V, res);
+    }
   }
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(kBlock) bias_add_kernel(const T* __restrict__ in, const T* __restrict__ bias,
+__global__ void __launch_bounds__(kBlock) bias_add_kernel(const T* in, const T* bias,
                                                           T* __restrict__ out, size_t n_packets, int cvecs, int act) {
   overlap_wait();
   for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n_packets; i += (size_t)gridDim.x * kBlock) {
@@ -1215,7 +1231,7 @@ template <>
 struct Packet<__half> {
   __half2 v[4];
   static __device__ __forceinline__ Packet load(const __half* p) {
-    const uint4 r = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 r = *reinterpret_cast<const uint4*>(p);
     Packet o;
     o.v[0] = *reinterpret_cast<const __half2*>(&r.x);
     o.v[1] = *reinterpret_cast<const __half2*>(&r.y);
@@ -1281,7 +1297,7 @@ template <>
 struct Packet<__nv_bfloat16> {  // maxima only: bf16 products would lose too much in a packed sum
   __nv_bfloat162 v[4];
   static __device__ __forceinline__ Packet load(const __nv_bfloat16* p) {
-    const uint4 r = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 r = *reinterpret_cast<const uint4*>(p);
     Packet o;
     o.v[0] = *reinterpret_cast<const __nv_bfloat162*>(&r.x);
     o.v[1] = *reinterpret_cast<const __nv_bfloat162*>(&r.y);
@@ -1335,7 +1351,7 @@ template <>
 struct Packet<float> {
   float v[4];
   static __device__ __forceinline__ Packet load(const float* p) {
-    const float4 r = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 r = *reinterpret_cast<const float4*>(p);
     Packet o;
     o.v[0] = r.x;
     o.v[1] = r.y;
@@ -1532,7 +1548,7 @@ __global__ void __launch_bounds__(kStripBlock)
 // 0.074 -> 0.067 ms, 56x56x144 0.068 -> 0.046 ms, the 17 layers 0.46 -> 0.36 ms.
 template <typename T, int ST, int PF>
 __global__ void __launch_bounds__(kStripBlock, 3)
-    depthwise3_async_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, StripGeometry g,
+    depthwise3_async_kernel(const T* x, const T* w, T* __restrict__ y, StripGeometry g,
                             size_t n_threads) {
   using P = Packet<T>;
   constexpr int V = 16 / sizeof(T);
@@ -2241,7 +2257,7 @@ struct BinaryGeometry {
 };
 
 template <typename T, int V>
-__global__ void __launch_bounds__(kBlock) binaryop_kernel(int op, const T* __restrict__ lhs, const T* __restrict__ rhs,
+__global__ void __launch_bounds__(kBlock) binaryop_kernel(int op, const T* lhs, const T* rhs,
                                                           T* __restrict__ out, BinaryGeometry g, size_t n_packets) {
   overlap_wait();
   const unsigned inner_packets = g.od[3] / V;

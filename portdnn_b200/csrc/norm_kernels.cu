@@ -37,7 +37,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <typename T, int V>
 __device__ __forceinline__ void load_v(const T* p, float (&v)[V]) {
   if constexpr (V == 1) {
-    v[0] = to_f32(__ldg(p));
+    v[0] = to_f32(*p);
   } else {
     const Vec16<T> pk = load16(p);
 #pragma unroll
@@ -59,7 +59,7 @@ __device__ __forceinline__ void store_v(T* p, const float (&v)[V]) {
 // One warp per pixel, packets of V channels, at most R packets per lane (C <= 32 * R * V): the
 // pixel is read once and stays in registers through the three steps.
 template <typename T, int V, int R>
-__global__ void __launch_bounds__(kBlock) softmax_forward_vec_kernel(const T* __restrict__ x, T* __restrict__ y,
+__global__ void __launch_bounds__(kBlock) softmax_forward_vec_kernel(const T* x, T* __restrict__ y,
                                                                      size_t rows, int C) {
   overlap_wait();
   const int lane = threadIdx.x & 31, packets = C / V;
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kBlock) softmax_forward_kernel(const T* __rest
 // dx = (dy - sum_c(dy * y)) * y, y = the forward output, on packets: both rows are read once and stay in
 // registers.  The form below reads them twice, a value at a time.  250 x 1000 f16: 13.3 -> 3.7 us.
 template <typename T, int V, int R>
-__global__ void __launch_bounds__(kBlock) softmax_grad_vec_kernel(const T* __restrict__ y, const T* __restrict__ dy,
+__global__ void __launch_bounds__(kBlock) softmax_grad_vec_kernel(const T* y, const T* dy,
                                                                   T* __restrict__ dx, size_t rows, int C) {
   overlap_wait();
   const int lane = threadIdx.x & 31, packets = C / V;
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(kBlock) softmax_grad_kernel(const T* __restric
 // packets.  The per-channel operands are read as packets too (they stay in L1).
 template <typename T, int V>
 __global__ void __launch_bounds__(kBlock)
-    batchnorm_apply_vec_kernel(const T* __restrict__ x, const T* __restrict__ beta, const T* __restrict__ gamma,
-                               const T* __restrict__ mean, const T* __restrict__ var, T* __restrict__ out, size_t n,
+    batchnorm_apply_vec_kernel(const T* x, const T* beta, const T* gamma,
+                               const T* mean, const T* var, T* __restrict__ out, size_t n,
                                int C, float eps) {
   overlap_wait();
   const size_t cvecs = (size_t)(C / V);
@@ -197,14 +197,20 @@ __global__ void __launch_bounds__(kBlock)
     // instruction-bound; the product differs from the quotient by at most one ulp of fp32
 #pragma unroll
     for (int k = 0; k < V; ++k) sd[k] = 1.f / sqrtf(sd[k] + eps);
-#pragma unroll 4
-    for (; i < n; i += step) {
-      float xv[V], o[V];
-      load_v<T, V>(x + i * V, xv);
+    auto put = [&](size_t at, const Vec16<T>& xv) {
+      float o[V];
 #pragma unroll
-      for (int k = 0; k < V; ++k) o[k] = (xv[k] - m[k]) * sd[k] * g[k] + b[k];
-      store_v<T, V>(out + i * V, o);
+      for (int k = 0; k < V; ++k) o[k] = (to_f32(xv.get(k)) - m[k]) * sd[k] * g[k] + b[k];
+      store_v<T, V>(out + at * V, o);
+    };
+    for (; i + 3 * step < n; i += 4 * step) {  // four packets requested together
+      Vec16<T> xv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) xv[u] = load16(x + (i + u * step) * V);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) put(i + u * step, xv[u]);
     }
+    for (; i < n; i += step) put(i, load16(x + i * V));
     return;
   }
   for (; i < n; i += step) {
@@ -223,8 +229,8 @@ __global__ void __launch_bounds__(kBlock)
 
 template <typename T, int V>
 __global__ void __launch_bounds__(kBlock)
-    batchnorm_grad_training_vec_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ gamma,
-                                       const float* __restrict__ stats0, const float* __restrict__ stats1,
+    batchnorm_grad_training_vec_kernel(const T* x, const T* dy, const T* gamma,
+                                       const float* stats0, const float* stats1,
                                        T* __restrict__ out, size_t n, int C, float rows, float eps) {
   overlap_wait();
   const size_t cvecs = (size_t)(C / V);
@@ -243,15 +249,23 @@ __global__ void __launch_bounds__(kBlock)
       mx[k] = stats0[c + k];
       mdy[k] = stats0[C + c + k];
     }
-#pragma unroll 4
-    for (; i < n; i += step) {
-      float xv[V], gv[V], o[V];
-      load_v<T, V>(x + i * V, xv);
-      load_v<T, V>(dy + i * V, gv);
+    auto put = [&](size_t at, const Vec16<T>& xv, const Vec16<T>& gv) {
+      float o[V];
 #pragma unroll
-      for (int k = 0; k < V; ++k) o[k] = ((gv[k] - mdy[k]) - (xv[k] - mx[k]) * kk[k]) * sd[k];
-      store_v<T, V>(out + i * V, o);
+      for (int k = 0; k < V; ++k) o[k] = ((to_f32(gv.get(k)) - mdy[k]) - (to_f32(xv.get(k)) - mx[k]) * kk[k]) * sd[k];
+      store_v<T, V>(out + at * V, o);
+    };
+    for (; i + 3 * step < n; i += 4 * step) {  // four packets of either tensor requested together
+      Vec16<T> xv[4], gv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        xv[u] = load16(x + (i + u * step) * V);
+        gv[u] = load16(dy + (i + u * step) * V);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) put(i + u * step, xv[u], gv[u]);
     }
+    for (; i < n; i += step) put(i, load16(x + i * V), load16(dy + i * V));
     return;
   }
   for (; i < n; i += step) {
@@ -533,10 +547,10 @@ struct Moments {
 template <typename T>
 __device__ __forceinline__ void load_four(const T* p, float (&v)[kMomentChannels]) {
   if constexpr (sizeof(T) == 4) {
-    const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 q = *reinterpret_cast<const float4*>(p);
     v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
   } else {
-    const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 q = *reinterpret_cast<const uint2*>(p);
     const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = to_f32(e[k]);
@@ -548,8 +562,8 @@ __device__ __forceinline__ void load_four(const T* p, float (&v)[kMomentChannels
 // out = (x - mean) / sqrt(var + eps) * gamma + beta with the given mean and variance.
 template <typename T, bool DY, bool APPLY>
 __global__ void __launch_bounds__(kBlock, 3)
-    batchnorm_moments_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ beta,
-                             const T* __restrict__ gamma, const T* __restrict__ mean, const T* __restrict__ var,
+    batchnorm_moments_kernel(const T* x, const T* dy, const T* beta,
+                             const T* gamma, const T* mean, const T* var,
                              T* __restrict__ out, float* __restrict__ partial, size_t rows, int C, size_t rows_per_slice, float eps) {
   overlap_wait();
   constexpr int NC = kMomentChannels, NS = Moments<DY>::N;
@@ -688,7 +702,7 @@ __global__ void __launch_bounds__(kBlock, 3)
 constexpr int kMergeChannels = 8, kMergeLanes = 64, kMergeWarps = kMergeChannels * kMergeLanes / 32;
 template <typename T, bool DY, typename Finish>
 __global__ void __launch_bounds__(kMergeChannels * kMergeLanes)
-    batchnorm_merge_kernel(const float* __restrict__ partial, const T* __restrict__ x, const T* __restrict__ dy, int slices, int C,
+    batchnorm_merge_kernel(const float* partial, const T* x, const T* dy, int slices, int C,
                            size_t rows, size_t rows_per_slice, Finish finish) {
   overlap_wait();
   constexpr int NS = Moments<DY>::N;
@@ -704,7 +718,7 @@ __global__ void __launch_bounds__(kMergeChannels * kMergeLanes)
       for (int i = 0; i < 4; ++i) {
         const float* at = partial + (size_t)min(s0 + kMergeLanes * i, slices - 1) * NS * C + c;
 #pragma unroll
-        for (int j = 0; j < NS; ++j) b[i].v[j] = __ldg(at + (size_t)j * C);
+        for (int j = 0; j < NS; ++j) b[i].v[j] = at[(size_t)j * C];
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {

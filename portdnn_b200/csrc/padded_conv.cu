@@ -60,7 +60,7 @@ __device__ __forceinline__ void repitch(const RepitchJob& j, unsigned first, uns
       if (i < j.items) {
         const unsigned row = i / cv, c = i - row * cv;
         const unsigned a = row / bo, b = row - a * bo;
-        if (c < civ && b < bi) v[u] = __ldg(in + ((size_t)a * bi + b) * civ + c);
+        if (c < civ && b < bi) v[u] = in[((size_t)a * bi + b) * civ + c];
       }
     }
 #pragma unroll
@@ -104,13 +104,22 @@ int run_jobs(const RepitchJobs& jobs, cudaStream_t s) {
 // out[a][b][c] (+)= in[a][b][c] with another element type; in has bi x ci elements per matrix, out bo x co.
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(kBlock)
-    cut_kernel(const InT* __restrict__ in, OutT* __restrict__ out, unsigned n, int bo, int bi, int co, int ci, bool accumulate) {
+    cut_kernel(const InT* in, OutT* __restrict__ out, unsigned n, int bo, int bi, int co, int ci, bool accumulate) {
   overlap_wait();
-  for (unsigned i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
-    const unsigned row = i / (unsigned)co, c = i - row * (unsigned)co, a = row / (unsigned)bo, b = row - a * (unsigned)bo;
-    float v = to_f32(in[((size_t)a * bi + b) * ci + c]);
-    if (accumulate) v += to_f32(out[i]);
-    out[i] = from_f32<OutT>(v);
+  const unsigned step = gridDim.x * kBlock;
+  for (unsigned i0 = blockIdx.x * kBlock + threadIdx.x; i0 < n; i0 += kUnroll * step) {
+    float v[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const unsigned i = i0 + u * step;
+      if (i >= n) break;
+      const unsigned row = i / (unsigned)co, c = i - row * (unsigned)co, a = row / (unsigned)bo, b = row - a * (unsigned)bo;
+      v[u] = to_f32(in[((size_t)a * bi + b) * ci + c]);
+      if (accumulate) v[u] += to_f32(out[i]);
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (i0 + u * step < n) out[i0 + u * step] = from_f32<OutT>(v[u]);
   }
 }
 

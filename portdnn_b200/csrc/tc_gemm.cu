@@ -226,7 +226,7 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& a, const uint32_t (&
     if (bias != nullptr) {
 #pragma unroll
       for (int i = 0; i < P; ++i)
-        if (c + i < a.ext_cols) v[i] += to_f32(__ldg(bias + c + i));
+        if (c + i < a.ext_cols) v[i] += to_f32(bias[c + i]);
     }
     if (a.act != PDNN_ACT_NONE) {
 #pragma unroll
@@ -349,7 +349,7 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmArgs& a, const TileC
 #pragma unroll
           for (int i = 0; i < P; ++i) {
             const int c = colbase + g * P + i;
-            if (c < a.ext_cols) v[i] += to_f32(__ldg(bias + c));
+            if (c < a.ext_cols) v[i] += to_f32(bias[c]);
           }
         }
         if (a.act != PDNN_ACT_NONE) {
@@ -540,7 +540,7 @@ __device__ __forceinline__ bool epilogue_tile_tma_fast(const GemmArgs& a, const 
 #pragma unroll
       for (int b = 0; b < 4; ++b)
         if (b * 64 < a.bn && t.nf0 + b * 64 < a.ext_cols)
-          pre[b] = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(a.mask_bits) + ((row_off + t.nf0 + b * 64) >> 3)));
+          pre[b] = *(reinterpret_cast<const uint2*>(static_cast<const uint8_t*>(a.mask_bits) + ((row_off + t.nf0 + b * 64) >> 3)));
     }
   }
 #pragma unroll 1
@@ -765,7 +765,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
       const int chunks = a.bias_smem_bytes >> 4;
       for (int i = threadIdx.x; i < chunks; i += blockDim.x) {
         const int col = bias_col0 + i * 8;
-        dst[i] = (col + 8 <= a.ext_cols) ? __ldg(reinterpret_cast<const uint4*>(bias + col)) : make_uint4(0u, 0u, 0u, 0u);
+        dst[i] = (col + 8 <= a.ext_cols) ? *reinterpret_cast<const uint4*>(bias + col) : make_uint4(0u, 0u, 0u, 0u);
       }
     }
   };
@@ -1329,7 +1329,7 @@ __global__ void __launch_bounds__(192, 1) umma_gemm_pair2_kernel(const __grid_co
     const int chunks = a.bias_smem_bytes >> 4;
     for (int i = threadIdx.x; i < chunks; i += blockDim.x) {
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (i * 8 + 8 <= a.ext_cols) v = __ldg(reinterpret_cast<const uint4*>(bias) + i);
+      if (i * 8 + 8 <= a.ext_cols) v = *(reinterpret_cast<const uint4*>(bias) + i);
       dst[i] = v;
     }
   }
@@ -2713,7 +2713,7 @@ int finish_forward(GemmArgs& g, int dtype, void* y, const PdnnConv2DParams& p, c
 // repacked the same way ([R][8][CP][K], zeros in the padding).
 // One thread per packed pixel; the grid is (row segments, padded rows, images), so no thread divides.
 template <typename T>
-__global__ void __launch_bounds__(256) pack_small_c_input_kernel(const T* __restrict__ x, uint4* __restrict__ xp, int N,
+__global__ void __launch_bounds__(256) pack_small_c_input_kernel(const T* x, uint4* __restrict__ xp, int N,
                                                                 int H, int W, int C, int Hp, int Wp, int pad_top,
                                                                 int pad_left) {
   overlap_wait();
@@ -2731,7 +2731,7 @@ __global__ void __launch_bounds__(256) pack_small_c_input_kernel(const T* __rest
 }
 
 // The same with 4 channels of 16 bits per pixel (8 bytes): half the bytes for a 3-channel image.
-__global__ void __launch_bounds__(256) pack_small_c_input_narrow_kernel(const unsigned short* __restrict__ x,
+__global__ void __launch_bounds__(256) pack_small_c_input_narrow_kernel(const unsigned short* x,
                                                                        uint2* __restrict__ xp, int N, int H, int W,
                                                                        int C, int Hp, int Wp, int pad_top,
                                                                        int pad_left) {
@@ -2749,7 +2749,7 @@ __global__ void __launch_bounds__(256) pack_small_c_input_narrow_kernel(const un
 
 // Filter [R][S][C][K] -> [R][8][CP][K], zeros for s >= S and c >= C.
 template <typename T>
-__global__ void __launch_bounds__(256) pack_small_c_filter_kernel(const T* __restrict__ w, T* __restrict__ wp, int R,
+__global__ void __launch_bounds__(256) pack_small_c_filter_kernel(const T* w, T* __restrict__ wp, int R,
                                                                  int S, int C, int K, int CP) {
   overlap_wait();
   const size_t total = (size_t)R * 8 * CP * K;
@@ -2925,7 +2925,7 @@ int conv_forward_small_c(int dtype, const void* x, const void* w, void* y, const
 
 // The lo part of a 3xTF32 operand: the tensor core reads the 19 leading bits of an fp32 word (hi, which
 // therefore needs no copy); lo = x - hi is exact in fp32.
-__global__ void __launch_bounds__(256) split_lo_kernel(const float* __restrict__ x, float* __restrict__ lo, size_t n) {
+__global__ void __launch_bounds__(256) split_lo_kernel(const float* x, float* __restrict__ lo, size_t n) {
   overlap_wait();
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
     const float v = x[i];
@@ -3122,7 +3122,7 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
 // packed[tap][nt * Kg + k][j * Cg + c] = feature (nt * per_tile + j) * Kg + k of channel c of its group, zero for
 // groups that do not exist and channels beyond per_tile * Cg.
 __global__ void __launch_bounds__(256)
-    pack_grouped_filter_kernel(const unsigned short* __restrict__ w, unsigned short* __restrict__ packed, int taps, int Cg, int Kg, int groups,
+    pack_grouped_filter_kernel(const unsigned short* w, unsigned short* __restrict__ packed, int taps, int Cg, int Kg, int groups,
                                int per_tile, int rows, bool fhwc) {
   overlap_wait();
   const unsigned total = (unsigned)taps * (unsigned)rows * 64u, K = (unsigned)(groups * Kg);
@@ -3530,7 +3530,7 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool
 // the final kernel sums the pixel splits and drops the padding entries.
 template <typename T, typename OutT = T>
 __global__ void __launch_bounds__(256)
-    unpack_small_c_filter_grad_kernel(const float* __restrict__ partial, OutT* __restrict__ dw, int splits, int R, int S,
+    unpack_small_c_filter_grad_kernel(const float* partial, OutT* __restrict__ dw, int splits, int R, int S,
                                       int C, int K, int rows_per_tap, bool accumulate) {
   overlap_wait();
   constexpr int CP = 16 / sizeof(T);
