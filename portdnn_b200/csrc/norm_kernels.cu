@@ -557,7 +557,8 @@ __device__ __forceinline__ void load_four(const T* p, float (&v)[kMomentChannels
   }
 }
 
-// Block: 32 lanes x 4 channels, 8 row lanes; blockIdx.x the slice of rows, blockIdx.y the channel tile.
+// Block: 32 lanes x 4 channels, 8 row lanes; blockIdx.x the channel tile (the extent of a grid that has no practical
+// limit), blockIdx.y the slice of rows.
 // partial[slice][value of the set][c].  APPLY: the forward output is written on the way,
 // out = (x - mean) / sqrt(var + eps) * gamma + beta with the given mean and variance.
 template <typename T, bool DY, bool APPLY>
@@ -569,8 +570,8 @@ __global__ void __launch_bounds__(kBlock, 3)
   constexpr int NC = kMomentChannels, NS = Moments<DY>::N;
   __shared__ float red[8][NS][NC][32];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int c = (blockIdx.y * 32 + tx) * NC;
-  const size_t begin = (size_t)blockIdx.x * rows_per_slice;
+  const int c = (blockIdx.x * 32 + tx) * NC;
+  const size_t begin = (size_t)blockIdx.y * rows_per_slice;
   const size_t end = begin + rows_per_slice < rows ? begin + rows_per_slice : rows;
   // the subtracted values, and sums of d, d^2 and x (h, d h and dy), d = x - hx, h = dy - hy
   float hx[NC] = {}, s1[NC] = {}, s2[NC] = {}, sx[NC] = {}, hy[NC] = {}, t1[NC] = {}, sxy[NC] = {}, sy[NC] = {};
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(kBlock, 3)
       t.merge(b, nt, nb);
       nt += nb;
     }
-    float* to = partial + (size_t)blockIdx.x * NS * C + c + ty;
+    float* to = partial + (size_t)blockIdx.y * NS * C + c + ty;
 #pragma unroll
     for (int i = 0; i < NS; ++i) to[(size_t)i * C] = t.v[i];
   }
@@ -938,7 +939,7 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
       Scratch sc;
       const int st = get_scratch(&sc, Moments<false>::N / 2 * slices, C, s);
       if (st != PDNN_OK) return st;
-      const dim3 grid((unsigned)slices, (unsigned)((C / kMomentChannels + 31) / 32));
+      const dim3 grid((unsigned)((C / kMomentChannels + 31) / 32), (unsigned)slices);
       const T *mt = static_cast<const T*>(mean), *vt = static_cast<const T*>(variance);
       launch_overlapped(batchnorm_moments_kernel<T, false, true>, grid, kBlock, s, static_cast<const T*>(input), nullptr,
           static_cast<const T*>(beta), static_cast<const T*>(gamma), mt, vt,
@@ -1013,7 +1014,7 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
     const unsigned c1grid = (C + kBlock - 1) / kBlock;
     const T *x = static_cast<const T*>(input), *dy = static_cast<const T*>(gradient), *g = static_cast<const T*>(gamma);
     if (one_pass) {
-      const dim3 mgrid((unsigned)slices, (unsigned)((C / kMomentChannels + 31) / 32));
+      const dim3 mgrid((unsigned)((C / kMomentChannels + 31) / 32), (unsigned)slices);
       launch_overlapped(batchnorm_moments_kernel<T, true, false>, mgrid, kBlock, s, x, dy, nullptr, nullptr, nullptr, nullptr,
           nullptr, sc.partial,
                                                                        rows, C, per_slice, 0.f);

@@ -3,6 +3,7 @@ few rows of partial sums (one thread per column), row counts around the 32 lanes
 lane has in flight, and column counts that leave the last block ragged."""
 import numpy as np
 import pytest
+import torch
 
 import portdnn_b200 as pd
 from gpu_util import to_dev, to_host
@@ -174,3 +175,18 @@ def test_batchnorm_infinities(rows, channels):
     for t, r in zip(got[:4], ref):
         assert np.allclose(t[6:], r[6:], rtol=1e-4, atol=1e-4)
     assert np.all(np.isfinite(dx[:, 6:])) and not np.any(np.isfinite(dx[:, :2]))
+
+
+def test_batchnorm_of_very_many_channels():
+    """More channel tiles than a grid's second extent holds (65535 of 128 channels)."""
+    rows, channels = 3, 65536 * 128 + 8
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, dy = (torch.randn(rows, channels, device="cuda", generator=g).half() for _ in range(2))
+    one, zero = torch.ones(channels, device="cuda").half(), torch.zeros(channels, device="cuda").half()
+    p = pd.batchnorm_params(1, 1, rows, channels, True, 1e-3, 0.0)
+    _, mean, var = pd.batchnorm_forward(x.view(-1), zero, one, zero, one, p)
+    _, dbeta, _ = pd.batchnorm_gradient(x.view(-1), dy.view(-1), one, p)
+    v, m = torch.var_mean(x.float(), 0, correction=0)
+    # one rounding of fp32 sums of three terms
+    for got, ref in ((mean, m), (var, v), (dbeta, dy.float().sum(0))):
+        assert ((got.float() - ref).abs() <= 2.0 ** -11 * 1.01 * ref.abs() + 2.0 ** -20).all()
