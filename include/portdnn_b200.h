@@ -338,6 +338,10 @@ const char* pdnn_last_error(void);
 /* Number of kernels this library has launched in the calling process; host only. */
 unsigned long long pdnn_launch_count(void);
 
+/* Name of the tensor-core kernel that the calling thread launched last ("" before the first): which of the
+ * plans a call has taken. */
+const char* pdnn_last_gemm_kernel(void);
+
 #ifdef __cplusplus
 }
 #endif

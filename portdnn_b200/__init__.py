@@ -20,5 +20,5 @@ from .api import (  # noqa: F401
     conv2d, conv2d_workspace_size, conv2d_validate, depthwise_conv2d, pooling, pooling_max_grad,
     pointwise, pointwise_grad, bias_add, binaryop, scale_blend, matmul, transpose,
     softmax, batchnorm_params, batchnorm_forward, batchnorm_gradient,
-    device_error_record, launch_count, lib, library_path,
+    device_error_record, last_gemm_kernel, launch_count, lib, library_path,
 )

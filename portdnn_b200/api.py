@@ -90,6 +90,7 @@ def lib():
         L = ctypes.CDLL(path)
         L.pdnn_last_error.restype = ctypes.c_char_p
         L.pdnn_launch_count.restype = ctypes.c_ulonglong
+        L.pdnn_last_gemm_kernel.restype = ctypes.c_char_p
         L.pdnn_depthwise_workspace_bytes.restype = ctypes.c_size_t
         L.pdnn_noalloc_scratch_bytes.restype = ctypes.c_size_t
         _LIB = L
@@ -344,3 +345,8 @@ def device_error_record(clear=True):
 
 def launch_count():
     return int(lib().pdnn_launch_count())
+
+
+def last_gemm_kernel():
+    """Name of the tensor-core kernel that the calling thread launched last."""
+    return lib().pdnn_last_gemm_kernel().decode()

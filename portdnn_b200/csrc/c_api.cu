@@ -469,4 +469,6 @@ const char* pdnn_last_error(void) { return last_error_buffer(); }
 
 unsigned long long pdnn_launch_count(void) { return g_launches.load(); }
 
+const char* pdnn_last_gemm_kernel(void) { return tc_last_kernel(); }
+
 }  // extern "C"

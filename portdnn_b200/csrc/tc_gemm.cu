@@ -2263,6 +2263,8 @@ GemmKernel select_grouped_kernel(int epi, int out_dtype) {
   return nullptr;
 }
 
+thread_local const char* t_last_kernel = "";
+
 // Launch of the CTA-pair kernel: clusters of two CTAs, one cluster per pair of SMs.
 int launch_gemm_pair2(const GemmArgs& g, long long total_pairs, cudaStream_t s) {
   const bool bits = g.bitmask_out != nullptr;
@@ -2317,6 +2319,7 @@ int launch_gemm_pair2(const GemmArgs& g, long long total_pairs, cudaStream_t s) 
     return fail(PDNN_ALLOCATION_PROBLEM, "tensor-core gemm (CTA pairs): launch failed: %s", cudaGetErrorString(le));
   }
   if (g.bitmask_out != nullptr) bitmask_written_flag() = true;
+  t_last_kernel = g.a_mn ? "umma_gemm_filter_pair_kernel" : "umma_gemm_pair2_kernel";
   return check_launch("tensor-core gemm (CTA pairs)");
 }
 
@@ -2398,6 +2401,7 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
     return fail(PDNN_ALLOCATION_PROBLEM, "tensor-core gemm: launch failed: %s", cudaGetErrorString(le));
   }
   if (g.bitmask_out != nullptr) bitmask_written_flag() = true;
+  t_last_kernel = g.group_k != 0 ? "umma_gemm_grouped_kernel" : "umma_gemm_kernel";
   return check_launch("tensor-core gemm");
 }
 
@@ -2543,6 +2547,7 @@ int launch_gemm_multi(const GemmArgs* list, int count, cudaStream_t s) {
     cudaGetLastError();
     return fail(PDNN_ALLOCATION_PROBLEM, "tensor-core gemm: launch failed: %s", cudaGetErrorString(le));
   }
+  t_last_kernel = "umma_gemm_multi_kernel";
   return check_launch("tensor-core gemm (several GEMMs)");
 }
 
@@ -2619,6 +2624,7 @@ int launch_gemm_cluster(const GemmArgs& g, int splits, cudaStream_t s) {
     return fail(PDNN_ALLOCATION_PROBLEM, "tensor-core gemm (clusters): launch failed: %s", cudaGetErrorString(le));
   }
   if (g.bitmask_out != nullptr) bitmask_written_flag() = true;
+  t_last_kernel = "umma_gemm_cluster_kernel";
   return check_launch("tensor-core gemm (clusters)");
 }
 
@@ -4124,6 +4130,8 @@ int simt_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, voi
     return fail(PDNN_INVALID_PARAMETER, "unknown dtype %d", dtype);
   return check_launch("simt matmul");
 }
+
+const char* tc_last_kernel() { return t_last_kernel; }
 
 int tc_read_error_record(unsigned out[4], int clear) {
   if (cudaMemcpyFromSymbol(out, g_error_record, sizeof(unsigned) * 4) != cudaSuccess) {

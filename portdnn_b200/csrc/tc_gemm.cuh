@@ -38,6 +38,9 @@ int tc_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, void*
 int simt_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, void* out, int batches, int m, int k, int n,
                 float beta, cudaStream_t s, bool out_f32 = false);
 
+// Name of the tensor-core kernel that the calling thread launched last ("" before the first).
+const char* tc_last_kernel();
+
 // Copies the device-side error record (4 words; word 0 == 0 means no error) to the host.
 // Synchronises the device.
 int tc_read_error_record(unsigned out[4], int clear);

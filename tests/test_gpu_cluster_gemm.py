@@ -54,6 +54,7 @@ def test_conv(shape, dtype, fhwc, any_order):
     ref = torch.nn.functional.conv2d(xp, w64, stride=st).permute(0, 2, 3, 1)
     mag = torch.nn.functional.conv2d(xp.abs(), w64.abs(), stride=st).permute(0, 2, 3, 1)
     y = pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, any_order=any_order).view(ref.shape)
+    assert pd.last_gemm_kernel() == ("umma_gemm_cluster_kernel" if any_order else "umma_gemm_kernel")
     _check(y, ref, mag, dtype)
     assert torch.equal(y, pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, constant_filter=True,
                                     any_order=any_order).view(ref.shape))
@@ -81,7 +82,7 @@ def test_an_image_alone_and_in_a_batch(shape, dtype):
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])
-@pytest.mark.parametrize("shape", [s for s in SHAPES if s[6] == 1] + [(1, 12, 10, 24, 520, 1, 1), (3, 5, 6, 136, 72, 5, 1)])
+@pytest.mark.parametrize("shape", [s for s in SHAPES if s[6] == 1] + [(1, 12, 10, 24, 520, 1, 1), (3, 5, 6, 136, 72, 5, 1), (1, 14, 14, 256, 1024, 1, 1)])
 def test_input_backprop(shape, dtype):
     n, h, w, c, k, win, _ = shape
     dt, g = TORCH_DTYPES[dtype], torch.Generator(device="cuda").manual_seed(h + c + k)
@@ -92,6 +93,8 @@ def test_input_backprop(shape, dtype):
     ref, mag = back(dy.double(), w64), back(dy.double().abs(), w64.abs())
     call = lambda **kw: pd.conv2d(pd.INPUT_BACKPROP, dy.reshape(-1), wt.reshape(-1), p, **kw).view(ref.shape)
     plain = call()
+    # (fewer than eight blocks of 64 features, one tap: nothing to share)
+    assert pd.last_gemm_kernel() == ("umma_gemm_kernel" if win == 1 and k <= 7 * 64 else "umma_gemm_cluster_kernel")
     _check(plain, ref, mag, dtype)
     fwd, before = _rand(g, n, h, w, c).relu().to(dt), _rand(g, n, h, w, c).to(dt)
     keep = fwd > 0
@@ -111,4 +114,5 @@ def test_matmul(batches, m, k, n, tr, dtype):
     a, b = _rand(g, batches, m, k).to(dt), (_rand(g, batches, k, n) / k ** 0.5).to(dt)
     bd = b.transpose(1, 2).contiguous() if tr else b
     out = pd.matmul(a.reshape(-1), bd.reshape(-1), batches, m, k, n, transpose_rhs=tr).view(batches, m, n)
+    assert pd.last_gemm_kernel() == "umma_gemm_cluster_kernel"
     _check(out, a.double() @ b.double(), a.double().abs() @ b.double().abs(), dtype)

@@ -1,6 +1,7 @@
-"""Filter gradients on clusters of two CTAs (umma_gemm_filter_pair_kernel): one and several splits, the last of
-them shorter, several tiles either way, stride 2, partial pixel boxes, and the three ways the sums end
-(added to an fp32 gradient, written as fp32, reduced to the tensors' type)."""
+"""Filter gradients of whole 256 x 256 tiles.  On clusters of two CTAs (umma_gemm_filter_pair_kernel), where every
+split has 16 pixel boxes or more: one and several splits, the last of them shorter, several tiles either way,
+stride 2, pixel boxes cut at each edge, and the three ways the sums end (added to an fp32 gradient, written as
+fp32, reduced to the tensors' type); and on tiles of one CTA below that."""
 import pytest
 import torch
 
@@ -16,11 +17,20 @@ SHAPES = [
     (33, 15, 17, 512, 256, 3, 2),
     (17, 8, 8, 768, 768, 3, 1),  # more tiles than clusters: one split
 ]
+# at 148 SMs: splits, boxes of the others / of the last split; edges at which boxes of 64 pixels are cut
+PAIR_SHAPES = [
+    (17, 8, 8, 768, 768, 3, 1),     # 1, 17
+    (43, 14, 14, 256, 256, 3, 1),   # 8, 19 / 14; images
+    (131, 21, 19, 256, 512, 1, 1),  # 36, 26 / 25; columns, rows, images
+    (67, 11, 13, 512, 512, 3, 2),   # 2, 26 / 25; columns, images
+    (37, 29, 27, 512, 256, 3, 2),   # 4, 34 / 31; rows, images
+]
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape", SHAPES + PAIR_SHAPES[1:])
 def test_filter_gradient(shape, dtype):
+    kernel = "umma_gemm_filter_pair_kernel" if shape in PAIR_SHAPES else "umma_gemm_kernel"
     n, h, w, c, k, win, st = shape
     dt, g = TORCH_DTYPES[dtype], torch.Generator(device="cuda").manual_seed(c + k)
     p = pd.conv_params(n, h, w, c, k, win, st)
@@ -37,11 +47,14 @@ def test_filter_gradient(shape, dtype):
     # fp32 sums that lose at most 2^-20 of the magnitudes of their terms, then at most one rounding
     slack = 2.0 ** -20 * mag
     f32 = pd.conv2d(pd.FILTER_BACKPROP, x.reshape(-1), dy.reshape(-1), p, output_f32=True).view(ref.shape)
+    assert pd.last_gemm_kernel() == kernel
     assert ((f32.double() - ref).abs() <= slack).all()
     own = pd.conv2d(pd.FILTER_BACKPROP, x.reshape(-1), dy.reshape(-1), p).view(ref.shape)
+    assert pd.last_gemm_kernel() == kernel
     unit = 2.0 ** -11 if dtype == "f16" else 2.0 ** -8
     assert ((own.double() - ref).abs() <= slack + 1.01 * unit * ref.abs()).all()
     total = torch.ones_like(f32).reshape(-1)
     pd.conv2d(pd.FILTER_BACKPROP, x.reshape(-1), dy.reshape(-1), p, out=total, output_f32=True, accumulate=True)
+    assert pd.last_gemm_kernel() == kernel
     assert ((total.view(ref.shape).double() - 1.0 - ref).abs() <= slack + 2.0 ** -20).all()
     assert_no_device_error()

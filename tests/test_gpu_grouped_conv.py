@@ -18,7 +18,8 @@ SHAPES = [
     (2, 15, 14, 8, 32, 32, 3, 2),   # parity maps
     (1, 9, 10, 7, 32, 64, 1, 1),    # a last tile of one group
     (2, 12, 12, 5, 48, 64, 3, 1),   # three slices of a step
-    (2, 14, 14, 6, 64, 64, 5, 1),
+    (2, 14, 14, 6, 64, 64, 3, 1),
+    (2, 14, 14, 6, 64, 64, 5, 1),   # a filter too large to stay in shared memory: one GEMM per group
     (1, 1, 1, 5, 16, 64, 1, 1),     # tiles of 256 features, one pixel
 ]
 
@@ -44,6 +45,7 @@ def test_grouped_forward(shape, fhwc, dtype):
     before = pd.launch_count()
     y = pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p).view(n, p.out_rows, p.out_cols, k)[..., kg:].double()
     assert pd.launch_count() - before == 2
+    assert pd.last_gemm_kernel() == ("umma_gemm_multi_kernel" if win == 5 else "umma_gemm_grouped_kernel")
     yb = pd.conv2d(pd.FORWARD, x.reshape(-1), wd.reshape(-1), p, bias=b, activation=pd.ACT_RELU)
     yb = yb.view(n, p.out_rows, p.out_cols, k)[..., kg:].double()
     assert_no_device_error()
