@@ -1802,10 +1802,10 @@ int launch_pooling(int op, int direction, int dtype, const void* in, void* out, 
       const unsigned words = (unsigned)p.channels / E, items0 = (unsigned)p.batch * words;
       if (direction == 0)
         launch_overlapped(pool_avg_global_kernel<T>, grid_for(items0, kBlock, sms), kBlock, s, from, static_cast<T*>(out),
-            words, px, items0);
+                          words, px, items0);
       else
         launch_overlapped(pool_avg_grad_global_kernel<T, VN>, blocks, 32 * kGlobalPoolLanes, s, from, static_cast<T*>(out),
-            cvecs, tiles, px, n_blocks);
+                          cvecs, tiles, px, n_blocks);
       return check_launch(direction == 0 ? "pooling average (global)" : "pooling average gradient (global)");
     }
     const unsigned grid = grid_for(items, kBlock, sms);
@@ -1879,10 +1879,10 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
       const unsigned g1 = grid_for(out_items, kBlock, sms);
       if (op == PDNN_POOL_MAX)
         launch_overlapped(pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX, VN, unsigned>, g1, kBlock, s, xt, yt, dyt, dxt, p,
-            (unsigned)out_items);
+                          (unsigned)out_items);
       else
-        launch_overlapped(pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX_WITH_NAN, VN, unsigned>, g1, kBlock, s, xt, yt, dyt, dxt,
-            p, (unsigned)out_items);
+        launch_overlapped(pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX_WITH_NAN, VN, unsigned>, g1, kBlock, s, xt, yt, dyt,
+                          dxt, p, (unsigned)out_items);
       return check_launch("pooling max gradient (tiling windows)");
     }
     if (vec && small && p.window_rows * p.window_cols < 255) {
@@ -1918,7 +1918,7 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
           g.strips = (g.M + g.rows - 1) / g.rows;
           const size_t n_items = columns * g.strips;
           launch_overlapped(pool_max_grad_s2_kernel<T, VN>, grid_for(n_items, kBlock, sms), kBlock, s, winner, dyt, dxt, g,
-                                                                                         (unsigned)n_items);
+                            (unsigned)n_items);
           st = check_launch("pooling max gradient (3x3 / 2 gather)");
         } else if (st == PDNN_OK) {
           pool_max_grad_from_winner_kernel<T, VN, unsigned><<<g2, kBlock, 0, s>>>(winner, dyt, dxt, p, (unsigned)in_items);
@@ -2038,10 +2038,11 @@ int launch_fbp_partials(bool vec, const T* in, const T* dy, float* partial, cons
     while (segs < 4 && units * segs < (long long)gx * kFbpRowsWarps * 12 && (p.out_cols + 2 * segs - 1) / (2 * segs) >= 2 * trip) segs *= 2;
     const int seg_cols = ((p.out_cols + segs - 1) / segs + trip - 1) / trip * trip;
     segs = (p.out_cols + seg_cols - 1) / seg_cols;
-    if (p.stride_rows == 1) launch_overlapped(depthwise_filter_backprop_rows_kernel<T, 1>, grid, kFbpRowsWarps * 32, s, in, dy,
-        partial, p, segs, seg_cols, (int)gx, (int)g_tail);
-    else launch_overlapped(depthwise_filter_backprop_rows_kernel<T, 2>, grid, kFbpRowsWarps * 32, s, in, dy, partial, p, segs,
-        seg_cols, (int)gx, (int)g_tail);
+    if (p.stride_rows == 1) launch_overlapped(
+        depthwise_filter_backprop_rows_kernel<T, 1>, grid, kFbpRowsWarps * 32, s, in, dy, partial, p, segs, seg_cols,
+        (int)gx, (int)g_tail);
+    else launch_overlapped(depthwise_filter_backprop_rows_kernel<T, 2>, grid, kFbpRowsWarps * 32, s, in, dy, partial, p,
+                           segs, seg_cols, (int)gx, (int)g_tail);
     return (int)gx;
   }
   if (fbp_all_taps(p, V)) {
@@ -2135,8 +2136,8 @@ int launch_depthwise(int pass, int dtype, const void* in, const void* fil, void*
       g.strips = (g.M + g.rows - 1) / g.rows;
       const size_t n_items = columns * g.strips;
       if (n_items < 0xFFFF0000ull) {
-        launch_overlapped(depthwise_ibp_s2_kernel<T, VN>, grid_for(n_items, kBlock, sms), kBlock, s, static_cast<const T*>(in),
-            static_cast<const T*>(fil), static_cast<T*>(out), g, (unsigned)n_items);
+        launch_overlapped(depthwise_ibp_s2_kernel<T, VN>, grid_for(n_items, kBlock, sms), kBlock, s,
+                          static_cast<const T*>(in), static_cast<const T*>(fil), static_cast<T*>(out), g, (unsigned)n_items);
         return check_launch("depthwise input backprop (3x3, stride 2)");
       }
     }
@@ -2177,10 +2178,10 @@ int launch_pointwise(int op, int dtype, const void* in, void* out, size_t n, cud
     // the reference picks the widest vector that divides n (src/pointwise/launch_pointwise_forward.cc:32-70)
     if (n % VN == 0 && aligned16(in) && aligned16(out))
       launch_overlapped(pointwise_kernel<T, VN, 0>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(in),
-          nullptr, static_cast<T*>(out), n / VN);
+                        nullptr, static_cast<T*>(out), n / VN);
     else
-      launch_overlapped(pointwise_kernel<T, 1, 0>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(in), nullptr,
-                                                                            static_cast<T*>(out), n);
+      launch_overlapped(pointwise_kernel<T, 1, 0>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(in),
+                        nullptr, static_cast<T*>(out), n);
     return check_launch("pointwise");
   });
 }
@@ -2195,11 +2196,11 @@ int launch_pointwise_grad(int op, int dtype, const void* fwd, const void* err, v
     using T = decltype(tag);
     constexpr int VN = Vec16<T>::N;
     if (n % VN == 0 && aligned16(fwd) && aligned16(err) && aligned16(out))
-      launch_overlapped(pointwise_kernel<T, VN, 1>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(fwd),
-          static_cast<const T*>(err), static_cast<T*>(out), n / VN);
+      launch_overlapped(pointwise_kernel<T, VN, 1>, grid_for(n / VN, kBlock, sms), kBlock, s, op,
+                        static_cast<const T*>(fwd), static_cast<const T*>(err), static_cast<T*>(out), n / VN);
     else
       launch_overlapped(pointwise_kernel<T, 1, 1>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(fwd),
-          static_cast<const T*>(err), static_cast<T*>(out), n);
+                        static_cast<const T*>(err), static_cast<T*>(out), n);
     return check_launch("pointwise gradient");
   });
 }
@@ -2217,10 +2218,10 @@ int launch_bias_add(int dtype, const void* in, const void* bias, void* out, size
     const size_t n = rows * (size_t)channels;
     if (channels % VN == 0 && aligned16(in) && aligned16(bias) && aligned16(out))
       launch_overlapped(bias_add_kernel<T, VN>, grid_for(n / VN, kBlock, sms), kBlock, s, static_cast<const T*>(in),
-          static_cast<const T*>(bias), static_cast<T*>(out), n / VN, channels / VN, act);
+                        static_cast<const T*>(bias), static_cast<T*>(out), n / VN, channels / VN, act);
     else
       launch_overlapped(bias_add_kernel<T, 1>, grid_for(n, kBlock, sms), kBlock, s, static_cast<const T*>(in),
-          static_cast<const T*>(bias), static_cast<T*>(out), n, channels, act);
+                        static_cast<const T*>(bias), static_cast<T*>(out), n, channels, act);
     return check_launch("bias add");
   });
 }
@@ -2355,10 +2356,10 @@ int launch_binaryop(int op, int dtype, const void* lhs, const int* lhs_dims, int
     const size_t n = (size_t)total;
     if (vec)
       launch_overlapped(binaryop_kernel<T, VN>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(lhs),
-          static_cast<const T*>(rhs), static_cast<T*>(out), g, n / VN);
+                        static_cast<const T*>(rhs), static_cast<T*>(out), g, n / VN);
     else
       launch_overlapped(binaryop_kernel<T, 1>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(lhs),
-          static_cast<const T*>(rhs), static_cast<T*>(out), g, n);
+                        static_cast<const T*>(rhs), static_cast<T*>(out), g, n);
     return check_launch("binaryop");
   });
 }

@@ -891,21 +891,19 @@ int launch_softmax(int direction, int dtype, const void* input, const void* grad
     const bool vec = p.channels % VN == 0 && aligned16(input) && aligned16(output);
     if (direction == 0 && vec && p.channels <= 32 * VN)
       launch_overlapped(softmax_forward_vec_kernel<T, VN, 1>, grid, kBlock, s, static_cast<const T*>(input),
-                                                                  static_cast<T*>(output), rows, p.channels);
+                        static_cast<T*>(output), rows, p.channels);
     else if (direction == 0 && vec && p.channels <= 128 * VN)
       launch_overlapped(softmax_forward_vec_kernel<T, VN, 4>, grid, kBlock, s, static_cast<const T*>(input),
-                                                                  static_cast<T*>(output), rows, p.channels);
+                        static_cast<T*>(output), rows, p.channels);
     else if (direction == 0)
       softmax_forward_kernel<T><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), static_cast<T*>(output), rows,
                                                         p.channels);
     else if (vec && aligned16(gradient) && p.channels <= 32 * VN)
       launch_overlapped(softmax_grad_vec_kernel<T, VN, 1>, grid, kBlock, s, static_cast<const T*>(input),
-          static_cast<const T*>(gradient),
-                                                                static_cast<T*>(output), rows, p.channels);
+                        static_cast<const T*>(gradient), static_cast<T*>(output), rows, p.channels);
     else if (vec && aligned16(gradient) && p.channels <= 128 * VN)
       launch_overlapped(softmax_grad_vec_kernel<T, VN, 4>, grid, kBlock, s, static_cast<const T*>(input),
-          static_cast<const T*>(gradient),
-                                                                static_cast<T*>(output), rows, p.channels);
+                        static_cast<const T*>(gradient), static_cast<T*>(output), rows, p.channels);
     else
       softmax_grad_kernel<T><<<grid, kBlock, 0, s>>>(static_cast<const T*>(input), static_cast<const T*>(gradient),
                                                      static_cast<T*>(output), rows, p.channels);
@@ -942,19 +940,21 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
       const dim3 grid((unsigned)((C / kMomentChannels + 31) / 32), (unsigned)slices);
       const T *mt = static_cast<const T*>(mean), *vt = static_cast<const T*>(variance);
       launch_overlapped(batchnorm_moments_kernel<T, false, true>, grid, kBlock, s, static_cast<const T*>(input), nullptr,
-          static_cast<const T*>(beta), static_cast<const T*>(gamma), mt, vt,
-          static_cast<T*>(output), sc.partial, rows, C, per, p.epsilon);
-      launch_overlapped(batchnorm_merge_kernel<T, false, StoreRunning<T>>, (C + kMergeChannels - 1) / kMergeChannels, kMergeChannels * kMergeLanes, s,
-          sc.partial, static_cast<const T*>(input), nullptr, slices, C, rows, per,
-          StoreRunning<T>{mt, vt, static_cast<T*>(running_mean), static_cast<T*>(running_variance), (float)rows, p.momentum});
+                        static_cast<const T*>(beta), static_cast<const T*>(gamma), mt, vt, static_cast<T*>(output),
+                        sc.partial, rows, C, per, p.epsilon);
+      launch_overlapped(batchnorm_merge_kernel<T, false, StoreRunning<T>>, (C + kMergeChannels - 1) / kMergeChannels,
+                        kMergeChannels * kMergeLanes, s, sc.partial, static_cast<const T*>(input), nullptr, slices, C, rows,
+                        per,
+                        StoreRunning<T>{mt, vt, static_cast<T*>(running_mean), static_cast<T*>(running_variance), (float)rows, p.momentum});
       count_launch();
       cudaFreeAsync(sc.base, s);
       return check_launch("batchnorm forward (training)");
     }
     if (vec)
       launch_overlapped(batchnorm_apply_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s,
-          static_cast<const T*>(input), static_cast<const T*>(beta), static_cast<const T*>(gamma),
-          static_cast<const T*>(mean), static_cast<const T*>(variance), static_cast<T*>(output), n / VN, C, p.epsilon);
+                        static_cast<const T*>(input), static_cast<const T*>(beta), static_cast<const T*>(gamma),
+                        static_cast<const T*>(mean), static_cast<const T*>(variance), static_cast<T*>(output), n / VN, C,
+                        p.epsilon);
     else
       batchnorm_apply_kernel<T><<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(
           static_cast<const T*>(input), static_cast<const T*>(beta), static_cast<const T*>(gamma),
@@ -1015,14 +1015,13 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
     const T *x = static_cast<const T*>(input), *dy = static_cast<const T*>(gradient), *g = static_cast<const T*>(gamma);
     if (one_pass) {
       const dim3 mgrid((unsigned)((C / kMomentChannels + 31) / 32), (unsigned)slices);
-      launch_overlapped(batchnorm_moments_kernel<T, true, false>, mgrid, kBlock, s, x, dy, nullptr, nullptr, nullptr, nullptr,
-          nullptr, sc.partial,
-                                                                       rows, C, per_slice, 0.f);
-      launch_overlapped(batchnorm_merge_kernel<T, true, StoreGradStats<T>>, (C + kMergeChannels - 1) / kMergeChannels, kMergeChannels * kMergeLanes,
-          s, sc.partial, x, dy, slices, C, rows, per_slice,
-          StoreGradStats<T>{sc.stats0, sc.stats1, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), C, (float)rows, p.epsilon});
-      launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s, x, dy,
-          g, sc.stats0, sc.stats1, static_cast<T*>(output), n / VN, C, (float)rows, p.epsilon);
+      launch_overlapped(batchnorm_moments_kernel<T, true, false>, mgrid, kBlock, s, x, dy, nullptr, nullptr, nullptr,
+                        nullptr, nullptr, sc.partial, rows, C, per_slice, 0.f);
+      launch_overlapped(batchnorm_merge_kernel<T, true, StoreGradStats<T>>, (C + kMergeChannels - 1) / kMergeChannels,
+                        kMergeChannels * kMergeLanes, s, sc.partial, x, dy, slices, C, rows, per_slice,
+                        StoreGradStats<T>{sc.stats0, sc.stats1, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), C, (float)rows, p.epsilon});
+      launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s, x,
+                        dy, g, sc.stats0, sc.stats1, static_cast<T*>(output), n / VN, C, (float)rows, p.epsilon);
       count_launch(2);
       cudaFreeAsync(sc.base, s);
       return check_launch("batchnorm gradient (training)");

@@ -280,12 +280,11 @@ int padded_conv(int pass, int dtype, const void* in, const void* fil, void* out,
       if (fusion != nullptr && fusion->accumulate) {
         if (dtype == PDNN_F16)
           launch_overlapped(cut_kernel<__half, __half>, grid_for(n, kBlock, sms), kBlock, s, static_cast<const __half*>(dx),
-              static_cast<__half*>(out), n, px_in,
-                                                                 px_in, p.channels, q.channels, true);
+                            static_cast<__half*>(out), n, px_in, px_in, p.channels, q.channels, true);
         else
           launch_overlapped(cut_kernel<__nv_bfloat16, __nv_bfloat16>, grid_for(n, kBlock, sms), kBlock, s,
-              static_cast<const __nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(out),
-                                                                 n, px_in, px_in, p.channels, q.channels, true);
+                            static_cast<const __nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(out), n, px_in, px_in,
+                            p.channels, q.channels, true);
         st = check_launch("conv2d input gradient");
       } else {
         RepitchJobs back = {};
@@ -311,7 +310,7 @@ int padded_conv(int pass, int dtype, const void* in, const void* fil, void* out,
       const bool add = fusion != nullptr && fusion->accumulate;
       auto cut = [&](auto* to) {
         launch_overlapped(cut_kernel<float, std::remove_pointer_t<decltype(to)>>, grid, kBlock, s, dw, to, n, p.channels,
-            q.channels, p.features, q.features, add);
+                          q.channels, p.features, q.features, add);
       };
       if (fusion != nullptr && fusion->output_f32) cut(static_cast<float*>(out));
       else if (dtype == PDNN_F16) cut(static_cast<__half*>(out));

@@ -2904,22 +2904,26 @@ int conv_forward_small_c(int dtype, const void* x, const void* w, void* y, const
   }
   const size_t n_fil = (size_t)p.window_rows * krows * p.features;
   if (dtype == PDNN_F32) {
-    launch_overlapped(pack_small_c_input_kernel<float>, dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, s, static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, sp.Hp,
-        sp.Wp, p.pad_rows, p.pad_cols);
+    launch_overlapped(pack_small_c_input_kernel<float>,
+                      dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, s,
+                      static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
+                      sp.Hp, sp.Wp, p.pad_rows, p.pad_cols);
     launch_overlapped(pack_small_c_filter_kernel<float>, grid_for(n_fil, 256, sms), 256, s, static_cast<const float*>(w),
-        reinterpret_cast<float*>(wpk), p.window_rows, p.window_cols, p.channels, p.features, 4);
+                      reinterpret_cast<float*>(wpk), p.window_rows, p.window_cols, p.channels, p.features, 4);
   } else {
     // fp16 and bf16 are both moved as 16-bit words
     if (narrow)
-      launch_overlapped(pack_small_c_input_narrow_kernel, dim3((unsigned)ceil_div(Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch),
-          256, s, static_cast<const unsigned short*>(x), reinterpret_cast<uint2*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
-          sp.Hp, Wp, p.pad_rows, p.pad_cols);
+      launch_overlapped(pack_small_c_input_narrow_kernel,
+                        dim3((unsigned)ceil_div(Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, s,
+                        static_cast<const unsigned short*>(x), reinterpret_cast<uint2*>(xp), p.batch, p.in_rows, p.in_cols,
+                        p.channels, sp.Hp, Wp, p.pad_rows, p.pad_cols);
     else
-      launch_overlapped(pack_small_c_input_kernel<__half>, dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, s, static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, sp.Hp,
-          sp.Wp, p.pad_rows, p.pad_cols);
+      launch_overlapped(pack_small_c_input_kernel<__half>,
+                        dim3((unsigned)ceil_div(sp.Wp, 256), (unsigned)sp.Hp, (unsigned)p.batch), 256, s,
+                        static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols,
+                        p.channels, sp.Hp, sp.Wp, p.pad_rows, p.pad_cols);
     launch_overlapped(pack_small_c_filter_kernel<__half>, grid_for(n_fil, 256, sms), 256, s, static_cast<const __half*>(w),
-        reinterpret_cast<__half*>(wpk), p.window_rows, p.window_cols, p.channels, p.features,
-        narrow ? 4 : 8);
+                      reinterpret_cast<__half*>(wpk), p.window_rows, p.window_cols, p.channels, p.features, narrow ? 4 : 8);
   }
   int st = check_launch("conv2d small-channel packing");
   count_launch();
@@ -3077,7 +3081,7 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
       (!hwcf || w_ld == (uint64_t)p.features)) {  // (a column slice of a wider filter is not one contiguous run)
     if (cudaMallocAsync(reinterpret_cast<void**>(&w_split), filter_elems * sizeof(float), s) == cudaSuccess) {
       launch_overlapped(split_lo_kernel, grid_for(filter_elems, 256, sms), 256, s, static_cast<const float*>(w), w_split,
-          filter_elems);
+                        filter_elems);
       count_launch();
       g.b_presplit = 1;
     } else {
@@ -3229,8 +3233,8 @@ int conv_forward_grouped(int dtype, const void* x, const void* w, void* y, const
   if (status == PDNN_OK && !plan.tma_store) status = PDNN_INVALID_PARAMETER;
   if (status == PDNN_OK) {
     launch_overlapped(pack_grouped_filter_kernel, grid_for(packed_bytes / 2, 256, sms), 256, s,
-        static_cast<const unsigned short*>(w), static_cast<unsigned short*>(packed), taps, Cg, Kg, p.groups, per_tile, rows,
-        p.filter_format == 2);
+                      static_cast<const unsigned short*>(w), static_cast<unsigned short*>(packed), taps, Cg, Kg, p.groups,
+                      per_tile, rows, p.filter_format == 2);
     status = check_launch("conv2d grouped filter packing");
     if (status == PDNN_OK) status = launch_gemm(plan, dtype, s);
     if (own) cudaFreeAsync(packed, s);
@@ -3260,7 +3264,7 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
   if (dtype == PDNN_F32 && (size_t)p.batch * p.in_rows * p.in_cols >= 2048 && aligned16(w) &&
       cudaMallocAsync(reinterpret_cast<void**>(&w_split), filter_elems * sizeof(float), s) == cudaSuccess) {
     launch_overlapped(split_lo_kernel, grid_for(filter_elems, 256, sms), 256, s, static_cast<const float*>(w), w_split,
-        filter_elems);
+                      filter_elems);
     count_launch();
   } else if (dtype == PDNN_F32) {
     cudaGetLastError();
@@ -3681,11 +3685,15 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
     }
   }
   if (dtype == PDNN_F32)
-    launch_overlapped(pack_small_c_input_kernel<float>, dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, s, static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels, q.sp.Hp,
-        q.sp.Wp, p.pad_rows, p.pad_cols);
+    launch_overlapped(pack_small_c_input_kernel<float>,
+                      dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, s,
+                      static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
+                      q.sp.Hp, q.sp.Wp, p.pad_rows, p.pad_cols);
   else
-    launch_overlapped(pack_small_c_input_kernel<__half>, dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, s, static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols, p.channels,
-        q.sp.Hp, q.sp.Wp, p.pad_rows, p.pad_cols);
+    launch_overlapped(pack_small_c_input_kernel<__half>,
+                      dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)q.sp.Hp, (unsigned)p.batch), 256, s,
+                      static_cast<const __half*>(x), reinterpret_cast<uint4*>(xp), p.batch, p.in_rows, p.in_cols,
+                      p.channels, q.sp.Hp, q.sp.Wp, p.pad_rows, p.pad_cols);
   int st = check_launch("conv2d small-channel packing");
   if (st == PDNN_OK) st = launch_gemm(g, dtype, s);
   if (st == PDNN_OK) {
@@ -3693,16 +3701,17 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
     const unsigned grid = grid_for(n_out, 256, sms);
     if (dtype == PDNN_F32)
       launch_overlapped(unpack_small_c_filter_grad_kernel<float>, grid, 256, s, partial, static_cast<float*>(dw), f.splits,
-                                                                    p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
+                        p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
     else if (out_f32)  // 16-bit tensors (8 channels per packed pixel), fp32 gradient
       launch_overlapped(unpack_small_c_filter_grad_kernel<__half, float>, grid, 256, s, partial, static_cast<float*>(dw),
-          f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
+                        f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
     else if (dtype == PDNN_F16)
-      launch_overlapped(unpack_small_c_filter_grad_kernel<__half>, grid, 256, s, partial, static_cast<__half*>(dw), f.splits,
-                                                                     p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
+      launch_overlapped(unpack_small_c_filter_grad_kernel<__half>, grid, 256, s, partial, static_cast<__half*>(dw),
+                        f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
     else
       launch_overlapped(unpack_small_c_filter_grad_kernel<__nv_bfloat16>, grid, 256, s, partial,
-          static_cast<__nv_bfloat16*>(dw), f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
+                        static_cast<__nv_bfloat16*>(dw), f.splits, p.window_rows, p.window_cols, p.channels, p.features,
+                        epr, accumulate);
     st = check_launch("conv2d small-channel filter gradient unpack");
   }
   release();
