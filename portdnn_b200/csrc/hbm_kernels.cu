@@ -1793,7 +1793,7 @@ int launch_pooling(int op, int direction, int dtype, const void* in, void* out, 
     const size_t items = pixels * (p.channels / (vec ? VN : 1));
     if (op == PDNN_POOL_AVERAGE && vec && p.out_rows == 1 && p.out_cols == 1 && p.pad_rows == 0 && p.pad_cols == 0 &&
         p.window_rows == p.in_rows && p.window_cols == p.in_cols &&
-        (size_t)p.batch * p.in_rows * p.in_cols * p.channels < 0xFF000000ull) {
+        (size_t)p.batch * p.channels < 0xFF000000ull) {  // (indices of channels; pixels are counted in 64 bits)
       const unsigned cvecs = (unsigned)(p.channels / VN), tiles = (cvecs + 31u) / 32u, px = (unsigned)(p.in_rows * p.in_cols);
       const unsigned n_blocks = (unsigned)p.batch * tiles, most = (unsigned)sms * 32u;
       const unsigned blocks = n_blocks < most ? n_blocks : most;

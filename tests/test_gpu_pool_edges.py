@@ -56,3 +56,18 @@ def test_global_average(n, rows, cols, c, dtype):
     assert ((y.view(n, c).double() - ref).abs() <= bound).all()
     share = (dy.float() / torch.full_like(dy, rows * cols, dtype=torch.float32)).to(dy.dtype)
     assert torch.equal(dx.view(n, rows * cols, c), share.expand(n, rows * cols, c))
+
+
+def test_global_average_of_more_than_four_billion_elements():
+    """8.6 GB on the image side: offsets beyond 32 bits in both directions."""
+    n, rows, cols, c = 21000, 10, 10, 2048
+    p = pd.pool_params(n, rows, cols, c, 1, 1, False)
+    p.window_rows, p.window_cols, p.out_rows, p.out_cols = rows, cols, 1, 1
+    dy = torch.randn(n, c, device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).half()
+    dx = pd.pooling(pd.POOL_AVERAGE, 1, dy.reshape(-1), p).view(n, rows * cols, c)
+    share = (dy.float() / torch.full_like(dy, 100.0, dtype=torch.float32)).half()
+    for i in (0, 1, 10485, 10486, 20971, 20972, n - 1):  # about the images at 2^31 and 2^32 elements
+        assert torch.equal(dx[i], share[i].expand(rows * cols, c))
+    y = pd.pooling(pd.POOL_AVERAGE, 0, dx.reshape(-1), p).view(n, c)
+    # a hundred equal values: exact products of the sum up to 100 fp32 roundings, one division and one rounding
+    assert ((y.float() - share.float()).abs() <= 2.0 ** -11 * 1.1 * share.float().abs() + 2.0 ** -25).all()
