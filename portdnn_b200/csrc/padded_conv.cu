@@ -161,22 +161,31 @@ size_t scratch_bytes(int pass, int dtype, const Plan& plan) {
 
 // Where the direct kernel, one launch that walks each output's terms one after another, is still the better
 // one.  Measured (bf16, us, direct / padded copies):
-//   images, size, channels, window | forward     | input backprop | filter backprop
-//   1 x 7x7    20 -> 30   3x3      |  17 / 20    |  21 / 20       |    7 / 20
-//   1 x 14x14  20 -> 30   3x3      |  17 / 20    |  21 / 17       |   15 / 17
-//   1 x 28x28  20 -> 30   3x3      |  17 / 17    |  21 / 17       |   50 / 19
-//   4 x 28x28  20 -> 30   3x3      |  22 / 17    |  23 / 17       |  189 / 23
-//   1 x 7x7    100 -> 150 3x3      |  66 / 19    | 107 / 21       |   33 / 17
-//   8 x 28x28  100 -> 150 1x1      |  79 / 18    | 128 / 18       |  517 / 28
-//   7 x 45x45  100 -> 150 3x3      | 1371 / 39   | 2523 / 40      | 7574 / 60
-// Forward and input backprop move over by the terms of a sum or by the work of the layer, the filter
-// gradient (one block per input channel, tap and 32 features) the work alone.
+//   forward                          |  1 image    | 4 images    | 64 images   | 256 images
+//    7x7   12 -> 12  1x1             |  4.7 / 10.1 |  4.7 / 10.0 |  4.7 / 10.1 |   6.2 / 10.2
+//   14x14  12 -> 12  1x1             | 10.5 / 10.4 |  4.7 / 10.0 |  6.2 / 10.2 |  14.4 / 12.0
+//   28x28  12 -> 20  1x1             |  4.7 / 10.0 |  4.6 / 10.0 | 22.6 / 15.5 |  71.7 / 21.1
+//    7x7  100 -> 20  1x1             | 10.3 / 10.1 | 10.3 / 10.1 | 12.3 / 10.2 |  24.6 / 12.9
+//    3x3   20 -> 30  3x3             | 12.3 / 10.2 | 12.3 / 12.2 | 14.4 / 12.5 |  14.4 / 13.0
+//   28x28  20 -> 30  3x3             | 16.5 / 11.6 | 20.8 / 12.0 | 224  / 21.7 | 874   / 48.6
+//   images, size, channels, window   | input backprop | filter backprop
+//   1 x 7x7    20 -> 30   3x3        |  21 / 20       |    7 / 20
+//   1 x 14x14  20 -> 30   3x3        |  21 / 17       |   15 / 17
+//   1 x 28x28  20 -> 30   3x3        |  21 / 17       |   50 / 19
+//   4 x 28x28  20 -> 30   3x3        |  23 / 17       |  189 / 23
+//   1 x 7x7    100 -> 150 3x3        | 107 / 21       |   33 / 17
+//   8 x 28x28  100 -> 150 1x1        | 128 / 18       |  517 / 28
+//   7 x 45x45  100 -> 150 3x3        | 2523 / 40      | 7574 / 60
+// The forward pass moves over by the terms of a sum or by the work of one image, not of the batch: the two kernels
+// add up in different orders, and an image has the same result alone and in any batch.  The input backprop moves
+// over by the terms or by the work of the layer, the filter gradient (one block per input channel, tap and 32
+// features) by the work alone.
 bool direct_is_better(int pass, const PdnnConv2DParams& p) {
   const double taps = (double)p.window_rows * p.window_cols;
-  const double macs = (double)p.batch * p.out_rows * p.out_cols * taps * p.channels * p.features;
+  const double per_image = (double)p.out_rows * p.out_cols * taps * p.channels * p.features, macs = per_image * p.batch;
+  if (pass == PDNN_FORWARD) return per_image < 1e5 && taps * p.channels < 64;
   if (pass == PDNN_FILTER_BACKPROP) return macs < 1.5e6;
-  const double terms = taps * (pass == PDNN_FORWARD ? p.channels : p.features);
-  return macs < 8e6 && terms < 256;
+  return macs < 8e6 && taps * p.features < 256;
 }
 
 }  // namespace

@@ -93,3 +93,23 @@ def test_fused_backprop_forms(channels, features):
     pd.conv2d(pd.FILTER_BACKPROP, x, dy, p, out=dw, output_f32=True, accumulate=1)
     plain = pd.conv2d(pd.FILTER_BACKPROP, x, dy, p, algorithm=pd.ALGO_DIRECT)
     _close(dw - 1.0, plain, "f16")
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("size,c,k,win", [(7, 20, 30, 3), (14, 20, 30, 3), (28, 20, 30, 3), (28, 12, 20, 1), (9, 100, 150, 1)])
+def test_an_image_alone_and_in_a_batch(size, c, k, win, dtype):
+    """Whichever kernel a ragged layer runs on, it is the same one for every batch: an image's result has the same
+    bits whatever is beside it."""
+    g = torch.Generator(device="cuda").manual_seed(size * c)
+    dt = torch.float16 if dtype == "f16" else torch.bfloat16
+    x, w, b = (torch.randn(n, device="cuda", generator=g).to(dt) for n in (64 * size * size * c, win * win * c * k, k))
+    x = x.view(64, -1)
+
+    def call(images):
+        p = pd.conv_params(len(images), size, size, c, k, win, 1)
+        return pd.conv2d(pd.FORWARD, images.reshape(-1), w, p, bias=b, activation=pd.ACT_RELU).view(len(images), -1)
+
+    together = call(x)
+    for first, many in ((0, 1), (5, 1), (8, 2), (30, 9)):
+        assert torch.equal(together[first:first + many], call(x[first:first + many]))
+    assert_no_device_error()
