@@ -47,9 +47,10 @@ typedef enum PdnnPass { PDNN_FORWARD = 0, PDNN_INPUT_BACKPROP = 1, PDNN_FILTER_B
  * needs no im2col buffer); Winograd and WinogradLarge run Winograd F(2x2,3x3) (transforms around
  * a batched tcgen05 matmul) on 3x3 stride-1 forward / input-backprop layers when the caller
  * passes the workspace pdnn_conv2d_workspace_size recommends, and the implicit-GEMM kernel
- * otherwise.  A shape the tensor-core kernels cannot take
- * (channel or feature count not a multiple of 8 elements of 16 bits / 4 of 32 bits) is routed
- * to the direct kernel whatever the algorithm. */
+ * otherwise.  16-bit tensors whose channel or feature count is not a multiple of 8, or that start off a
+ * 16-byte boundary, run on the tensor cores through padded copies; a shape they cannot take otherwise
+ * (32-bit tensors with a count off a multiple of 4, strides above 2, more than 64 taps) is routed to the
+ * direct kernel whatever the algorithm. */
 typedef enum PdnnAlgorithm {
   PDNN_ALGO_NOT_SUPPORTED = 0,
   PDNN_ALGO_DIRECT = 1,

@@ -3,8 +3,8 @@
 The product is ``libportdnn_b200.so`` (hand-written sm_100a CUDA behind the C ABI of
 ``include/portdnn_b200.h``) plus the C++ headers under ``include/portdnn/`` that rebuild
 portDNN's ``sycldnn::`` API on top of it.  This package is the Python front end used by
-the tests and the benchmark: thin ctypes calls on torch CUDA tensors, named after the
-reference's operators.  There is no CPU path: without the built library, or without a
+the tests and the benchmark: thin calls on torch CUDA tensors, named after the reference's
+operators (the operators through a small extension module, queries through ctypes).  There is no CPU path: without the built library, or without a
 B200, every call raises.
 """
 from .api import (  # noqa: F401

@@ -1,5 +1,6 @@
-// Second stage of the split reductions (filter gradients over pixel splits or slices, batch statistics
-// over row slices): the columns of a rows x n fp32 matrix of partial sums are added in a fixed order.
+// Second stage of the split reductions (filter gradients over pixel splits or slices; batch statistics over row
+// slices where the tensors are not in 16-byte packets, and with frozen parameters): the columns of a
+// rows x n fp32 matrix of partial sums are added in a fixed order.
 #pragma once
 
 #include "common.cuh"
@@ -11,9 +12,9 @@ constexpr int kSumFlat = 256;  // threads of a block without row lanes
 
 // Bound by latency: the matrix is in L2 and a thread that walks a column alone waits for one load after
 // another.  Here a block takes 32 columns with LANES (8 or 32) threads to a column, each with four loads
-// in flight, and adds their results through shared memory, in a fixed order.  Batch normalisation in
-// training, forward and backward, between its convolutions (four sums of 784 x 512, on two blocks before):
-// 364 -> 221 us; depthwise filter gradient of 56x56x144 at 128 images (444 x 1296): 8 us less.
+// in flight, and adds their results through shared memory, in a fixed order.  Four sums of 784 x 512 of a batch
+// normalisation, on two blocks before: 36 us less each; depthwise filter gradient of 56x56x144 at 128 images
+// (444 x 1296): 8 us less.
 // finish(i, sum): what becomes of column i.
 template <int LANES, typename Finish>
 __global__ void __launch_bounds__(32 * LANES)

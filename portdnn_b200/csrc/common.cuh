@@ -112,7 +112,8 @@ int device_sm_count();   // SM count of the current device; -1 if it is not an s
 // nothing under an ordinary launch.)  The life of such a kernel begins while its predecessor still writes what it
 // will read, so the read-only path is not open to it, which asks for data that nobody writes meanwhile and
 // promises nothing else: its inputs are plain pointers (const without __restrict__, from which the compiler would
-// infer read-only loads) and plain loads, which stay behind the wait.  Grids of fewer than four waves only: beside a kernel of that length
+// infer read-only loads) and plain loads, which stay behind the wait.  (The compiler moves no plain load ahead of a
+// store, so kernels that want several in flight request them before they write.)  Grids of fewer than four waves only: beside a kernel of that length
 // the gap is nothing, and long ones chained this way cost the kernels around them.  All launches ordinary /
 // grids below four waves / all overlapped, us: MobileNet-v2 forward at 64 images (80 launches) 824 / 785 / 782,
 // 7x45x61 100 -> 150 3x3 with gradients 152 / 135 / 135, two max pools with gradients 121 / 114 / 114, one

@@ -1229,8 +1229,7 @@ __global__ void __launch_bounds__(SPLIT ? 320 : 384, 1) umma_gemm_kernel(const _
 // channels share a tile, so that a step's 128-byte rows of A are full and one launch has all groups.  Every slice
 // of 16 channels multiplies its own group's filter only: no zeros of a block-diagonal filter, nothing of one
 // group ever meets another.  Bound by the A tiles an MMA reads from shared memory (4 KB for 16 columns) and by
-// HBM.  32 x 28x28x512, 32 groups, 3x3, f16: 141 -> 27 us (3 of
-// them the packing of the filter).
+// HBM.  32 x 28x28x512, 32 groups, 3x3, f16: 141 -> 24 us (3 of them the packing of the filter).
 template <int EPI, typename OutT>
 __global__ void __launch_bounds__(384, 1) umma_gemm_grouped_kernel(const __grid_constant__ GemmArgs args) {
   umma_gemm_body<false, EPI, OutT, true>(args, (int)blockIdx.x, (int)gridDim.x);
@@ -2335,8 +2334,11 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
                          : g.halo ? g.halo_stage_bytes
                                   : g.b_res ? (unsigned)kABytes : (kABytes + (unsigned)g.bn * 128u) * (split ? 2u : 1u);
   const int rings = g.pair ? 1 : g.groups;
-  // At least 120 KB, so that two CTAs never share an SM: the second one would wait for TMEM
-  // columns the first one holds.
+  // At least 120 KB, so that two such CTAs never share an SM: the second one would wait for TMEM columns that the
+  // first one holds, and tcgen05.alloc has no limit.  A CTA of umma_gemm_cluster_kernel is small enough to
+  // share an SM with one of that size.  Whichever of them is placed second waits for the first, which waits for
+  // nobody behind it: a successor is placed only once all CTAs of its predecessor, all ranks of its clusters
+  // among them, hold their columns (they allocate before they let it be launched).
   size_t smem = 1024 + (size_t)g.b_res_bytes + (size_t)rings * g.stages * stage +
                 (g.tma_store ? (size_t)g.groups * (g.nsw + g.mask_slots) * 4 * 4096 : 0) + kBarBlockBytes +
                 (size_t)g.bias_smem_bytes + (size_t)g.mask_smem_bytes;
@@ -2429,8 +2431,6 @@ size_t gemm_smem_bytes(const GemmArgs& g, bool split) {
   const size_t smem = 1024 + (size_t)g.b_res_bytes + (size_t)rings * g.stages * stage +
                       (g.tma_store ? (size_t)g.groups * (g.nsw + g.mask_slots) * 4 * 4096 : 0) + kBarBlockBytes +
                       (size_t)g.bias_smem_bytes + (size_t)g.mask_smem_bytes;
-  // At least 120 KB, so that two CTAs never share an SM: the second one would wait for TMEM
-  // columns the first one holds.
   return std::max<size_t>(smem, 120 * 1024);
 }
 
