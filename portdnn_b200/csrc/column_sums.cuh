@@ -32,7 +32,12 @@ __global__ void __launch_bounds__(32 * LANES)
         const float c = m[(size_t)(r + 2 * LANES) * n + i], d = m[(size_t)(r + 3 * LANES) * n + i];
         sum += (a + b) + (c + d);
       }
-      for (; r < rows; r += LANES) sum += m[(size_t)r * n + i];
+      float rest[3];  // the last ones requested together, too (7x45x61 104 -> 152 3x3 filter gradient: 40.8 -> 39.0 us)
+#pragma unroll
+      for (int u = 0; u < 3; ++u) rest[u] = r + u * LANES < rows ? m[(size_t)(r + u * LANES) * n + i] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 3; ++u)
+        if (r + u * LANES < rows) sum += rest[u];
     }
     red[ty][tx] = sum;
     __syncthreads();
