@@ -417,10 +417,8 @@ struct PoolS2Geometry {
 };
 
 template <typename T, int V>
-__global__ void __launch_bounds__(kBlock)
-    pool_max_grad_s2_kernel(const unsigned char* winner, const T* dy, T* __restrict__ dx,
-                            PoolS2Geometry g, unsigned n_items) {
-  overlap_wait();
+__device__ __forceinline__ void pool_max_grad_s2(const unsigned char* winner, const T* dy, T* dx, const PoolS2Geometry& g,
+                                                 unsigned n_items) {
   const unsigned cvecs = (unsigned)(g.C / V);
   for (unsigned idx = blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += gridDim.x * kBlock) {
     const unsigned cv = idx % cvecs;
@@ -512,6 +510,21 @@ __global__ void __launch_bounds__(kBlock)
       }
     }
   }
+}
+
+// Ordinary launch, read-only loads: those of the next row are on their way before this one is stored.
+template <typename T, int V>
+__global__ void __launch_bounds__(kBlock)
+    pool_max_grad_s2_kernel(const unsigned char* __restrict__ winner, const T* __restrict__ dy, T* __restrict__ dx,
+                            PoolS2Geometry g, unsigned n_items) {
+  pool_max_grad_s2<T, V>(winner, dy, dx, g, n_items);
+}
+// Placed beside the end of the winner kernel, plain loads.
+template <typename T, int V>
+__global__ void __launch_bounds__(kBlock)
+    pool_max_grad_s2_overlapped_kernel(const unsigned char* winner, const T* dy, T* dx, PoolS2Geometry g, unsigned n_items) {
+  overlap_wait();
+  pool_max_grad_s2<T, V>(winner, dy, dx, g, n_items);
 }
 
 // Average-pool gradient (src/pooling/kernels.h:312-366): dx[i] = sum_o dy[o] / valid(o).
@@ -1917,8 +1930,15 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
           while (g.rows > 4 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 2048) g.rows = (g.rows + 1) / 2;
           g.strips = (g.M + g.rows - 1) / g.rows;
           const size_t n_items = columns * g.strips;
-          launch_overlapped(pool_max_grad_s2_kernel<T, VN>, grid_for(n_items, kBlock, sms), kBlock, s, winner, dyt, dxt, g,
-                            (unsigned)n_items);
+          // Below three quarters of a wave the overlap is worth more, above it the read-only loads (us, overlapped /
+          // ordinary: 2 x 56x56x128 f32 10.8 / 12.4, 16 x 113x151x64 f16 (0.5 waves) 30.8 / 33.2, f32 (1.0) 46.3 / 45.7,
+          // 64 x 112x112x64 f32 118.1 / 116.5, f16 80.3 / 74.3).
+          const unsigned grid = grid_for(n_items, kBlock, sms);
+          if (n_items < (size_t)sms * 1536)
+            launch_overlapped(pool_max_grad_s2_overlapped_kernel<T, VN>, grid, kBlock, s, winner, dyt, dxt, g,
+                              (unsigned)n_items);
+          else
+            pool_max_grad_s2_kernel<T, VN><<<grid, kBlock, 0, s>>>(winner, dyt, dxt, g, (unsigned)n_items);
           st = check_launch("pooling max gradient (3x3 / 2 gather)");
         } else if (st == PDNN_OK) {
           pool_max_grad_from_winner_kernel<T, VN, unsigned><<<g2, kBlock, 0, s>>>(winner, dyt, dxt, p, (unsigned)in_items);
