@@ -5,7 +5,7 @@
 // are in order are read, and results written, in place.
 //
 // Bound by the convolution itself, then by the launches around it.  7 x 45x61, 100 -> 150 channels, 3x3, bf16,
-// all three passes: 15580 us on the direct kernel, 139 us here.
+// all three passes: 15580 us on the direct kernel, 137 us here.
 #include "padded_conv.cuh"
 #include "tc_gemm.cuh"
 
