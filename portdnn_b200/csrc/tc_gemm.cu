@@ -12,12 +12,12 @@
 // main loop of the next) and are written to global memory by four epilogue warps with bias,
 // activation and alpha/beta applied on the way.
 //
-// fp32 tensors are multiplied as three TF32 products (hi*hi + hi*lo + lo*hi): four extra warps
-// split each landed stage into its high and low parts in shared memory before the MMA warp
-// consumes it.
+// fp32 tensors are multiplied as three TF32 products (hi*hi + hi*lo + lo*hi): eight extra warps
+// split each landed stage into its high and low parts, A into tensor memory and B in shared memory, before
+// the MMA warp consumes it.
 //
-// Warp roles (192 threads; 320 with the split): warp 0 TMA producer, warp 1 MMA issuer and TMEM
-// owner, warps 2-5 epilogue, warps 6-9 hi/lo split.
+// Warp roles of a pipeline: warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-5 epilogue;
+// with the split warps 6-13 hi/lo.
 #include "column_sums.cuh"
 #include "tc_gemm.cuh"
 #include "umma.cuh"
@@ -37,6 +37,8 @@ constexpr int kMaxTaps = 64;
 constexpr int kTileM = 128;
 constexpr int kABytes = kTileM * 128;  // one A stage: 128 rows of 128 bytes
 constexpr int kMaxStages = 8;
+constexpr int kSplitThreads = 448;       // fp32 variant: producer, issuer, four epilogue and eight split warps
+constexpr uint32_t kSplitAColumns = 64;  // fp32 variant: tensor-memory columns of a stage's A tile, hi and lo
 constexpr int kSmemBudget = 227 * 1024;
 constexpr int kBarsPerGroup = 3 * kMaxStages + 4;  // full, empty, ready per stage; accumulator full / empty x 2
 constexpr int kBarBlockBytes = 512;                // barriers of two groups, the resident-B barrier, TMEM slot, abort flag
@@ -334,31 +336,39 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmArgs& a, const TileC
     uint8_t* row_ptr = ws.buf + slot * 4096u + (size_t)lane * 128;
 #pragma unroll
     for (int half = 0; half < CPB / 32; ++half) {
-      uint32_t acc[32];
-      if (!zero) {
-        tmem_ld_32x32(tmem_acc + (uint32_t)(c0 + half * 32), acc);
-        tmem_wait_ld();
-      }
       const int colbase = t.nf0 + c0 + half * 32;
+      uint32_t acc[32];
+      if (!zero) tmem_ld_32x32(tmem_acc + (uint32_t)(c0 + half * 32), acc);
+      // all of the bias in flight beside the accumulators (columns beyond the last one are not stored)
+      float b[32];
+      if (bias != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) b[i] = to_f32(bias[min(colbase + i, a.ext_cols - 1)]);
+      }
+      if (!zero) tmem_wait_ld();
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = zero ? 0.f : a.alpha * __uint_as_float(acc[i]);
+      if (bias != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] += b[i];
+      }
+      if (a.act == PDNN_ACT_TANH) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = apply_activation(v[i], PDNN_ACT_TANH);
+      } else if (a.act != PDNN_ACT_NONE) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = apply_activation(v[i], PDNN_ACT_RELU);
+        if (a.act == PDNN_ACT_RELU6) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = fminf(v[i], 6.f);
+        }
+      }
 #pragma unroll
       for (int g = 0; g < 32 / P; ++g) {
-        float v[P];
-#pragma unroll
-        for (int i = 0; i < P; ++i) v[i] = zero ? 0.f : a.alpha * __uint_as_float(acc[g * P + i]);
-        if (bias != nullptr) {
-#pragma unroll
-          for (int i = 0; i < P; ++i) {
-            const int c = colbase + g * P + i;
-            if (c < a.ext_cols) v[i] += to_f32(bias[c]);
-          }
-        }
-        if (a.act != PDNN_ACT_NONE) {
-#pragma unroll
-          for (int i = 0; i < P; ++i) v[i] = apply_activation(v[i], a.act);
-        }
         Vec16<OutT> pk;
 #pragma unroll
-        for (int i = 0; i < P; ++i) pk.set(i, from_f32<OutT>(v[i]));
+        for (int i = 0; i < P; ++i) pk.set(i, from_f32<OutT>(v[g * P + i]));
         const int chunk = half * (32 / P) + g;  // 0..7 within the 128-byte row
         *reinterpret_cast<uint4*>(row_ptr + ((chunk ^ (lane & 7)) << 4)) = pk.raw;
       }
@@ -618,7 +628,7 @@ __device__ __forceinline__ bool epilogue_tile_tma_fast(const GemmArgs& a, const 
 // MMAs are counted, which is two to three times the time the tensor pipe needs for a 128 x 64 or
 // 128 x 128 MMA; two issuers keep the pipe busy, and two epilogue teams halve the time a tile's
 // accumulator waits to be drained.  The resident B tiles, the bias copy and the TMEM allocation
-// are shared.  The fp32 (3xTF32) variant runs one group plus the four hi/lo split warps.
+// are shared.  The fp32 (3xTF32) variant runs one group plus the eight hi/lo split warps.
 //
 // The role loops carry `#pragma unroll 1`: left alone the compiler unrolls them fourfold, the
 // kernel grows from 59 to 80 KB, and the instruction-cache hit rate drops (92% measured on the
@@ -628,7 +638,7 @@ __device__ __forceinline__ bool epilogue_tile_tma_fast(const GemmArgs& a, const 
 //   warp 6g + 0      producer of group g
 //   warp 6g + 1      MMA issuer of group g (warp 1 also owns the TMEM allocation)
 //   warps 6g + 2..5  epilogue of group g (warp % 4 selects the TMEM lane quarter)
-//   SPLIT: warps 6..9 are the hi/lo split warps of the only group
+//   SPLIT: warps 6..13 are the hi/lo split warps of the only group
 // The body of the kernel for CTA `cta` of `n_ctas` that work on the GEMM `a` (the whole grid, or the share
 // of it that umma_gemm_multi_kernel gives to one of its GEMMs).
 template <bool SPLIT, int EPI, typename OutT, bool GROUPED = false>
@@ -647,7 +657,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
   // for.
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int grp = SPLIT ? 0 : warp / 6;
-  const int role = SPLIT ? warp : warp - grp * 6;  // 0 producer, 1 issuer, 2..5 epilogue, 6..9 split (SPLIT)
+  const int role = SPLIT ? warp : warp - grp * 6;  // 0 producer, 1 issuer, 2..5 epilogue, 6..13 split (SPLIT)
 
   const uint32_t b_bytes = a.b_step_bytes;
   const uint32_t part_bytes = kABytes + b_bytes;              // one A tile + one B tile
@@ -655,7 +665,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
   const uint32_t res_bytes = b_res ? a.b_res_bytes : 0u;      // resident B tiles come first
   const bool halo = !SPLIT && a.halo != 0;
   const bool pair = !SPLIT && a.pair != 0;
-  const uint32_t stage_bytes = SPLIT  ? 2u * part_bytes
+  const uint32_t stage_bytes = SPLIT  ? part_bytes + b_bytes  // A, the landed B, the lo part of B
                                : pair ? part_bytes + (uint32_t)kABytes
                                : halo ? a.halo_stage_bytes
                                       : (b_res ? (uint32_t)kABytes : part_bytes);
@@ -857,7 +867,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
                   load_b(sa + 2u * kABytes, fb, kc, t.nf0, btap);
                 } else if (!b_res) {
                   load_b(sa + kABytes, fb, kc, t.nf0, btap);
-                  if (presplit) load_b_from(&a.b_map_lo, sa + part_bytes + kABytes, fb, kc, t.nf0, btap);
+                  if (presplit) load_b_from(&a.b_map_lo, sa + part_bytes, fb, kc, t.nf0, btap);
                 }
               }
               next_stage();
@@ -866,7 +876,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
         } else {
           const TapEntry e = a.taps[t.tap];
           const CUtensorMap* amap = &a.a_map[e.a_map];
-          // packed taps: the second box holds the same channels as seen by the next tap (none: a box
+          // packed taps: the second half of the boxes holds the same channels as seen by the next tap (none: boxes
           // beyond the last channel, which TMA fills with zeros)
           const bool packed = a.tap_pack > 1, second = packed && t.tap + 1 < a.num_taps;
           const TapEntry e2 = a.taps[second ? t.tap + 1 : t.tap];
@@ -889,8 +899,11 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
               const uint32_t sb = sa + kABytes;
               const int kw = iw * a.tw, kh = ih * a.th, kn = in * a.tn + batch;
               if (packed) {
-                warp_tma_load_4d(sa, amap, fb, t.w0, kw + e.dw, kh + e.dh, kn);
-                warp_tma_load_4d(sa + a_box_bytes, amap2, fb, c2nd, kw + e2.dw, kh + e2.dh, kn);
+                const int half = a_boxes >> 1;
+                for (int j = 0; j < half; ++j) {
+                  warp_tma_load_4d(sa + (uint32_t)j * a_box_bytes, amap, fb, t.w0 + j * epr, kw + e.dw, kh + e.dh, kn);
+                  warp_tma_load_4d(sa + (uint32_t)(half + j) * a_box_bytes, amap2, fb, c2nd + j * epr, kw + e2.dw, kh + e2.dh, kn);
+                }
               } else {
 #pragma unroll 1
                 for (int j = 0; j < a_boxes; ++j)
@@ -925,7 +938,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
       const uint64_t a_desc0 = make_smem_desc(0, a.a_lbo, a.a_sbo, a.a_layout);
       const uint64_t b_desc0 = make_smem_desc(0, a.b_lbo, a.b_sbo, a.b_layout);
       const uint32_t a_kadv = a.a_kadv >> 4, b_kadv = a.b_kadv >> 4, idesc = a.idesc;
-      const uint32_t lo_off = part_bytes >> 4;
+      const uint32_t lo_off = b_bytes >> 4;
       int s = 0;
       uint32_t ph = 0;
       uint32_t buf = 0, aph = 0;  // accumulator buffer of this tile and the parity of its barriers
@@ -1068,12 +1081,13 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
             const uint32_t sa = ring_base + (uint32_t)s * stage_bytes;
             uint64_t da = a_desc0 + (uint64_t)(sa >> 4);
             uint64_t db = b_desc0 + (uint64_t)((sa + kABytes) >> 4);
+            const uint32_t ta = tmem_base + acc_bufs * acc_stride + (uint32_t)s * kSplitAColumns;  // SPLIT: hi, then lo of A
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               if (SPLIT) {
-                warp_mma_tf32(d_tmem, da + lo_off, db, idesc, accumulate);
-                warp_mma_tf32(d_tmem, da, db + lo_off, idesc, 1u);
-                warp_mma_tf32(d_tmem, da, db, idesc, 1u);
+                warp_mma_tf32_ts(d_tmem, ta + 32u + 8u * (uint32_t)k, db, idesc, accumulate);
+                warp_mma_tf32_ts(d_tmem, ta + 8u * (uint32_t)k, db + lo_off, idesc, 1u);
+                warp_mma_tf32_ts(d_tmem, ta + 8u * (uint32_t)k, db, idesc, 1u);
               } else {
                 warp_mma_f16(d_tmem, da, db, idesc, accumulate);
               }
@@ -1162,12 +1176,22 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     if (EPI != 0 && lane == 0) bulk_wait_group<0>();
   } else if (SPLIT) {
     // ------------------------------- hi/lo split (fp32 as 3xTF32) ----------------------------
-    // hi is the 19 leading bits of an fp32 word, which is all the tensor core reads of it, so the
-    // landed tile serves as the hi part as it is; lo = x - hi is exact in fp32 and is written to the
-    // second part of the stage.  Element positions do not change, so the swizzle is irrelevant here.
-    const int tid = threadIdx.x - 6 * 32;  // 0..127
-    const int chunks = (int)((a.b_presplit ? (uint32_t)kABytes : part_bytes) >> 4);  // A comes first in a part
-    int s = 0;
+    // hi is the 19 leading bits of an fp32 word, which is all the tensor core reads of it; lo = x - hi is exact
+    // in fp32.  Both parts of A go to tensor memory, a row to a lane, from where the MMAs read them without
+    // touching shared memory; rows that lie along the reduction in shared memory (A MN-major) are transposed by
+    // the way they are read.  The landed B serves as its own hi part; its lo part, where it did not arrive by
+    // TMA, is written behind it (element positions do not change, so the swizzle is irrelevant there).
+    // Two teams of four warps take every second stage each.
+    // What bounds the kernel is shared memory, 128 bytes a cycle: per step of 32 and 128 columns TMA writes 32 KB, A is
+    // read once (16), B read and its lo part written (32), and the three products read 48 KB of B - 128 KB, 1000
+    // cycles, for 768 cycles of math, and 0.53 us are measured.  With both parts of A in shared memory the products
+    // read 96 KB and lo of A was written there too, 176 KB and 0.72 us.  8 images, us before / now:
+    // VGG-16 training step 6905 / 4243; 3x3 56x56 256 -> 256 forward 278 / 120, filter gradient 205 / 120.
+    const int team = (warp - 6) >> 2, q = warp & 3;  // q: the TMEM lanes [32q, 32q+32) this warp may write
+    const int row = q * 32 + lane, tid = threadIdx.x - (6 + 4 * team) * 32;
+    const int chunks = a.b_presplit ? 0 : (int)(b_bytes >> 4);
+    const uint32_t a_tmem = tmem_base + ((uint32_t)(q * 32) << 16) + acc_bufs * acc_stride;
+    int s = 0, turn = 0;
     uint32_t ph = 0;
     bool ok = true;
     TileWalker walker;
@@ -1176,28 +1200,52 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
       const TileCoord t = walker.coord(a);
 #pragma unroll 1
-      for (int ks = t.ks_begin; ks < t.ks_end; ++ks) {
-        if (!mbar_wait(full_bar(s), ph, abort_flag, g_error_record, a.wait_limit_ns, 0x500u + (unsigned)s)) {
-          ok = false;
-          break;
+      for (int ks = t.ks_begin; ks < t.ks_end; ++ks, turn ^= 1) {
+        if (turn == team) {
+          if (!mbar_wait(full_bar(s), ph, abort_flag, g_error_record, a.wait_limit_ns, 0x500u + (unsigned)s)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();  // the MMAs that read this slot of tensor memory before are done (the stage was free)
+          const uint8_t* at = ring_mem + (size_t)s * stage_bytes;
+          uint32_t v[32];
+          if (!a.a_mn) {  // the row's 128 bytes, 16-byte chunk j at j ^ (row % 8)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint4 c = *reinterpret_cast<const uint4*>(at + row * 128 + ((j ^ (row & 7)) << 4));
+              v[4 * j] = c.x, v[4 * j + 1] = c.y, v[4 * j + 2] = c.z, v[4 * j + 3] = c.w;
+            }
+          } else {  // column `lane` of the 32 reduction rows of box q, 32-byte chunk j of row k at j ^ (k % 4)
+            const uint8_t* box = at + q * 4096 + ((lane & 7) << 2);
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = *reinterpret_cast<const uint32_t*>(box + k * 128 + (((lane >> 3) ^ (k & 3)) << 5));
+          }
+          uint32_t hi[32];
+#pragma unroll
+          for (int k = 0; k < 32; ++k) {
+            hi[k] = v[k] & 0xFFFFE000u;
+            v[k] = __float_as_uint(__uint_as_float(v[k]) - __uint_as_float(hi[k]));
+          }
+          const uint32_t slot = a_tmem + (uint32_t)s * kSplitAColumns;
+          tmem_st_32x32(slot, hi);
+          tmem_st_32x32(slot + 32u, v);
+          const uint4* b_hi = reinterpret_cast<const uint4*>(at + kABytes);
+          uint4* b_lo = reinterpret_cast<uint4*>(ring_mem + (size_t)s * stage_bytes + part_bytes);
+          for (int c = tid; c < chunks; c += 128) {
+            const uint4 w = b_hi[c];
+            uint4 l;
+            l.x = __float_as_uint(__uint_as_float(w.x) - __uint_as_float(w.x & 0xFFFFE000u));
+            l.y = __float_as_uint(__uint_as_float(w.y) - __uint_as_float(w.y & 0xFFFFE000u));
+            l.z = __float_as_uint(__uint_as_float(w.z) - __uint_as_float(w.z & 0xFFFFE000u));
+            l.w = __float_as_uint(__uint_as_float(w.w) - __uint_as_float(w.w & 0xFFFFE000u));
+            b_lo[c] = l;
+          }
+          fence_proxy_async_smem();
+          tmem_wait_st();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(ready_bar(s));
         }
-        uint4* hi = reinterpret_cast<uint4*>(ring_mem + (size_t)s * stage_bytes);
-        uint4* lo = reinterpret_cast<uint4*>(ring_mem + (size_t)s * stage_bytes + part_bytes);
-        for (int c = tid; c < chunks; c += 128) {
-          uint4 v = hi[c], h, l;
-          h.x = v.x & 0xFFFFE000u;
-          h.y = v.y & 0xFFFFE000u;
-          h.z = v.z & 0xFFFFE000u;
-          h.w = v.w & 0xFFFFE000u;
-          l.x = __float_as_uint(__uint_as_float(v.x) - __uint_as_float(h.x));
-          l.y = __float_as_uint(__uint_as_float(v.y) - __uint_as_float(h.y));
-          l.z = __float_as_uint(__uint_as_float(v.z) - __uint_as_float(h.z));
-          l.w = __float_as_uint(__uint_as_float(v.w) - __uint_as_float(h.w));
-          lo[c] = l;  // the hi part stays as it is: the tensor core reads the 19 leading bits of an fp32 word only
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(ready_bar(s));
         if (++s == S) {
           s = 0;
           ph ^= 1u;
@@ -1221,7 +1269,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
 }
 
 template <bool SPLIT, int EPI, typename OutT>
-__global__ void __launch_bounds__(SPLIT ? 320 : 384, 1) umma_gemm_kernel(const __grid_constant__ GemmArgs args) {
+__global__ void __launch_bounds__(SPLIT ? kSplitThreads : 384, 1) umma_gemm_kernel(const __grid_constant__ GemmArgs args) {
   umma_gemm_body<SPLIT, EPI, OutT>(args, (int)blockIdx.x, (int)gridDim.x);
 }
 
@@ -2024,10 +2072,13 @@ bool choose_box_halo(int W, int H, int rows, int* tw, int* th) {
 // 128 leave room for two accumulator buffers per pipeline, so that the next tile's MMAs overlap it.
 bool want_narrow(int ksteps, int cols) { return ksteps <= 4 || cols <= 128; }
 
-int pick_bn(long long row_tiles, int cols, int unit, int max_bn, int sms, int ksteps = 1 << 30) {
+int pick_bn(int dtype, long long row_tiles, int cols, int unit, int max_bn, int sms, int ksteps = 1 << 30) {
   if (want_narrow(ksteps, cols)) max_bn = std::min(max_bn, 128);
-  sms *= 2;  // two pipelines per CTA work on two tiles at a time
-  // cost ~ waves * (bn + fixed overhead); unit: granularity the B loader needs
+  if (dtype != PDNN_F32) sms *= 2;  // two pipelines per CTA work on two tiles at a time
+  // cost ~ waves * (bn + fixed overhead); unit: granularity the B loader needs.  fp32: a step of 128 columns takes
+  // 0.53 us, one of 64 0.39 (in-kernel split), which is where the 110 comes from: 8 images, 28x28 512 -> 512 3x3,
+  // 196 tiles of 128 columns 154 us, 392 of 64 171; 14x14, 56 of 128 78 us, 112 of 64 64.
+  const double overhead = dtype == PDNN_F32 ? 110.0 : 40.0;
   int best_bn = unit;
   double best = 1e30;
   for (int bn = unit; bn <= max_bn; bn += unit) {
@@ -2035,7 +2086,7 @@ int pick_bn(long long row_tiles, int cols, int unit, int max_bn, int sms, int ks
     if (cols >= 64 && bn % 64 != 0) continue;  // whole 128-byte output blocks for the TMA-store epilogue
     const long long tiles = row_tiles * ceil_div(cols, bn);
     const double waves = (double)((tiles + sms - 1) / sms);
-    const double cost = waves * (bn + 40.0);
+    const double cost = waves * (bn + overhead);
     if (cost < best - 1e-9) {
       best = cost;
       best_bn = bn;
@@ -2090,7 +2141,7 @@ void set_operand_layout(GemmArgs& g, int dtype, int b_mn) {
   g.a_row_bytes = 128;
   g.kmmas = 4;
   g.b_step_bytes = (unsigned)g.bn * 128u;
-  g.idesc = make_idesc(dtype == PDNN_F32 ? 2 : (dtype == PDNN_BF16 ? 1 : 0), g.a_mn, b_mn, g.bn);
+  g.idesc = make_idesc(f32 ? 2 : (dtype == PDNN_BF16 ? 1 : 0), f32 ? 0 : g.a_mn, b_mn, g.bn);  // (fp32: A comes from tensor memory, a row to a lane)
   g.tmem_cols = next_pow2(2 * g.bn);
 }
 
@@ -2132,7 +2183,7 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
   }
   g.acc_stride = std::max(32, next_pow2(g.bn));
   g.acc_bufs = g.groups * 2 * g.acc_stride <= 512 ? 2 : 1;
-  g.tmem_cols = next_pow2(g.groups * g.acc_bufs * g.acc_stride);
+  g.tmem_cols = split ? 512 : next_pow2(g.groups * g.acc_bufs * g.acc_stride);  // (split: the rest holds A tiles)
   g.bias_smem_bytes = 0;
   g.bias_tile_only = 0;
   if (!g.epi_fast) g.relu_mask = nullptr;  // only the fast epilogue applies the mask; the caller checks
@@ -2149,7 +2200,7 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
       g.bias_smem_bytes = padded * 2;
     }
   }
-  unsigned stage = (kABytes + (unsigned)g.bn * 128u) * (split ? 2u : 1u);
+  unsigned stage = kABytes + (unsigned)g.bn * 128u * (split ? 2u : 1u);
   int ksteps = g.a_mn ? g.slabs_per_split : g.num_taps * g.cblocks;
   if (!g.halo) g.res_taps = g.num_taps;
   else ksteps = g.res_taps * g.cblocks;
@@ -2215,6 +2266,7 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
     if (stages_with(g.nsw) < 4) g.mask_slots = 1;
   }
   g.stages = std::min(kMaxStages, stages_with(g.nsw));
+  if (split) g.stages = std::min(g.stages, (512 - g.acc_bufs * g.acc_stride) / (int)kSplitAColumns);
   if (g.stages < 2 && g.groups == 2) {  // very wide stages: one pipeline with a deeper ring
     g.groups = 1;
     g.acc_bufs = 2 * g.acc_stride <= 512 ? 2 : 1;
@@ -2332,7 +2384,7 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
   if (g.cta_pair) return launch_gemm_pair2(g, total, s);
   const unsigned stage = g.pair   ? 2u * kABytes + (unsigned)g.bn * 128u
                          : g.halo ? g.halo_stage_bytes
-                                  : g.b_res ? (unsigned)kABytes : (kABytes + (unsigned)g.bn * 128u) * (split ? 2u : 1u);
+                                  : g.b_res ? (unsigned)kABytes : kABytes + (unsigned)g.bn * 128u * (split ? 2u : 1u);
   const int rings = g.pair ? 1 : g.groups;
   // At least 120 KB, so that two such CTAs never share an SM: the second one would wait for TMEM columns that the
   // first one holds, and tcgen05.alloc has no limit.  A CTA of umma_gemm_cluster_kernel is small enough to
@@ -2386,7 +2438,7 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
   // in the stream (the kernel waits for that kernel before it touches any tensor it wrote).
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(split ? 320 : 384);
+  cfg.blockDim = dim3(split ? kSplitThreads : 384);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -2426,7 +2478,7 @@ int gemm_epilogue_kind(const GemmArgs& g) {
 size_t gemm_smem_bytes(const GemmArgs& g, bool split) {
   const unsigned stage = g.pair   ? 2u * kABytes + (unsigned)g.bn * 128u
                          : g.halo ? g.halo_stage_bytes
-                                  : g.b_res ? (unsigned)kABytes : (kABytes + (unsigned)g.bn * 128u) * (split ? 2u : 1u);
+                                  : g.b_res ? (unsigned)kABytes : kABytes + (unsigned)g.bn * 128u * (split ? 2u : 1u);
   const int rings = g.pair ? 1 : g.groups;
   const size_t smem = 1024 + (size_t)g.b_res_bytes + (size_t)rings * g.stages * stage +
                       (g.tma_store ? (size_t)g.groups * (g.nsw + g.mask_slots) * 4 * 4096 : 0) + kBarBlockBytes +
@@ -2838,7 +2890,7 @@ int conv_forward_small_c(int dtype, const void* x, const void* w, void* y, const
   g.tiles_w = ceil_div(p.out_cols, g.tw);
   g.tiles_h = ceil_div(p.out_rows, g.th);
   g.tiles_n = ceil_div(p.batch, g.tn);
-  g.bn = pick_bn((long long)g.tiles_w * g.tiles_h * g.tiles_n, p.features, epr, dtype == PDNN_F32 ? 128 : 256, sms);
+  g.bn = pick_bn(dtype, (long long)g.tiles_w * g.tiles_h * g.tiles_n, p.features, epr, dtype == PDNN_F32 ? 128 : 256, sms);
   g.n_tiles = ceil_div(p.features, g.bn);
   set_operand_layout(g, dtype, 1);
   // Narrow layout (16-bit, at most 4 channels, even column stride, halo mode): 4 channels per pixel,
@@ -2946,7 +2998,6 @@ __global__ void __launch_bounds__(256) split_lo_kernel(const float* x, float* __
 int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnConv2DParams& p,
                  const PdnnConvEpilogue* epi, cudaStream_t s, bool try_halo = true, bool try_cta_pair = true,
                  const ConvLd* ld = nullptr, GemmArgs* plan_out = nullptr, bool try_cluster = true) {
-  if (plan_out != nullptr && dtype == PDNN_F32) return PDNN_INVALID_PARAMETER;  // (the fp32 plan owns scratch)
   const int x_ld = ld != nullptr ? ld->x : 0, y_ld = ld != nullptr ? ld->y : 0;
   const uint64_t w_ld = ld != nullptr && ld->w > 0 ? (uint64_t)ld->w : (uint64_t)p.features;
   GemmArgs g;
@@ -3024,7 +3075,7 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   } else if (cluster != 0) {
     g.bn = kClusterColumns;
   } else {
-    g.bn = pick_bn(row_tiles, p.features, hwcf ? epr : 16, dtype == PDNN_F32 ? 128 : 256, sms, ksteps_all);
+    g.bn = pick_bn(dtype, row_tiles, p.features, hwcf ? epr : 16, dtype == PDNN_F32 ? 128 : 256, sms, ksteps_all);
     // A single tap with a long reduction into exactly 256 features: one 256-column tile per row tile
     // reads the input once instead of twice and runs as one double-buffered pipeline (measured 12%
     // faster than two 128-column pipelines on 14x14x1024 -> 256).
@@ -3072,23 +3123,6 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   g.num_taps = nt;
   g.cblocks = ceil_div(p.channels, epr);
   const uint64_t taps = (uint64_t)p.window_rows * p.window_cols;
-  // fp32 (3xTF32) with enough work to pay for one extra pass over the filter: the lo part of the filter
-  // is computed once, ahead of the GEMM, and arrives by TMA like the filter itself (whose words serve as
-  // the hi part); the kernel's split warps then only have the A tiles to split.
-  const size_t filter_elems = (size_t)taps * p.channels * p.features;
-  float* w_split = nullptr;
-  if (dtype == PDNN_F32 && (size_t)p.batch * p.out_rows * p.out_cols >= 2048 && aligned16(w) &&
-      (!hwcf || w_ld == (uint64_t)p.features)) {  // (a column slice of a wider filter is not one contiguous run)
-    if (cudaMallocAsync(reinterpret_cast<void**>(&w_split), filter_elems * sizeof(float), s) == cudaSuccess) {
-      launch_overlapped(split_lo_kernel, grid_for(filter_elems, 256, sms), 256, s, static_cast<const float*>(w), w_split,
-                        filter_elems);
-      count_launch();
-      g.b_presplit = 1;
-    } else {
-      cudaGetLastError();
-      w_split = nullptr;
-    }
-  }
   auto make_b_map = [&](CUtensorMap* map, const void* base) {
     if (hwcf && p.features % epr == 0) {
       // All 128-byte column blocks of the tile in one copy: the block index is a tensor dimension
@@ -3114,13 +3148,8 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
     const uint32_t box[4] = {(uint32_t)epr, 1, (uint32_t)g.bn, 1};
     return make_map(map, dtype, false, base, dims, st, box);
   };
-  const bool maps_ok = make_b_map(&g.b_map, w) && (w_split == nullptr || make_b_map(&g.b_map_lo, w_split));
-  if (!maps_ok) {
-    if (w_split != nullptr) cudaFreeAsync(w_split, s);
-    return PDNN_INVALID_PARAMETER;
-  }
+  if (!make_b_map(&g.b_map, w)) return PDNN_INVALID_PARAMETER;
   const int status = finish_forward(g, dtype, y, p, epi, s, y_ld, plan_out, cluster);
-  if (w_split != nullptr) cudaFreeAsync(w_split, s);
   if (status == kPlanAgain && cluster != 0) return conv_forward(dtype, x, w, y, p, epi, s, try_halo, try_cta_pair, ld, plan_out, false);
   if (status == kPlanAgain)  // first without the CTA pairs, then without halo / pair mode
     return g.cta_pair ? conv_forward(dtype, x, w, y, p, epi, s, try_halo, false, ld, plan_out, try_cluster)
@@ -3258,10 +3287,15 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
   const int sms = device_sm_count();
   const bool hwcf = p.filter_format == 0;
   const int epr = dtype == PDNN_F32 ? 32 : 64;
-  // fp32: the lo part of the filter computed ahead of the GEMMs, as in the forward pass
+  // fp32 (3xTF32) with enough work to pay for one extra pass over the filter: the lo part of the filter is computed
+  // once, ahead of the GEMMs, and arrives by TMA like the filter itself, whose words serve as the hi part.  The split
+  // warps then neither read nor write B: 16 of the 128 KB a step of 128 columns moves through shared memory (8 images,
+  // 56x56 256 -> 256 3x3: 121 -> 109 us, 28x28 512 -> 512 155 -> 139).  With 64 columns and fewer the bytes that pass
+  // from L2 count for more (224x224 64 -> 64: 153 -> 166 us), as they do in the forward pass, whose filter tiles lie
+  // across the reduction: 56x56 256 -> 256 122 us without and 144 with it, 28x28 512 -> 512 154 and 182.
   const size_t filter_elems = (size_t)p.window_rows * p.window_cols * p.channels * p.features;
   float* w_split = nullptr;
-  if (dtype == PDNN_F32 && (size_t)p.batch * p.in_rows * p.in_cols >= 2048 && aligned16(w) &&
+  if (dtype == PDNN_F32 && hwcf && p.channels > 64 && (size_t)p.batch * p.in_rows * p.in_cols >= 2048 && aligned16(w) &&
       cudaMallocAsync(reinterpret_cast<void**>(&w_split), filter_elems * sizeof(float), s) == cudaSuccess) {
     launch_overlapped(split_lo_kernel, grid_for(filter_elems, 256, sms), 256, s, static_cast<const float*>(w), w_split,
                       filter_elems);
@@ -3346,7 +3380,7 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
       } else if (cluster != 0) {
         g.bn = kClusterColumns;
       } else {
-        g.bn = pick_bn(row_tiles, p.channels, hwcf ? 16 : epr, 128, sms, ksteps_all);
+        g.bn = pick_bn(dtype, row_tiles, p.channels, hwcf ? 16 : epr, 128, sms, ksteps_all);
       }
       g.n_tiles = ceil_div(p.channels, g.bn);
       set_operand_layout(g, dtype, hwcf ? 0 : 1);
@@ -3404,8 +3438,6 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
         const uint64_t st[3] = {(uint64_t)p.channels * es, taps * p.channels * es, taps * p.channels * p.features * es};
         const uint32_t box[4] = {(uint32_t)epr, 1, (uint32_t)epr, 1};
         if (!make_map(&g.b_map, dtype, true, w, dims, st, box)) return PDNN_INVALID_PARAMETER;
-        if (w_split != nullptr && !make_map(&g.b_map_lo, dtype, true, w_split, dims, st, box))
-          return PDNN_INVALID_PARAMETER;
       }
       g.b_presplit = w_split != nullptr ? 1 : 0;
       set_epilogue(g, nullptr);
@@ -3521,7 +3553,7 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool
   f.n_tiles = ceil_div(p.features, f.bn);
   // At most 64 channels and several taps: a tile holds two taps, the second 64 accumulator rows being
   // the same channels as the next tap sees them, instead of rows that no channel uses.
-  f.tap_pack = (dtype != PDNN_F32 && p.channels <= 64 && p.window_rows * p.window_cols >= 2) ? 2 : 1;
+  f.tap_pack = (p.channels <= 64 && p.window_rows * p.window_cols >= 2) ? 2 : 1;
   const long long out_tiles = (long long)f.m_tiles * f.n_tiles * ceil_div(p.window_rows * p.window_cols, f.tap_pack);
   const long long total_slabs = (long long)f.slabs_w * f.slabs_h * f.slabs_n;
   long long want = std::max<long long>(1, (2ll * sms) / out_tiles);
@@ -3576,7 +3608,7 @@ SmallCFbpPlan plan_small_c_fbp(int dtype, const PdnnConv2DParams& p, int sms) {
   f.slabs_h = ceil_div(p.out_rows, f.th);
   f.slabs_n = ceil_div(p.batch, f.tn);
   f.m_tiles = 1;
-  f.tap_pack = (dtype != PDNN_F32 && p.window_rows >= 2) ? 2 : 1;  // 64 packed rows per filter row: two per tile
+  f.tap_pack = p.window_rows >= 2 ? 2 : 1;  // at most 64 packed rows per filter row: two per tile
   f.bn = std::min(dtype == PDNN_F32 ? 128 : 256, ceil_div(p.features, epr) * epr);
   f.n_tiles = ceil_div(p.features, f.bn);
   const long long out_tiles = (long long)f.n_tiles * ceil_div(p.window_rows, f.tap_pack);
@@ -4024,7 +4056,7 @@ int tc_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, void*
   const int cluster =
       (!tl && beta == 0.f && !out_f32) ? cluster_splits(dtype, (long long)m_tiles * batches, n, ceil_div(k, epr), sms) : 0;
   g.bn = cluster != 0 ? kClusterColumns
-                 : pick_bn((long long)m_tiles * batches, n, b_mn ? epr : 16, dtype == PDNN_F32 ? 128 : 256, sms, ceil_div(k, epr));
+                 : pick_bn(dtype, (long long)m_tiles * batches, n, b_mn ? epr : 16, dtype == PDNN_F32 ? 128 : 256, sms, ceil_div(k, epr));
   g.n_tiles = ceil_div(n, g.bn);
   set_operand_layout(g, dtype, b_mn);
   g.taps[0] = TapEntry{0, 0, 0, 0};
