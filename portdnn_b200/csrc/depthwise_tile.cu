@@ -1,4 +1,4 @@
-// Depthwise 3x3 filter gradient on tiles that TMA brings into shared memory.
+// Depthwise 3x3 convolutions, all three passes, on tiles that TMA brings into shared memory.
 #include "column_sums.cuh"
 #include "depthwise_tile.cuh"
 #include "tc_gemm.cuh"
@@ -23,6 +23,7 @@ struct Lanes {
   using V = unsigned long long;
   static __device__ __forceinline__ V zero() { return 0ull; }
   static __device__ __forceinline__ V unpack(unsigned w);
+  static __device__ __forceinline__ unsigned pack(V v);
   static __device__ __forceinline__ void fma(V& acc, V a, V b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
   static __device__ __forceinline__ float get(V v, int e) { return __uint_as_float(e ? (unsigned)(v >> 32) : (unsigned)v); }
 };
@@ -40,46 +41,62 @@ __device__ __forceinline__ unsigned long long Lanes<__nv_bfloat16>::unpack(unsig
   return v;
 }
 template <>
+__device__ __forceinline__ unsigned Lanes<__half>::pack(unsigned long long v) {
+  const __half2 h = __floats2half2_rn(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
+  return *reinterpret_cast<const unsigned*>(&h);
+}
+template <>
+__device__ __forceinline__ unsigned Lanes<__nv_bfloat16>::pack(unsigned long long v) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
+  return *reinterpret_cast<const unsigned*>(&h);
+}
+template <>
 struct Lanes<float> {
   static constexpr int E = 1;
   using V = float;
   static __device__ __forceinline__ V zero() { return 0.f; }
   static __device__ __forceinline__ V unpack(unsigned w) { return __uint_as_float(w); }
+  static __device__ __forceinline__ unsigned pack(V v) { return __float_as_uint(v); }
   static __device__ __forceinline__ void fma(V& acc, V a, V b) { acc = fmaf(a, b, acc); }
   static __device__ __forceinline__ float get(V v, int) { return v; }
 };
 
-constexpr int kTileThreads = 288;            // most threads that multiply; one warp more requests the tiles
-constexpr int kTileStages = 2;
-constexpr int kTileStageBytes = 54 * 1024;   // two blocks of two stages to an SM
+// One block to an SM.  Filter gradient, us, 128 images, f16, 56x56x144 / 112x112x32 / 28x28x192 / 7x7x960: two blocks of
+// two stages of 54 KB 67 / 47 / 22 / 16, one block of three of 72 KB 49 / 45 / 21 / 13, four of 54 KB 57 / 49 / 22 /
+// 13: larger tiles read fewer rows twice, and a block's stages are filled one after another, not in bursts.
+constexpr int kTileThreads = 512;            // most threads that multiply; one warp more requests the tiles
+constexpr int kTileStages = 3;
+constexpr int kTileStageBytes = 72 * 1024;
 constexpr unsigned kTileHead = 128;          // barriers and the abort flag
-template <int ST>
-struct TileCols { static constexpr int value = ST == 1 ? 8 : 4; };  // output columns of a tile
 
-struct FilterTiles {
+struct Tiles {
   int words, strips;       // 32-bit words of channels to a block, strips of two output rows
   int chunks, slices;      // blocks along the channels, blocks that share the tiles of a chunk
-  int tiles_w, tiles_h;
+  int tw, tiles_w, tiles_h;
   unsigned tiles;          // of one chunk: tiles_w * tiles_h * images
-  int channels, out_rows, out_cols, pad_rows, pad_cols;
+  int channels, in_rows, in_cols, out_rows, out_cols, pad_rows, pad_cols;
+  int mirrored;            // the filter's taps in reverse order (input gradient)
   unsigned x_bytes, dy_off, dy_bytes, stage_bytes;
   unsigned* error_record;
 };
 
 // dW[r][s][c] = sum of x[h * ST + r][w * ST + s][c] * dy[h][w][c].  What bounds the nine multiply-adds per word
-// is everything around them: loads, conversions and bounds checks.  Here a
-// warp of its own has TMA bring tiles of TW columns x 2 * strips rows with their halo, zeros outside the image, so
-// that the multiplying warps check nothing and only read shared memory; a thread owns a word of channels and
-// a strip of two output rows, walks the columns of the tile with a window of 3 columns x (ST + 3) rows in
-// registers, converts every word once, and multiplies two channels to an instruction.  Its 9 sums stay in
-// registers over all tiles of the block; the block's partial sums go to partial[slice][tap][channel].
-template <typename T, int ST>
-__global__ void __launch_bounds__(kTileThreads + 32, 2)
+// is everything around them: loads, conversions and bounds checks (56x56x144, 128 images, f16: 71 million warp
+// instructions with the rows in registers, 27 million here).  A warp of its own has TMA bring tiles of TW columns x
+// 2 * strips rows with their halo, zeros outside the image, so that the multiplying warps check nothing and only read
+// shared memory; a thread owns a word of channels and a strip of two output rows, walks the columns of the tile with
+// a window of 3 columns x (ST + 3) rows in registers, converts every word once, and multiplies two channels to an
+// instruction.  Its 9 sums stay in registers over all tiles of the block; the block's partial sums go to
+// partial[slice][tap][channel].  What is left is the bytes: 5.1 TB/s of the tensors, 5.6 with the halo.
+// us with the second stage, before / now, 128 images, f16: 56x56x144 86 / 45, 112x112x96 / 2 85 / 60, 112x112x32 69 / 45,
+// 14x14x384 20 / 13, 7x7x960 19 / 13.
+template <typename T, int ST, int TW>
+__global__ void __launch_bounds__(kTileThreads + 32, 1)
     depthwise_filter_tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap dy_map,
-                                 float* partial, const FilterTiles g) {
+                                 float* partial, const Tiles g) {
   using L = Lanes<T>;
   using V = typename L::V;
-  constexpr int E = L::E, TW = TileCols<ST>::value, XW = (TW - 1) * ST + 3, ROWS = ST + 3;
+  constexpr int E = L::E, XW = (TW - 1) * ST + 3, ROWS = ST + 3;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw), base = (raw + 127u) & ~127u;
   uint8_t* smem = smem_raw + (base - raw);
@@ -198,14 +215,141 @@ __global__ void __launch_bounds__(kTileThreads + 32, 2)
   }
 }
 
+// Forward pass, and the input gradient of stride 1 as the forward pass of dy with the filter mirrored and the padding
+// complemented, on the same tiles and walk: nine multiply-adds in fp32 to a pair of channels, one rounding.  Bound by
+// HBM; one thread to an output packet with nine loads of it, as these layers ran before, by the loads.  bf16, us, 128
+// images: 56x56x144 forward 184 -> 44, input gradient 285 -> 44; 112x112x96 / 2 forward 134 -> 64; 7x7x960 20 -> 8.5.
+// (fp16 and fp32 have the strip kernels with sums in the tensors' type, 45.6 us for 56x56x144; on these tiles fp16
+// measured between 13 % slower, 61x61x88, and 10 % faster, 14x14x576.)
+template <typename T, int ST, int TW>
+__global__ void __launch_bounds__(kTileThreads + 32, 1)
+    depthwise_forward_tile_kernel(const __grid_constant__ CUtensorMap x_map, const T* filter, T* out, const Tiles g) {
+  using L = Lanes<T>;
+  using V = typename L::V;
+  constexpr int E = L::E, XW = (TW - 1) * ST + 3, ROWS = ST + 3;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw), base = (raw + 127u) & ~127u;
+  uint8_t* smem = smem_raw + (base - raw);
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = (int)(threadIdx.x & 31);
+  const int workers = (int)(blockDim.x >> 5) - 1;
+  auto full_bar = [&](int s) { return base + 8u * (uint32_t)s; };
+  auto empty_bar = [&](int s) { return base + 8u * (uint32_t)(kTileStages + s); };
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 16 * kTileStages);
+  if (threadIdx.x < 2 * kTileStages) {
+    mbar_init(base + 8u * threadIdx.x, threadIdx.x < kTileStages ? 1u : (unsigned)workers);
+    if (threadIdx.x == 0) *abort_flag = 0;
+    fence_barrier_init();
+  }
+  __syncthreads();
+  overlap_wait();
+  const int chunk = (int)blockIdx.x % g.chunks, slice = (int)blockIdx.x / g.chunks;
+  const int words = g.words, strips = g.strips;
+  const int word = (int)threadIdx.x % words, strip = (int)threadIdx.x / words;
+  const int pixel_words = g.channels / E, channel_word = chunk * words + word;
+
+  int s = 0;
+  uint32_t ph = 0;
+  if (warp == workers) {
+    if (lane == 0) prefetch_tensormap(&x_map);
+#pragma unroll 1
+    for (unsigned tile = (unsigned)slice; tile < g.tiles; tile += (unsigned)g.slices) {
+      const int tw = (int)(tile % (unsigned)g.tiles_w);
+      const unsigned rest = tile / (unsigned)g.tiles_w;
+      const int w0 = tw * TW, h0 = (int)(rest % (unsigned)g.tiles_h) * 2 * strips, n = (int)(rest / (unsigned)g.tiles_h);
+      if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g.error_record, kWaitLimitNs, 0x1700u + (unsigned)s)) break;
+      warp_arrive_expect_tx(full_bar(s), g.x_bytes);
+      warp_tma_load_4d(base + kTileHead + (uint32_t)s * g.stage_bytes, &x_map, full_bar(s), chunk * words * E, w0 * ST - g.pad_cols,
+                       h0 * ST - g.pad_rows, n);
+      if (++s == kTileStages) {
+        s = 0;
+        ph ^= 1u;
+      }
+    }
+  } else {
+    const bool live = strip < strips && channel_word < pixel_words;
+    V f[9];
+    bool finite = true;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      f[t] = live ? L::unpack(reinterpret_cast<const unsigned*>(filter)[(g.mirrored ? 8 - t : t) * pixel_words + channel_word]) : L::zero();
+#pragma unroll
+      for (int e = 0; e < E; ++e) finite = finite && isfinite(L::get(f[t], e));
+    }
+    const int row = XW * words;
+    const size_t image_words = (size_t)g.out_rows * g.out_cols * pixel_words;
+#pragma unroll 1
+    for (unsigned tile = (unsigned)slice; tile < g.tiles; tile += (unsigned)g.slices) {
+      if (!mbar_wait(full_bar(s), ph, abort_flag, g.error_record, kWaitLimitNs, 0x1800u + (unsigned)s)) break;
+      const int tw = (int)(tile % (unsigned)g.tiles_w);
+      const unsigned rest = tile / (unsigned)g.tiles_w;
+      const int w0 = tw * TW, h0 = ((int)(rest % (unsigned)g.tiles_h) * strips + strip) * 2, n = (int)(rest / (unsigned)g.tiles_h);
+      if (live && h0 < g.out_rows) {
+        const unsigned* xp = reinterpret_cast<const unsigned*>(smem + kTileHead + (size_t)s * g.stage_bytes) + 2 * ST * strip * row + word;
+        unsigned* yp = reinterpret_cast<unsigned*>(out) + (size_t)n * image_words + ((size_t)h0 * g.out_cols + w0) * pixel_words + channel_word;
+        const int cols_left = g.out_cols - w0, y_row = g.out_cols * pixel_words;
+        const bool second = h0 + 1 < g.out_rows;
+        auto walk = [&](auto every_tap) {
+          V win[3][ROWS];  // column c of the tile in win[c % 3]
+#pragma unroll
+          for (int c = 0; c < 3 - ST; ++c)
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) win[c][r] = L::unpack(xp[r * row + c * words]);
+#pragma unroll
+          for (int j = 0; j < TW; ++j) {
+#pragma unroll
+            for (int c = j * ST + 3 - ST; c < j * ST + 3; ++c)
+#pragma unroll
+              for (int r = 0; r < ROWS; ++r) win[c % 3][r] = L::unpack(xp[r * row + c * words]);
+            if (j < cols_left) {
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                V acc = L::zero();
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+#pragma unroll
+                  for (int c = 0; c < 3; ++c) {
+                    // a tap outside the image is no term of the sum: the zero there and an infinite weight would be one
+                    if (!decltype(every_tap)::value) {
+                      const int ih = (h0 + k) * ST - g.pad_rows + r, iw = (w0 + j) * ST - g.pad_cols + c;
+                      if (ih < 0 || ih >= g.in_rows || iw < 0 || iw >= g.in_cols) continue;
+                    }
+                    L::fma(acc, win[(j * ST + c) % 3][k * ST + r], f[r * 3 + c]);
+                  }
+                if (k == 0 || second) yp[k * y_row + j * pixel_words] = L::pack(acc);
+              }
+            }
+          }
+        };
+        if (finite) walk(std::true_type{});
+        else walk(std::false_type{});
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty_bar(s));
+      if (++s == kTileStages) {
+        s = 0;
+        ph ^= 1u;
+      }
+    }
+  }
+  __syncthreads();
+  if (*abort_flag) {  // copies already requested may still be landing in shared memory
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) {
+    }
+  }
+}
+
 int up(int v, int to) { return (v + to - 1) / to * to; }
 
 // Words and strips of a block: the split of the channels into equal chunks (of whole 16-byte packets, for TMA) and
-// of the rows into equal tiles that leaves the fewest threads without work, with tiles of at most
-// kTileStageBytes.
-bool plan_filter_tiles(const PdnnDepthwiseConv2DParams& p, int elems, FilterTiles* out) {
-  const int total = p.channels / elems, row_pairs = (p.out_rows + 1) / 2, st = p.stride_rows;
-  const int tw = st == 1 ? TileCols<1>::value : TileCols<2>::value, xw = (tw - 1) * st + 3;
+// of the rows into equal tiles that takes the least time by the estimate below, with tiles of at most
+// kTileStageBytes.  p: the geometry as the walk sees it; filter_gradient: a stage holds a tile of dy, too.
+bool plan_tiles(const PdnnDepthwiseConv2DParams& p, int elems, bool filter_gradient, Tiles* out) {
+  const int sms = device_sm_count(), total = p.channels / elems, row_pairs = (p.out_rows + 1) / 2, st = p.stride_rows;
+  // 14 columns (the sizes of networks for 224 x 224 pixels are its multiples) or 8, whichever leaves less of the last
+  // tile empty; two columns of the window are read again for every tile.  56x56x144, 128 images: 44 and 49 us; 7x7x960: 19 and 13.
+  const int tw = st == 2 ? 4 : (p.out_cols + 13) / 14 * 16 < (p.out_cols + 7) / 8 * 10 ? 14 : 8;
+  const int xw = (tw - 1) * st + 3;
   double best = 1e30;
   for (int chunks = 1; chunks <= total / 4; ++chunks) {
     const int words = up((total + chunks - 1) / chunks, 4);
@@ -213,70 +357,118 @@ bool plan_filter_tiles(const PdnnDepthwiseConv2DParams& p, int elems, FilterTile
     if (words < 16 && chunks > 1) break;  // rows of less than 64 bytes: only where a pixel has no more
     auto bytes = [&](int strips) {
       const int x = up(((2 * strips - 1) * st + 3) * xw * words * 4, 128);
-      return up(x + 2 * strips * tw * words * 4, 128);
+      return filter_gradient ? up(x + 2 * strips * tw * words * 4, 128) : x;
     };
     int most = std::min(kTileThreads / words, row_pairs);
     while (most > 1 && (bytes(most) > kTileStageBytes || (2 * most - 1) * st + 3 > 256)) --most;
     if (most < 1 || bytes(most) > kTileStageBytes) continue;
-    const int tiles_h = (row_pairs + most - 1) / most, strips = (row_pairs + tiles_h - 1) / tiles_h;
-    // thread slots spent on a column of the image, and the rows above and below a tile that are read again
-    const double cost = (double)chunks * tiles_h * (up(words * strips, 32) + 32) * (1.0 + 0.1 / strips);
-    if (cost < best - 1e-9) {
-      best = cost;
-      out->words = words;
-      out->strips = strips;
-      out->chunks = chunks;
-      out->tiles_h = tiles_h;
-      out->x_bytes = (unsigned)(((2 * strips - 1) * st + 3) * xw * words * 4);
-      out->dy_bytes = (unsigned)(2 * strips * tw * words * 4);
-      out->dy_off = (unsigned)up((int)out->x_bytes, 128);
-      out->stage_bytes = (unsigned)bytes(strips);
+    const int slices = std::max(1, sms / chunks), least_h = (row_pairs + most - 1) / most;
+    for (int tiles_h = least_h; tiles_h <= std::min(8 * least_h, row_pairs); tiles_h *= 2) {
+      const int strips = (row_pairs + tiles_h - 1) / tiles_h;
+      const long long tiles = (long long)((p.out_cols + tw - 1) / tw) * tiles_h * p.batch;
+      // tiles one block after another works off, each its warps' instructions and what a tile costs besides (about six
+      // warps' worth: its barriers, the first reads), and the rows above and below a tile that are read again
+      const double rounds = tiles > 8ll * slices ? (double)tiles / slices : (double)((tiles + slices - 1) / slices);
+      // (rows of a box that are no multiple of 64 bytes share their memory sectors with the next chunk's block)
+      const double split_rows = chunks == 1 || words % 16 == 0 ? 1.0 : words % 8 == 0 ? 1.08 : 1.15;
+      const double cost = rounds * (up(words * strips, 32) / 32 + 6) * (1.0 + 0.1 / strips) * split_rows;
+      if (cost < best - 1e-9) {
+        best = cost;
+        out->words = words;
+        out->strips = strips;
+        out->chunks = chunks;
+        out->tiles_h = (row_pairs + strips - 1) / strips;
+        out->x_bytes = (unsigned)(((2 * strips - 1) * st + 3) * xw * words * 4);
+        out->dy_bytes = (unsigned)(2 * strips * tw * words * 4);
+        out->dy_off = (unsigned)up((int)out->x_bytes, 128);
+        out->stage_bytes = (unsigned)bytes(strips);
+      }
     }
   }
   if (best > 1e29) return false;
+  out->tw = tw;
   out->tiles_w = (p.out_cols + tw - 1) / tw;
   const unsigned long long tiles = (unsigned long long)out->tiles_w * out->tiles_h * p.batch;
   if (tiles > 0x3FFFFFFFull) return false;
   out->tiles = (unsigned)tiles;
   out->channels = p.channels;
+  out->in_rows = p.in_rows;
+  out->in_cols = p.in_cols;
   out->out_rows = p.out_rows;
   out->out_cols = p.out_cols;
   out->pad_rows = p.pad_rows;
   out->pad_cols = p.pad_cols;
+  out->mirrored = 0;
+  out->error_record = tc_error_record_address();
+  return out->error_record != nullptr;
+}
+
+bool tile_layer(const PdnnDepthwiseConv2DParams& p, int es) {
+  return p.window_rows == 3 && p.window_cols == 3 && p.channel_multiplier == 1 && p.stride_rows == p.stride_cols && p.stride_rows <= 2 &&
+         p.channels * es % 16 == 0;
+}
+
+bool x_tile_map(CUtensorMap* map, int dtype, const void* x, const PdnnDepthwiseConv2DParams& p, const Tiles& g, int elems) {
+  const int st = p.stride_rows;
+  const uint32_t box[4] = {(uint32_t)(g.words * elems), (uint32_t)((g.tw - 1) * st + 3), (uint32_t)((2 * g.strips - 1) * st + 3), 1};
+  return tc_dense_nhwc_map(map, dtype, x, p.batch, p.in_rows, p.in_cols, p.channels, box);
+}
+
+template <typename... Params>
+bool opt_in(void (*kernel)(Params...), std::mutex& mu, bool (&done)[kMaxDevices]) {
+  const int dev = current_device();
+  if (dev < 0 || dev >= kMaxDevices) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!done[dev]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 + kTileStages * kTileStageBytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    done[dev] = true;
+  }
   return true;
 }
 
-template <typename T, int ST>
-int launch_filter_tiles(const CUtensorMap& x_map, const CUtensorMap& dy_map, float* partial, const FilterTiles& g, cudaStream_t s) {
-  auto kernel = depthwise_filter_tile_kernel<T, ST>;
-  const size_t sums = (size_t)9 * g.words * g.strips * Lanes<T>::E * 4;
-  const size_t smem = 128 + kTileHead + std::max((size_t)kTileStages * g.stage_bytes, sums);
-  {
-    static std::mutex mu;
-    static bool opted_in[kMaxDevices] = {};
-    const int dev = current_device();
-    if (dev < 0 || dev >= kMaxDevices) return 0;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!opted_in[dev]) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 + kTileStages * kTileStageBytes) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-      }
-      opted_in[dev] = true;
-    }
-  }
+template <typename... Params, typename... Args>
+bool launch_tiles(void (*kernel)(Params...), const Tiles& g, size_t least_smem, cudaStream_t s, const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(g.slices * g.chunks));
   cfg.blockDim = dim3((unsigned)up(g.words * g.strips, 32) + 32);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = 128 + kTileHead + std::max((size_t)kTileStages * g.stage_bytes, least_smem);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, x_map, dy_map, partial, g);  // (the caller's check_launch() reads the error)
+  return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+
+template <typename T, int ST, int TW>
+int launch_filter_tiles(const CUtensorMap& x_map, const CUtensorMap& dy_map, float* partial, const Tiles& g, cudaStream_t s) {
+  static std::mutex mu;
+  static bool done[kMaxDevices] = {};
+  if (!opt_in(depthwise_filter_tile_kernel<T, ST, TW>, mu, done)) return 0;
+  const size_t sums = (size_t)9 * g.words * g.strips * Lanes<T>::E * 4;
+  launch_tiles(depthwise_filter_tile_kernel<T, ST, TW>, g, sums, s, x_map, dy_map, partial, g);  // (the caller's check_launch() reads the error)
   return g.slices;
+}
+
+template <typename T, int ST, int TW>
+bool launch_forward_tiles(const CUtensorMap& x_map, const void* filter, void* out, const Tiles& g, cudaStream_t s) {
+  static std::mutex mu;
+  static bool done[kMaxDevices] = {};
+  if (!opt_in(depthwise_forward_tile_kernel<T, ST, TW>, mu, done)) return false;
+  launch_tiles(depthwise_forward_tile_kernel<T, ST, TW>, g, 0, s, x_map, static_cast<const T*>(filter), static_cast<T*>(out), g);
+  return true;
+}
+
+// f(stride, columns) as integral constants
+template <typename F>
+auto with_tile_shape(int stride, int tw, F f) {
+  if (stride == 2) return f(std::integral_constant<int, 2>{}, std::integral_constant<int, 4>{});
+  if (tw == 14) return f(std::integral_constant<int, 1>{}, std::integral_constant<int, 14>{});
+  return f(std::integral_constant<int, 1>{}, std::integral_constant<int, 8>{});
 }
 
 }  // namespace
@@ -284,28 +476,36 @@ int launch_filter_tiles(const CUtensorMap& x_map, const CUtensorMap& dy_map, flo
 int launch_depthwise_filter_tiles(int dtype, const void* x, const void* dy, float* partial, const PdnnDepthwiseConv2DParams& p,
                                   int max_slices, cudaStream_t s) {
   const int es = (int)dtype_size(dtype), elems = 4 / es;
-  if (p.window_rows != 3 || p.window_cols != 3 || p.channel_multiplier != 1 || p.stride_rows != p.stride_cols || p.stride_rows > 2 ||
-      p.channels * es % 16 != 0 || !aligned16(x) || !aligned16(dy))
-    return 0;
-  FilterTiles g;
-  if (!plan_filter_tiles(p, elems, &g)) return 0;
-  g.error_record = tc_error_record_address();
-  if (g.error_record == nullptr) return 0;
-  const int st = p.stride_rows, tw = st == 1 ? TileCols<1>::value : TileCols<2>::value;
-  // two blocks to an SM, all channels of a tile side by side
-  g.slices = std::max(1, std::min<int>({max_slices, 2 * device_sm_count() / g.chunks, (int)std::min<unsigned>(g.tiles, 1u << 20)}));
-  const uint32_t x_box[4] = {(uint32_t)(g.words * elems), (uint32_t)((tw - 1) * st + 3), (uint32_t)((2 * g.strips - 1) * st + 3), 1};
-  const uint32_t dy_box[4] = {(uint32_t)(g.words * elems), (uint32_t)tw, (uint32_t)(2 * g.strips), 1};
+  Tiles g;
+  if (!tile_layer(p, es) || !aligned16(x) || !aligned16(dy) || !plan_tiles(p, elems, true, &g)) return 0;
+  // Few tiles leave all but a few SMs idle, which the kernel that spreads rows over warps does not (3 images, 7x7x960:
+  // 8.1 us on three tiles, 7.2 there; 4 images, 14x14x384, eight tiles: 6.6 and 8.3).
+  if (g.tiles < 8) return 0;
+  g.slices = std::max(1, std::min<int>({max_slices, device_sm_count() / g.chunks, (int)std::min<unsigned>(g.tiles, 1u << 20)}));
+  const uint32_t dy_box[4] = {(uint32_t)(g.words * elems), (uint32_t)g.tw, (uint32_t)(2 * g.strips), 1};
   CUtensorMap x_map, dy_map;
-  if (!tc_dense_nhwc_map(&x_map, dtype, x, p.batch, p.in_rows, p.in_cols, p.channels, x_box) ||
+  if (!x_tile_map(&x_map, dtype, x, p, g, elems) ||
       !tc_dense_nhwc_map(&dy_map, dtype, dy, p.batch, p.out_rows, p.out_cols, p.channels, dy_box))
     return 0;
-  if (dtype == PDNN_F32)
-    return st == 1 ? launch_filter_tiles<float, 1>(x_map, dy_map, partial, g, s) : launch_filter_tiles<float, 2>(x_map, dy_map, partial, g, s);
-  if (dtype == PDNN_F16)
-    return st == 1 ? launch_filter_tiles<__half, 1>(x_map, dy_map, partial, g, s) : launch_filter_tiles<__half, 2>(x_map, dy_map, partial, g, s);
-  return st == 1 ? launch_filter_tiles<__nv_bfloat16, 1>(x_map, dy_map, partial, g, s)
-                 : launch_filter_tiles<__nv_bfloat16, 2>(x_map, dy_map, partial, g, s);
+  return with_tile_shape(p.stride_rows, g.tw, [&](auto st, auto tw) {
+    constexpr int ST = decltype(st)::value, TW = decltype(tw)::value;
+    return dtype == PDNN_F32   ? launch_filter_tiles<float, ST, TW>(x_map, dy_map, partial, g, s)
+           : dtype == PDNN_F16 ? launch_filter_tiles<__half, ST, TW>(x_map, dy_map, partial, g, s)
+                               : launch_filter_tiles<__nv_bfloat16, ST, TW>(x_map, dy_map, partial, g, s);
+  });
+}
+
+bool launch_depthwise_forward_tiles_bf16(const void* x, const void* filter, void* out, const PdnnDepthwiseConv2DParams& p,
+                                         bool mirrored, cudaStream_t s) {
+  Tiles g;
+  if (!tile_layer(p, 2) || !aligned16(x) || !aligned16(filter) || !aligned16(out) || !plan_tiles(p, 2, false, &g)) return false;
+  g.mirrored = mirrored ? 1 : 0;
+  g.slices = std::max(1, std::min<int>(device_sm_count() / g.chunks, (int)std::min<unsigned>(g.tiles, 1u << 20)));
+  CUtensorMap x_map;
+  if (!x_tile_map(&x_map, PDNN_BF16, x, p, g, 2)) return false;
+  return with_tile_shape(p.stride_rows, g.tw, [&](auto st, auto tw) {
+    return launch_forward_tiles<__nv_bfloat16, decltype(st)::value, decltype(tw)::value>(x_map, filter, out, g, s);
+  });
 }
 
 }  // namespace pdnn

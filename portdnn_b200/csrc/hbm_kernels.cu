@@ -9,6 +9,7 @@
 // src/depthwise_conv2d/kernels.h, src/pointwise/kernels.h, src/binaryop/kernels.h.
 #include "column_sums.cuh"
 #include "common.cuh"
+#include "depthwise_tile.cuh"
 
 #include <cfloat>
 #include <mutex>
@@ -2027,6 +2028,9 @@ int launch_fbp_partials(bool vec, const T* in, const T* dy, float* partial, cons
                          int slices, cudaStream_t s) {
   constexpr int VN = Vec16<T>::N;
   const int V = vec ? VN : 1, F = p.channels * p.channel_multiplier;
+  if (const int tiled = launch_depthwise_filter_tiles(std::is_same<T, float>::value ? PDNN_F32 : std::is_same<T, __half>::value ? PDNN_F16 : PDNN_BF16,
+                                                      in, dy, partial, p, slices, s))
+    return tiled;
   const long long pixels = (long long)p.batch * p.out_rows * p.out_cols;
   const long long per_slice = (pixels + slices - 1) / slices;
   constexpr int E = 4 / (int)sizeof(T);
@@ -2125,6 +2129,17 @@ int launch_depthwise(int pass, int dtype, const void* in, const void* fil, void*
       }
       if (own) cudaFreeAsync(partial, s);
       return st;
+    }
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      if (pass == PDNN_FORWARD && launch_depthwise_forward_tiles_bf16(in, fil, out, p, false, s))
+        return check_launch("depthwise conv2d (3x3 tiles)");
+      if (pass == PDNN_INPUT_BACKPROP && p.window_rows == 3 && p.window_cols == 3 && p.stride_rows == 1 && p.stride_cols == 1 &&
+          p.pad_rows <= 2 && p.pad_cols <= 2) {
+        PdnnDepthwiseConv2DParams q = p;  // as below: dx[h][w] = sum dy[h + pad - r][w + pad - s] * w[r][s]
+        q.in_rows = p.out_rows, q.in_cols = p.out_cols, q.out_rows = p.in_rows, q.out_cols = p.in_cols;
+        q.pad_rows = 2 - p.pad_rows, q.pad_cols = 2 - p.pad_cols;
+        if (launch_depthwise_forward_tiles_bf16(in, fil, out, q, true, s)) return check_launch("depthwise input backprop (3x3 tiles)");
+      }
     }
     if constexpr (!std::is_same<T, __nv_bfloat16>::value) {
       if (pass == PDNN_FORWARD && vec && p.window_rows == 3 && p.window_cols == 3 && p.stride_rows == p.stride_cols &&

@@ -1987,9 +1987,11 @@ EncodeTiledFn encode_fn() {
 // 4-D tiled map with a 128-byte swizzle and zero fill outside the tensor.  dims[0] is the
 // contiguous dimension; strides_bytes[i] is the stride of dims[i+1].  A 32-bit operand that the
 // MMA reads MN-major must be swizzled in 32-byte units (the only MN-major layout tcgen05 accepts
-// for tf32); everything else uses the ordinary 16-byte-unit pattern.
+// for tf32); everything else uses the ordinary 16-byte-unit pattern.  `forced`: the swizzle of boxes that are not
+// 128 bytes wide.
+constexpr CUtensorMapSwizzle kDefaultSwizzle = (CUtensorMapSwizzle)-1;
 bool make_map(CUtensorMap* map, int dtype, bool mn_major, const void* base, const uint64_t dims[4],
-              const uint64_t strides_bytes[3], const uint32_t box[4], bool rows64 = false) {
+              const uint64_t strides_bytes[3], const uint32_t box[4], CUtensorMapSwizzle forced = kDefaultSwizzle) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) {
     fail(PDNN_ALLOCATION_PROBLEM, "cuTensorMapEncodeTiled is unavailable");
@@ -2005,8 +2007,7 @@ bool make_map(CUtensorMap* map, int dtype, bool mn_major, const void* base, cons
     b[i] = box[i];
   }
   for (int i = 0; i < 3; ++i) st[i] = strides_bytes[i];
-  // rows64: the box is 64 bytes wide and lands as 64-byte rows swizzled in 16-byte units
-  const CUtensorMapSwizzle sw = rows64 ? CU_TENSOR_MAP_SWIZZLE_64B
+  const CUtensorMapSwizzle sw = forced != kDefaultSwizzle ? forced
                                 : (dtype == PDNN_F32 && mn_major) ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
                                                                   : CU_TENSOR_MAP_SWIZZLE_128B;
   CUresult r = fn(map, dt, 4, const_cast<void*>(base), d, st, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
@@ -2920,7 +2921,7 @@ int conv_forward_small_c(int dtype, const void* x, const void* w, void* y, const
     // filter rows q, q + stride, ... read this parity class
     const int cnt = (p.window_rows - q + p.stride_rows - 1) / p.stride_rows;
     const uint32_t box[4] = {(uint32_t)krows, (uint32_t)g.tw, (uint32_t)(halo ? g.th + cnt - 1 : g.th), (uint32_t)g.tn};
-    if (!make_map(&g.a_map[q], dtype, false, xp + (size_t)q * row_pitch, dims, st, box, narrow)) {
+    if (!make_map(&g.a_map[q], dtype, false, xp + (size_t)q * row_pitch, dims, st, box, narrow ? CU_TENSOR_MAP_SWIZZLE_64B : kDefaultSwizzle)) {
       release();
       return -1;
     }
@@ -4173,6 +4174,30 @@ int simt_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, voi
 }
 
 const char* tc_last_kernel() { return t_last_kernel; }
+
+bool tc_dense_nhwc_map(CUtensorMap* map, int dtype, const void* base, int n, int h, int w, int c, const uint32_t box[4]) {
+  const uint64_t es = dtype_size(dtype);
+  const uint64_t dims[4] = {(uint64_t)c, (uint64_t)w, (uint64_t)h, (uint64_t)n};
+  const uint64_t st[3] = {c * es, (uint64_t)w * c * es, (uint64_t)h * w * c * es};
+  return make_map(map, dtype, false, base, dims, st, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
+unsigned* tc_error_record_address() {
+  static std::mutex mu;
+  static unsigned* address[kMaxDevices] = {};
+  const int dev = current_device();
+  if (dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (address[dev] == nullptr) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_error_record) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    address[dev] = static_cast<unsigned*>(p);
+  }
+  return address[dev];
+}
 
 int tc_read_error_record(unsigned out[4], int clear) {
   if (cudaMemcpyFromSymbol(out, g_error_record, sizeof(unsigned) * 4) != cudaSuccess) {

@@ -1,6 +1,8 @@
 // Interface of the tcgen05 implicit-GEMM engine (tc_gemm.cu).
 #pragma once
 
+#include <cuda.h>  // CUtensorMap
+
 #include "common.cuh"
 
 namespace pdnn {
@@ -40,6 +42,13 @@ int simt_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, voi
 
 // Name of the tensor-core kernel that the calling thread launched last ("" before the first).
 const char* tc_last_kernel();
+
+// Tensor map of a dense NHWC tensor whose box lands in shared memory as it is (no swizzle), zeros outside the tensor.
+// False, with the error text set, where it cannot be encoded.
+bool tc_dense_nhwc_map(CUtensorMap* map, int dtype, const void* base, int n, int h, int w, int c, const uint32_t box[4]);
+
+// Device address of the error record, for kernels outside this file that wait on barriers; nullptr on error.
+unsigned* tc_error_record_address();
 
 // Copies the device-side error record (4 words; word 0 == 0 means no error) to the host.
 // Synchronises the device.

@@ -1,0 +1,92 @@
+"""The depthwise 3x3 filter gradient on TMA tiles against the oracle: sizes around its tiles of 8 (stride 1) or 4
+(stride 2) columns and two rows to a strip, one and several chunks of channels, and values at the image's far edge
+that belong to no product."""
+import numpy as np
+import pytest
+import torch
+
+import portdnn_b200 as pd
+from gpu_util import assert_no_device_error, rounded, to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+
+# n, h, w, c, stride, same
+SHAPES = [
+    (1, 3, 3, 8, 1, False),      # one output
+    (9, 7, 7, 24, 1, True),      # odd rows: the last strip has one
+    (8, 8, 8, 40, 1, True),
+    (4, 9, 17, 144, 1, True),    # one column beyond two tiles
+    (5, 33, 16, 72, 1, False),
+    (8, 6, 7, 960, 1, True),     # several chunks
+    (4, 5, 5, 520, 2, True),     # the last chunk partly beyond the channels
+    (3, 15, 18, 32, 2, True),
+    (2, 64, 9, 16, 2, False),
+    (40, 14, 14, 64, 1, True),   # several tiles to a block
+]
+# Products of 16-bit values are exact in fp32; a sum of m terms in any order is off by at most m * 2^-24 of the sum of
+# magnitudes, the rounding of the result by 2^-11 or 2^-8 of its value.
+ULP = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8, "f32": 2.0 ** -24}
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_filter_gradient(orc, dtype, shape):
+    n, h, w, c, st, same = shape
+    rng = np.random.default_rng(3)
+    p, po = pd.depthwise_params(n, h, w, c, 1, 3, st, same), orc.depthwise_params(n, h, w, c, 1, 3, st, same)
+    x = rounded(rng.standard_normal(n * h * w * c).astype(np.float32), dtype)
+    dy = rounded(rng.standard_normal(n * p.out_rows * p.out_cols * c).astype(np.float32), dtype)
+    got = to_host(pd.depthwise_conv2d(pd.FILTER_BACKPROP, to_dev(x, dtype), to_dev(dy, dtype), p))
+    assert_no_device_error()
+    ref = orc.depthwise_conv2d(orc.FILTER_BACKPROP, x, dy, po)
+    size = orc.depthwise_conv2d(orc.FILTER_BACKPROP, np.abs(x), np.abs(dy), po)
+    terms = n * p.out_rows * p.out_cols
+    # (the oracle's own fp32 sums are off by as much again)
+    assert np.all(np.abs(got - ref) <= 2 * (terms + 1) * 2.0 ** -24 * size + ULP[dtype] * np.abs(ref) + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "f32"])
+def test_edge_values_stay_out_of_other_taps(dtype):
+    """VALID windows on 10 x 11 pixels: the last row and column are read by the last tap of each direction only."""
+    n, h, w, c = 16, 10, 11, 16
+    p = pd.depthwise_params(n, h, w, c, 1, 3, 1, False)
+    x = torch.zeros(n, h, w, c)
+    x[:, -1] = float("inf")
+    x[:, :, -1] = float("inf")
+    dy = torch.ones(n, p.out_rows, p.out_cols, c)
+    dw = pd.depthwise_conv2d(pd.FILTER_BACKPROP, to_dev(x.numpy().ravel(), dtype), to_dev(dy.numpy().ravel(), dtype), p)
+    dw = dw.float().cpu().view(3, 3, c)
+    assert_no_device_error()
+    assert torch.equal(dw[:2, :2], torch.zeros(2, 2, c))
+    assert torch.isinf(dw[2]).all() and torch.isinf(dw[:, 2]).all()
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_forward_and_input_gradient(orc, dtype, shape):
+    n, h, w, c, st, same = shape
+    rng = np.random.default_rng(4)
+    p, po = pd.depthwise_params(n, h, w, c, 1, 3, st, same), orc.depthwise_params(n, h, w, c, 1, 3, st, same)
+    x = rounded(rng.standard_normal(n * h * w * c).astype(np.float32), dtype)
+    f = rounded(rng.standard_normal(9 * c).astype(np.float32), dtype)
+    dy = rounded(rng.standard_normal(n * p.out_rows * p.out_cols * c).astype(np.float32), dtype)
+    y = to_host(pd.depthwise_conv2d(pd.FORWARD, to_dev(x, dtype), to_dev(f, dtype), p))
+    dx = to_host(pd.depthwise_conv2d(pd.INPUT_BACKPROP, to_dev(dy, dtype), to_dev(f, dtype), p))
+    assert_no_device_error()
+    # nine products: at most nine roundings of partial sums (fp16 kernels may hold them in fp16) and one of the result
+    for got, ref, size in ((y, orc.depthwise_conv2d(orc.FORWARD, x, f, po), orc.depthwise_conv2d(orc.FORWARD, np.abs(x), np.abs(f), po)),
+                           (dx, orc.depthwise_conv2d(orc.INPUT_BACKPROP, dy, f, po),
+                            orc.depthwise_conv2d(orc.INPUT_BACKPROP, np.abs(dy), np.abs(f), po))):
+        assert np.all(np.abs(got - ref) <= 10 * (2.0 ** -24 if dtype == "bf16" else ULP[dtype]) * size + ULP[dtype] * np.abs(ref) + 2.0 ** -24)
+
+
+def test_infinite_weight_meets_the_image_only():
+    """bf16: a tap outside the image is no term of the sum, whatever its weight."""
+    n, h, w, c = 1, 9, 10, 16
+    p = pd.depthwise_params(n, h, w, c, 1, 3, 1, True)
+    f = torch.zeros(3, 3, c)
+    f[0, 0] = float("inf")
+    y = pd.depthwise_conv2d(pd.FORWARD, to_dev(np.ones(n * h * w * c), "bf16"), to_dev(f.numpy().ravel(), "bf16"), p)
+    y = y.float().cpu().view(h, w, c)
+    assert torch.equal(y[0], torch.zeros(w, c)) and torch.equal(y[:, 0], torch.zeros(h, c))
+    assert torch.isinf(y[1:, 1:]).all()
