@@ -130,7 +130,7 @@ typedef struct PdnnConvEpilogue {
                           (programmatic dependent launch) and then waits for it before it touches a tensor;
                           with this flag it fetches the filter and the bias before that wait.  0 is always safe. */
   int any_order; /* non-zero: the order in which the products of an output are added may depend on the batch.  A
-                    single image then takes the kernel that splits a long sum among several SMs where a layer
+                    small batch then takes the kernel that splits a long sum among several SMs where a layer
                     has too few tiles for all of them.  0: one order for all batches, so that an image has the
                     same result, bit by bit, alone and beside others. */
 } PdnnConvEpilogue;

@@ -222,7 +222,7 @@ def conv2d(pass_, inp, fil, params, algorithm=ALGO_IM2COL, out=None, workspace=N
     constant_filter (Forward, InputBackprop): filter and bias were not written by the kernel that precedes this
     call in the stream, so the kernel may fetch them while that kernel is still finishing.
     any_order (Forward): the order in which the products of an output are added may depend on the batch, which
-    lets a single image take a faster kernel; without it an image's result is the same, bit by bit, alone and
+    lets a small batch take a faster kernel; without it an image's result is the same, bit by bit, alone and
     beside others."""
     return (_F or _front()).conv2d(pass_, inp, fil, params, algorithm, out, workspace, bias, activation, alpha, beta,
                                    relu_forward_output, output_f32, accumulate, relu_bitmask, constant_filter, any_order)

@@ -3032,12 +3032,13 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   g.tiles_n = ceil_div(p.batch, g.tn);
   const long long row_tiles = (long long)g.tiles_w * g.tiles_h * g.tiles_n;
   const int ksteps_all = p.window_rows * p.window_cols * ceil_div(p.channels, epr);
-  // One image, few tiles and a long reduction: clusters that share a tile's steps, if the caller leaves the order
-  // of the sums open.  All other plans add the terms of a sum in the same order, so that an image's result
+  // Few tiles and a long reduction: clusters that share a tile's steps, if the caller leaves the order of the sums open
+  // (f16, 3x3 512 -> 512 at 7x7, us: 2 images 27.8 -> 7.4, 8 images 28.1 -> 10.1; 256 -> 256 at 14x14: 16.3 -> 7.6 and
+  // 16.7 -> 9.6; 1x1 2048 -> 512 at 7x7, 8 images: 14.3 -> 7.5).  All other plans add the terms of a sum in the same order, so that an image's result
   // does not depend on how many others are in its batch (running the first layers in slices of the batch,
   // of one image or more, relies on it).
   const bool any_order = epi != nullptr && epi->any_order != 0;
-  const int cluster = (try_cluster && any_order && !halo && plan_out == nullptr && p.batch == 1)
+  const int cluster = (try_cluster && any_order && !halo && plan_out == nullptr)
                           ? cluster_splits(dtype, row_tiles, p.features, ksteps_all, sms) : 0;
   // Long reductions over filters too large to keep in shared memory are bound by the bytes that
   // pass through an SM's shared memory per MMA (the operand reads of the tensor core and the TMA
@@ -3083,6 +3084,12 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
     if (dtype != PDNN_F32 && !halo && p.window_rows * p.window_cols == 1 &&
         ksteps_all >= 16 && p.features == 256 && row_tiles >= 2 * sms)
       g.bn = 256;
+    // A long reduction into a little more than 128 or up to 256 features: one column tile reads the input once where two or
+    // three tiles of 64 and 128 columns read it again for columns that are partly not there.  From one row tile to an SM
+    // on (bf16, us, before / now): 7x45x61 100 -> 150 3x3 32.6 / 25.5, 128 -> 192 19.3 / 14.8; 20x20x25 200 -> 200 5x5
+    // 85.7 / 74.1.  Whole multiples of 128 gain nothing (16x28x28 256 -> 256 3x3 19.3, as one tile 20.1).
+    if (dtype != PDNN_F32 && !halo && ksteps_all >= 8 && p.features > 128 && p.features < 256 && row_tiles >= sms)
+      g.bn = ceil_div(p.features, 64) * 64;
     // One or two reduction steps over pixels narrower than 64 bytes (MobileNet-v2's 24 -> 144 expansions):
     // with two column tiles the input tile is fetched twice, and fetching such short rows is what the layer
     // spends its time on; one wide tile reads it once (measured 0.053 -> 0.035 ms on 56x56x24 -> 144; layers

@@ -127,7 +127,7 @@ class ConvStackRunner:
     same way on the host (tools/network.h)."""
 
     def __init__(self, layers, device, seed, training=False, dtype=None, chunk=None, chunk_layers=0,
-                 fuse_accumulate=True, bitmasks=True):
+                 fuse_accumulate=True, bitmasks=True, any_order=True):
         """bitmasks (training, 16-bit): every convolution with a ReLU also writes the sign bits of its output (one
         bit per element), and the input backprops read those instead of the output tensor for the ReLU mask.
         fuse_accumulate (training): a gradient with several contributions is summed (and masked) inside the
@@ -137,11 +137,13 @@ class ConvStackRunner:
         slices of ``chunk`` images - all those layers on images 0..chunk-1, then on the next slice, and so
         on - with their intermediate activations in slice-sized buffers that every slice reuses, so that a
         layer's output is still in the L2 cache when the next layer reads it.  Results are identical to
-        the layer-by-layer order: every operator of the path is independent per image."""
+        the layer-by-layer order of a runner with any_order=False: every operator of the path is independent per image.
+        any_order (forward): the sums of a small batch may be split among SMs, in an order that depends on the batch."""
         import torch
         from . import dist as pdist
         self.torch, self.layers, self.training, self.device = torch, layers, training, device
         self.fuse_accumulate = fuse_accumulate
+        self.any_order = any_order and not chunk  # (slices of a batch agree with the whole of it)
         self.use_bits = bool(bitmasks and training and self.dtype_is_16bit(dtype, torch))
         self.dtype = dtype or torch.float16
         self.code = api.F16 if self.dtype == torch.float16 else api.BF16 if self.dtype == torch.bfloat16 else api.F32
@@ -250,7 +252,7 @@ class ConvStackRunner:
                        bias=self.biases[i], activation=l.activation, workspace=self.workspaces.get(i),
                        relu_bitmask=self.bits.get(i) if self.training else None,
                        constant_filter=True,  # the weights are not written inside a step
-                       any_order=True)  # (a single image is a network of its own here: no slices of it to agree with)
+                       any_order=self.any_order)
         else:
             api.pooling(l.op, 0, self._in(i), p, out=self._out(i))
 

@@ -116,3 +116,39 @@ def test_matmul(batches, m, k, n, tr, dtype):
     out = pd.matmul(a.reshape(-1), bd.reshape(-1), batches, m, k, n, transpose_rhs=tr).view(batches, m, n)
     assert pd.last_gemm_kernel() == "umma_gemm_cluster_kernel"
     _check(out, a.double() @ b.double(), a.double().abs() @ b.double().abs(), dtype)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("batch", [2, 5])
+@pytest.mark.parametrize("shape", [(7, 7, 512, 512, 3, 1), (13, 11, 72, 40, 3, 1), (15, 17, 256, 200, 3, 2), (14, 14, 1024, 256, 1, 1)])
+def test_small_batches_in_any_order(shape, batch, dtype):
+    """Several images to a row tile, and a last row tile that is not full."""
+    h, w, c, k, win, st = shape
+    dt, g = TORCH_DTYPES[dtype], torch.Generator(device="cuda").manual_seed(h * c + k + batch)
+    p = pd.conv_params(batch, h, w, c, k, win, st)
+    x, wt = _rand(g, batch, h, w, c).to(dt), (_rand(g, win, win, c, k) / (win * win * c) ** 0.5).to(dt)
+    below, right = (max((o - 1) * st + win - s - pad, 0) for o, s, pad in ((p.out_rows, h, p.pad_rows), (p.out_cols, w, p.pad_cols)))
+    xp = torch.nn.functional.pad(x.double().permute(0, 3, 1, 2), (p.pad_cols, right, p.pad_rows, below))
+    w64 = wt.double().permute(3, 2, 0, 1)
+    ref = torch.nn.functional.conv2d(xp, w64, stride=st).permute(0, 2, 3, 1)
+    mag = torch.nn.functional.conv2d(xp.abs(), w64.abs(), stride=st).permute(0, 2, 3, 1)
+    y = pd.conv2d(pd.FORWARD, x.reshape(-1), wt.reshape(-1), p, any_order=True).view(ref.shape)
+    assert pd.last_gemm_kernel() == "umma_gemm_cluster_kernel"
+    _check(y, ref, mag, dtype)
+    assert_no_device_error()
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("shape", [(3, 90, 71, 64, 136, 3), (2, 100, 100, 520, 248, 1), (3, 80, 80, 72, 192, 3)])
+def test_one_wide_column_tile(shape, dtype):
+    """129 to 255 features and a row tile for every SM: one column tile of 192 or 256, its last columns not there."""
+    n, h, w, c, k, win = shape
+    dt, g = TORCH_DTYPES[dtype], torch.Generator(device="cuda").manual_seed(h * c + k)
+    p = pd.conv_params(n, h, w, c, k, win, 1)
+    x, wt = _rand(g, n, h, w, c).to(dt), (_rand(g, win, win, c, k) / (win * win * c) ** 0.5).to(dt)
+    w64 = wt.double().permute(3, 2, 0, 1)
+    xp = x.double().permute(0, 3, 1, 2)
+    ref = torch.nn.functional.conv2d(xp, w64, padding=win // 2).permute(0, 2, 3, 1)
+    mag = torch.nn.functional.conv2d(xp.abs(), w64.abs(), padding=win // 2).permute(0, 2, 3, 1)
+    _check(pd.conv2d(pd.FORWARD, x.reshape(-1), wt.reshape(-1), p).view(ref.shape), ref, mag, dtype)
+    assert_no_device_error()
