@@ -324,12 +324,32 @@ __device__ __forceinline__ void issue_slice_store(const GemmArgs& a, const TileC
   }
 }
 
-template <typename OutT>
-__device__ __forceinline__ void epilogue_tile_tma(const GemmArgs& a, const TileCoord& t, uint32_t tmem_acc, int lane,
+// (volatile, as ld_shared_v4 below: issued where it is written)
+__device__ __forceinline__ uint4 ld_global_v4(const void* ptr) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(ptr));
+  return v;
+}
+
+// Element offset of the lane's row of the tile in the output tensor (row = q32 + lane), or -1 if the row
+// lies outside the tensor.
+__device__ __forceinline__ long long row_element_offset(const GemmArgs& a, const TileCoord& t, int q32, int lane) {
+  const int sh_w = __ffs(a.etw) - 1, sh_h = __ffs(a.eth) - 1, row = q32 + lane;
+  const int w = t.w0 + (row & (a.etw - 1)), h = t.h0 + ((row >> sh_w) & (a.eth - 1)), n = t.n0 + (row >> (sh_w + sh_h));
+  if (!(w < a.ext_w && h < a.ext_h && n < a.ext_n)) return -1;
+  return (long long)n * a.stride_n + (long long)h * a.stride_h + (long long)w * a.stride_w;
+}
+
+// MASK (fp32): a.relu_mask, laid out like the output, zeroes the result wherever it is not positive - the ReLU gradient that
+// would otherwise be a pass of its own over dx (8 images of VGG-16 in training: 4243 -> 4160 us).  Its words take
+// the registers of the bias, which is never there beside it; both in one instantiation spilled.
+template <typename OutT, bool MASK = false>
+__device__ __forceinline__ void epilogue_tile_tma(const GemmArgs& a, const TileCoord& t, uint32_t tmem_acc, int q32, int lane,
                                                   bool zero, const WarpStore& ws, uint32_t& store_count) {
   constexpr int CPB = 128 / sizeof(OutT);  // columns per block
   constexpr int P = 16 / sizeof(OutT);     // columns per 16-byte chunk
   const OutT* bias = static_cast<const OutT*>(a.bias);
+  const long long mask_off = MASK ? row_element_offset(a, t, q32, lane) : -1;  // -1: a row that is not stored
   for (int c0 = 0; c0 < a.bn; c0 += CPB, ++store_count) {
     const uint32_t slot = store_count & (uint32_t)(ws.nsw - 1);
     wait_slice_free(ws, lane);
@@ -339,38 +359,54 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmArgs& a, const TileC
       const int colbase = t.nf0 + c0 + half * 32;
       uint32_t acc[32];
       if (!zero) tmem_ld_32x32(tmem_acc + (uint32_t)(c0 + half * 32), acc);
-      // all of the bias in flight beside the accumulators (columns beyond the last one are not stored)
-      float b[32];
-      if (bias != nullptr) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) b[i] = to_f32(bias[min(colbase + i, a.ext_cols - 1)]);
-      }
-      if (!zero) tmem_wait_ld();
-      float v[32];
+      for (int part = 0; part < 2; ++part) {  // 16 columns at a time: what is added or masks them is in flight together
+        const int col = colbase + 16 * part;
+        float b[16];
+        if constexpr (MASK) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = zero ? 0.f : a.alpha * __uint_as_float(acc[i]);
-      if (bias != nullptr) {
+          for (int g = 0; g < 4; ++g) {
+            uint4 m = make_uint4(0u, 0u, 0u, 0u);
+            if (mask_off >= 0 && col + 4 * g < a.ext_cols) m = ld_global_v4(static_cast<const float*>(a.relu_mask) + mask_off + col + 4 * g);
+            b[4 * g] = __uint_as_float(m.x), b[4 * g + 1] = __uint_as_float(m.y);
+            b[4 * g + 2] = __uint_as_float(m.z), b[4 * g + 3] = __uint_as_float(m.w);
+          }
+        } else if (bias != nullptr) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] += b[i];
-      }
-      if (a.act == PDNN_ACT_TANH) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = apply_activation(v[i], PDNN_ACT_TANH);
-      } else if (a.act != PDNN_ACT_NONE) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = apply_activation(v[i], PDNN_ACT_RELU);
-        if (a.act == PDNN_ACT_RELU6) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = fminf(v[i], 6.f);
+          for (int i = 0; i < 16; ++i) b[i] = to_f32(bias[min(col + i, a.ext_cols - 1)]);  // (columns beyond the last are not stored)
         }
-      }
+        if (part == 0 && !zero) tmem_wait_ld();
+        float v[16];
 #pragma unroll
-      for (int g = 0; g < 32 / P; ++g) {
-        Vec16<OutT> pk;
+        for (int i = 0; i < 16; ++i) v[i] = zero ? 0.f : a.alpha * __uint_as_float(acc[16 * part + i]);
+        if constexpr (MASK) {
 #pragma unroll
-        for (int i = 0; i < P; ++i) pk.set(i, from_f32<OutT>(v[g * P + i]));
-        const int chunk = half * (32 / P) + g;  // 0..7 within the 128-byte row
-        *reinterpret_cast<uint4*>(row_ptr + ((chunk ^ (lane & 7)) << 4)) = pk.raw;
+          for (int i = 0; i < 16; ++i) v[i] = b[i] > 0.f ? v[i] : 0.f;
+        } else {
+          if (bias != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += b[i];
+          }
+          if (a.act == PDNN_ACT_TANH) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = apply_activation(v[i], PDNN_ACT_TANH);
+          } else if (a.act != PDNN_ACT_NONE) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = apply_activation(v[i], PDNN_ACT_RELU);
+            if (a.act == PDNN_ACT_RELU6) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) v[i] = fminf(v[i], 6.f);
+            }
+          }
+        }
+#pragma unroll
+        for (int g = 0; g < 16 / P; ++g) {
+          Vec16<OutT> pk;
+#pragma unroll
+          for (int i = 0; i < P; ++i) pk.set(i, from_f32<OutT>(v[g * P + i]));
+          const int chunk = half * (32 / P) + part * (16 / P) + g;  // 0..7 within the 128-byte row
+          *reinterpret_cast<uint4*>(row_ptr + ((chunk ^ (lane & 7)) << 4)) = pk.raw;
+        }
       }
     }
     issue_slice_store(a, t, ws, slot, t.nf0 + c0, lane);
@@ -406,11 +442,6 @@ __device__ __forceinline__ P2 bits_pair(uint32_t v) {
 // loads of a column block are batched ahead of the wait for the accumulators, and their latencies
 // overlap instead of each load sitting directly in front of its first use (a lone warp stalls on
 // every one of them: eight round trips cost more than the arithmetic of the block).
-__device__ __forceinline__ uint4 ld_global_v4(const void* ptr) {
-  uint4 v;
-  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(ptr));
-  return v;
-}
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -458,15 +489,6 @@ __device__ __forceinline__ uint32_t fast_convert_store(const uint32_t (&acc)[32]
     *reinterpret_cast<uint4*>(row_ptr + (((chunk_base + g) ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
   }
   return bits;
-}
-
-// Element offset of the lane's row of the tile in the output tensor (row = q32 + lane), or -1 if the row
-// lies outside the tensor.
-__device__ __forceinline__ long long row_element_offset(const GemmArgs& a, const TileCoord& t, int q32, int lane) {
-  const int sh_w = __ffs(a.etw) - 1, sh_h = __ffs(a.eth) - 1, row = q32 + lane;
-  const int w = t.w0 + (row & (a.etw - 1)), h = t.h0 + ((row >> sh_w) & (a.eth - 1)), n = t.n0 + (row >> (sh_w + sh_h));
-  if (!(w < a.ext_w && h < a.ext_h && n < a.ext_n)) return -1;
-  return (long long)n * a.stride_n + (long long)h * a.stride_h + (long long)w * a.stride_w;
 }
 
 // 64 mask bits of a row -> keep masks of the eight 16-byte chunks (0xFFFF per kept halfword).
@@ -618,7 +640,8 @@ __device__ __forceinline__ bool epilogue_tile_tma_fast(const GemmArgs& a, const 
 // EPI selects the epilogue compiled into the instantiation: 0 = direct stores from registers,
 // 1 = staged TMA store with fp32 arithmetic, 2 = staged TMA store with packed 16-bit arithmetic,
 // 3 = as 2 with the ReLU-gradient mask (GemmArgs::relu_mask), 4 = as 2 writing the sign bits of the
-// result (GemmArgs::bitmask_out), 5 = as 3 with the mask as one bit per element (GemmArgs::mask_bits).
+// result (GemmArgs::bitmask_out), 5 = as 3 with the mask as one bit per element (GemmArgs::mask_bits), 6 (fp32) = as 1
+// with the ReLU-gradient mask.
 // One epilogue per instantiation keeps each kernel's register allocation tight.
 //
 // A CTA runs up to two independent pipelines ("groups") side by side, each with its own TMA
@@ -695,7 +718,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
   // indexing by absolute column still works
   const int bias_col0 = a.bias_tile_only ? (cta % a.n_tiles) * a.bn : 0;
   const uint32_t bias_s =
-      (EPI >= 2 && a.bias != nullptr) ? bar_base + kBarBlockBytes - (uint32_t)bias_col0 * 2u : 0u;
+      (EPI >= 2 && EPI != 6 && a.bias != nullptr) ? bar_base + kBarBlockBytes - (uint32_t)bias_col0 * 2u : 0u;
 
   // One barrier per thread (a single thread initialising all of them costs about a microsecond of
   // every launch): full, empty and ready per stage, accumulator full / empty per buffer, per group.
@@ -768,7 +791,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
       }
   };
   auto copy_bias = [&] {
-    if (EPI >= 2 && a.bias != nullptr) {
+    if (EPI >= 2 && EPI != 6 && a.bias != nullptr) {
       // the CTA's copy of the bias vector, zero beyond the last column
       const OutT* bias = static_cast<const OutT*>(a.bias);
       uint4* dst = reinterpret_cast<uint4*>(bar_mem + kBarBlockBytes);
@@ -1155,12 +1178,12 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
       tc_fence_after_sync();
       const uint32_t tmem_acc = grp_tmem + ((uint32_t)(q * 32) << 16) + buf * acc_stride;
       const bool zero = !(t.ks_end > t.ks_begin);
-      if constexpr (EPI >= 2) {
+      if constexpr (EPI >= 2 && EPI != 6) {
         if (!epilogue_tile_tma_fast<OutT, EPI == 3 || EPI == 5, EPI == 4, EPI == 5>(a, t, tmem_acc, lane, zero, ws, store_count, bias_s, q * 32, mask_slot,
                                                     abort_flag))
           break;
-      } else if constexpr (EPI == 1) {
-        epilogue_tile_tma<OutT>(a, t, tmem_acc, lane, zero, ws, store_count);
+      } else if constexpr (EPI == 1 || EPI == 6) {
+        epilogue_tile_tma<OutT, EPI == 6>(a, t, tmem_acc, q * 32, lane, zero, ws, store_count);
       } else {
         epilogue_tile<OutT>(a, t, tmem_acc, row, zero);
       }
@@ -1688,7 +1711,7 @@ __global__ void __launch_bounds__(192, 1) umma_gemm_filter_pair_kernel(const __g
       const TileCoord t = coord();
       if (!mbar_wait(acc_full_bar((int)buf), aph, abort_flag, g_error_record, a.wait_limit_ns, 0x1400u + buf)) break;
       tc_fence_after_sync();
-      epilogue_tile_tma<float>(a, t, tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256u, lane, false, ws, store_count);
+      epilogue_tile_tma<float>(a, t, tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256u, q * 32, lane, false, ws, store_count);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty_bar((int)buf) & kPeerBitMask);  // rank 0 collects both CTAs
@@ -2187,8 +2210,10 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
   g.tmem_cols = split ? 512 : next_pow2(g.groups * g.acc_bufs * g.acc_stride);  // (split: the rest holds A tiles)
   g.bias_smem_bytes = 0;
   g.bias_tile_only = 0;
-  if (!g.epi_fast) g.relu_mask = nullptr;  // only the fast epilogue applies the mask; the caller checks
-  g.mask_smem_bytes = g.relu_mask != nullptr ? 128 : 0;  // the mask slots' barriers; the slots count as staging
+  // only the fast epilogue and the staged fp32 one apply the mask; the caller checks
+  if (!g.epi_fast && !(g.tma_store && compute_dtype == PDNN_F32)) g.relu_mask = nullptr;
+  const bool mask_tma = g.epi_fast && g.relu_mask != nullptr;
+  g.mask_smem_bytes = mask_tma ? 128 : 0;  // the mask slots' barriers; the slots count as staging
   if (g.pair && !g.cta_pair && (split || g.groups != 2 || !g.tma_store)) return false;  // the caller plans again without pairing
   if (g.epi_fast && g.bias != nullptr) {
     const int padded = ceil_div(g.n_tiles * g.bn, 64) * 64;
@@ -2208,7 +2233,7 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
   g.b_res = 0;
   g.b_res_bytes = 0;
   const int fixed = 1024 + kBarBlockBytes + g.bias_smem_bytes + g.mask_smem_bytes;
-  g.mask_slots = (g.relu_mask != nullptr && g.mask_bits == nullptr) ? 1 : 0;
+  g.mask_slots = (mask_tma && g.mask_bits == nullptr) ? 1 : 0;
   auto staging = [&](int nsw) { return g.tma_store ? g.groups * 4 * (nsw + g.mask_slots) * 4096 : 0; };
   // A small filter (all taps, all column tiles) is kept in shared memory for the whole kernel:
   // the filter tiles are the part of the L2 -> SM traffic that never changes.
@@ -2286,7 +2311,8 @@ using GemmKernelMulti = void (*)(const GemmArgsMulti);
 GemmKernel select_kernel(bool split, int epi, int out_dtype) {
   if (split) {
     if (out_dtype != PDNN_F32) return nullptr;
-    return epi == 1 ? umma_gemm_kernel<true, 1, float> : epi == 0 ? umma_gemm_kernel<true, 0, float> : nullptr;
+    return epi == 6 ? umma_gemm_kernel<true, 6, float> : epi == 1 ? umma_gemm_kernel<true, 1, float>
+           : epi == 0 ? umma_gemm_kernel<true, 0, float> : nullptr;
   }
   switch (out_dtype) {
     case PDNN_F16:
@@ -2407,7 +2433,7 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
     std::lock_guard<std::mutex> lock(mu);
     if (!opted_in[dev]) {
       for (int sp = 0; sp < 2; ++sp)
-        for (int epi = 0; epi < 6; ++epi)
+        for (int epi = 0; epi < 7; ++epi)
           for (int dt = 0; dt < 3; ++dt) {
             GemmKernel k = select_kernel(sp != 0, epi, dt);
             if (k != nullptr && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) != cudaSuccess) {
@@ -2425,7 +2451,7 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
     }
   }
   const int epi = g.epi_fast ? (g.mask_bits != nullptr ? 5 : g.relu_mask != nullptr ? 3 : g.bitmask_out != nullptr ? 4 : 2)
-                             : (g.tma_store ? 1 : 0);
+                             : (g.tma_store ? (g.relu_mask != nullptr ? 6 : 1) : 0);
   GemmKernel kernel = g.group_k != 0 ? select_grouped_kernel(epi, g.out_dtype) : select_kernel(split, epi, g.out_dtype);
   if (kernel == nullptr) return fail(PDNN_INVALID_PARAMETER, "tensor-core gemm: no kernel for this output type");
   const int sms = device_sm_count();
@@ -2473,7 +2499,7 @@ GemmKernelMulti select_multi_kernel(int epi, int out_dtype) {
 
 int gemm_epilogue_kind(const GemmArgs& g) {
   return g.epi_fast ? (g.mask_bits != nullptr ? 5 : g.relu_mask != nullptr ? 3 : g.bitmask_out != nullptr ? 4 : 2)
-                    : (g.tma_store ? 1 : 0);
+                    : (g.tma_store ? (g.relu_mask != nullptr ? 6 : 1) : 0);
 }
 
 size_t gemm_smem_bytes(const GemmArgs& g, bool split) {

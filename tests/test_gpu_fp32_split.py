@@ -3,6 +3,7 @@ the tiles (channel boxes of 32, two filter taps to a tile, column tiles of 64 an
 the kernel and inside it) and the fp32 epilogue's bias and activations beside the last column."""
 import numpy as np
 import pytest
+import torch
 
 import portdnn_b200 as pd
 from conftest import rel_err
@@ -55,3 +56,18 @@ def test_backprops(orc, shape):
     dx = to_host(pd.conv2d(pd.INPUT_BACKPROP, to_dev(dy, "f32"), to_dev(wt, "f32"), p))
     assert rel_err(dx, orc.conv2d(orc.INPUT_BACKPROP, dy, wt, po)) <= TOL["f32"]
     assert_no_device_error()
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_relu_gradient_in_the_epilogue(shape):
+    """The masked input gradient is the unmasked one with zeros wherever the forward output is not positive."""
+    n, h, w, c, k, win, st = shape
+    rng = np.random.default_rng(5)
+    p = pd.conv_params(n, h, w, c, k, win, st)
+    fwd = to_dev(rng.standard_normal(n * h * w * c).astype(np.float32), "f32")
+    wt = to_dev(rng.standard_normal(win * win * c * k).astype(np.float32), "f32")
+    dy = to_dev(rng.standard_normal(n * p.out_rows * p.out_cols * k).astype(np.float32), "f32")
+    plain = pd.conv2d(pd.INPUT_BACKPROP, dy, wt, p)
+    masked = pd.conv2d(pd.INPUT_BACKPROP, dy, wt, p, relu_forward_output=fwd)
+    assert_no_device_error()
+    assert torch.equal(masked, torch.where(fwd > 0, plain, torch.zeros_like(plain)))
