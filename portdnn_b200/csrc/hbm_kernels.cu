@@ -78,19 +78,30 @@ __global__ void __launch_bounds__(kBlock) pool_forward_kernel(const T* x, T* __r
 #pragma unroll
     for (int i = 0; i < V; ++i) acc[i] = (OP == PDNN_POOL_AVERAGE) ? 0.f : lowest_of<T>();
     const T* xn = x + (size_t)n * p.in_rows * p.in_cols * p.channels + (size_t)cv * V;
-    for (int r = r0; r < r1; ++r) {
-      for (int c = c0; c < c1; ++c) {
-        float v[V];
-        load_vec<T, V>(xn + ((size_t)r * p.in_cols + c) * p.channels, v);
+    auto take = [&](const float (&v)[V]) {
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          if (OP == PDNN_POOL_MAX) {
-            if (v[i] > acc[i]) acc[i] = v[i];
-          } else if (OP == PDNN_POOL_MAX_WITH_NAN) {
-            if (isnan(v[i]) || v[i] > acc[i]) acc[i] = v[i];
-          } else {
-            acc[i] += v[i];
-          }
+      for (int i = 0; i < V; ++i) {
+        if (OP == PDNN_POOL_MAX) {
+          if (v[i] > acc[i]) acc[i] = v[i];
+        } else if (OP == PDNN_POOL_MAX_WITH_NAN) {
+          if (isnan(v[i]) || v[i] > acc[i]) acc[i] = v[i];
+        } else {
+          acc[i] += v[i];
+        }
+      }
+    };
+    if (r1 - r0 == 2 && c1 - c0 == 2) {  // four packets requested together; the loops below wait for each in turn
+      float v[4][V];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) load_vec<T, V>(xn + ((size_t)(r0 + (k >> 1)) * p.in_cols + c0 + (k & 1)) * p.channels, v[k]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) take(v[k]);
+    } else {
+      for (int r = r0; r < r1; ++r) {
+        for (int c = c0; c < c1; ++c) {
+          float v[V];
+          load_vec<T, V>(xn + ((size_t)r * p.in_cols + c) * p.channels, v);
+          take(v);
         }
       }
     }
