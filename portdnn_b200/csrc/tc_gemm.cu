@@ -3125,8 +3125,9 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
     // A long reduction into a little more than 128 or up to 256 features: one column tile reads the input once where two or
     // three tiles of 64 and 128 columns read it again for columns that are partly not there.  From one row tile to an SM
     // on (bf16, us, before / now): 7x45x61 100 -> 150 3x3 32.6 / 25.5, 128 -> 192 19.3 / 14.8; 20x20x25 200 -> 200 5x5
-    // 85.7 / 74.1.  Whole multiples of 128 gain nothing (16x28x28 256 -> 256 3x3 19.3, as one tile 20.1).
-    if (dtype != PDNN_F32 && !halo && ksteps_all >= 8 && p.features > 128 && p.features < 256 && row_tiles >= sms)
+    // 85.7 / 74.1.  Whole multiples of 128 gain nothing (16x28x28 256 -> 256 3x3 19.3, as one tile 20.1), nor do pixels of
+    // 16 channels, which cost little to read again (39x59x62 16 -> 136 3x3 / 2: 18.5, as one tile 20.5).
+    if (dtype != PDNN_F32 && !halo && ksteps_all >= 8 && p.channels >= 32 && p.features > 128 && p.features < 256 && row_tiles >= sms)
       g.bn = ceil_div(p.features, 64) * 64;
     // One or two reduction steps over pixels narrower than 64 bytes (MobileNet-v2's 24 -> 144 expansions):
     // with two column tiles the input tile is fetched twice, and fetching such short rows is what the layer
