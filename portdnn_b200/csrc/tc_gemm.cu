@@ -3597,12 +3597,17 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool
   // 128-column tiles: two accumulator buffers per pipeline, so the fp32 epilogue of one tile overlaps the
   // reduction of the next (measured over the ResNet-50 layers: 9% less time than 256-column tiles)
   f.bn = std::min(std::min(max_bn, 128), ceil_div(p.features, epr) * epr);
-  f.n_tiles = ceil_div(p.features, f.bn);
   // At most 64 channels and several taps: a tile holds two taps, the second 64 accumulator rows being
   // the same channels as the next tap sees them, instead of rows that no channel uses.
   f.tap_pack = (p.channels <= 64 && p.window_rows * p.window_cols >= 2) ? 2 : 1;
-  const long long out_tiles = (long long)f.m_tiles * f.n_tiles * ceil_div(p.window_rows * p.window_cols, f.tap_pack);
+  const long long units = (long long)f.m_tiles * ceil_div(p.window_rows * p.window_cols, f.tap_pack);
   const long long total_slabs = (long long)f.slabs_w * f.slabs_h * f.slabs_n;
+  // 129 to 192 features: one column tile reads x once where two of 128 read it for columns that are partly not there,
+  // if there are steps enough (17 to an SM) to pay for its single accumulator buffer (bf16, us, before / now: 7x45x61
+  // 104 -> 152 3x3 37.0 / 30.1, 18x50x61 96 -> 176 5x5 / 2 35.9 / 27.1; 12 to an SM: 7x21x43 224 -> 184 3x3 20.5 / 21.8).
+  if (dtype != PDNN_F32 && p.features > 128 && p.features <= 192 && units * total_slabs >= 17ll * sms) f.bn = 192;
+  f.n_tiles = ceil_div(p.features, f.bn);
+  const long long out_tiles = units * f.n_tiles;
   long long want = std::max<long long>(1, (2ll * sms) / out_tiles);
   want = std::min<long long>(want, std::max<long long>(1, total_slabs / 8));  // at least 8 slabs per split
   want = std::min<long long>(want, 512);
