@@ -19,6 +19,7 @@
 // Warp roles of a pipeline: warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-5 epilogue;
 // with the split warps 6-13 hi/lo.
 #include "column_sums.cuh"
+#include "split_ring.cuh"
 #include "tc_gemm.cuh"
 #include "umma.cuh"
 
@@ -37,7 +38,7 @@ constexpr int kMaxTaps = 64;
 constexpr int kTileM = 128;
 constexpr int kABytes = kTileM * 128;  // one A stage: 128 rows of 128 bytes
 constexpr int kMaxStages = 8;
-constexpr int kSplitThreads = 448;       // fp32 variant: producer, issuer, four epilogue and eight split warps
+constexpr int kSplitThreads = (6 + 4 * kSplitTeams) * 32;  // fp32 variant: producer, issuer, four epilogue and eight split warps
 constexpr uint32_t kSplitAColumns = 64;  // fp32 variant: tensor-memory columns of a stage's A tile, hi and lo
 constexpr int kSmemBudget = 227 * 1024;
 constexpr int kBarsPerGroup = 3 * kMaxStages + 4;  // full, empty, ready per stage; accumulator full / empty x 2
@@ -1204,7 +1205,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     // touching shared memory; rows that lie along the reduction in shared memory (A MN-major) are transposed by
     // the way they are read.  The landed B serves as its own hi part; its lo part, where it did not arrive by
     // TMA, is written behind it (element positions do not change, so the swizzle is irrelevant there).
-    // Two teams of four warps take every second stage each.
+    // Two teams of four warps take every second stage each (split_ring.cuh).
     // What bounds the kernel is shared memory, 128 bytes a cycle: per step of 32 and 128 columns TMA writes 32 KB, A is
     // read once (16), B read and its lo part written (32), and the three products read 48 KB of B - 128 KB, 1000
     // cycles, for 768 cycles of math, and 0.53 us are measured.  With both parts of A in shared memory the products
@@ -1214,7 +1215,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     const int row = q * 32 + lane, tid = threadIdx.x - (6 + 4 * team) * 32;
     const int chunks = a.b_presplit ? 0 : (int)(b_bytes >> 4);
     const uint32_t a_tmem = tmem_base + ((uint32_t)(q * 32) << 16) + acc_bufs * acc_stride;
-    int s = 0, turn = 0;
+    int s = 0;
     uint32_t ph = 0;
     bool ok = true;
     TileWalker walker;
@@ -1223,8 +1224,8 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
       const TileCoord t = walker.coord(a);
 #pragma unroll 1
-      for (int ks = t.ks_begin; ks < t.ks_end; ++ks, turn ^= 1) {
-        if (turn == team) {
+      for (int ks = t.ks_begin; ks < t.ks_end; ++ks) {
+        if (split_team_of_stage(s) == team) {
           if (!mbar_wait(full_bar(s), ph, abort_flag, g_error_record, a.wait_limit_ns, 0x500u + (unsigned)s)) {
             ok = false;
             break;

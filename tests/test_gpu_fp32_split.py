@@ -22,6 +22,11 @@ SHAPES = [
     (2, 40, 40, 68, 64, 1, 1),    # ... and 68: ahead of it
     (3, 56, 56, 128, 128, 3, 1),  # several tiles to a CTA
     (4, 16, 16, 3, 64, 3, 1),     # packed few-channel form, filter rows two to a tile
+    # column tiles of 16 and 32: rings of seven stages
+    (2, 20, 20, 128, 16, 3, 1),   # one tile of 36 steps
+    (8, 64, 64, 96, 24, 3, 1),    # forward: two tiles to a CTA; filter gradient: 1024 steps
+    (8, 64, 64, 24, 96, 3, 1),    # input gradient: two tiles to a CTA
+    (3, 65, 63, 128, 32, 1, 1),
 ]
 
 
