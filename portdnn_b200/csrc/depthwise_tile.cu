@@ -25,6 +25,7 @@ struct Lanes {
   static __device__ __forceinline__ V unpack(unsigned w);
   static __device__ __forceinline__ unsigned pack(V v);
   static __device__ __forceinline__ void fma(V& acc, V a, V b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+  static __device__ __forceinline__ void add(V& acc, V a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
   static __device__ __forceinline__ float get(V v, int e) { return __uint_as_float(e ? (unsigned)(v >> 32) : (unsigned)v); }
 };
 template <>
@@ -58,6 +59,7 @@ struct Lanes<float> {
   static __device__ __forceinline__ V unpack(unsigned w) { return __uint_as_float(w); }
   static __device__ __forceinline__ unsigned pack(V v) { return __float_as_uint(v); }
   static __device__ __forceinline__ void fma(V& acc, V a, V b) { acc = fmaf(a, b, acc); }
+  static __device__ __forceinline__ void add(V& acc, V a) { acc += a; }
   static __device__ __forceinline__ float get(V v, int) { return v; }
 };
 
@@ -86,8 +88,9 @@ struct Tiles {
 // 2 * strips rows with their halo, zeros outside the image, so that the multiplying warps check nothing and only read
 // shared memory; a thread owns a word of channels and a strip of two output rows, walks the columns of the tile with
 // a window of 3 columns x (ST + 3) rows in registers, converts every word once, and multiplies two channels to an
-// instruction.  Its 9 sums stay in registers over all tiles of the block; the block's partial sums go to
-// partial[slice][tap][channel].  What is left is the bytes: 5.1 TB/s of the tensors, 5.6 with the halo.
+// instruction.  Its 9 sums are taken tile by tile and added up in registers over the tiles of the block (one chain of up
+// to 1800 products had four times the error: 56x56x144, 128 images, fp32, products of random sign, 7.5e-7 -> 1.9e-7 of the
+// root of the number of terms, at the same time); the block's partial sums go to partial[slice][tap][channel].  What is left is the bytes: 5.1 TB/s of the tensors, 5.6 with the halo.
 // us with the second stage, before / now, 128 images, f16: 56x56x144 86 / 45, 112x112x96 / 2 85 / 60, 112x112x32 69 / 45,
 // 14x14x384 20 / 13, 7x7x960 19 / 13.
 template <typename T, int ST, int TW>
@@ -153,6 +156,9 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
         const unsigned* dp = reinterpret_cast<const unsigned*>(at + g.dy_off) + 2 * strip * TW * words + word;
         const int tw = (int)(tile % (unsigned)g.tiles_w), th = (int)(tile / (unsigned)g.tiles_w % (unsigned)g.tiles_h);
         const int cols_left = g.out_cols - tw * TW, rows_left = g.out_rows - 2 * (th * strips + strip);
+        V sum[9];  // of this tile
+#pragma unroll
+        for (int t = 0; t < 9; ++t) sum[t] = L::zero();
         auto walk = [&](auto whole) {
           V win[3][ROWS];  // column c of the tile in win[c % 3]
 #pragma unroll
@@ -174,12 +180,14 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
 #pragma unroll
               for (int r = 0; r < 3; ++r)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) L::fma(acc[r * 3 + c], win[(j * ST + c) % 3][k * ST + r], d);
+                for (int c = 0; c < 3; ++c) L::fma(sum[r * 3 + c], win[(j * ST + c) % 3][k * ST + r], d);
             }
           }
         };
         if (cols_left >= TW && rows_left >= 2) walk(std::true_type{});
         else walk(std::false_type{});
+#pragma unroll
+        for (int t = 0; t < 9; ++t) L::add(acc[t], sum[t]);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty_bar(s));

@@ -45,6 +45,22 @@ def test_filter_gradient(orc, dtype, shape):
     assert np.all(np.abs(got - ref) <= 2 * (terms + 1) * 2.0 ** -24 * size + ULP[dtype] * np.abs(ref) + 2.0 ** -24)
 
 
+@pytest.mark.parametrize("size,c", [(56, 144), (112, 32)])
+def test_error_of_long_fp32_sums(size, c):
+    """128 images, products of random sign, against float64.  A chain of L additions of products of variance one leaves an
+    error of 0.45 * 2^-24 * sqrt(L / 2) of the root of the number of terms: 2e-7 for sums of up to 28 products that are
+    then added up over the 64 tiles of a thread, 3e-7 for chains of 500, 8e-7 for one of 1800."""
+    n = 128
+    p = pd.depthwise_params(n, size, size, c, 1, 3, 1, True)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, dy = (torch.randn(n, size, size, c, device="cuda", generator=g) for _ in range(2))
+    dw = pd.depthwise_conv2d(pd.FILTER_BACKPROP, x.view(-1), dy.view(-1), p).view(3, 3, c)
+    assert_no_device_error()
+    xp = torch.nn.functional.pad(x, (0, 0, 1, 1, 1, 1))
+    ref = torch.stack([torch.stack([(xp[:, r:r + size, s:s + size].double() * dy).sum((0, 1, 2)) for s in range(3)]) for r in range(3)])
+    assert (dw - ref).square().mean().sqrt() <= 3.2e-7 * (n * size * size) ** 0.5
+
+
 @pytest.mark.parametrize("dtype", ["f16", "f32"])
 def test_edge_values_stay_out_of_other_taps(dtype):
     """VALID windows on 10 x 11 pixels: the last row and column are read by the last tap of each direction only."""
