@@ -96,7 +96,7 @@ struct Tiles {
 template <typename T, int ST, int TW>
 __global__ void __launch_bounds__(kTileThreads + 32, 1)
     depthwise_filter_tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap dy_map,
-                                 float* partial, const Tiles g) {
+                                 const unsigned* x, const unsigned* dy, float* partial, const Tiles g) {
   using L = Lanes<T>;
   using V = typename L::V;
   constexpr int E = L::E, XW = (TW - 1) * ST + 3, ROWS = ST + 3;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
         V sum[9];  // of this tile
 #pragma unroll
         for (int t = 0; t < 9; ++t) sum[t] = L::zero();
-        auto walk = [&](auto whole) {
+        auto walk = [&](auto whole) {  // (false: without the products of outputs that do not exist)
           V win[3][ROWS];  // column c of the tile in win[c % 3]
 #pragma unroll
           for (int c = 0; c < 3 - ST; ++c)
@@ -174,8 +174,6 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
               const V d = L::unpack(dp[(k * TW + j) * words]);
-              // (where there is no such output, the zero that stands for dy meets values of x that are not its own:
-              // an infinity among them must not become a NaN)
               if (!decltype(whole)::value && (j >= cols_left || k >= rows_left)) continue;
 #pragma unroll
               for (int r = 0; r < 3; ++r)
@@ -195,6 +193,44 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
         s = 0;
         ph ^= 1u;
       }
+    }
+  }
+  // The zeros that stand for pixels outside the image and for outputs that do not exist are no terms of the sums, and
+  // make NaNs of infinities: a thread with a NaN takes its products once more, from memory and only those that there are.
+  // (56x56x144, 128 images, f16: 43.8 us; with a look at every tile's sums while it is in shared memory 48.5.)
+  V all[9];  // their sum is a NaN if one of them is
+#pragma unroll
+  for (int t = 0; t < 9; ++t) all[t] = acc[t];
+#pragma unroll
+  for (int step = 1; step < 9; step *= 2)
+#pragma unroll
+    for (int t = 0; t + step < 9; t += 2 * step) L::add(all[t], all[t + step]);
+  const int pixel_words = g.channels / E, channel_word = chunk * words + word;
+  if ((isnan(L::get(all[0], 0)) || isnan(L::get(all[0], E - 1))) && live && channel_word < pixel_words) {
+#pragma unroll
+    for (int t = 0; t < 9; ++t) acc[t] = L::zero();
+#pragma unroll 1
+    for (unsigned tile = (unsigned)slice; tile < g.tiles; tile += (unsigned)g.slices) {
+      const unsigned rest = tile / (unsigned)g.tiles_w;
+      const int w0 = (int)(tile % (unsigned)g.tiles_w) * TW, n = (int)(rest / (unsigned)g.tiles_h);
+      const int h0 = 2 * ((int)(rest % (unsigned)g.tiles_h) * strips + strip);
+      V sum[9];
+#pragma unroll
+      for (int t = 0; t < 9; ++t) sum[t] = L::zero();
+#pragma unroll 1
+      for (int j = 0; j < min(TW, g.out_cols - w0); ++j)
+#pragma unroll 1
+        for (int k = 0; k < min(2, g.out_rows - h0); ++k) {
+          const V d = L::unpack(dy[(((size_t)n * g.out_rows + h0 + k) * g.out_cols + w0 + j) * pixel_words + channel_word]);
+#pragma unroll
+          for (int t = 0; t < 9; ++t) {
+            const int ih = (h0 + k) * ST - g.pad_rows + t / 3, iw = (w0 + j) * ST - g.pad_cols + t % 3;
+            if (ih >= 0 && ih < g.in_rows && iw >= 0 && iw < g.in_cols)
+              L::fma(sum[t], L::unpack(x[(((size_t)n * g.in_rows + ih) * g.in_cols + iw) * pixel_words + channel_word]), d);
+          }
+        }
+#pragma unroll
+      for (int t = 0; t < 9; ++t) L::add(acc[t], sum[t]);
     }
   }
   __syncthreads();
@@ -453,12 +489,14 @@ bool launch_tiles(void (*kernel)(Params...), const Tiles& g, size_t least_smem, 
 }
 
 template <typename T, int ST, int TW>
-int launch_filter_tiles(const CUtensorMap& x_map, const CUtensorMap& dy_map, float* partial, const Tiles& g, cudaStream_t s) {
+int launch_filter_tiles(const CUtensorMap& x_map, const CUtensorMap& dy_map, const void* x, const void* dy, float* partial,
+                        const Tiles& g, cudaStream_t s) {
   static std::mutex mu;
   static bool done[kMaxDevices] = {};
   if (!opt_in(depthwise_filter_tile_kernel<T, ST, TW>, mu, done)) return 0;
   const size_t sums = (size_t)9 * g.words * g.strips * Lanes<T>::E * 4;
-  launch_tiles(depthwise_filter_tile_kernel<T, ST, TW>, g, sums, s, x_map, dy_map, partial, g);  // (the caller's check_launch() reads the error)
+  launch_tiles(depthwise_filter_tile_kernel<T, ST, TW>, g, sums, s, x_map, dy_map, static_cast<const unsigned*>(x),
+               static_cast<const unsigned*>(dy), partial, g);  // (the caller's check_launch() reads the error)
   return g.slices;
 }
 
@@ -497,9 +535,9 @@ int launch_depthwise_filter_tiles(int dtype, const void* x, const void* dy, floa
     return 0;
   return with_tile_shape(p.stride_rows, g.tw, [&](auto st, auto tw) {
     constexpr int ST = decltype(st)::value, TW = decltype(tw)::value;
-    return dtype == PDNN_F32   ? launch_filter_tiles<float, ST, TW>(x_map, dy_map, partial, g, s)
-           : dtype == PDNN_F16 ? launch_filter_tiles<__half, ST, TW>(x_map, dy_map, partial, g, s)
-                               : launch_filter_tiles<__nv_bfloat16, ST, TW>(x_map, dy_map, partial, g, s);
+    return dtype == PDNN_F32   ? launch_filter_tiles<float, ST, TW>(x_map, dy_map, x, dy, partial, g, s)
+           : dtype == PDNN_F16 ? launch_filter_tiles<__half, ST, TW>(x_map, dy_map, x, dy, partial, g, s)
+                               : launch_filter_tiles<__nv_bfloat16, ST, TW>(x_map, dy_map, x, dy, partial, g, s);
   });
 }
 

@@ -903,7 +903,7 @@ __global__ void __launch_bounds__(kFbpLanesF* kFbpLanesP)
         for (int c = 0; c < 3; ++c) {
           const bool ok = row_ok && iw0 + c >= 0 && iw0 + c < p.in_cols;
 #pragma unroll
-          for (int i = 0; i < V; ++i) acc[r * 3 + c][i] = fmaf(ok ? xv[c][i] : 0.f, dv[i], acc[r * 3 + c][i]);
+          for (int i = 0; i < V; ++i) acc[r * 3 + c][i] = ok ? fmaf(xv[c][i], dv[i], acc[r * 3 + c][i]) : acc[r * 3 + c][i];
         }
       }
       ow += lanes_p;
@@ -1131,6 +1131,36 @@ __global__ void __launch_bounds__(kFbpRowsWarps * 32, kFbpRowsBlocks)
       for (int k = 0; k < CARRY; ++k)
 #pragma unroll
         for (int r = 0; r < 3; ++r) win[k][r] = win[NEW + k][r];
+    }
+  }
+  // The zeros above that stand for pixels outside the image and for outputs that do not exist are no terms of the sums,
+  // and make NaNs of infinities: where there is a NaN the products are taken once more, only those that there are.
+  bool again = false;
+#pragma unroll
+  for (int t = 0; t < 9; ++t)
+#pragma unroll
+    for (int e = 0; e < E; ++e) again = again || isnan(acc[t][e]);
+  if (again) {
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[t][e] = 0.f;
+#pragma unroll 1
+    for (unsigned u = (unsigned)bx * (unsigned)kFbpRowsWarps + (unsigned)warp; u < units; u += (unsigned)nbx * (unsigned)kFbpRowsWarps) {
+      const unsigned row = (u / (unsigned)segs) * (unsigned)rows_here + (unsigned)sub;
+      if (sub >= rows_here || row >= all_rows) continue;
+      const int oh = (int)(row % (unsigned)p.out_rows), n = (int)(row / (unsigned)p.out_rows);
+      const int ow_begin = (int)(u % (unsigned)segs) * seg_cols, ow_end = min(ow_begin + seg_cols, p.out_cols);
+#pragma unroll 1
+      for (int ow = ow_begin; ow < ow_end; ++ow) {
+        const unsigned d = dw[(unsigned)((n * p.out_rows + oh) * p.out_cols + ow) * wstride + lw];
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+          const int ih = oh * ST - p.pad_rows + t / 3, iw = ow * ST - p.pad_cols + t % 3;
+          if (ih >= 0 && ih < p.in_rows && iw >= 0 && iw < p.in_cols)
+            WordOf<T>::fma(acc[t], xw[(unsigned)((n * p.in_rows + ih) * p.in_cols + iw) * wstride + lw], d);
+        }
+      }
     }
   }
 #pragma unroll

@@ -78,6 +78,38 @@ def test_edge_values_stay_out_of_other_taps(dtype):
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("shape", [(16, 10, 11, 16, 1), (9, 9, 15, 24, 2),  # tiles
+                                   (1, 5, 6, 16, 1), (2, 7, 9, 10, 2),      # rows: few tiles, no whole packets
+                                   (3, 11, 10, 16, 3)])                     # packets, all taps to a thread
+def test_infinities_meet_their_own_products_only(dtype, shape):
+    """SAME windows: what stands outside the image, and for outputs that do not exist, is no term of a sum."""
+    n, h, w, c, st = shape
+    p = pd.depthwise_params(n, h, w, c, 1, 3, st, True)
+    rng = np.random.default_rng(6)
+    x = rounded(rng.standard_normal(n * h * w * c).astype(np.float32), dtype).reshape(n, h, w, c)
+    dy = rounded(rng.standard_normal(n * p.out_rows * p.out_cols * c).astype(np.float32), dtype).reshape(n, p.out_rows, p.out_cols, c)
+    dy[0, 0, 0, 0] = dy[-1, 0, -1, 2] = dy[0, -1, 0, 4] = dy[-1, -1, -1, 6] = np.inf
+    x[0, 0, 0, 1] = x[-1, 0, -1, 3] = x[0, -1, 0, 5] = x[-1, -1, -1, 7] = -np.inf
+    dw = pd.depthwise_conv2d(pd.FILTER_BACKPROP, to_dev(x.ravel(), dtype), to_dev(dy.ravel(), dtype), p)
+    dw = dw.float().cpu().numpy().reshape(3, 3, c)
+    assert_no_device_error()
+    ref, size = np.zeros((3, 3, c)), np.zeros((3, 3, c))
+    for r in range(3):
+        for s in range(3):
+            oh = [o for o in range(p.out_rows) if 0 <= o * st - p.pad_rows + r < h]
+            ow = [o for o in range(p.out_cols) if 0 <= o * st - p.pad_cols + s < w]
+            a = x[:, [o * st - p.pad_rows + r for o in oh]][:, :, [o * st - p.pad_cols + s for o in ow]].astype(np.float64)
+            b = dy[:, oh][:, :, ow].astype(np.float64)
+            ref[r, s], size[r, s] = (a * b).sum((0, 1, 2)), np.abs(a * b).sum((0, 1, 2))
+    finite = np.isfinite(ref)
+    assert finite.sum() >= 9 * (c - 8) and not finite.all()
+    assert np.array_equal(dw[~finite], ref[~finite], equal_nan=True)
+    terms = n * p.out_rows * p.out_cols
+    dw, ref, size = dw[finite], ref[finite], size[finite]
+    assert np.all(np.abs(dw - ref) <= (terms + 1) * 2.0 ** -24 * size + ULP[dtype] * np.abs(ref) + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_forward_and_input_gradient(orc, dtype, shape):
     n, h, w, c, st, same = shape
