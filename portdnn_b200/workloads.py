@@ -136,11 +136,12 @@ class ConvStackRunner:
         chunk / chunk_layers (forward only): the first ``chunk_layers`` layers run depth-first over
         slices of ``chunk`` images - all those layers on images 0..chunk-1, then on the next slice, and so
         on - with their intermediate activations in slice-sized buffers that every slice reuses, so that a
-        layer's output is still in the L2 cache when the next layer reads it.  Results are identical to
-        the layer-by-layer order of a runner with any_order=False: every operator of the path is independent per image.
+        layer's output is still in the L2 cache when the next layer reads it.
         any_order (forward, layers that run on the whole batch): sums may be split among SMs where a layer has too few
-        tiles for all of them, in an order that depends on the batch (none of the first 25 layers of ResNet-50 has from
-        eight images on, so that there the results are identical with any_order, too)."""
+        tiles for all of them, which depends on the batch and on the device (ResNet-50, f16, us without / with: 2 images
+        508 / 344, 8 images 602 / 479, 16 images 649 / 593).  An image's bits then depend on the batch it is in, and slices
+        change them, both within the rounding of the sums.  any_order=False: an image has the same bits in all batches, and
+        slices change nothing, since every operator is independent per image and adds up in one order."""
         import torch
         from . import dist as pdist
         self.torch, self.layers, self.training, self.device = torch, layers, training, device

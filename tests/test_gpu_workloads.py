@@ -95,6 +95,28 @@ def test_resnet50_depth_first_slices_equal_layer_by_layer():
     assert_no_device_error()
 
 
+def test_resnet50_images_do_not_depend_on_the_batch():
+    """With one order of the sums an image has the same bits in every batch, sliced or not; with the order left open
+    it may not, within rounding."""
+    dev = torch.device("cuda", 0)
+    whole = workloads.ConvStackRunner(workloads.resnet50_v15(8), dev, seed=7, any_order=False)
+    ref = whole.forward().clone().view(8, -1)
+    for batch, any_order, chunk in ((1, False, None), (2, False, None), (2, False, 1), (4, False, None), (4, False, 2), (2, True, None),
+                                    (4, True, 2)):
+        part = workloads.ConvStackRunner(workloads.resnet50_v15(batch), dev, seed=7, any_order=any_order, chunk=chunk,
+                                         chunk_layers=25 if chunk else 0)
+        part.input.copy_(whole.input[:part.input.numel()])
+        for i in part.weights:
+            part.weights[i].copy_(whole.weights[i])
+            part.biases[i].copy_(whole.biases[i])
+        out = part.forward().view(batch, -1)
+        assert_no_device_error()
+        if any_order:  # (53 layers of sums in another order: 6e-4 measured between any two fp16 orders)
+            assert (out.double() - ref[:batch].double()).norm() <= 4e-3 * ref[:batch].double().norm()
+        else:
+            assert torch.equal(out, ref[:batch]), (batch, chunk)
+
+
 def test_vgg16_fp32_forward_every_layer(orc):
     net = workloads.ConvStackRunner(workloads.vgg16(1), torch.device("cuda", 0), seed=3, training=True,
                                     dtype=torch.float32)
