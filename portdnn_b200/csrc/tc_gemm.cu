@@ -3566,7 +3566,7 @@ struct FbpPlan {
 
 constexpr long long kMinPairSlabs = 16;
 
-FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool try_pair = true) {
+FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool try_pair = true, bool try_split = true) {
   FbpPlan f;
   const int epr = dtype == PDNN_F32 ? 32 : 64;
   choose_box(epr, p.out_cols, p.out_rows, p.batch, &f.tw, &f.th, &f.tn);
@@ -3611,7 +3611,7 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool
   const long long out_tiles = units * f.n_tiles;
   long long want = std::max<long long>(1, (2ll * sms) / out_tiles);
   want = std::min<long long>(want, std::max<long long>(1, total_slabs / 8));  // at least 8 slabs per split
-  want = std::min<long long>(want, 512);
+  want = try_split ? std::min<long long>(want, 512) : 1;
   f.slabs_per_split = (int)((total_slabs + want - 1) / want);
   f.splits = (int)((total_slabs + f.slabs_per_split - 1) / f.slabs_per_split);
   return f;
@@ -3810,11 +3810,11 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
 // otherwise the split reduction adds to what dW held.
 int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, const PdnnConv2DParams& p, bool out_f32,
                          bool accumulate, void* ws, size_t ws_elems, cudaStream_t s, bool try_reduce = true,
-                         bool try_pair = true) {
+                         bool try_pair = true, bool try_split = true) {
   const size_t es = dtype_size(dtype);
   const int sms = device_sm_count();
   const int epr = dtype == PDNN_F32 ? 32 : 64;
-  const FbpPlan f = plan_filter_backprop(dtype, p, sms, try_pair);
+  const FbpPlan f = plan_filter_backprop(dtype, p, sms, try_pair, try_split);
   GemmArgs g;
   std::memset(&g, 0, sizeof(g));
   g.a_mn = 1;
@@ -3874,8 +3874,11 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
     } else {
       if (cudaMallocAsync(reinterpret_cast<void**>(&partial), need_bytes, s) != cudaSuccess) {
         cudaGetLastError();
-        // (whole tiles of the tensors' own type need no partial sums outside the CTA pairs)
+        // (whole tiles of the tensors' own type need no partial sums outside the CTA pairs, nor does any layer in one
+        // piece; what is added to dw needs those of one piece)
         if (f.pair) return conv_filter_backprop(dtype, x, dy, dw, p, out_f32, accumulate, ws, ws_elems, s, try_reduce, false);
+        if (f.splits > 1)
+          return conv_filter_backprop(dtype, x, dy, dw, p, out_f32, accumulate, ws, ws_elems, s, try_reduce, false, false);
         return fail(PDNN_ALLOCATION_PROBLEM, "filter backprop: cannot allocate %zu bytes of scratch", need_bytes);
       }
       own = true;
@@ -3911,7 +3914,7 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
       return PDNN_INVALID_PARAMETER;
     }
     // only the staged TMA epilogue can add; anything else goes through partial sums
-    if (reduce && !g.tma_store) return conv_filter_backprop(dtype, x, dy, dw, p, out_f32, accumulate, ws, ws_elems, s, false, try_pair);
+    if (reduce && !g.tma_store) return conv_filter_backprop(dtype, x, dy, dw, p, out_f32, accumulate, ws, ws_elems, s, false, try_pair, try_split);
   }
   int st = launch_gemm(g, dtype, s);
   if (st == PDNN_OK && use_partial) {

@@ -97,3 +97,23 @@ def test_partial_sums_of_whole_filter_tiles():
     with no_memory():
         got = pd.conv2d(pd.FILTER_BACKPROP, x, dy, p)
     _near(got, ref)
+
+
+@pytest.mark.parametrize("dtype,layer", [
+    (torch.float32, (2, 16, 16, 64, 768, 5)),  # two taps to a tile: two pieces of 4.9 MB
+    (torch.half, (8, 16, 16, 400, 192, 5)),    # one column tile of 192: two pieces of 7.7 MB
+    (torch.half, (8, 56, 56, 64, 64, 3))])     # many pieces
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_partial_sums_of_a_split_filter_gradient(dtype, layer, accumulate):
+    """Without memory the reduction runs in one piece."""
+    p = pd.conv_params(*layer, 1)
+    n_in, n_fil, n_out = api.conv_sizes(pd.FILTER_BACKPROP, p)
+    x, dy = _rand(n_in).to(dtype), _rand(n_fil, 0.02).to(dtype)
+    _, elems = pd.conv2d_workspace_size(pd.FILTER_BACKPROP, pd.F32 if dtype == torch.float32 else pd.F16, p, pd.ALGO_IM2COL)
+    assert elems > 0
+    kw = {"accumulate": True, "output_f32": True} if accumulate else {}
+    out = [torch.zeros(n_out, device="cuda", dtype=torch.float32 if accumulate else dtype) for _ in range(2)]
+    pd.conv2d(pd.FILTER_BACKPROP, x, dy, p, out=out[0], **kw)
+    with no_memory():
+        pd.conv2d(pd.FILTER_BACKPROP, x, dy, p, out=out[1], **kw)
+    _near(out[1], out[0])
