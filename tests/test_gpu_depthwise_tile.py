@@ -138,3 +138,21 @@ def test_infinite_weight_meets_the_image_only():
     y = y.float().cpu().view(h, w, c)
     assert torch.equal(y[0], torch.zeros(w, c)) and torch.equal(y[:, 0], torch.zeros(h, c))
     assert torch.isinf(y[1:, 1:]).all()
+
+
+def test_rows_of_more_than_four_billion_elements():
+    """bf16: the second of two rows starts more than 2^31 words into the output."""
+    w, c = 2 ** 22 + 5, 1024
+    if torch.cuda.get_device_properties(0).total_memory < 50e9:
+        pytest.skip("needs two tensors of 17 GB")
+    p = pd.depthwise_params(1, 2, w, c, 1, 3, 1, True)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.empty(2, w, c, device="cuda", dtype=torch.bfloat16).normal_(generator=g)
+    f = torch.randn(3, 3, c, device="cuda", generator=g).bfloat16()
+    y = pd.depthwise_conv2d(pd.FORWARD, x.view(-1), f.view(-1), p).view(2, w, c)
+    assert_no_device_error()
+    for at in (0, w // 2, w - 40):
+        part = torch.nn.functional.pad(x[:, max(at - 1, 0):at + 41].double(), (0, 0, at == 0, at + 40 == w, 1, 1))
+        terms = torch.stack([part[r:r + 2, s:s + 40] * f[r, s].double() for r in range(3) for s in range(3)])
+        ref, size = terms.sum(0), terms.abs().sum(0)
+        assert ((y[:, at:at + 40].double() - ref).abs() <= 10 * 2.0 ** -24 * size + 2.0 ** -8 * ref.abs() + 2.0 ** -24).all()
