@@ -229,7 +229,9 @@ __global__ void __launch_bounds__(kBlock)
 
 // A thread has five packets of 50176 x 256 f16 or so: with the square root and the two divisions of its eight channels
 // to do, as long as the packets took it, it ran at 3.5 TB/s of L2 (21.8 us).  The merging kernel does them once per
-// channel, with the same operations: terms[c] = mean x, mean dy, sum dy * xc / rows / variance, gamma / deviation.
+// channel: terms[c] = mean x, mean dy, sum dy * xc / rows / variance, gamma / deviation.  (Where a thread's channels change,
+// below, the division by the deviation used to come after the multiplication by gamma; the last factor is now
+// rounded first, as it always was where they do not.)
 template <typename T, int V>
 __global__ void __launch_bounds__(kBlock)
     batchnorm_grad_training_vec_kernel(const T* x, const T* dy, const float4* terms, T* __restrict__ out, size_t n, int C) {
@@ -842,14 +844,17 @@ unsigned channel_stable_grid(size_t packets, int cvecs, int sms) {
 
 bool params_ok(int batch, int rows, int cols, int channels) { return batch > 0 && rows > 0 && cols > 0 && channels > 0; }
 
-// Scratch of one call: [partial: slices * 2 * C][stats0: 2C][stats1: 2C][shift: C][scale: C] floats.
+// Scratch of one call: [partial: slices * 2 * C][stats0: 2C][stats1: 2C][shift: C][scale: C] floats.  terms: C float4 from
+// the first 16-byte boundary of stats0 on, in the place of all that follows it (the training gradient in packets,
+// which has no other statistics).
 struct Scratch {
   float *partial, *stats0, *stats1, *shift, *scale;
+  float4* terms;
   void* base;
 };
 
 int get_scratch(Scratch* sc, int slices, int C, cudaStream_t s) {
-  const size_t floats = (size_t)slices * 2 * C + 6 * (size_t)C;
+  const size_t floats = (size_t)slices * 2 * C + 6 * (size_t)C + 3;  // (terms begin up to three floats later)
   if (cudaMallocAsync(&sc->base, floats * sizeof(float), s) != cudaSuccess) {
     cudaGetLastError();
     return fail(PDNN_ALLOCATION_PROBLEM, "batchnorm: cannot allocate %zu bytes of scratch", floats * sizeof(float));
@@ -859,6 +864,7 @@ int get_scratch(Scratch* sc, int slices, int C, cudaStream_t s) {
   sc->stats1 = sc->stats0 + 2 * C;
   sc->shift = sc->stats1 + 2 * C;
   sc->scale = sc->shift + C;
+  sc->terms = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(sc->stats0) + 15) & ~(uintptr_t)15);
   return PDNN_OK;
 }
 
@@ -1010,9 +1016,9 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
                         nullptr, nullptr, sc.partial, rows, C, per_slice, 0.f);
       launch_overlapped(batchnorm_merge_kernel<T, true, StoreGradStats<T>>, (C + kMergeChannels - 1) / kMergeChannels,
                         kMergeChannels * kMergeLanes, s, sc.partial, x, dy, slices, C, rows, per_slice,
-                        StoreGradStats<T>{reinterpret_cast<float4*>(sc.stats0), g, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), (float)rows, p.epsilon});
+                        StoreGradStats<T>{sc.terms, g, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), (float)rows, p.epsilon});
       launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s, x,
-                        dy, reinterpret_cast<const float4*>(sc.stats0), static_cast<T*>(output), n / VN, C);
+                        dy, static_cast<const float4*>(sc.terms), static_cast<T*>(output), n / VN, C);
       count_launch(2);
       cudaFreeAsync(sc.base, s);
       return check_launch("batchnorm gradient (training)");
