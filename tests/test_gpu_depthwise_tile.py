@@ -1,6 +1,6 @@
-"""The depthwise 3x3 filter gradient on TMA tiles against the oracle: sizes around its tiles of 8 (stride 1) or 4
-(stride 2) columns and two rows to a strip, one and several chunks of channels, and values at the image's far edge
-that belong to no product."""
+"""The depthwise 3x3 kernels on TMA tiles against the oracle: sizes around their tiles of 14 or 8 (stride 1) or 4
+(stride 2) columns and two rows to a strip, one and several chunks of channels, and values at the image's edges
+that belong to no product.  Which kernel ran is read from a trace."""
 import numpy as np
 import pytest
 import torch
@@ -12,13 +12,17 @@ pytestmark = pytest.mark.gpu
 
 # n, h, w, c, stride, same
 SHAPES = [
-    (1, 3, 3, 8, 1, False),      # one output
+    (1, 3, 3, 8, 1, False),      # one output: too few tiles for the filter gradient
     (9, 7, 7, 24, 1, True),      # odd rows: the last strip has one
     (8, 8, 8, 40, 1, True),
     (4, 9, 17, 144, 1, True),    # one column beyond two tiles
     (5, 33, 16, 72, 1, False),
     (8, 6, 7, 960, 1, True),     # several chunks
-    (4, 5, 5, 520, 2, True),     # the last chunk partly beyond the channels
+    (8, 5, 5, 520, 2, True),     # the last chunk partly beyond the channels
+    (9, 5, 5, 520, 1, True),
+    (2, 9, 28, 40, 1, True),     # two whole tiles of 14 columns
+    (2, 9, 27, 40, 1, True),     # ... the second one short of a column
+    (1, 30, 40, 24, 1, True),    # three, the last of 12 columns
     (3, 15, 18, 32, 2, True),
     (2, 64, 9, 16, 2, False),
     (40, 14, 14, 64, 1, True),   # several tiles to a block
@@ -26,6 +30,16 @@ SHAPES = [
 # Products of 16-bit values are exact in fp32; a sum of m terms in any order is off by at most m * 2^-24 of the sum of
 # magnitudes, the rounding of the result by 2^-11 or 2^-8 of its value.
 ULP = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8, "f32": 2.0 ** -24}
+
+
+def traced(call, kernel, ran=True):
+    """What the call returns; kernel was launched by it, or was not.  (Without a tracer nothing is known of it.)"""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as trace:
+        out = call()
+        torch.cuda.synchronize()
+    names = [e.key for e in trace.key_averages() if "kernel<" in e.key]
+    assert not names or any(kernel in n for n in names) == ran, names
+    return out
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
@@ -36,7 +50,8 @@ def test_filter_gradient(orc, dtype, shape):
     p, po = pd.depthwise_params(n, h, w, c, 1, 3, st, same), orc.depthwise_params(n, h, w, c, 1, 3, st, same)
     x = rounded(rng.standard_normal(n * h * w * c).astype(np.float32), dtype)
     dy = rounded(rng.standard_normal(n * p.out_rows * p.out_cols * c).astype(np.float32), dtype)
-    got = to_host(pd.depthwise_conv2d(pd.FILTER_BACKPROP, to_dev(x, dtype), to_dev(dy, dtype), p))
+    xd, dyd = to_dev(x, dtype), to_dev(dy, dtype)
+    got = to_host(traced(lambda: pd.depthwise_conv2d(pd.FILTER_BACKPROP, xd, dyd, p), "depthwise_filter_tile_kernel", shape != SHAPES[0]))
     assert_no_device_error()
     ref = orc.depthwise_conv2d(orc.FILTER_BACKPROP, x, dy, po)
     size = orc.depthwise_conv2d(orc.FILTER_BACKPROP, np.abs(x), np.abs(dy), po)
@@ -78,10 +93,13 @@ def test_edge_values_stay_out_of_other_taps(dtype):
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16", "f32"])
-@pytest.mark.parametrize("shape", [(16, 10, 11, 16, 1), (9, 9, 15, 24, 2),  # tiles
-                                   (1, 5, 6, 16, 1), (2, 7, 9, 10, 2),      # rows: few tiles, no whole packets
-                                   (3, 11, 10, 16, 3)])                     # packets, all taps to a thread
-def test_infinities_meet_their_own_products_only(dtype, shape):
+@pytest.mark.parametrize("shape,kernel", [
+    ((16, 10, 11, 16, 1), "depthwise_filter_tile_kernel"),
+    ((9, 9, 15, 24, 2), "depthwise_filter_tile_kernel"),
+    ((1, 5, 6, 16, 1), "depthwise_filter_backprop_rows_kernel"),  # few tiles
+    ((2, 7, 9, 10, 2), "depthwise_filter_backprop_rows_kernel"),  # no whole packets
+    ((3, 11, 10, 16, 3), "depthwise_filter_backprop_partial9_kernel")])
+def test_infinities_meet_their_own_products_only(dtype, shape, kernel):
     """SAME windows: what stands outside the image, and for outputs that do not exist, is no term of a sum."""
     n, h, w, c, st = shape
     p = pd.depthwise_params(n, h, w, c, 1, 3, st, True)
@@ -90,8 +108,8 @@ def test_infinities_meet_their_own_products_only(dtype, shape):
     dy = rounded(rng.standard_normal(n * p.out_rows * p.out_cols * c).astype(np.float32), dtype).reshape(n, p.out_rows, p.out_cols, c)
     dy[0, 0, 0, 0] = dy[-1, 0, -1, 2] = dy[0, -1, 0, 4] = dy[-1, -1, -1, 6] = np.inf
     x[0, 0, 0, 1] = x[-1, 0, -1, 3] = x[0, -1, 0, 5] = x[-1, -1, -1, 7] = -np.inf
-    dw = pd.depthwise_conv2d(pd.FILTER_BACKPROP, to_dev(x.ravel(), dtype), to_dev(dy.ravel(), dtype), p)
-    dw = dw.float().cpu().numpy().reshape(3, 3, c)
+    xd, dyd = to_dev(x.ravel(), dtype), to_dev(dy.ravel(), dtype)
+    dw = to_host(traced(lambda: pd.depthwise_conv2d(pd.FILTER_BACKPROP, xd, dyd, p), kernel)).reshape(3, 3, c)
     assert_no_device_error()
     ref, size = np.zeros((3, 3, c)), np.zeros((3, 3, c))
     for r in range(3):
@@ -118,8 +136,10 @@ def test_forward_and_input_gradient(orc, dtype, shape):
     x = rounded(rng.standard_normal(n * h * w * c).astype(np.float32), dtype)
     f = rounded(rng.standard_normal(9 * c).astype(np.float32), dtype)
     dy = rounded(rng.standard_normal(n * p.out_rows * p.out_cols * c).astype(np.float32), dtype)
-    y = to_host(pd.depthwise_conv2d(pd.FORWARD, to_dev(x, dtype), to_dev(f, dtype), p))
-    dx = to_host(pd.depthwise_conv2d(pd.INPUT_BACKPROP, to_dev(dy, dtype), to_dev(f, dtype), p))
+    xd, fd, dyd = to_dev(x, dtype), to_dev(f, dtype), to_dev(dy, dtype)
+    tiles = "depthwise_forward_tile_kernel"
+    y = to_host(traced(lambda: pd.depthwise_conv2d(pd.FORWARD, xd, fd, p), tiles, dtype == "bf16"))
+    dx = to_host(traced(lambda: pd.depthwise_conv2d(pd.INPUT_BACKPROP, dyd, fd, p), tiles, dtype == "bf16" and st == 1))
     assert_no_device_error()
     # nine products: at most nine roundings of partial sums (fp16 kernels may hold them in fp16) and one of the result
     for got, ref, size in ((y, orc.depthwise_conv2d(orc.FORWARD, x, f, po), orc.depthwise_conv2d(orc.FORWARD, np.abs(x), np.abs(f), po)),
