@@ -90,9 +90,10 @@ struct Tiles {
 // a window of 3 columns x (ST + 3) rows in registers, converts every word once, and multiplies two channels to an
 // instruction.  Its 9 sums are taken tile by tile and added up in registers over the tiles of the block (one chain of up
 // to 1800 products had four times the error: 56x56x144, 128 images, fp32, products of random sign, 7.5e-7 -> 1.9e-7 of the
-// root of the number of terms, at the same time); the block's partial sums go to partial[slice][tap][channel].  What is left is the bytes: 5.1 TB/s of the tensors, 5.6 with the halo.
-// us with the second stage, before / now, 128 images, f16: 56x56x144 86 / 45, 112x112x96 / 2 85 / 60, 112x112x32 69 / 45,
-// 14x14x384 20 / 13, 7x7x960 19 / 13.
+// root of the number of terms, at the same time); the block's partial sums go to partial[slice][tap][channel].  What is left is the bytes: 5.3 TB/s of the
+// tensors, 5.8 with the halo.
+// us with the second stage, before / now, 128 images, f16: 56x56x144 86 / 44, 112x112x96 / 2 85 / 60, 112x112x32 69 / 42,
+// 14x14x384 20 / 13, 7x7x960 19 / 14.
 template <typename T, int ST, int TW>
 __global__ void __launch_bounds__(kTileThreads + 32, 1)
     depthwise_filter_tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap dy_map,

@@ -2799,7 +2799,8 @@ int finish_forward(GemmArgs& g, int dtype, void* y, const PdnnConv2DParams& p, c
 // repacked the same way ([R][8][CP][K], zeros in the padding).
 // The grid is (row segments, groups of kPackRows padded rows, images), so no thread divides.  A thread packs one column of a
 // group, all its reads requested before the first write: with one pixel to a thread and a loop over its channels
-// the launch was 58 880 blocks of three loads each at 256 images.  MobileNet-v2 forward, 64 images: 786 -> 781 us.
+// the launch was 58 880 blocks of three loads each at 256 images.  f16, the layer's us: 64 images 3x3 / 2 3 -> 32 45.0 -> 41.4,
+// 256 images 7x7 / 2 3 -> 64 181.9 -> 162.8 (whole networks: 0 to 0.6 %).
 constexpr int kPackRows = 4;
 template <typename T>
 __global__ void __launch_bounds__(256) pack_small_c_input_kernel(const T* x, uint4* __restrict__ xp, int H, int W, int C, int Hp,
@@ -3604,8 +3605,9 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool
   const long long units = (long long)f.m_tiles * ceil_div(p.window_rows * p.window_cols, f.tap_pack);
   const long long total_slabs = (long long)f.slabs_w * f.slabs_h * f.slabs_n;
   // 129 to 192 features: one column tile reads x once where two of 128 read it for columns that are partly not there,
-  // if there are steps enough (17 to an SM) to pay for its single accumulator buffer (bf16, us, before / now: 7x45x61
-  // 104 -> 152 3x3 37.0 / 30.1, 18x50x61 96 -> 176 5x5 / 2 35.9 / 27.1; 12 to an SM: 7x21x43 224 -> 184 3x3 20.5 / 21.8).
+  // if there are steps enough to pay for its single accumulator buffer: 17 to an SM.  120 layers drawn over sizes, windows
+  // and strides, bf16, time with two tiles over time with one, on average: 12 steps to an SM 0.96, 14 0.98, 16 1.05, 18 1.06,
+  // 20 1.09, 25 1.16 (single layers 0.8 to 1.4).  7x45x61 104 -> 152 3x3 37.0 -> 30.1 us, 18x50x61 96 -> 176 5x5 / 2 35.9 -> 27.1.
   if (dtype != PDNN_F32 && p.features > 128 && p.features <= 192 && units * total_slabs >= 17ll * sms) f.bn = 192;
   f.n_tiles = ceil_div(p.features, f.bn);
   const long long out_tiles = units * f.n_tiles;
