@@ -84,7 +84,7 @@ struct Tiles {
 
 // dW[r][s][c] = sum of x[h * ST + r][w * ST + s][c] * dy[h][w][c].  What bounds the nine multiply-adds per word
 // is everything around them: loads, conversions and bounds checks (56x56x144, 128 images, f16: 71 million warp
-// instructions with the rows in registers, 27 million here).  A warp of its own has TMA bring tiles of TW columns x
+// instructions with the rows in registers, 24 million here).  A warp of its own has TMA bring tiles of TW columns x
 // 2 * strips rows with their halo, zeros outside the image, so that the multiplying warps check nothing and only read
 // shared memory; a thread owns a word of channels and a strip of two output rows, walks the columns of the tile with
 // a window of 3 columns x (ST + 3) rows in registers, converts every word once, and multiplies two channels to an
