@@ -1153,14 +1153,20 @@ __global__ void __launch_bounds__(kFbpRowsWarps * 32, kFbpRowsBlocks)
       if (sub >= rows_here || row >= all_rows) continue;
       const int oh = (int)(row % (unsigned)p.out_rows), n = (int)(row / (unsigned)p.out_rows);
       const int ow_begin = (int)(u % (unsigned)segs) * seg_cols, ow_end = min(ow_begin + seg_cols, p.out_cols);
-#pragma unroll 1
+#pragma unroll 2
       for (int ow = ow_begin; ow < ow_end; ++ow) {
         const unsigned d = dw[(unsigned)((n * p.out_rows + oh) * p.out_cols + ow) * wstride + lw];
+        unsigned xv[9];
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {  // (requested together, where there is nothing from the nearest pixel)
+          const int ih = min(max(oh * ST - p.pad_rows + t / 3, 0), p.in_rows - 1);
+          const int iw = min(max(ow * ST - p.pad_cols + t % 3, 0), p.in_cols - 1);
+          xv[t] = xw[(unsigned)((n * p.in_rows + ih) * p.in_cols + iw) * wstride + lw];
+        }
 #pragma unroll
         for (int t = 0; t < 9; ++t) {
           const int ih = oh * ST - p.pad_rows + t / 3, iw = ow * ST - p.pad_cols + t % 3;
-          if (ih >= 0 && ih < p.in_rows && iw >= 0 && iw < p.in_cols)
-            WordOf<T>::fma(acc[t], xw[(unsigned)((n * p.in_rows + ih) * p.in_cols + iw) * wstride + lw], d);
+          if (ih >= 0 && ih < p.in_rows && iw >= 0 && iw < p.in_cols) WordOf<T>::fma(acc[t], xv[t], d);
         }
       }
     }
