@@ -128,6 +128,10 @@ __device__ __forceinline__ void bulk_wait_group() {
 __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// The part of such a barrier for warps that others wait for and that wait for nobody.
+__device__ __forceinline__ void named_barrier_arrive(uint32_t id, uint32_t count) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
