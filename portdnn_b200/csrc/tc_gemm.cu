@@ -844,22 +844,19 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     // a group that is switched off has nothing to do
   } else if (role == 0) {
     // ------------------------------- TMA producer ------------------------------------------
-    // One thread; the loop body is kept to a wait, an expect_tx and the copies, with all
-    // coordinates advanced incrementally: a lone thread issues an instruction every few cycles
-    // at best, so every division or table lookup per step would show up as pipeline bubbles.
+    // A lone warp issues an instruction every few cycles at best, so what stands in the loop over the reduction steps is
+    // what a step costs: a wait, an expect_tx and the copies take about 220 cycles, and every division, switch or loop of
+    // run-time length beside them shows (with a switch over the filter's layouts and a division in it a step took 615 cycles,
+    // twice what its MMAs need).  Coordinates are therefore advanced by constants chosen outside, and the copies a
+    // step has in nearly every plan are written out.
     // The whole warp walks the tiles and waits on the barriers (every value stays warp-uniform); the
     // warp_* wrappers elect the one lane that issues each copy.
     if (!(pair && grp != 0)) {  // pair mode: group 0's producer fills the shared ring
-      const int epr = a.epr, b_mode = a.b_mode, b_boxes = a.b_boxes, a_boxes = a.a_boxes, cblocks = a.cblocks;
+      const int epr = a.epr, b_mode = a.b_mode, cblocks = a.cblocks;
       const bool presplit = SPLIT && a.b_presplit != 0;
       const uint32_t a_box_bytes = a.a_box_bytes, b_box_bytes = a.b_box_bytes,
                      tx_bytes = pair ? 2u * kABytes + b_bytes
                                      : (b_res ? (uint32_t)kABytes : kABytes + (presplit ? 2u * b_bytes : b_bytes));
-      // pair mode: where the second row tile of the pair starts, relative to the first
-      const int pair_dw = a.pair_dim == 1 ? a.tw : 0, pair_dh = a.pair_dim == 2 ? a.th : 0,
-                pair_dn = a.pair_dim == 3 ? a.tn : 0;
-      const CUtensorMap* bmap = &a.b_map;
-      auto load_b = [&](uint32_t sb, uint32_t fb, int kc, int nf0, int btap) { load_b_from(bmap, sb, fb, kc, nf0, btap); };
       // (the filter of constant_filter is not written by the preceding kernel: requested ahead of the wait)
       if (b_res && early_b && grp == 0 && cta < total_tiles) load_resident_b();
       auto wait_for_tensors = [&] {
@@ -867,20 +864,30 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
         if (b_res && !early_b && grp == 0) load_resident_b();
       };
       int s = 0;
-      uint32_t ph = 0;
+      uint32_t ph = 0, sa = ring_base;
       bool ok = true;
       auto next_stage = [&] {
+        sa += stage_bytes;
         if (++s == S) {
           s = 0;
+          sa = ring_base;
           ph ^= 1u;
         }
       };
       TileWalker walker;
       walker.init(a, first_tile, tile_step);
+      if (!a.a_mn) {
+        // pair mode: where the second row tile of the pair starts, relative to the first
+        const int pair_dw = a.pair_dim == 1 ? a.tw : 0, pair_dh = a.pair_dim == 2 ? a.th : 0,
+                  pair_dn = a.pair_dim == 3 ? a.tn : 0;
+        // Coordinates of a B tile: what a reduction block adds to each, and how many copies a tile takes.
+        const bool b_blocks = b_mode == B_MN_3 || b_mode == B_MN_FHWC;  // one copy per 128-byte column block
+        const int inc0 = (b_mode == B_K_3 || b_mode == B_K_FHWC) ? epr : 0, inc1 = (b_mode == B_MN_3X || b_mode == B_MN_3) ? epr : 0,
+                  inc2 = b_mode == B_MN_FHWC ? epr : 0, b_copies = b_blocks ? a.b_boxes : 1;
+        const uint32_t b_off = pair ? 2u * kABytes : (uint32_t)kABytes;
 #pragma unroll 1
-      for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
-        const TileCoord t = walker.coord(a);
-        if (!a.a_mn) {
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
+          const TileCoord t = walker.coord(a);
           if (tile == first_tile) wait_for_tensors();
 #pragma unroll 1
           for (int tap = 0; tap < a.num_taps && ok; ++tap) {
@@ -889,41 +896,61 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
             const int aw = t.w0 + e.dw, ah = t.h0 + e.dh;
             const int btap = e.b_tap + t.n0 * a.b_batch_mul;
             const uint32_t tx = halo ? (uint32_t)(a.th + e.cnt - 1) * (uint32_t)(a.tw * a.a_row_bytes) : tx_bytes;
+            int b0 = b_blocks ? t.nf0 : 0, b1 = 0, b2 = 0, b3 = 0;  // B_MN_3: nf0, kc, tap
+            switch (b_mode) {
+              case B_MN_3X: b2 = t.nt * a.b_boxes, b3 = btap; break;  // 0, kc, column block, tap
+              case B_MN_3: b2 = btap; break;
+              case B_K_3: b1 = t.nf0, b2 = btap; break;               // kc, nf0, tap
+              case B_K_FHWC: b1 = btap, b2 = t.nf0; break;            // kc, tap, nf0
+              default: b1 = btap; break;                              // B_MN_FHWC: nf0, tap, kc
+            }
 #pragma unroll 1
             for (int cb = 0, kc = GROUPED ? t.nt * a.group_c : 0; cb < cblocks; ++cb, kc += epr) {
               if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g_error_record, a.wait_limit_ns, 0x100u + (unsigned)s)) {
                 ok = false;
                 break;
               }
-              {
-                const uint32_t fb = full_bar(s);
-                warp_arrive_expect_tx(fb, tx);
-                const uint32_t sa = ring_base + (uint32_t)s * stage_bytes;
-                warp_tma_load_4d(sa, amap, fb, kc, aw, ah, t.n0);
-                if (pair) {
-                  warp_tma_load_4d(sa + kABytes, amap, fb, kc, aw + pair_dw, ah + pair_dh, t.n0 + pair_dn);
-                  load_b(sa + 2u * kABytes, fb, kc, t.nf0, btap);
-                } else if (!b_res) {
-                  load_b(sa + kABytes, fb, kc, t.nf0, btap);
-                  if (presplit) load_b_from(&a.b_map_lo, sa + part_bytes, fb, kc, t.nf0, btap);
+              const uint32_t fb = full_bar(s);
+              warp_arrive_expect_tx(fb, tx);
+              warp_tma_load_4d(sa, amap, fb, kc, aw, ah, t.n0);
+              if (!b_res) {
+                if (pair) warp_tma_load_4d(sa + kABytes, amap, fb, kc, aw + pair_dw, ah + pair_dh, t.n0 + pair_dn);
+                const uint32_t sb = sa + b_off;
+                warp_tma_load_4d(sb, &a.b_map, fb, b0, b1, b2, b3);
+#pragma unroll 1
+                for (int j = 1; j < b_copies; ++j)
+                  warp_tma_load_4d(sb + (uint32_t)j * b_box_bytes, &a.b_map, fb, b0 + j * epr, b1, b2, b3);
+                if (presplit) {
+                  warp_tma_load_4d(sa + part_bytes, &a.b_map_lo, fb, b0, b1, b2, b3);
+#pragma unroll 1
+                  for (int j = 1; j < b_copies; ++j)
+                    warp_tma_load_4d(sa + part_bytes + (uint32_t)j * b_box_bytes, &a.b_map_lo, fb, b0 + j * epr, b1, b2, b3);
                 }
+                b0 += inc0, b1 += inc1, b2 += inc2;
               }
               next_stage();
             }
           }
-        } else {
+        }
+      } else {
+        const int a_boxes = a.a_boxes, b_boxes = b_mode == B_MN_4 ? a.b_boxes : 1;
+#pragma unroll 1
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
+          const TileCoord t = walker.coord(a);
           const TapEntry e = a.taps[t.tap];
           const CUtensorMap* amap = &a.a_map[e.a_map];
           // packed taps: the second half of the boxes holds the same channels as seen by the next tap (none: boxes
           // beyond the last channel, which TMA fills with zeros)
           const bool packed = a.tap_pack > 1, second = packed && t.tap + 1 < a.num_taps;
           const TapEntry e2 = a.taps[second ? t.tap + 1 : t.tap];
+          const int half = packed ? a_boxes >> 1 : a_boxes;  // boxes of the first tap
           const CUtensorMap* amap2 = &a.a_map[e2.a_map];
           const int c2nd = second ? t.w0 : 0x40000000;
           const int batch = a.split_is_batch ? t.split : 0;
           // slab coordinates of ks_begin, then advanced like an odometer
           const int line = t.ks_begin / a.slabs_w;
           int iw = t.ks_begin - line * a.slabs_w, in = line / a.slabs_h, ih = line - in * a.slabs_h;
+          int kw = iw * a.tw, kh = ih * a.th, kn = in * a.tn + batch;
           if (tile == first_tile) wait_for_tensors();
 #pragma unroll 1
           for (int ks = t.ks_begin; ks < t.ks_end; ++ks) {
@@ -931,36 +958,36 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
               ok = false;
               break;
             }
-            {
-              const uint32_t fb = full_bar(s);
-              warp_arrive_expect_tx(fb, tx_bytes);
-              const uint32_t sa = ring_base + (uint32_t)s * stage_bytes;
-              const uint32_t sb = sa + kABytes;
-              const int kw = iw * a.tw, kh = ih * a.th, kn = in * a.tn + batch;
+            const uint32_t fb = full_bar(s), sb = sa + kABytes;
+            warp_arrive_expect_tx(fb, tx_bytes);
+            warp_tma_load_4d(sa, amap, fb, t.w0, kw + e.dw, kh + e.dh, kn);
+            if (packed) warp_tma_load_4d(sa + (uint32_t)half * a_box_bytes, amap2, fb, c2nd, kw + e2.dw, kh + e2.dh, kn);
+            else warp_tma_load_4d(sa + a_box_bytes, amap, fb, t.w0 + epr, kw + e.dw, kh + e.dh, kn);
+            if constexpr (SPLIT) {  // four boxes of 32 fp32 words
               if (packed) {
-                const int half = a_boxes >> 1;
-                for (int j = 0; j < half; ++j) {
-                  warp_tma_load_4d(sa + (uint32_t)j * a_box_bytes, amap, fb, t.w0 + j * epr, kw + e.dw, kh + e.dh, kn);
-                  warp_tma_load_4d(sa + (uint32_t)(half + j) * a_box_bytes, amap2, fb, c2nd + j * epr, kw + e2.dw, kh + e2.dh, kn);
-                }
+                warp_tma_load_4d(sa + a_box_bytes, amap, fb, t.w0 + epr, kw + e.dw, kh + e.dh, kn);
+                warp_tma_load_4d(sa + 3u * a_box_bytes, amap2, fb, c2nd + epr, kw + e2.dw, kh + e2.dh, kn);
               } else {
-#pragma unroll 1
-                for (int j = 0; j < a_boxes; ++j)
-                  warp_tma_load_4d(sa + (uint32_t)j * a_box_bytes, amap, fb, t.w0 + j * epr, kw + e.dw, kh + e.dh, kn);
-              }
-              if (b_mode == B_MN_4) {
-#pragma unroll 1
-                for (int j = 0; j < b_boxes; ++j)
-                  warp_tma_load_4d(sb + (uint32_t)j * b_box_bytes, bmap, fb, t.nf0 + j * epr, kw, kh, kn);
-              } else {  // B_K_4
-                warp_tma_load_4d(sb, bmap, fb, kw, t.nf0, 0, kn);
+                warp_tma_load_4d(sa + 2u * a_box_bytes, amap, fb, t.w0 + 2 * epr, kw + e.dw, kh + e.dh, kn);
+                warp_tma_load_4d(sa + 3u * a_box_bytes, amap, fb, t.w0 + 3 * epr, kw + e.dw, kh + e.dh, kn);
               }
             }
+            if (b_mode == B_MN_4) {
+              warp_tma_load_4d(sb, &a.b_map, fb, t.nf0, kw, kh, kn);
+              if (b_boxes > 1) warp_tma_load_4d(sb + b_box_bytes, &a.b_map, fb, t.nf0 + epr, kw, kh, kn);
+#pragma unroll 1
+              for (int j = 2; j < b_boxes; ++j)
+                warp_tma_load_4d(sb + (uint32_t)j * b_box_bytes, &a.b_map, fb, t.nf0 + j * epr, kw, kh, kn);
+            } else {  // B_K_4
+              warp_tma_load_4d(sb, &a.b_map, fb, kw, t.nf0, 0, kn);
+            }
+            kw += a.tw;
             if (++iw == a.slabs_w) {
-              iw = 0;
+              iw = kw = 0;
+              kh += a.th;
               if (++ih == a.slabs_h) {
-                ih = 0;
-                ++in;
+                ih = kh = 0;
+                kn += a.tn;
               }
             }
             next_stage();
@@ -1038,8 +1065,8 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
         tc_fence_after_sync();
         const uint32_t d_tmem = grp_tmem + buf * acc_stride;
         uint32_t accumulate = 0u;
-        if (!SPLIT && !a.a_mn) {
-          // Forward-style GEMM: one stage per (tap entry, reduction block); in halo mode a stage
+        if (!SPLIT && b_res) {
+          // Resident B: one stage per (tap entry, reduction block); in halo mode a stage
           // feeds the MMAs of all cnt taps of its entry.  Everything in this loop is kept to
           // 32-bit additions on values prepared outside it: the lone issuing thread is what bounds
           // tiles of 64 or 128 columns, and it needs the tile's nt only (the walker's digit 0).
@@ -1058,7 +1085,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
               // start addresses stay below 2^18, so adding to the low descriptor word never carries
               // into the neighbouring field
               uint32_t a_lo = fw.a_lo0 + sa16 + fw.my_a16;
-              uint32_t b_lo = b_res ? fw.b_lo0 + res16 + (uint32_t)cb * fw.b_bytes16 : fw.b_lo0 + sa16 + fw.my_b16;
+              uint32_t b_lo = fw.b_lo0 + res16 + (uint32_t)cb * fw.b_bytes16;
               if constexpr (GROUPED) {
                 // one MMA per slice of 16 channels, into the columns of the slice's group
 #pragma unroll 1
@@ -1122,28 +1149,32 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
               ok = false;
               break;
             }
-            tc_fence_after_sync();
-            const uint32_t sa = ring_base + (uint32_t)s * stage_bytes;
-            uint64_t da = a_desc0 + (uint64_t)(sa >> 4);
-            uint64_t db = b_desc0 + (uint64_t)((sa + kABytes) >> 4);
-            const uint32_t ta = tmem_base + acc_bufs * acc_stride + (uint32_t)s * kSplitAColumns;  // SPLIT: hi, then lo of A
+            const uint64_t da = ((uint64_t)fw.a_hi << 32) | (fw.a_lo0 + sa16 + fw.my_a16);
+            const uint64_t db = ((uint64_t)fw.b_hi << 32) | (fw.b_lo0 + sa16 + fw.my_b16);
+            if constexpr (SPLIT) {
+              tc_fence_after_sync();
+              const uint32_t ta = tmem_base + acc_bufs * acc_stride + (uint32_t)s * kSplitAColumns;  // hi, then lo of A
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              if (SPLIT) {
-                warp_mma_tf32_ts(d_tmem, ta + 32u + 8u * (uint32_t)k, db, idesc, accumulate);
-                warp_mma_tf32_ts(d_tmem, ta + 8u * (uint32_t)k, db + lo_off, idesc, 1u);
-                warp_mma_tf32_ts(d_tmem, ta + 8u * (uint32_t)k, db, idesc, 1u);
-              } else {
-                warp_mma_f16(d_tmem, da, db, idesc, accumulate);
+              for (int k = 0; k < 4; ++k) {
+                const uint64_t dbk = db + (uint32_t)k * b_kadv;
+                warp_mma_tf32_ts(d_tmem, ta + 32u + 8u * (uint32_t)k, dbk, idesc, accumulate);
+                warp_mma_tf32_ts(d_tmem, ta + 8u * (uint32_t)k, dbk + lo_off, idesc, 1u);
+                warp_mma_tf32_ts(d_tmem, ta + 8u * (uint32_t)k, dbk, idesc, 1u);
+                accumulate = 1u;
               }
+            } else {  // (as above: TMA and MMA are ordered by the mbarrier)
+              warp_mma_f16(d_tmem, da, db, idesc, accumulate);
+              warp_mma_f16(d_tmem, da + a_kadv, db + b_kadv, idesc, 1u);
+              warp_mma_f16(d_tmem, da + 2 * a_kadv, db + 2 * b_kadv, idesc, 1u);
+              warp_mma_f16(d_tmem, da + 3 * a_kadv, db + 3 * b_kadv, idesc, 1u);
               accumulate = 1u;
-              da += a_kadv;
-              db += b_kadv;
             }
             warp_commit(empty_bar(s));  // frees the stage once these MMAs have read it
+            sa16 += fw.stage16;
             if (++s == S) {
               s = 0;
               ph ^= 1u;
+              sa16 = fw.ring16;
             }
           }
         }
@@ -1454,7 +1485,7 @@ __global__ void __launch_bounds__(192, 1) umma_gemm_pair2_kernel(const __grid_co
           if (leader) warp_arrive_expect_tx(fb, 2u * kStage);  // the bytes of both CTAs
           const uint32_t sa = base + (uint32_t)s * kStage;
           warp_tma_load_4d_pair(sa, amap, fb, kc, aw, ah, an);
-          warp_tma_load_4d_pair(sa + kABytes, bmap, fb, 0, kc, nf0 / epr, e.b_tap);  // two 64-column blocks
+          warp_tma_load_4d_pair(sa + kABytes, bmap, fb, 0, kc, nf0 >> 6, e.b_tap);  // two 64-column blocks
           if (++s == S) {
             s = 0;
             ph ^= 1u;
@@ -1894,7 +1925,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) umma_gemm_cluster_kernel(c
       const uint32_t sb = ring + (uint32_t)s * stage_bytes + (uint32_t)kABytes, fb = full_bar(s);
       const int kc = cb * a.epr, btap = a.taps[tap].b_tap + t.n0 * a.b_batch_mul;
       switch (a.b_mode) {
-        case B_MN_3X: warp_tma_load_4d(sb, &a.b_map, fb, 0, kc, t.nf0 / a.epr, btap); break;
+        case B_MN_3X: warp_tma_load_4d(sb, &a.b_map, fb, 0, kc, t.nt * a.b_boxes, btap); break;
         case B_K_3: warp_tma_load_4d(sb, &a.b_map, fb, kc, t.nf0, btap, 0); break;
         case B_K_FHWC: warp_tma_load_4d(sb, &a.b_map, fb, kc, btap, t.nf0, 0); break;
         default:  // B_MN_3, B_MN_FHWC: one copy per 64 columns
