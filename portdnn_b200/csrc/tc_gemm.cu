@@ -141,6 +141,9 @@ struct alignas(64) GemmArgs {
   int accumulate;  // packed 16-bit epilogues, no bias: the block already in the output is added (before the mask)
   int reduce_add;  // staged fp32 epilogue of the filter backprop: every pixel split adds its tile to the output
   int mask_smem_bytes;  // the barriers of the epilogue warps' mask slots (the slots themselves follow the staging slices)
+  // 1: one tile to a CTA, one pipeline, 192 threads and under half of an SM's shared memory (see plan_solo): the staging
+  // slices take the ring's place once the accumulators are complete
+  int solo;
   unsigned long long walk_magic[3];  // TileWalker: ceil(2^32 / radix) (set_walk_magic)
   // Time limit of one barrier wait; a wait that lasts longer means a lost arrival, and the CTA
   // gives up (see umma::mbar_wait).
@@ -527,15 +530,18 @@ struct MaskSlot {
   uint32_t bar;        // mbarrier of the first slot (one per slot, 8 bytes apart)
   uint32_t nslots;     // 1 or 2: how many blocks ahead the requests run
   uint32_t issued, consumed;
-  // the block the next request is for: the warp's blocks in the order it will work on them
-  TileWalker walker;
+  // the block the next request is for: the warp's blocks in the order it will work on them (digits of its tile; radices and
+  // step are those of the epilogue's own walker)
+  int d0, d1, d2, d3;
   int tile, c0, tile_step, total_tiles, sub_w, sub_h, sub_n;
 };
 
 // Requests the mask of the next block that has none yet (if any is left).
-__device__ __forceinline__ void request_mask_block(const GemmArgs& a, const WarpStore& ws, MaskSlot& ms) {
+__device__ __forceinline__ void request_mask_block(const GemmArgs& a, const WarpStore& ws, MaskSlot& ms, const TileWalker& walker) {
   if (ms.tile >= ms.total_tiles) return;
-  const TileCoord t = ms.walker.coord(a);
+  TileWalker at = walker;
+  at.d0 = ms.d0, at.d1 = ms.d1, at.d2 = ms.d2, at.d3 = ms.d3;
+  const TileCoord t = at.coord(a);
   const uint32_t slot = ms.issued % ms.nslots;
   if (elect_one()) {
     mbar_arrive_expect_tx(ms.bar + 8u * slot, 4096u);
@@ -547,7 +553,8 @@ __device__ __forceinline__ void request_mask_block(const GemmArgs& a, const Warp
   if (ms.c0 >= a.bn) {
     ms.c0 = 0;
     ms.tile += ms.tile_step;
-    ms.walker.advance();
+    at.advance();
+    ms.d0 = at.d0, ms.d1 = at.d1, ms.d2 = at.d2, ms.d3 = at.d3;
   }
 }
 
@@ -562,7 +569,7 @@ template <typename OutT, bool MASK, bool BITS = false, bool MBITS = false>
 __device__ __forceinline__ bool epilogue_tile_tma_fast(const GemmArgs& a, const TileCoord& t, uint32_t tmem_acc,
                                                        int lane, bool zero, const WarpStore& ws,
                                                        uint32_t& store_count, uint32_t bias_s, int q32, MaskSlot& ms,
-                                                       volatile int* abort_flag) {
+                                                       const TileWalker& walker, volatile int* abort_flag) {
   const int act = a.act;
   static_assert(!(MASK && BITS) && (MASK || !MBITS), "one form per instantiation");
   constexpr bool bit_mask = MBITS;  // the mask arrives as one bit per element (a.mask_bits), not as a tensor
@@ -628,7 +635,7 @@ __device__ __forceinline__ bool epilogue_tile_tma_fast(const GemmArgs& a, const 
       }
       __syncwarp();  // every lane holds its masks: the slot may be overwritten
       ++ms.consumed;
-      request_mask_block(a, ws, ms);
+      request_mask_block(a, ws, ms, walker);
      }
     }
     wait_slice_free(ws, lane);
@@ -708,8 +715,10 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
   // staging slices for the TMA-store epilogue (per group: 4 warps x nsw slices), then the barrier
   // block, then the bias copy
   const uint32_t group_staging = a.tma_store ? ((uint32_t)a.nsw + (EPI == 3 ? (uint32_t)a.mask_slots : 0u)) * 4u * 4096u : 0u;
-  const uint32_t staging_off = res_bytes + (uint32_t)rings * ring_bytes;
-  const uint32_t bar_off = staging_off + (uint32_t)groups * group_staging;
+  const bool solo = !SPLIT && a.solo != 0;
+  const uint32_t solo_masks = EPI == 3 ? (uint32_t)a.mask_slots * 4u * 4096u : 0u;  // (a solo CTA's mask slots follow its ring)
+  const uint32_t staging_off = solo ? 0u : res_bytes + (uint32_t)rings * ring_bytes;
+  const uint32_t bar_off = solo ? ring_bytes + solo_masks : staging_off + (uint32_t)groups * group_staging;
   uint8_t* bar_mem = smem + bar_off;
   const uint32_t bar_base = base + bar_off;
   auto gbar = [&](int g, int i) { return bar_base + 8u * (uint32_t)(g * kBarsPerGroup + i); };
@@ -808,8 +817,9 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
       }
   };
   // the CTA's copy of the bias vector, zero beyond the last column (all epilogue warps together)
+  constexpr bool kPackedBias = EPI == 2 || EPI == 4;  // (the forms with a mask have none)
   auto copy_bias = [&] {
-    if (EPI >= 2 && EPI != 6 && a.bias != nullptr) {
+    if (kPackedBias && a.bias != nullptr) {
       const OutT* bias = static_cast<const OutT*>(a.bias);
       uint4* dst = reinterpret_cast<uint4*>(bar_mem + kBarBlockBytes);
       const int chunks = a.bias_smem_bytes >> 4;
@@ -885,6 +895,39 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
         const int inc0 = (b_mode == B_K_3 || b_mode == B_K_FHWC) ? epr : 0, inc1 = (b_mode == B_MN_3X || b_mode == B_MN_3) ? epr : 0,
                   inc2 = b_mode == B_MN_FHWC ? epr : 0, b_copies = b_blocks ? a.b_boxes : 1;
         const uint32_t b_off = pair ? 2u * kABytes : (uint32_t)kABytes;
+        struct BCoord {
+          int c0, c1, c2, c3;
+        };
+        auto b_coord = [&](const TileCoord& t, int btap) {  // of the tap's first reduction block
+          BCoord b{b_blocks ? t.nf0 : 0, 0, 0, 0};
+          switch (b_mode) {
+            case B_MN_3X: b.c2 = t.nt * a.b_boxes, b.c3 = btap; break;  // 0, kc, column block, tap
+            case B_MN_3: b.c2 = btap; break;                            // nf0, kc, tap
+            case B_K_3: b.c1 = t.nf0, b.c2 = btap; break;               // kc, nf0, tap
+            case B_K_FHWC: b.c1 = btap, b.c2 = t.nf0; break;            // kc, tap, nf0
+            default: b.c1 = btap; break;                                // B_MN_FHWC: nf0, tap, kc
+          }
+          return b;
+        };
+        auto load_b = [&](const CUtensorMap* map, uint32_t sb, uint32_t fb, const BCoord& b) {
+          warp_tma_load_4d(sb, map, fb, b.c0, b.c1, b.c2, b.c3);
+#pragma unroll 1
+          for (int j = 1; j < b_copies; ++j)
+            warp_tma_load_4d(sb + (uint32_t)j * b_box_bytes, map, fb, b.c0 + j * epr, b.c1, b.c2, b.c3);
+        };
+        // filter tiles of the first stages that are requested before the preceding kernel has ended
+        int ahead = 0;
+        if (early_b && !b_res && first_tile < total_tiles) {
+          const TileCoord t = walker.coord(a);
+          for (int tap = 0; tap < a.num_taps && ahead < S; ++tap) {
+            BCoord b = b_coord(t, a.taps[tap].b_tap + t.n0 * a.b_batch_mul);
+            for (int cb = 0; cb < cblocks && ahead < S; ++cb, ++ahead) {
+              warp_arrive_expect_tx(full_bar(ahead), tx_bytes);
+              load_b(&a.b_map, ring_base + (uint32_t)ahead * stage_bytes + b_off, full_bar(ahead), b);
+              b.c0 += inc0, b.c1 += inc1, b.c2 += inc2;
+            }
+          }
+        }
 #pragma unroll 1
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
           const TileCoord t = walker.coord(a);
@@ -896,38 +939,29 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
             const int aw = t.w0 + e.dw, ah = t.h0 + e.dh;
             const int btap = e.b_tap + t.n0 * a.b_batch_mul;
             const uint32_t tx = halo ? (uint32_t)(a.th + e.cnt - 1) * (uint32_t)(a.tw * a.a_row_bytes) : tx_bytes;
-            int b0 = b_blocks ? t.nf0 : 0, b1 = 0, b2 = 0, b3 = 0;  // B_MN_3: nf0, kc, tap
-            switch (b_mode) {
-              case B_MN_3X: b2 = t.nt * a.b_boxes, b3 = btap; break;  // 0, kc, column block, tap
-              case B_MN_3: b2 = btap; break;
-              case B_K_3: b1 = t.nf0, b2 = btap; break;               // kc, nf0, tap
-              case B_K_FHWC: b1 = btap, b2 = t.nf0; break;            // kc, tap, nf0
-              default: b1 = btap; break;                              // B_MN_FHWC: nf0, tap, kc
-            }
+            BCoord b = b_coord(t, btap);
 #pragma unroll 1
             for (int cb = 0, kc = GROUPED ? t.nt * a.group_c : 0; cb < cblocks; ++cb, kc += epr) {
-              if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g_error_record, a.wait_limit_ns, 0x100u + (unsigned)s)) {
-                ok = false;
-                break;
-              }
               const uint32_t fb = full_bar(s);
-              warp_arrive_expect_tx(fb, tx);
-              warp_tma_load_4d(sa, amap, fb, kc, aw, ah, t.n0);
-              if (!b_res) {
-                if (pair) warp_tma_load_4d(sa + kABytes, amap, fb, kc, aw + pair_dw, ah + pair_dh, t.n0 + pair_dn);
-                const uint32_t sb = sa + b_off;
-                warp_tma_load_4d(sb, &a.b_map, fb, b0, b1, b2, b3);
-#pragma unroll 1
-                for (int j = 1; j < b_copies; ++j)
-                  warp_tma_load_4d(sb + (uint32_t)j * b_box_bytes, &a.b_map, fb, b0 + j * epr, b1, b2, b3);
-                if (presplit) {
-                  warp_tma_load_4d(sa + part_bytes, &a.b_map_lo, fb, b0, b1, b2, b3);
-#pragma unroll 1
-                  for (int j = 1; j < b_copies; ++j)
-                    warp_tma_load_4d(sa + part_bytes + (uint32_t)j * b_box_bytes, &a.b_map_lo, fb, b0 + j * epr, b1, b2, b3);
+              const bool have_b = b_res || ahead > 0;
+              if (ahead > 0) {
+                --ahead;
+              } else {
+                if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, g_error_record, a.wait_limit_ns, 0x100u + (unsigned)s)) {
+                  ok = false;
+                  break;
                 }
-                b0 += inc0, b1 += inc1, b2 += inc2;
+                warp_arrive_expect_tx(fb, tx);
               }
+              warp_tma_load_4d(sa, amap, fb, kc, aw, ah, t.n0);
+              if (pair) warp_tma_load_4d(sa + kABytes, amap, fb, kc, aw + pair_dw, ah + pair_dh, t.n0 + pair_dn);
+              if (!have_b) {
+                load_b(&a.b_map, sa + b_off, fb, b);
+                if constexpr (SPLIT) {
+                  if (presplit) load_b(&a.b_map_lo, sa + part_bytes, fb, b);
+                }
+              }
+              b.c0 += inc0, b.c1 += inc1, b.c2 += inc2;
               next_stage();
             }
           }
@@ -997,8 +1031,8 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     }
   } else if (role == 1) {
     // ------------------------------- MMA issuer ---------------------------------------------
-    // The successor may be placed once every CTA of this grid has got here: the grid is a single wave, so nothing of it
-    // is still waiting for an SM, and the columns of tensor memory are taken.
+    // The successor may be placed once every CTA of this grid has got here: nothing of the grid is still waiting for an SM
+    // then, and its columns of tensor memory are taken.
     if (grp == 0) {
       grid_dependency_wait();
       grid_launch_dependents();
@@ -1196,11 +1230,13 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     WarpStore ws;
     ws.nsw = a.nsw;
     const uint32_t warp_slices = (uint32_t)a.nsw + (EPI == 3 ? (uint32_t)a.mask_slots : 0u);  // the last ones are the mask slots
-    const uint32_t my_staging = staging_off + (uint32_t)grp * group_staging + (uint32_t)wslot * warp_slices * 4096u;
+    const uint32_t my_staging = solo ? (uint32_t)wslot * (uint32_t)a.nsw * 4096u
+                                     : staging_off + (uint32_t)grp * group_staging + (uint32_t)wslot * warp_slices * 4096u;
     ws.buf = smem + my_staging;
     ws.buf_addr = base + my_staging;
     [[maybe_unused]] MaskSlot mask_slot;
-    mask_slot.addr = base + my_staging + (uint32_t)a.nsw * 4096u;
+    mask_slot.addr = solo ? base + ring_bytes + (uint32_t)wslot * (uint32_t)a.mask_slots * 4096u
+                          : base + my_staging + (uint32_t)a.nsw * 4096u;
     mask_slot.bar = bar_base + (uint32_t)kBarBlockBytes + (uint32_t)a.bias_smem_bytes + 16u * (uint32_t)(grp * 4 + wslot);
     mask_slot.nslots = (uint32_t)a.mask_slots;
     mask_slot.issued = mask_slot.consumed = 0;
@@ -1213,9 +1249,9 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     if (early_b) copy_bias();
     grid_dependency_wait();
     if (!early_b) copy_bias();
-    if (EPI >= 2 && EPI != 6 && a.bias != nullptr) named_barrier_sync(2, (uint32_t)groups * 128u);
+    if (kPackedBias && a.bias != nullptr) named_barrier_sync(2, (uint32_t)groups * 128u);
     if constexpr (EPI == 3) {
-      mask_slot.walker = walker;
+      mask_slot.d0 = walker.d0, mask_slot.d1 = walker.d1, mask_slot.d2 = walker.d2, mask_slot.d3 = walker.d3;
       mask_slot.tile = first_tile;
       mask_slot.c0 = 0;
       mask_slot.tile_step = tile_step;
@@ -1223,7 +1259,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
       mask_slot.sub_w = sub_w;
       mask_slot.sub_h = sub_h;
       mask_slot.sub_n = sub_n;
-      for (uint32_t i = 0; i < mask_slot.nslots; ++i) request_mask_block(a, ws, mask_slot);
+      for (uint32_t i = 0; i < mask_slot.nslots; ++i) request_mask_block(a, ws, mask_slot, walker);
     }
 #pragma unroll 1
     for (int tile = first_tile; tile < total_tiles; tile += tile_step, walker.advance()) {
@@ -1237,7 +1273,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
       const bool zero = !(t.ks_end > t.ks_begin);
       if constexpr (EPI >= 2 && EPI != 6) {
         if (!epilogue_tile_tma_fast<OutT, EPI == 3 || EPI == 5, EPI == 4, EPI == 5>(a, t, tmem_acc, lane, zero, ws, store_count, bias_s, q * 32, mask_slot,
-                                                    abort_flag))
+                                                    walker, abort_flag))
           break;
       } else if constexpr (EPI == 1 || EPI == 6) {
         epilogue_tile_tma<OutT, EPI == 6>(a, t, tmem_acc, q * 32, lane, zero, ws, store_count);
@@ -1577,7 +1613,7 @@ __global__ void __launch_bounds__(192, 1) umma_gemm_pair2_kernel(const __grid_co
       tc_fence_after_sync();
       const uint32_t tmem_acc = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256u;
       if (!epilogue_tile_tma_fast<OutT, false, BITS>(a, t, tmem_acc, lane, false, ws, store_count, bias_s, q * 32, unused_mask,
-                                               abort_flag))
+                                               walker, abort_flag))
         break;
       tc_fence_before_sync();
       __syncwarp();
@@ -2234,7 +2270,45 @@ void set_operand_layout(GemmArgs& g, int dtype, int b_mn) {
 // Chooses the store path of the epilogue and sizes the pipeline; call once the output fields of
 // `g` are set.  out_dims / out_strides describe the output as a 4-D tensor whose dimension 0 is
 // the column (feature) axis and whose other dimensions are the ones the row-tile box spans.
-bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], const uint64_t out_strides[3]) {
+//
+// plan_solo: GEMMs of at most two tiles to an SM, 16-bit operands.  What bounds them is not their few steps but what stands
+// around them: a CTA of the persistent form takes an SM's shared memory, so it starts where the preceding
+// kernel's CTA ends, 2.6 us before its first MMA.  A solo CTA has one tile, one pipeline of 192 threads, one accumulator and
+// less than half of an SM's shared memory: two share an SM, of one launch or of two that follow each other, and the
+// set-up of the second - and under constant_filter its first filter tiles - run beside the first.
+// us at 24 images, f16, persistent / solo: 28x28 512 -> 128 forward 8.5 / 6.7, its filter gradient 8.1 / 6.4; 7x7 512 -> 2048 7.3 / 6.6
+// forward, 9.4 / 8.4 and 8.5 / 7.1 backward; 14x14 256 -> 256 3x3 12.0 / 12.3 (168 tiles), 12.6 / 13.0, 10.9 / 10.3.  ResNet-50
+// backward 1437 -> 1300, with the shorter loops.  More than two tiles to an SM are worked off by persistent CTAs.
+constexpr int kSoloSmem = 113 * 1024, kSoloSmemMin = 108 * 1024;  // (the minimum: see launch_gemm)
+bool plan_solo(GemmArgs& g, bool mask_tma) {
+  const int tap_pack = std::max(g.tap_pack, 1);
+  const long long tiles = g.a_mn ? (long long)g.n_tiles * g.tiles_w * ((g.num_taps + tap_pack - 1) / tap_pack) * g.splits
+                                 : (long long)g.n_tiles * g.tiles_w * g.tiles_h * g.tiles_n;
+  if (tiles > 2ll * device_sm_count()) return false;
+  GemmArgs t = g;
+  t.solo = 1;
+  t.groups = t.acc_bufs = 1;
+  t.acc_stride = std::max(32, next_pow2(t.bn));
+  t.tmem_cols = t.acc_stride;
+  t.bias_tile_only = 1;
+  t.bias_smem_bytes = (t.epi_fast && t.bias != nullptr) ? ceil_div(t.bn, 64) * 128 : 0;
+  t.res_taps = t.num_taps;
+  t.b_res = 0;
+  t.b_res_bytes = 0;
+  const int blocks = ceil_div(t.bn, t.cpb), stage = kABytes + t.bn * 128, fixed = 1024 + kBarBlockBytes + t.bias_smem_bytes + t.mask_smem_bytes;
+  const int steps = t.a_mn ? t.slabs_per_split : t.num_taps * t.cblocks;
+  auto stages = [&] { return std::min(kMaxStages, (kSoloSmem - fixed - t.mask_slots * 4 * 4096) / stage); };
+  t.mask_slots = (mask_tma && t.mask_bits == nullptr) ? std::min(2, blocks) : 0;
+  if (t.mask_slots == 2 && stages() < 3) t.mask_slots = 1;
+  t.stages = stages();
+  if (t.stages < std::min(3, steps)) return false;
+  t.nsw = blocks > 2 ? 4 : blocks;
+  while (t.nsw > 1 && t.nsw * 4 * 4096 > t.stages * stage) t.nsw /= 2;
+  g = t;
+  return true;
+}
+
+bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], const uint64_t out_strides[3], bool allow_solo = true) {
   g.cpb = 128 / (int)dtype_size(g.out_dtype);
   g.tma_store = 0;
   if (g.beta == 0.f && g.bn % g.cpb == 0 && aligned16(g.out)) {
@@ -2276,6 +2350,8 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
   if (!g.epi_fast && !(g.tma_store && compute_dtype == PDNN_F32)) g.relu_mask = nullptr;
   const bool mask_tma = g.epi_fast && g.relu_mask != nullptr;
   g.mask_smem_bytes = mask_tma ? 128 : 0;  // the mask slots' barriers; the slots count as staging
+  g.solo = 0;
+  if (allow_solo && !split && g.tma_store && !g.pair && !g.cta_pair && !g.halo && g.group_k == 0 && plan_solo(g, mask_tma)) return true;
   if (g.pair && !g.cta_pair && (split || g.groups != 2 || !g.tma_store)) return false;  // the caller plans again without pairing
   if (g.epi_fast && g.bias != nullptr) {
     const int padded = ceil_div(g.n_tiles * g.bn, 64) * 64;
@@ -2492,6 +2568,11 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
                 (g.tma_store ? (size_t)g.groups * (g.nsw + g.mask_slots) * 4 * 4096 : 0) + kBarBlockBytes +
                 (size_t)g.bias_smem_bytes + (size_t)g.mask_smem_bytes;
   smem = std::max<size_t>(smem, 120 * 1024);
+  // (a solo CTA of at least 108 KB shares an SM with another one or with a CTA of the cluster kernel, whose columns of
+  // tensor memory fit beside its own, and with nothing larger)
+  if (g.solo)
+    smem = std::max<size_t>(1024 + (size_t)g.stages * stage + (size_t)g.mask_slots * 4 * 4096 + kBarBlockBytes +
+                                (size_t)g.bias_smem_bytes + (size_t)g.mask_smem_bytes, (size_t)kSoloSmemMin);
   if (smem > (size_t)kSmemBudget) return fail(PDNN_INVALID_PARAMETER, "tensor-core gemm: plan needs %zu bytes of shared memory", smem);
   // The opt-in to large dynamic shared memory is a per-device attribute of each kernel: it is made
   // once for every device this process launches on, with that device current.
@@ -2506,7 +2587,9 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
         for (int epi = 0; epi < 7; ++epi)
           for (int dt = 0; dt < 3; ++dt) {
             GemmKernel k = select_kernel(sp != 0, epi, dt);
-            if (k != nullptr && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) != cudaSuccess) {
+            // (the whole of an SM's memory as shared memory: two CTAs of a solo plan are to fit)
+            if (k != nullptr && (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) != cudaSuccess ||
+                                 cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)) {
               cudaGetLastError();
               return fail(PDNN_ALLOCATION_PROBLEM, "cannot opt in to %d bytes of shared memory", kSmemBudget);
             }
@@ -2525,8 +2608,8 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
   GemmKernel kernel = g.group_k != 0 ? select_grouped_kernel(epi, g.out_dtype) : select_kernel(split, epi, g.out_dtype);
   if (kernel == nullptr) return fail(PDNN_INVALID_PARAMETER, "tensor-core gemm: no kernel for this output type");
   const int sms = device_sm_count();
-  unsigned grid = (unsigned)std::min<long long>(total, (long long)sms);
-  if (g.b_res == 2 || g.bias_tile_only) {
+  unsigned grid = (unsigned)(g.solo ? total : std::min<long long>(total, (long long)sms));
+  if (!g.solo && (g.b_res == 2 || g.bias_tile_only)) {
     // every CTA stays on one column tile: tiles advance by a multiple of n_tiles
     if (grid < (unsigned)g.n_tiles) return fail(PDNN_INVALID_PARAMETER, "tensor-core gemm: grid smaller than the column tiles");
     grid -= grid % (unsigned)g.n_tiles;
@@ -2535,7 +2618,7 @@ int launch_gemm(const GemmArgs& g, int dtype, cudaStream_t s) {
   // in the stream (the kernel waits for that kernel before it touches any tensor it wrote).
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(split ? kSplitThreads : 384);
+  cfg.blockDim = dim3(split ? kSplitThreads : g.groups == 1 ? 192 : 384);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -2599,7 +2682,7 @@ bool multi_launchable(const GemmArgs* list, int count, int sms) {
   int min_ctas = 0;
   for (int i = 0; i < count; ++i) {
     const GemmArgs& g = list[i];
-    if (gemm_epilogue_kind(g) != epi || g.out_dtype != list[0].out_dtype || g.cta_pair || g.a_mn) return false;
+    if (gemm_epilogue_kind(g) != epi || g.out_dtype != list[0].out_dtype || g.cta_pair || g.a_mn || g.solo) return false;
     // a GEMM without reduction steps only writes zeros: side by side it would take SMs from the ones that
     // compute and finish no sooner (measured on a strided 1x1 layer: 0.31 against 0.21 ms)
     if (g.num_taps < 1) return false;
@@ -2853,7 +2936,7 @@ int finish_forward(GemmArgs& g, int dtype, void* y, const PdnnConv2DParams& p, c
   if (cluster != 0) return cluster_epilogue_ok(g) ? launch_gemm_cluster(g, cluster, s) : kPlanAgain;
   const uint64_t od[4] = {(uint64_t)p.features, (uint64_t)p.out_cols, (uint64_t)p.out_rows, (uint64_t)p.batch};
   const uint64_t os[3] = {(uint64_t)ld * es, (uint64_t)p.out_cols * ld * es, (uint64_t)p.out_rows * p.out_cols * ld * es};
-  if (!setup_store(g, dtype, od, os)) return (g.halo || g.pair) ? kPlanAgain : PDNN_INVALID_PARAMETER;
+  if (!setup_store(g, dtype, od, os, plan_out == nullptr)) return (g.halo || g.pair) ? kPlanAgain : PDNN_INVALID_PARAMETER;
   if (plan_out != nullptr) {
     *plan_out = g;
     return PDNN_OK;
@@ -3594,11 +3677,12 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
         // Accumulating form (dx += ...): inside the packed 16-bit epilogue when that runs, else through
         // the general epilogue's beta.
         g.accumulate = accumulate ? 1 : 0;
-        bool planned = setup_store(g, dtype, od, os);
+        const bool solo = p.stride_rows == 1 && p.stride_cols == 1;  // (several classes go side by side in one launch)
+        bool planned = setup_store(g, dtype, od, os, solo);
         if (planned && accumulate && !g.epi_fast) {
           g.accumulate = 0;
           g.beta = 1.f;
-          planned = setup_store(g, dtype, od, os);
+          planned = setup_store(g, dtype, od, os, solo);
         }
         if (!planned) {
           if (g.halo || g.pair) return conv_input_backprop(dtype, dy, w, dx, p, relu_mask, mask_bits, accumulate, constant_filter, s, false, try_cluster);  // plan again without the halo / pairing
