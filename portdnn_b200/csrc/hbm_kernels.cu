@@ -205,10 +205,11 @@ __global__ void __launch_bounds__(kBlock)
 template <typename T, int OP, int V, typename Index>
 __global__ void __launch_bounds__(kBlock)
     pool_max_grad_tiled_kernel(const T* x, const T* y, const T* dy,
-                               T* __restrict__ dx, PdnnPoolingParams p, Index n_items) {
+                               T* __restrict__ dx, PdnnPoolingParams p, Index n_items, bool down) {
   overlap_wait();
   const Index cvecs = (Index)(p.channels / V);
-  for (Index idx = (Index)blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += (Index)gridDim.x * kBlock) {
+  for (Index i0 = (Index)blockIdx.x * kBlock + threadIdx.x; i0 < n_items; i0 += (Index)gridDim.x * kBlock) {
+    const Index idx = down ? n_items - 1 - i0 : i0;
     const Index cv = idx % cvecs;
     Index t = idx / cvecs;
     const int ow = (int)(t % (Index)p.out_cols);
@@ -428,13 +429,15 @@ __global__ void __launch_bounds__(kBlock)
 struct PoolS2Geometry {
   int H, W, Ho, Wo, C, pad_r, pad_c, N;
   int M, K, rows, strips;
+  int down;  // the last images first (reads_from_the_end)
 };
 
 template <typename T, int V>
 __device__ __forceinline__ void pool_max_grad_s2(const unsigned char* winner, const T* dy, T* dx, const PoolS2Geometry& g,
                                                  unsigned n_items) {
   const unsigned cvecs = (unsigned)(g.C / V);
-  for (unsigned idx = blockIdx.x * kBlock + threadIdx.x; idx < n_items; idx += gridDim.x * kBlock) {
+  for (unsigned i0 = blockIdx.x * kBlock + threadIdx.x; i0 < n_items; i0 += gridDim.x * kBlock) {
+    const unsigned idx = g.down ? n_items - 1 - i0 : i0;
     const unsigned cv = idx % cvecs;
     unsigned t = idx / cvecs;
     const int k = (int)(t % (unsigned)g.K);
@@ -1480,6 +1483,7 @@ struct StripGeometry {
   int rows_per_thread, wgroups, hchunks;
   int flip;  // MODE 0: read the filter mirrored in both window axes (stride-1 input backprop)
   int positive_only;  // MODE 3 / 4: a window whose maximum is not positive has no winner
+  int down;           // the last images first (reads_from_the_end)
 };
 
 // MODE 0: depthwise 3x3 (needs Packet::fma); MODE 1: max ignoring NaN; MODE 2: max keeping NaN;
@@ -1495,7 +1499,7 @@ __global__ void __launch_bounds__(kStripBlock)
   constexpr int V = 16 / sizeof(T);
   constexpr int kStripW = StripWidth<ST>::value;
   constexpr int NIN = (kStripW - 1) * ST + 3;
-  const size_t idx = (size_t)blockIdx.x * kStripBlock + threadIdx.x;
+  const size_t idx = (size_t)(g.down ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * kStripBlock + threadIdx.x;
   if (idx >= n_threads) return;
   const int cvecs = g.channels / V;
   const int cv = (int)(idx % cvecs);
@@ -1626,7 +1630,7 @@ __global__ void __launch_bounds__(kStripBlock, 3)
   // these blocks has started.  (Both are no-ops under an ordinary launch.)
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const size_t idx = (size_t)blockIdx.x * kStripBlock + threadIdx.x;
+  const size_t idx = (size_t)(g.down ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * kStripBlock + threadIdx.x;
   if (idx >= n_threads) return;
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dw_async_smem) + threadIdx.x * 16u;
   const int cvecs = g.channels / V;
@@ -1789,6 +1793,7 @@ int launch_window3_strip(const T* x, const T* w, T* y, int stride, StripGeometry
     const size_t want = (size_t)sms * 1024;
     while (rows > 1 && per_row_chunk * ((g.out_rows + rows - 1) / rows) < want) rows >>= 1;
   }
+  g.down = MODE < 3 && reads_from_the_end((size_t)g.batch * g.in_rows * g.in_cols * g.channels * sizeof(T));
   g.rows_per_thread = rows;
   g.hchunks = (g.out_rows + rows - 1) / rows;
   const size_t n_threads = per_row_chunk * g.hchunks;
@@ -1939,13 +1944,14 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
         (p.out_cols - 1) * p.stride_cols < p.in_cols && p.in_rows < (p.out_rows + 1) * p.stride_rows &&
         p.in_cols < (p.out_cols + 1) * p.stride_cols) {
       // no window overlaps another, and less than a window is left over at the edges: one pass
+      const bool down = reads_from_the_end(in_items * VN * sizeof(T));
       const unsigned g1 = grid_for(out_items, kBlock, sms);
       if (op == PDNN_POOL_MAX)
         launch_overlapped(pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX, VN, unsigned>, g1, kBlock, s, xt, yt, dyt, dxt, p,
-                          (unsigned)out_items);
+                          (unsigned)out_items, down);
       else
         launch_overlapped(pool_max_grad_tiled_kernel<T, PDNN_POOL_MAX_WITH_NAN, VN, unsigned>, g1, kBlock, s, xt, yt, dyt,
-                          dxt, p, (unsigned)out_items);
+                          dxt, p, (unsigned)out_items, down);
       return check_launch("pooling max gradient (tiling windows)");
     }
     if (vec && small && p.window_rows * p.window_cols < 255) {
@@ -1974,7 +1980,8 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
         int st = check_launch("pooling max gradient (winners)");
         if (st == PDNN_OK && p.window_rows == 3 && p.window_cols == 3 && p.stride_rows == 2 && p.stride_cols == 2) {
           PoolS2Geometry g{p.in_rows, p.in_cols, p.out_rows, p.out_cols, p.channels, p.pad_rows, p.pad_cols, p.batch,
-                           (p.in_rows - 1 + p.pad_rows) / 2 + 1, (p.in_cols - 1 + p.pad_cols) / 2 + 1, 0, 0};
+                           (p.in_rows - 1 + p.pad_rows) / 2 + 1, (p.in_cols - 1 + p.pad_cols) / 2 + 1, 0, 0,
+                           reads_from_the_end(in_items * VN * sizeof(T))};
           const size_t columns = (size_t)p.batch * g.K * (p.channels / VN);
           g.rows = g.M;
           while (g.rows > 4 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 2048) g.rows = (g.rows + 1) / 2;

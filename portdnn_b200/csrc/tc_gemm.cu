@@ -74,6 +74,10 @@ struct alignas(64) GemmArgs {
   int tap_pack;      // a_mn == 1: taps per tile (2: the second 64 rows of the A tile are the next tap's channels)
   int cblocks;       // a_mn == 0: reduction blocks per tap
   int slabs_w, slabs_h, slabs_n, splits, slabs_per_split, split_is_batch;  // a_mn == 1
+  // a_mn == 1: slabs from one step of a split to the next (1, or as many as there are splits) and its digits; not 0 in a plan:
+  // the splits go through the batch side by side (reads_from_the_end)
+  int slab_step, step_w, step_h, step_n;
+  int images_down;   // a_mn == 0: the last images first (reads_from_the_end)
   int b_batch_mul;
   int stages, tmem_cols;
   unsigned idesc;
@@ -202,7 +206,8 @@ struct TileWalker {
       // in pair mode the paired dimension's digit counts pairs of tiles
       t.w0 = (a.pair_dim == 1 ? 2 * d1 : d1) * a.tw;
       t.h0 = (a.pair_dim == 2 ? 2 * d2 : d2) * a.th;
-      t.n0 = (a.pair_dim == 3 ? 2 * d3 : d3) * a.tn;
+      const int image = a.images_down ? a.tiles_n - 1 - d3 : d3;
+      t.n0 = (a.pair_dim == 3 ? 2 * image : image) * a.tn;
       t.tap = 0;
       t.split = 0;
       t.out_off = 0;
@@ -216,8 +221,13 @@ struct TileWalker {
       t.n0 = 0;
       t.out_off = (long long)t.split * a.split_stride + (a.tap_pack > 1 ? 0ll : (long long)t.tap * a.tap_stride);
       const int total = a.slabs_w * a.slabs_h * a.slabs_n;
-      t.ks_begin = a.split_is_batch ? 0 : t.split * a.slabs_per_split;
-      t.ks_end = min(t.ks_begin + a.slabs_per_split, total);
+      if (a.slab_step > 1) {  // slabs split, split + splits, ...: counted from the first
+        t.ks_begin = t.split;
+        t.ks_end = t.split + (total - t.split + a.slab_step - 1) / a.slab_step;
+      } else {
+        t.ks_begin = a.split_is_batch ? 0 : t.split * a.slabs_per_split;
+        t.ks_end = min(t.ks_begin + a.slabs_per_split, total);
+      }
     }
     return t;
   }
@@ -1015,15 +1025,15 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
             } else {  // B_K_4
               warp_tma_load_4d(sb, &a.b_map, fb, kw, t.nf0, 0, kn);
             }
-            kw += a.tw;
-            if (++iw == a.slabs_w) {
-              iw = kw = 0;
-              kh += a.th;
-              if (++ih == a.slabs_h) {
-                ih = kh = 0;
-                kn += a.tn;
-              }
-            }
+            iw += a.step_w;
+            const bool wrap_w = iw >= a.slabs_w;
+            iw -= wrap_w ? a.slabs_w : 0;
+            ih += a.step_h + (wrap_w ? 1 : 0);
+            const bool wrap_h = ih >= a.slabs_h;
+            ih -= wrap_h ? a.slabs_h : 0;
+            kn += (a.step_n + (wrap_h ? 1 : 0)) * a.tn;
+            kw = iw * a.tw;
+            kh = ih * a.th;
             next_stage();
           }
         }
@@ -1733,13 +1743,13 @@ __global__ void __launch_bounds__(192, 1) umma_gemm_filter_pair_kernel(const __g
         warp_tma_load_4d_pair(sa + kABytes / 2, amap, fb, t.w0 + 64, kw + e.dw, kh + e.dh, kn);
         warp_tma_load_4d_pair(sa + kABytes, &a.b_map, fb, f0, kw, kh, kn);
         warp_tma_load_4d_pair(sa + kABytes + kABytes / 2, &a.b_map, fb, f0 + 64, kw, kh, kn);
-        if (++iw == a.slabs_w) {
-          iw = 0;
-          if (++ih == a.slabs_h) {
-            ih = 0;
-            ++in;
-          }
-        }
+        iw += a.step_w;
+        const bool wrap_w = iw >= a.slabs_w;
+        iw -= wrap_w ? a.slabs_w : 0;
+        ih += a.step_h + (wrap_w ? 1 : 0);
+        const bool wrap_h = ih >= a.slabs_h;
+        ih -= wrap_h ? a.slabs_h : 0;
+        in += a.step_n + (wrap_h ? 1 : 0);
         if (++s == S) {
           s = 0;
           ph ^= 1u;
@@ -2481,8 +2491,16 @@ GemmKernel select_grouped_kernel(int epi, int out_dtype) {
 
 thread_local const char* t_last_kernel = "";
 
-// (after tap_pack has its final value)
+// (after tap_pack and the slabs have their final values)
+void set_slab_order(GemmArgs& g, bool interleaved) {
+  g.slab_step = (interleaved && g.splits > 1 && !g.split_is_batch) ? g.splits : 1;
+  g.step_w = g.slab_step % g.slabs_w;
+  g.step_h = g.slab_step / g.slabs_w % g.slabs_h;
+  g.step_n = g.slab_step / g.slabs_w / g.slabs_h;
+}
+
 void set_walk_magic(GemmArgs& g) {
+  if (g.a_mn) set_slab_order(g, g.slab_step != 0);
   const unsigned long long radix[3] = {(unsigned long long)g.n_tiles, (unsigned long long)g.tiles_w,
                                        (unsigned long long)(g.a_mn ? (g.num_taps + g.tap_pack - 1) / g.tap_pack : g.tiles_h)};
   for (int i = 0; i < 3; ++i) g.walk_magic[i] = ((1ull << 32) + radix[i] - 1) / std::max(radix[i], 1ull);
@@ -3300,6 +3318,8 @@ int conv_forward(int dtype, const void* x, const void* w, void* y, const PdnnCon
   const uint32_t abox[4] = {(uint32_t)epr, (uint32_t)g.tw, (uint32_t)(halo ? g.th + p.window_rows - 1 : g.th),
                             (uint32_t)g.tn};
   g.early_b = (epi != nullptr && epi->constant_filter != 0 && dtype != PDNN_F32) ? 1 : 0;
+  g.images_down = dtype != PDNN_F32 && p.window_rows * p.window_cols == 1 && p.features <= p.channels &&
+                  reads_from_the_end((size_t)p.batch * p.in_rows * p.in_cols * p.channels * es);
   if (!make_parity_maps(g, dtype, false, x, p, abox, x_ld)) return PDNN_INVALID_PARAMETER;
   // taps
   int nt = 0;
@@ -3528,6 +3548,8 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
       std::memset(&g, 0, sizeof(g));
       g.a_mn = 0;
       g.early_b = (constant_filter && dtype != PDNN_F32) ? 1 : 0;
+      g.images_down = dtype != PDNN_F32 && reads_from_the_end((size_t)p.batch * es * std::max((size_t)p.out_rows * p.out_cols * p.features,
+                                                                                             (size_t)p.in_rows * p.in_cols * p.channels));
       // Stride 1: the taps of one window column read overlapping rows of dy, as in the forward
       // pass (halo mode), if the whole filter can stay in shared memory.
       int hw = 0, hh = 0;
@@ -3874,6 +3896,8 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
   g.slabs_n = f.slabs_n;
   g.splits = f.splits;
   g.slabs_per_split = f.slabs_per_split;
+  g.slab_step = dtype != PDNN_F32 && reads_from_the_end((size_t)p.batch * es * std::max((size_t)p.out_rows * p.out_cols * p.features,
+                                                                                       (size_t)p.in_rows * p.in_cols * p.channels));
   set_operand_layout(g, dtype, 1);
   const size_t row_pitch = (size_t)q.sp.Wp * 16;
   const uint32_t box[4] = {(uint32_t)epr, (uint32_t)f.tw, (uint32_t)f.th, (uint32_t)f.tn};
@@ -3991,6 +4015,8 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
   g.slabs_n = f.slabs_n;
   g.splits = f.splits;
   g.slabs_per_split = f.slabs_per_split;
+  g.slab_step = dtype != PDNN_F32 && reads_from_the_end((size_t)p.batch * es * std::max((size_t)p.out_rows * p.out_cols * p.features,
+                                                                                       (size_t)p.in_rows * p.in_cols * p.channels));
   g.split_is_batch = 0;
   set_operand_layout(g, dtype, 1);
   if (f.pair) {
