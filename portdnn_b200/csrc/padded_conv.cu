@@ -1,6 +1,6 @@
 // Convolutions of 16-bit tensors whose channel or feature count is not a multiple of 8 (or whose tensors
 // start off a 16-byte boundary): TMA needs rows that start on 16 bytes, so the operands are copied into
-// rows padded with zeros to the next multiple of 8, the tensor-core kernels run on the copies, and what they
+// rows padded with zeros (padded_count), the tensor-core kernels run on the copies, and what they
 // wrote is cut back.  The padding adds zero terms to the sums and columns that are dropped; operands that
 // are in order are read, and results written, in place.
 //
@@ -123,6 +123,16 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
+// A count off a multiple of 8, padded.  A multiple of 8 would do, but rows that start inside a 32-byte sector cost the tiles' loads
+// one more sector and often a second line each (bf16, us, 7x45x61 3x3, input gradient: 128 -> 152 features 27.0, 160 16.5,
+// 192 13.1; forward pass, 104 -> 128 channels 14.5, 112 11.7, 128 10.1).  So whole lines of 64 where they
+// are hardly more to copy, else whole sectors of 16.
+int padded_count(int n) {
+  if (n % 8 == 0) return n;
+  const int lines = (int)round_up((size_t)n, 64);
+  return 10ll * lines <= 13ll * n ? lines : (int)round_up((size_t)n, 16);
+}
+
 struct Plan {
   PdnnConv2DParams q;          // the convolution the tensor-core kernels run
   size_t x, w, y;              // elements of the padded tensors
@@ -137,9 +147,9 @@ bool make_plan(int pass, int dtype, const PdnnConv2DParams& p, Plan* plan) {
   if (p.filter_format != 0 && p.filter_format != 2) return false;
   PdnnConv2DParams q = p;
   const void* aligned = reinterpret_cast<const void*>(uintptr_t(256));
-  q.features = (int)round_up((size_t)p.features, 8);
+  q.features = padded_count(p.features);
   if (!tc_conv_supported(pass, dtype, aligned, aligned, aligned, q)) {
-    q.channels = (int)round_up((size_t)p.channels, 8);
+    q.channels = padded_count(p.channels);
     if (!tc_conv_supported(pass, dtype, aligned, aligned, aligned, q)) return false;
   }
   const size_t px_in = (size_t)p.batch * p.in_rows * p.in_cols, px_out = (size_t)p.batch * p.out_rows * p.out_cols;
