@@ -63,6 +63,17 @@ struct Lanes<float> {
   static __device__ __forceinline__ float get(V v, int) { return v; }
 };
 
+// Two fp16 channels summed in fp16, tap by tile column, as window3_strip_kernel does: the same bits.
+struct HalfSums {
+  static constexpr int E = 2;
+  using V = __half2;
+  static __device__ __forceinline__ V zero() { return __float2half2_rn(0.f); }
+  static __device__ __forceinline__ V unpack(unsigned w) { return *reinterpret_cast<const __half2*>(&w); }
+  static __device__ __forceinline__ unsigned pack(V v) { return *reinterpret_cast<const unsigned*>(&v); }
+  static __device__ __forceinline__ void fma(V& acc, V a, V b) { acc = __hfma2(a, b, acc); }
+  static __device__ __forceinline__ float get(V v, int e) { return e ? __high2float(v) : __low2float(v); }
+};
+
 // One block to an SM.  Filter gradient, us, 128 images, f16, 56x56x144 / 112x112x32 / 28x28x192 / 7x7x960: two blocks of
 // two stages of 54 KB 67 / 47 / 22 / 16, one block of three of 72 KB 49 / 45 / 21 / 13, four of 54 KB 57 / 49 / 22 /
 // 13: larger tiles read fewer rows twice, and a block's stages are filled one after another, not in bursts.
@@ -78,6 +89,7 @@ struct Tiles {
   unsigned tiles;          // of one chunk: tiles_w * tiles_h * images
   int channels, in_rows, in_cols, out_rows, out_cols, pad_rows, pad_cols;
   int mirrored;            // the filter's taps in reverse order (input gradient)
+  int down;                // the last images first (reads_from_the_end)
   unsigned x_bytes, dy_off, dy_bytes, stage_bytes;
   unsigned* error_record;
 };
@@ -266,12 +278,13 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
 // complemented, on the same tiles and walk: nine multiply-adds in fp32 to a pair of channels, one rounding.  Bound by
 // HBM; one thread to an output packet with nine loads of it, as these layers ran before, by the loads.  bf16, us, 128
 // images: 56x56x144 forward 184 -> 44, input gradient 285 -> 44; 112x112x96 / 2 forward 134 -> 64; 7x7x960 20 -> 8.5.
-// (fp16 and fp32 have the strip kernels with sums in the tensors' type, 45.6 us for 56x56x144; on these tiles fp16
-// measured between 13 % slower, 61x61x88, and 10 % faster, 14x14x576.)
-template <typename T, int ST, int TW>
+// fp16 sums in fp16 (HalfSums), against the strips of depthwise3_async_kernel, whose 111 instructions to a 16-byte packet -
+// copies, slots, addresses - are twice what is left here; us, strips / tiles: 128 images 112x112x32 43.7 / 35.1, 56x56x144 45.9 /
+// 40.2 (5.8 TB/s), 14x14x576 16.3 / 11.9, 7x7x960 9.7 / 7.5; 64 images 112x112x96 / 2 38.5 / 34.2, 28x28x192 10.3 / 9.2.
+// (fp32 has the strips.)
+template <typename T, typename L, int ST, int TW>
 __global__ void __launch_bounds__(kTileThreads + 32, 1)
     depthwise_forward_tile_kernel(const __grid_constant__ CUtensorMap x_map, const T* filter, T* out, const Tiles g) {
-  using L = Lanes<T>;
   using V = typename L::V;
   constexpr int E = L::E, XW = (TW - 1) * ST + 3, ROWS = ST + 3;
   extern __shared__ uint8_t smem_raw[];
@@ -299,7 +312,8 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
   if (warp == workers) {
     if (lane == 0) prefetch_tensormap(&x_map);
 #pragma unroll 1
-    for (unsigned tile = (unsigned)slice; tile < g.tiles; tile += (unsigned)g.slices) {
+    for (unsigned i = (unsigned)slice; i < g.tiles; i += (unsigned)g.slices) {
+      const unsigned tile = g.down ? g.tiles - 1u - i : i;
       const int tw = (int)(tile % (unsigned)g.tiles_w);
       const unsigned rest = tile / (unsigned)g.tiles_w;
       const int w0 = tw * TW, h0 = (int)(rest % (unsigned)g.tiles_h) * 2 * strips, n = (int)(rest / (unsigned)g.tiles_h);
@@ -325,7 +339,8 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
     const int row = XW * words;
     const size_t image_words = (size_t)g.out_rows * g.out_cols * pixel_words;
 #pragma unroll 1
-    for (unsigned tile = (unsigned)slice; tile < g.tiles; tile += (unsigned)g.slices) {
+    for (unsigned i = (unsigned)slice; i < g.tiles; i += (unsigned)g.slices) {
+      const unsigned tile = g.down ? g.tiles - 1u - i : i;
       if (!mbar_wait(full_bar(s), ph, abort_flag, g.error_record, kWaitLimitNs, 0x1800u + (unsigned)s)) break;
       const int tw = (int)(tile % (unsigned)g.tiles_w);
       const unsigned rest = tile / (unsigned)g.tiles_w;
@@ -352,9 +367,9 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
               for (int k = 0; k < 2; ++k) {
                 V acc = L::zero();
 #pragma unroll
-                for (int r = 0; r < 3; ++r)
-#pragma unroll
-                  for (int c = 0; c < 3; ++c) {
+                for (int t = 0; t < 9; ++t) {
+                    constexpr bool by_column = std::is_same<L, HalfSums>::value;
+                    const int r = by_column ? t % 3 : t / 3, c = by_column ? t / 3 : t % 3;
                     // a tap outside the image is no term of the sum: the zero there and an infinite weight would be one
                     if (!decltype(every_tap)::value) {
                       const int ih = (h0 + k) * ST - g.pad_rows + r, iw = (w0 + j) * ST - g.pad_cols + c;
@@ -445,7 +460,7 @@ bool plan_tiles(const PdnnDepthwiseConv2DParams& p, int elems, bool filter_gradi
   out->out_cols = p.out_cols;
   out->pad_rows = p.pad_rows;
   out->pad_cols = p.pad_cols;
-  out->mirrored = 0;
+  out->mirrored = out->down = 0;
   out->error_record = tc_error_record_address();
   return out->error_record != nullptr;
 }
@@ -503,12 +518,12 @@ int launch_filter_tiles(const CUtensorMap& x_map, const CUtensorMap& dy_map, con
   return g.slices;
 }
 
-template <typename T, int ST, int TW>
+template <typename T, typename L, int ST, int TW>
 bool launch_forward_tiles(const CUtensorMap& x_map, const void* filter, void* out, const Tiles& g, cudaStream_t s) {
   static std::mutex mu;
   static bool done[kMaxDevices] = {};
-  if (!opt_in(depthwise_forward_tile_kernel<T, ST, TW>, mu, done)) return false;
-  launch_tiles(depthwise_forward_tile_kernel<T, ST, TW>, g, 0, s, x_map, static_cast<const T*>(filter), static_cast<T*>(out), g);
+  if (!opt_in(depthwise_forward_tile_kernel<T, L, ST, TW>, mu, done)) return false;
+  launch_tiles(depthwise_forward_tile_kernel<T, L, ST, TW>, g, 0, s, x_map, static_cast<const T*>(filter), static_cast<T*>(out), g);
   return true;
 }
 
@@ -544,18 +559,21 @@ int launch_depthwise_filter_tiles(int dtype, const void* x, const void* dy, floa
   });
 }
 
-bool launch_depthwise_forward_tiles_bf16(const void* x, const void* filter, void* out, const PdnnDepthwiseConv2DParams& p,
-                                         bool mirrored, cudaStream_t s) {
+bool launch_depthwise_forward_tiles(int dtype, const void* x, const void* filter, void* out, const PdnnDepthwiseConv2DParams& p,
+                                    bool mirrored, cudaStream_t s) {
   Tiles g;
   if (!tile_layer(p, 2) || !aligned16(x) || !aligned16(filter) || !aligned16(out) || !plan_tiles(p, 2, false, &g)) return false;
   // (offsets in a strip's two rows are 32-bit words in an int: in 64 bits 56x56x144, 128 images, took 44.4 us, not 43.2)
   if ((long long)p.out_cols * p.channels > 0x7FFFFFFFll) return false;
   g.mirrored = mirrored ? 1 : 0;
+  g.down = reads_from_the_end((size_t)p.batch * p.in_rows * p.in_cols * p.channels * 2);
   g.slices = std::max(1, std::min<int>(device_sm_count() / g.chunks, (int)std::min<unsigned>(g.tiles, 1u << 20)));
   CUtensorMap x_map;
-  if (!x_tile_map(&x_map, PDNN_BF16, x, p, g, 2)) return false;
+  if (!x_tile_map(&x_map, dtype, x, p, g, 2)) return false;
   return with_tile_shape(p.stride_rows, g.tw, [&](auto st, auto tw) {
-    return launch_forward_tiles<__nv_bfloat16, decltype(st)::value, decltype(tw)::value>(x_map, filter, out, g, s);
+    constexpr int ST = decltype(st)::value, TW = decltype(tw)::value;
+    return dtype == PDNN_F16 ? launch_forward_tiles<__half, HalfSums, ST, TW>(x_map, filter, out, g, s)
+                             : launch_forward_tiles<__nv_bfloat16, Lanes<__nv_bfloat16>, ST, TW>(x_map, filter, out, g, s);
   });
 }
 

@@ -11,9 +11,9 @@ namespace pdnn {
 int launch_depthwise_filter_tiles(int dtype, const void* x, const void* dy, float* partial, const PdnnDepthwiseConv2DParams& p,
                                   int max_slices, cudaStream_t s);
 
-// Forward pass of bf16 tensors; mirrored: with the filter's taps in reverse order, which with the tensors' and paddings' roles exchanged
+// Forward pass of 16-bit tensors; mirrored: with the filter's taps in reverse order, which with the tensors' and paddings' roles exchanged
 // in p is the input gradient of stride 1.  False where the layer is not for this kernel.
-bool launch_depthwise_forward_tiles_bf16(const void* x, const void* filter, void* out, const PdnnDepthwiseConv2DParams& p,
-                                         bool mirrored, cudaStream_t s);
+bool launch_depthwise_forward_tiles(int dtype, const void* x, const void* filter, void* out, const PdnnDepthwiseConv2DParams& p,
+                                    bool mirrored, cudaStream_t s);
 
 }  // namespace pdnn
