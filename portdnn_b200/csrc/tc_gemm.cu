@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace pdnn {
@@ -71,7 +72,7 @@ struct alignas(64) GemmArgs {
   int num_taps;
   int b_presplit;    // fp32 (3xTF32): the lo part of B arrives by TMA too (b_map_lo); only A is split in the kernel
   int cta_pair;      // 1: run by umma_gemm_pair2_kernel (clusters of two CTAs, 256 x 256 tiles)
-  int tap_pack;      // a_mn == 1: taps per tile (2: the second 64 rows of the A tile are the next tap's channels)
+  int tap_pack;      // a_mn == 1: taps per tile (2: the second 64 rows of the A tile are the next tap's channels; 4: 32 rows to a tap)
   int cblocks;       // a_mn == 0: reduction blocks per tap
   int slabs_w, slabs_h, slabs_n, splits, slabs_per_split, split_is_batch;  // a_mn == 1
   // a_mn == 1: slabs from one step of a split to the next (1, or as many as there are splits) and its digits; not 0 in a plan:
@@ -985,7 +986,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
           const CUtensorMap* amap = &a.a_map[e.a_map];
           // packed taps: the second half of the boxes holds the same channels as seen by the next tap (none: boxes
           // beyond the last channel, which TMA fills with zeros)
-          const bool packed = a.tap_pack > 1, second = packed && t.tap + 1 < a.num_taps;
+          const bool packed = a.tap_pack > 1, second = packed && t.tap + 1 < a.num_taps, narrow = !SPLIT && a.tap_pack == 4;
           const TapEntry e2 = a.taps[second ? t.tap + 1 : t.tap];
           const int half = packed ? a_boxes >> 1 : a_boxes;  // boxes of the first tap
           const CUtensorMap* amap2 = &a.a_map[e2.a_map];
@@ -1004,6 +1005,14 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
             }
             const uint32_t fb = full_bar(s), sb = sa + kABytes;
             warp_arrive_expect_tx(fb, tx_bytes);
+            if (narrow) {  // a box to a tap
+#pragma unroll 1
+              for (int j = 0; j < 4; ++j) {
+                const bool there = t.tap + j < a.num_taps;
+                const TapEntry ej = a.taps[there ? t.tap + j : t.tap];
+                warp_tma_load_4d(sa + (uint32_t)j * a_box_bytes, &a.a_map[ej.a_map], fb, there ? 0 : 0x40000000, kw + ej.dw, kh + ej.dh, kn);
+              }
+            } else {
             warp_tma_load_4d(sa, amap, fb, t.w0, kw + e.dw, kh + e.dh, kn);
             if (packed) warp_tma_load_4d(sa + (uint32_t)half * a_box_bytes, amap2, fb, c2nd, kw + e2.dw, kh + e2.dh, kn);
             else warp_tma_load_4d(sa + a_box_bytes, amap, fb, t.w0 + epr, kw + e.dw, kh + e.dh, kn);
@@ -1015,6 +1024,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
                 warp_tma_load_4d(sa + 2u * a_box_bytes, amap, fb, t.w0 + 2 * epr, kw + e.dw, kh + e.dh, kn);
                 warp_tma_load_4d(sa + 3u * a_box_bytes, amap, fb, t.w0 + 3 * epr, kw + e.dw, kh + e.dh, kn);
               }
+            }
             }
             if (b_mode == B_MN_4) {
               warp_tma_load_4d(sb, &a.b_map, fb, t.nf0, kw, kh, kn);
@@ -3820,31 +3830,49 @@ FbpPlan plan_filter_backprop(int dtype, const PdnnConv2DParams& p, int sms, bool
 // Xr is the 128-byte packed run of 8 pixels x CP channels that output pixel reads for filter
 // row r.  The 64 rows of the result are exactly [s (8)][c (CP)], i.e. the packed filter layout;
 // the final kernel sums the pixel splits and drops the padding entries.
-template <typename T, typename OutT = T>
+// A block has 32 outputs, its eight warps take every eighth split each: with one thread to an output the loop over 148 splits
+// is what the kernel waits for (24 images of 224x224x3, 7x7/2 to 64 features: the
+// gradient 48.6 -> 39.1 us).
+template <typename OutT>
 __global__ void __launch_bounds__(256)
     unpack_small_c_filter_grad_kernel(const float* partial, OutT* __restrict__ dw, int splits, int R, int S,
-                                      int C, int K, int rows_per_tap, bool accumulate) {
+                                      int C, int K, int CP, bool accumulate) {
   overlap_wait();
-  constexpr int CP = 16 / sizeof(T);
-  const size_t total = (size_t)R * S * C * K;
-  const size_t split_stride = (size_t)R * rows_per_tap * K;
-  for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (size_t)gridDim.x * 256) {
+  __shared__ float sums[8][32];
+  const int rows_per_tap = 8 * CP, lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+  const size_t total = (size_t)R * S * C * K, split_stride = (size_t)R * rows_per_tap * K;
+  const size_t idx = (size_t)blockIdx.x * 32 + lane;
+  float sum = 0.f;
+  if (idx < total) {
     const int k = (int)(idx % K);
     size_t t = idx / K;
     const int c = (int)(t % C);
     t /= C;
     const int sidx = (int)(t % S);
     const int r = (int)(t / S);
-    const size_t src = ((size_t)r * rows_per_tap + (size_t)sidx * CP + c) * K + k;
-    float sum = accumulate ? to_f32(dw[idx]) : 0.f;
-    for (int sp = 0; sp < splits; ++sp) sum += partial[(size_t)sp * split_stride + src];
-    dw[idx] = from_f32<OutT>(sum);
+    const float* src = partial + ((size_t)r * rows_per_tap + (size_t)sidx * CP + c) * K + k;
+#pragma unroll 4
+    for (int sp = warp; sp < splits; sp += 8) sum += src[(size_t)sp * split_stride];
   }
+  sums[warp][lane] = sum;
+  __syncthreads();
+  if (warp != 0 || idx >= total) return;
+  sum = accumulate ? to_f32(dw[idx]) : 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sum += sums[i][lane];
+  dw[idx] = from_f32<OutT>(sum);
 }
 
+// What bounds the stem is the rows that TMA brings in, of 128 or of 64 bytes alike, about one in two cycles: a 64-pixel step has 128
+// of A and 64 of dy, for every pair of filter rows again.  With 8 channels to a pixel two filter rows fill a tile
+// (tap_pack 2); with 4 channels - 64-byte rows, where an even column stride keeps them on 16 bytes - four do: 320 rows
+// for four instead of 384, half the MMAs, half the bytes to pack.  224x224x3, 7x7/2 to 64 features, f16, packing and second stage
+// included: 256 images 375 -> 285 us, 24 images 47 -> 39.
 struct SmallCFbpPlan {
   FbpPlan f;
   SmallCPlan sp;
+  bool narrow;  // 4 channels to a pixel
+  int rows;     // of a filter row's gradient: 8 pixels x channels
   size_t partial_bytes;
 };
 
@@ -3852,13 +3880,20 @@ SmallCFbpPlan plan_small_c_fbp(int dtype, const PdnnConv2DParams& p, int sms) {
   SmallCFbpPlan q;
   const int epr = dtype == PDNN_F32 ? 32 : 64;
   q.sp = plan_small_c(dtype, p);
+  q.narrow = dtype != PDNN_F32 && p.channels <= 4 && p.stride_cols % 2 == 0 && p.window_rows >= 3 &&
+             (size_t)p.batch * q.sp.Hp * (q.sp.Wp + 1) < 0x7FFFFFFFull;
+  if (q.narrow) {
+    q.sp.Wp = (q.sp.Wp + 1) / 2 * 2;  // rows stay 16-byte aligned
+    q.sp.xp_bytes = (((size_t)p.batch * q.sp.Hp * q.sp.Wp * 8) + 255) / 256 * 256;
+  }
+  q.rows = q.narrow ? 32 : epr;
   FbpPlan& f = q.f;
   choose_box(epr, p.out_cols, p.out_rows, p.batch, &f.tw, &f.th, &f.tn);
   f.slabs_w = ceil_div(p.out_cols, f.tw);
   f.slabs_h = ceil_div(p.out_rows, f.th);
   f.slabs_n = ceil_div(p.batch, f.tn);
   f.m_tiles = 1;
-  f.tap_pack = p.window_rows >= 2 ? 2 : 1;  // at most 64 packed rows per filter row: two per tile
+  f.tap_pack = q.narrow ? 4 : p.window_rows >= 2 ? 2 : 1;  // filter rows to a tile
   f.bn = std::min(dtype == PDNN_F32 ? 128 : 256, ceil_div(p.features, epr) * epr);
   f.n_tiles = ceil_div(p.features, f.bn);
   const long long out_tiles = (long long)f.n_tiles * ceil_div(p.window_rows, f.tap_pack);
@@ -3868,7 +3903,7 @@ SmallCFbpPlan plan_small_c_fbp(int dtype, const PdnnConv2DParams& p, int sms) {
   want = std::min<long long>(want, 512);
   f.slabs_per_split = (int)((total_slabs + want - 1) / want);
   f.splits = (int)((total_slabs + f.slabs_per_split - 1) / f.slabs_per_split);
-  q.partial_bytes = (((size_t)f.splits * p.window_rows * epr * p.features * sizeof(float)) + 255) / 256 * 256;
+  q.partial_bytes = (((size_t)f.splits * p.window_rows * q.rows * p.features * sizeof(float)) + 255) / 256 * 256;
   return q;
 }
 
@@ -3916,14 +3951,24 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
   g.slab_step = dtype != PDNN_F32 && reads_from_the_end((size_t)p.batch * es * std::max((size_t)p.out_rows * p.out_cols * p.features,
                                                                                        (size_t)p.in_rows * p.in_cols * p.channels));
   set_operand_layout(g, dtype, 1);
-  const size_t row_pitch = (size_t)q.sp.Wp * 16;
+  if (q.narrow) {  // A: blocks of 32 rows, 64 pixels of 64 bytes each, with the 64-byte swizzle
+    g.a_layout = 4;
+    g.a_lbo = g.a_box_bytes = 64u * 64u;
+    g.a_sbo = 8u * 64u;
+    g.a_kadv = 16u * 64u;
+    g.a_boxes = 4;
+  }
+  const int pix_bytes = q.narrow ? 8 : 16;
+  const size_t row_pitch = (size_t)q.sp.Wp * pix_bytes;
   const uint32_t box[4] = {(uint32_t)epr, (uint32_t)f.tw, (uint32_t)f.th, (uint32_t)f.tn};
+  const uint32_t a_box[4] = {(uint32_t)q.rows, (uint32_t)f.tw, (uint32_t)f.th, (uint32_t)f.tn};
   for (int r = 0; r < p.stride_rows; ++r) {
     const int Hq = ceil_div(q.sp.Hp - r, p.stride_rows);
-    const uint64_t dims[4] = {(uint64_t)epr, (uint64_t)p.out_cols, (uint64_t)std::max(Hq, 1), (uint64_t)p.batch};
-    const uint64_t st[3] = {(uint64_t)p.stride_cols * 16, (uint64_t)p.stride_rows * row_pitch,
+    const uint64_t dims[4] = {(uint64_t)q.rows, (uint64_t)p.out_cols, (uint64_t)std::max(Hq, 1), (uint64_t)p.batch};
+    const uint64_t st[3] = {(uint64_t)p.stride_cols * pix_bytes, (uint64_t)p.stride_rows * row_pitch,
                             (uint64_t)q.sp.Hp * row_pitch};
-    if (!make_map(&g.a_map[r], dtype, true, xp + (size_t)r * row_pitch, dims, st, box)) {
+    if (!make_map(&g.a_map[r], dtype, true, xp + (size_t)r * row_pitch, dims, st, a_box,
+                  q.narrow ? CU_TENSOR_MAP_SWIZZLE_64B : kDefaultSwizzle)) {
       release();
       return -1;
     }
@@ -3945,24 +3990,24 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
   set_epilogue(g, nullptr);
   g.out = partial;
   g.out_dtype = PDNN_F32;
-  g.ext_w = epr;  // the rows of a tap's result that exist: [s][c] of the packed filter
+  g.ext_w = q.rows;  // the rows of a tap's result that exist: [s][c] of the packed filter
   g.ext_h = g.ext_n = 1;
   g.ext_cols = p.features;
   g.stride_w = p.features;
-  g.tap_stride = (long long)epr * p.features;
-  g.split_stride = (long long)p.window_rows * epr * p.features;
+  g.tap_stride = (long long)q.rows * p.features;
+  g.split_stride = (long long)p.window_rows * q.rows * p.features;
   g.tap_pack = f.tap_pack;
-  if (f.tap_pack == 2) {  // two filter rows per tile: 2 x 64 accumulator rows
-    g.etw = 64;
-    g.eth = 2;
+  if (f.tap_pack > 1) {  // several filter rows to a tile: 2 x 64 or 4 x 32 accumulator rows
+    g.etw = kTileM / f.tap_pack;
+    g.eth = f.tap_pack;
     g.ext_h = p.window_rows;
     g.stride_h = g.tap_stride;
   }
   g.vec_ok = 1;
   {
-    const uint64_t od[4] = {(uint64_t)p.features, (uint64_t)epr, (uint64_t)p.window_rows, (uint64_t)f.splits};
-    const uint64_t os[3] = {(uint64_t)p.features * 4, (uint64_t)epr * p.features * 4,
-                            (uint64_t)p.window_rows * epr * p.features * 4};
+    const uint64_t od[4] = {(uint64_t)p.features, (uint64_t)q.rows, (uint64_t)p.window_rows, (uint64_t)f.splits};
+    const uint64_t os[3] = {(uint64_t)p.features * 4, (uint64_t)q.rows * p.features * 4,
+                            (uint64_t)p.window_rows * q.rows * p.features * 4};
     if (!setup_store(g, dtype, od, os)) {
       release();
       return -1;
@@ -3973,6 +4018,11 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
                       dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)ceil_div(q.sp.Hp, kPackRows), (unsigned)p.batch), 256, s,
                       static_cast<const float*>(x), reinterpret_cast<uint4*>(xp), p.in_rows, p.in_cols, p.channels,
                       q.sp.Hp, q.sp.Wp, p.pad_rows, p.pad_cols);
+  else if (q.narrow)
+    launch_overlapped(pack_small_c_input_narrow_kernel,
+                      dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)ceil_div(q.sp.Hp, kPackRows), (unsigned)p.batch), 256, s,
+                      static_cast<const unsigned short*>(x), reinterpret_cast<uint2*>(xp), p.in_rows, p.in_cols, p.channels,
+                      q.sp.Hp, q.sp.Wp, p.pad_rows, p.pad_cols);
   else
     launch_overlapped(pack_small_c_input_kernel<__half>,
                       dim3((unsigned)ceil_div(q.sp.Wp, 256), (unsigned)ceil_div(q.sp.Hp, kPackRows), (unsigned)p.batch), 256, s,
@@ -3982,20 +4032,14 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
   if (st == PDNN_OK) st = launch_gemm(g, dtype, s);
   if (st == PDNN_OK) {
     const size_t n_out = (size_t)p.window_rows * p.window_cols * p.channels * p.features;
-    const unsigned grid = grid_for(n_out, 256, sms);
-    if (dtype == PDNN_F32)
-      launch_overlapped(unpack_small_c_filter_grad_kernel<float>, grid, 256, s, partial, static_cast<float*>(dw), f.splits,
-                        p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
-    else if (out_f32)  // 16-bit tensors (8 channels per packed pixel), fp32 gradient
-      launch_overlapped(unpack_small_c_filter_grad_kernel<__half, float>, grid, 256, s, partial, static_cast<float*>(dw),
-                        f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
-    else if (dtype == PDNN_F16)
-      launch_overlapped(unpack_small_c_filter_grad_kernel<__half>, grid, 256, s, partial, static_cast<__half*>(dw),
-                        f.splits, p.window_rows, p.window_cols, p.channels, p.features, epr, accumulate);
-    else
-      launch_overlapped(unpack_small_c_filter_grad_kernel<__nv_bfloat16>, grid, 256, s, partial,
-                        static_cast<__nv_bfloat16*>(dw), f.splits, p.window_rows, p.window_cols, p.channels, p.features,
-                        epr, accumulate);
+    const unsigned grid = (unsigned)((n_out + 31) / 32);
+    auto unpack = [&](auto* to) {
+      launch_overlapped(unpack_small_c_filter_grad_kernel<std::remove_pointer_t<decltype(to)>>, grid, 256, s, partial, to, f.splits,
+                        p.window_rows, p.window_cols, p.channels, p.features, q.rows / 8, accumulate);
+    };
+    if (dtype == PDNN_F32 || out_f32) unpack(static_cast<float*>(dw));
+    else if (dtype == PDNN_F16) unpack(static_cast<__half*>(dw));
+    else unpack(static_cast<__nv_bfloat16*>(dw));
     st = check_launch("conv2d small-channel filter gradient unpack");
   }
   release();
