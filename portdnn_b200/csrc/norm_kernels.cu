@@ -801,11 +801,12 @@ struct StoreGradStats {
   }
 };
 
-// Slices of the moments kernel, a multiple of 32 rows each (whole batches of every row lane), two waves of
-// three blocks per SM at most.
+// Slices of the moments kernel, a multiple of 32 rows each (whole batches of every row lane): one wave of three blocks per SM,
+// all of which then end together, and half as many sets to merge as with two (us, forward / gradient, two waves / one: 64x28x28x256
+// f16 16.1 / 12.8 and 36.3 / 32.8, 128x56x56x64 41.9 / 37.3 and 75.2 / 70.5).
 int moment_slices(size_t rows, int C, int sms, size_t* rows_per_slice) {
   const size_t ctiles = (size_t)(C + 32 * kMomentChannels - 1) / (32 * kMomentChannels);
-  size_t want = ((size_t)sms * 6 + ctiles - 1) / ctiles;
+  size_t want = ((size_t)sms * 3 + ctiles - 1) / ctiles;
   size_t per = (rows + want - 1) / want;
   per = (per + 8 * kBatch - 1) / (8 * kBatch) * (8 * kBatch);
   if (per < 64) per = 64;
@@ -827,9 +828,11 @@ int slices_for(size_t rows, int C, int sms, int block_channels) {
 
 // Grid of an elementwise packet kernel whose threads should keep their channels: the number of
 // threads is made a multiple of the packets per pixel when that costs little, and no more of them than the
-// device holds at once, so that what a thread prepares for its channels serves several packets.
-unsigned channel_stable_grid(size_t packets, int cvecs, int sms) {
-  unsigned grid = std::min(grid_for(packets, kBlock, sms), (unsigned)sms * (2048u / kBlock));
+// device holds at once (blocks_per_sm), so that what a thread prepares for its channels serves several packets and no
+// second wave is left over.  us, 8 blocks to an SM / as they fit: training gradient, three kernels, 64x28x28x256 f16 (3) 32.9 / 26.0,
+// 128x56x56x64 69.7 / 62.1, f32 (4) 42.3 / 41.4; frozen forward (4) 8.4 / 7.0.  The frozen gradient is no better for it.
+unsigned channel_stable_grid(size_t packets, int cvecs, int sms, unsigned blocks_per_sm) {
+  unsigned grid = std::min(grid_for(packets, kBlock, sms), (unsigned)sms * blocks_per_sm);
   // threads = grid * kBlock must be a multiple of cvecs: grid a multiple of cvecs / gcd(cvecs, kBlock)
   int a = cvecs, b = kBlock;
   while (b != 0) {
@@ -948,7 +951,7 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
       return check_launch("batchnorm forward (training)");
     }
     if (vec)
-      launch_overlapped(batchnorm_apply_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s,
+      launch_overlapped(batchnorm_apply_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms, 4), kBlock, s,
                         static_cast<const T*>(input), static_cast<const T*>(beta), static_cast<const T*>(gamma),
                         static_cast<const T*>(mean), static_cast<const T*>(variance), static_cast<T*>(output), n / VN, C,
                         p.epsilon);
@@ -1017,7 +1020,7 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
       launch_overlapped(batchnorm_merge_kernel<T, true, StoreGradStats<T>>, (C + kMergeChannels - 1) / kMergeChannels,
                         kMergeChannels * kMergeLanes, s, sc.partial, x, dy, slices, C, rows, per_slice,
                         StoreGradStats<T>{sc.terms, g, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), (float)rows, p.epsilon});
-      launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms), kBlock, s, x,
+      launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms, VN == 8 ? 3 : 4), kBlock, s, x,
                         dy, static_cast<const float4*>(sc.terms), static_cast<T*>(output), n / VN, C);
       count_launch(2);
       cudaFreeAsync(sc.base, s);
@@ -1039,7 +1042,7 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
       else batchnorm_sums_kernel<T, 2><<<grid, kBlock, 0, s>>>(x, dy, sc.shift, sc.scale, sc.partial, rows, C, per_slice);
       launch_column_sums(sc.partial, slices, 2 * (size_t)C, sms, s, StoreTotals{sc.stats0, C, 1.f, 1.f});
       if (vec)
-        batchnorm_grad_frozen_vec_kernel<T, VN><<<channel_stable_grid(n / VN, C / VN, sms), kBlock, 0, s>>>(
+        batchnorm_grad_frozen_vec_kernel<T, VN><<<channel_stable_grid(n / VN, C / VN, sms, 2048 / kBlock), kBlock, 0, s>>>(
             dy, g, static_cast<const T*>(pop_variance), static_cast<T*>(output), n / VN, C, p.epsilon);
       else
         batchnorm_grad_frozen_kernel<T><<<grid_for(n, kBlock, sms), kBlock, 0, s>>>(
