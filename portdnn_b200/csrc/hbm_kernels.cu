@@ -1220,30 +1220,50 @@ __device__ __forceinline__ float pointwise_grad_value(float v, float e, int op) 
   }
 }
 
-template <typename T, int V, int MODE>  // MODE 0: forward, 1: gradient
+__device__ __forceinline__ float binary_value(float a, float b, int op) {
+  return op == PDNN_BINARY_ADD ? a + b : op == PDNN_BINARY_SUB ? a - b : op == PDNN_BINARY_MUL ? a * b : a / b;
+}
+
+// MODE 0: forward, 1: gradient, 2: a binary operator on tensors of one shape.  OP: the operator where it is one that networks run
+// between their convolutions, else -1 and the operator is any_op: with the choice in the loop a packet cost more instructions
+// than memory time.  Four packets in flight (two of either operand), 16 blocks to an SM, or 32 where the tensors
+// stream through L2 (256x56x56x256: 130 and 127 us).  f16, us, choice in the loop and two packets / here: ReLU6 64x14x14x576
+// 4.8 / 4.0, 64x28x28x256 6.6 / 5.6; ReLU gradient 5.5 / 4.1, 8.6 / 6.2; the sum of two tensors, through
+// binaryop_kernel's coordinates before, 6.4 / 4.1, 10.2 / 6.4.
+template <typename T, int V, int MODE, int OP>
 __global__ void __launch_bounds__(kBlock)
-    pointwise_kernel(int op, const T* a, const T* b, T* __restrict__ out, size_t n_packets) {
+    pointwise_kernel(int any_op, const T* a, const T* b, T* __restrict__ out, size_t n_packets) {
   overlap_wait();
+  constexpr int U = MODE == 0 ? 4 : 2;
+  const int op = OP >= 0 ? OP : any_op;
   const size_t step = (size_t)gridDim.x * kBlock;
-  for (size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x; i < n_packets; i += 2 * step) {
-    // two packets requested together
-    const int count = i + step < n_packets ? 2 : 1;
-    float av[2][V], bv[2][V], res[V];
+  auto put = [&](size_t i, const float (&av)[V], const float (&bv)[V]) {
+    float res[V];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u >= count) break;
+    for (int j = 0; j < V; ++j)
+      res[j] = MODE == 0 ? pointwise_forward_value(av[j], op) : MODE == 1 ? pointwise_grad_value(av[j], bv[j], op) : binary_value(av[j], bv[j], op);
+    store_vec<T, V>(out + i * V, res);
+  };
+  size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x;
+  for (; i + (U - 1) * step < n_packets; i += U * step) {
+    float av[U][V], bv[U][V];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
       load_vec<T, V>(a + (i + u * step) * V, av[u]);
-      if (MODE == 1) load_vec<T, V>(b + (i + u * step) * V, bv[u]);
+      if (MODE != 0) load_vec<T, V>(b + (i + u * step) * V, bv[u]);
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u >= count) break;
-#pragma unroll
-      for (int j = 0; j < V; ++j)
-        res[j] = MODE == 0 ? pointwise_forward_value(av[u][j], op) : pointwise_grad_value(av[u][j], bv[u][j], op);
-      store_vec<T, V>(out + (i + u * step) * V, res);
-    }
+    for (int u = 0; u < U; ++u) put(i + u * step, av[u], bv[u]);
   }
+  for (; i < n_packets; i += step) {
+    float av[V], bv[V];
+    load_vec<T, V>(a + i * V, av);
+    if (MODE != 0) load_vec<T, V>(b + i * V, bv);
+    put(i, av, bv);
+  }
+}
+unsigned pointwise_grid(size_t packets, size_t bytes, int sms) {
+  return std::min(grid_for(packets, kBlock, sms), (unsigned)sms * (bytes > kStreamedBytes ? 32u : 16u));
 }
 
 template <typename T, int V>
@@ -2271,12 +2291,17 @@ int launch_pointwise(int op, int dtype, const void* in, void* out, size_t n, cud
     using T = decltype(tag);
     constexpr int VN = Vec16<T>::N;
     // the reference picks the widest vector that divides n (src/pointwise/launch_pointwise_forward.cc:32-70)
-    if (n % VN == 0 && aligned16(in) && aligned16(out))
-      launch_overlapped(pointwise_kernel<T, VN, 0>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(in),
-                        nullptr, static_cast<T*>(out), n / VN);
+    const unsigned grid = pointwise_grid(n / VN, n * sizeof(T), sms);
+    const T *a = static_cast<const T*>(in), *none = nullptr;
+    T* to = static_cast<T*>(out);
+    if (n % VN != 0 || !aligned16(in) || !aligned16(out))
+      launch_overlapped(pointwise_kernel<T, 1, 0, -1>, grid_for(n, kBlock, sms), kBlock, s, op, a, none, to, n);
+    else if (op == PDNN_ACT_RELU)
+      launch_overlapped(pointwise_kernel<T, VN, 0, PDNN_ACT_RELU>, grid, kBlock, s, op, a, none, to, n / VN);
+    else if (op == PDNN_ACT_RELU6)
+      launch_overlapped(pointwise_kernel<T, VN, 0, PDNN_ACT_RELU6>, grid, kBlock, s, op, a, none, to, n / VN);
     else
-      launch_overlapped(pointwise_kernel<T, 1, 0>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(in),
-                        nullptr, static_cast<T*>(out), n);
+      launch_overlapped(pointwise_kernel<T, VN, 0, -1>, grid, kBlock, s, op, a, none, to, n / VN);
     return check_launch("pointwise");
   });
 }
@@ -2290,12 +2315,15 @@ int launch_pointwise_grad(int op, int dtype, const void* fwd, const void* err, v
   return dispatch_dtype(dtype, [&](auto tag) {
     using T = decltype(tag);
     constexpr int VN = Vec16<T>::N;
-    if (n % VN == 0 && aligned16(fwd) && aligned16(err) && aligned16(out))
-      launch_overlapped(pointwise_kernel<T, VN, 1>, grid_for(n / VN, kBlock, sms), kBlock, s, op,
-                        static_cast<const T*>(fwd), static_cast<const T*>(err), static_cast<T*>(out), n / VN);
+    const unsigned grid = pointwise_grid(n / VN, n * sizeof(T), sms);
+    const T *a = static_cast<const T*>(fwd), *b = static_cast<const T*>(err);
+    T* to = static_cast<T*>(out);
+    if (n % VN != 0 || !aligned16(fwd) || !aligned16(err) || !aligned16(out))
+      launch_overlapped(pointwise_kernel<T, 1, 1, -1>, grid_for(n, kBlock, sms), kBlock, s, op, a, b, to, n);
+    else if (op == PDNN_ACT_RELU)
+      launch_overlapped(pointwise_kernel<T, VN, 1, PDNN_ACT_RELU>, grid, kBlock, s, op, a, b, to, n / VN);
     else
-      launch_overlapped(pointwise_kernel<T, 1, 1>, grid_for(n, kBlock, sms), kBlock, s, op, static_cast<const T*>(fwd),
-                        static_cast<const T*>(err), static_cast<T*>(out), n);
+      launch_overlapped(pointwise_kernel<T, VN, 1, -1>, grid, kBlock, s, op, a, b, to, n / VN);
     return check_launch("pointwise gradient");
   });
 }
@@ -2384,8 +2412,7 @@ __global__ void __launch_bounds__(kBlock) binaryop_kernel(int op, const T* lhs, 
     }
 #pragma unroll
     for (int j = 0; j < V; ++j)
-      res[j] = op == PDNN_BINARY_ADD ? a[j] + b[j] : op == PDNN_BINARY_SUB ? a[j] - b[j]
-               : op == PDNN_BINARY_MUL ? a[j] * b[j] : a[j] / b[j];
+      res[j] = binary_value(a[j], b[j], op);
     store_vec<T, V>(out + i * V, res);
   }
 }
@@ -2449,7 +2476,15 @@ int launch_binaryop(int op, int dtype, const void* lhs, const int* lhs_dims, int
     // that runs along it is then a multiple of the packet too
     const bool vec = g.od[3] % VN == 0 && aligned16(lhs) && aligned16(rhs) && aligned16(out);
     const size_t n = (size_t)total;
-    if (vec)
+    const bool flat = vec && k <= 1 && g.ls[3] != 0 && g.rs[3] != 0;  // tensors of one shape
+    const unsigned grid = pointwise_grid(n / VN, n * sizeof(T), sms);
+    if (flat && op == PDNN_BINARY_ADD)
+      launch_overlapped(pointwise_kernel<T, VN, 2, PDNN_BINARY_ADD>, grid, kBlock, s, op, static_cast<const T*>(lhs),
+                        static_cast<const T*>(rhs), static_cast<T*>(out), n / VN);
+    else if (flat)
+      launch_overlapped(pointwise_kernel<T, VN, 2, -1>, grid, kBlock, s, op, static_cast<const T*>(lhs), static_cast<const T*>(rhs),
+                        static_cast<T*>(out), n / VN);
+    else if (vec)
       launch_overlapped(binaryop_kernel<T, VN>, grid_for(n / VN, kBlock, sms), kBlock, s, op, static_cast<const T*>(lhs),
                         static_cast<const T*>(rhs), static_cast<T*>(out), g, n / VN);
     else
