@@ -101,6 +101,46 @@ __global__ void __launch_bounds__(kBlock) softmax_forward_vec_kernel(const T* x,
   }
 }
 
+// Few pixels of many channels: a block of four warps per pixel, a packet to a thread, so that a quarter of the exponentials and
+// divisions stand one after another in a thread.  250 x 1000 f16: 3.05 -> 1.75 us.
+constexpr int kSoftmaxRow = 128;
+template <typename T, int V>
+__global__ void __launch_bounds__(kSoftmaxRow) softmax_forward_row_kernel(const T* x, T* __restrict__ y, int C) {
+  overlap_wait();
+  __shared__ float red[2][kSoftmaxRow / 32];
+  const int warp = threadIdx.x >> 5;
+  const bool here = (int)threadIdx.x < C / V;
+  const size_t at = (size_t)blockIdx.x * C + (size_t)threadIdx.x * V;
+  float v[V], m = -INFINITY, sum = 0.f;
+  if (here) {
+    load_v<T, V>(x + at, v);
+#pragma unroll
+    for (int k = 0; k < V; ++k) m = fmaxf(m, v[k]);
+  }
+  m = warp_max(m);
+  if ((threadIdx.x & 31) == 0) red[0][warp] = m;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kSoftmaxRow / 32; ++i) m = fmaxf(m, red[0][i]);
+  if (here) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      v[k] = expf(v[k] - m);
+      sum += v[k];
+    }
+  }
+  sum = warp_sum(sum);
+  if ((threadIdx.x & 31) == 0) red[1][warp] = sum;
+  __syncthreads();
+  sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < kSoftmaxRow / 32; ++i) sum += red[1][i];
+  if (!here) return;
+#pragma unroll
+  for (int k = 0; k < V; ++k) v[k] = v[k] / sum;
+  store_v<T, V>(y + at, v);
+}
+
 // One warp per pixel: y = exp(x - max) / sum exp(x - max) over the pixel's C channels.
 template <typename T>
 __global__ void __launch_bounds__(kBlock) softmax_forward_kernel(const T* __restrict__ x, T* __restrict__ y, size_t rows,
@@ -892,6 +932,9 @@ int launch_softmax(int direction, int dtype, const void* input, const void* grad
     if (direction == 0 && vec && p.channels <= 32 * VN)
       launch_overlapped(softmax_forward_vec_kernel<T, VN, 1>, grid, kBlock, s, static_cast<const T*>(input),
                         static_cast<T*>(output), rows, p.channels);
+    else if (direction == 0 && vec && p.channels <= kSoftmaxRow * VN && rows <= (size_t)sms * (2048 / kSoftmaxRow))  // (one wave)
+      launch_overlapped(softmax_forward_row_kernel<T, VN>, (unsigned)rows, kSoftmaxRow, s, static_cast<const T*>(input),
+                        static_cast<T*>(output), p.channels);
     else if (direction == 0 && vec && p.channels <= 128 * VN)
       launch_overlapped(softmax_forward_vec_kernel<T, VN, 4>, grid, kBlock, s, static_cast<const T*>(input),
                         static_cast<T*>(output), rows, p.channels);
