@@ -2005,6 +2005,9 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
           const size_t columns = (size_t)p.batch * g.K * (p.channels / VN);
           g.rows = g.M;
           while (g.rows > 4 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 2048) g.rows = (g.rows + 1) / 2;
+          // few columns: shorter walks still, each of which costs a thread 0.3 us a row (us, 4 rows / 1: one image 112x112x64 f16
+          // 8.6 / 5.7, four 60x80x96 9.0 / 6.8, both kernels)
+          while (g.rows > 1 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 512) g.rows = (g.rows + 1) / 2;
           g.strips = (g.M + g.rows - 1) / g.rows;
           const size_t n_items = columns * g.strips;
           // Below three quarters of a wave the overlap is worth more, above it the read-only loads (us, overlapped /
@@ -2248,6 +2251,7 @@ int launch_depthwise(int pass, int dtype, const void* in, const void* fil, void*
       const size_t columns = (size_t)p.batch * g.K * (p.channels / VN);
       g.rows = g.M;
       while (g.rows > 4 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 2048) g.rows = (g.rows + 1) / 2;
+      while (g.rows > 1 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 512) g.rows = (g.rows + 1) / 2;  // (as for the pools)
       g.strips = (g.M + g.rows - 1) / g.rows;
       const size_t n_items = columns * g.strips;
       if (n_items < 0xFFFF0000ull) {
