@@ -2170,18 +2170,26 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // Splits `total` (a power of two) rows into a box tw x th x tn of powers of two that wastes the
 // fewest rows when tiled over [W, H, N]; ties go to the widest box.
 void choose_box(int total, int W, int H, int N, int* tw, int* th, int* tn) {
-  double best = -1;
-  for (int w = total; w >= 1; w >>= 1)
-    for (int h = total / w; h >= 1; h >>= 1) {
-      const int n = total / (w * h);
-      if (w > 256 || h > 256 || n > 256) continue;
-      const double covered = (double)ceil_div(W, w) * w * (double)ceil_div(H, h) * h * (double)ceil_div(N, n) * n;
-      const double eff = ((double)W * H * N) / covered;
-      if (eff > best + 1e-9) {
-        best = eff;
-        *tw = w;
-        *th = h;
-        *tn = n;
+  // extents rounded up to the multiples of 1, 2, 4, ... (every convolution call comes through here, and the divisions of the
+  // 36 boxes of 128 rows took 0.3 us of its 4)
+  unsigned long long cw[9], ch[9], cn[9];
+  for (int i = 0; i < 9; ++i) {
+    const unsigned long long m = (1ull << i) - 1;
+    cw[i] = (W + m) & ~m, ch[i] = (H + m) & ~m, cn[i] = (N + m) & ~m;
+  }
+  int log2 = 0;
+  while ((1 << log2) < total) ++log2;
+  unsigned long long best = ~0ull;
+  for (int lw = std::min(log2, 8); lw >= 0; --lw)
+    for (int lh = std::min(log2 - lw, 8); lh >= 0; --lh) {
+      const int ln = log2 - lw - lh;
+      if (ln > 8) continue;
+      const unsigned long long covered = cw[lw] * ch[lh] * cn[ln];
+      if (covered < best) {
+        best = covered;
+        *tw = 1 << lw;
+        *th = 1 << lh;
+        *tn = 1 << ln;
       }
     }
 }
