@@ -21,7 +21,7 @@ OBJ = os.path.join(HERE, "_obj")
 LIB = os.path.join(HERE, "libportdnn_b200.so")
 FRONT_SOURCE = os.path.join(CSRC, "front.cpp")
 SOURCES = ["c_api.cu", "hbm_kernels.cu", "direct_conv.cu", "tc_gemm.cu", "winograd.cu", "norm_kernels.cu",
-           "layout_kernels.cu", "padded_conv.cu", "depthwise_tile.cu", "collective.cu"]
+           "layout_kernels.cu", "padded_conv.cu", "depthwise_tile.cu", "simt_gemm.cu", "collective.cu"]
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--expt-relaxed-constexpr",
          "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall"]
 

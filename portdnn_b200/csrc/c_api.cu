@@ -1,6 +1,7 @@
 // extern "C" entry points declared in include/portdnn_b200.h.
 #include "common.cuh"
 #include "padded_conv.cuh"
+#include "simt_gemm.cuh"
 #include "tc_gemm.cuh"
 
 #include <mutex>
@@ -126,11 +127,18 @@ __global__ void __launch_bounds__(256) widen_to_f32_kernel(const T* __restrict__
     out[i] = (accumulate ? out[i] : 0.f) + to_f32(in[i]);
 }
 
-// The direct kernel with the fused backprop forms applied afterwards (shapes the tensor-core engine
+// What no tensor-core kernel takes: fp32 tiles on the CUDA cores where they gain, else a thread to an output.
+int general_conv(int pass, int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
+                 const PdnnConvEpilogue* epi, bool tiled, cudaStream_t s) {
+  if (tiled && simt_conv_applicable(pass, p)) return simt_conv(pass, dtype, in, fil, out, p, epi, s);
+  return launch_direct_conv(pass, dtype, in, fil, out, p, epi, s);
+}
+
+// The general kernels with the fused backprop forms applied afterwards (shapes the tensor-core engine
 // does not take): the ReLU-gradient mask as a pointwise pass in place, an fp32 filter gradient
 // through a temporary in the tensors' own type.
 int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
-                        const PdnnBackpropFusion* fusion, cudaStream_t s) {
+                        const PdnnBackpropFusion* fusion, bool tiled, cudaStream_t s) {
   const size_t es = dtype_size(dtype);
   if (pass == PDNN_FILTER_BACKPROP && fusion != nullptr && fusion->accumulate && !(fusion->output_f32 && dtype != PDNN_F32)) {
     // dW += gradient in the tensors' own type: the gradient into a temporary, then one blend
@@ -140,7 +148,7 @@ int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, vo
       cudaGetLastError();
       return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for the filter gradient", n * es);
     }
-    int st = launch_direct_conv(pass, dtype, in, fil, tmp, p, nullptr, s);
+    int st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, s);
     if (st == PDNN_OK) st = launch_scale_blend(dtype, tmp, 1.f, out, 1.f, out, n, s);
     cudaFreeAsync(tmp, s);
     return st;
@@ -152,7 +160,7 @@ int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, vo
       cudaGetLastError();
       return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for the filter gradient", n * es);
     }
-    int st = launch_direct_conv(pass, dtype, in, fil, tmp, p, nullptr, s);
+    int st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, s);
     if (st == PDNN_OK) {
       const unsigned grid = grid_for(n, 256, device_sm_count());
       if (dtype == PDNN_F16) widen_to_f32_kernel<__half><<<grid, 256, 0, s>>>(static_cast<const __half*>(tmp), static_cast<float*>(out), n, fusion->accumulate != 0);
@@ -170,11 +178,11 @@ int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, vo
       cudaGetLastError();
       return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for the input gradient", n_dx * es);
     }
-    st = launch_direct_conv(pass, dtype, in, fil, tmp, p, nullptr, s);
+    st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, s);
     if (st == PDNN_OK) st = launch_scale_blend(dtype, tmp, 1.f, out, 1.f, out, n_dx, s);
     cudaFreeAsync(tmp, s);
   } else {
-    st = launch_direct_conv(pass, dtype, in, fil, out, p, nullptr, s);
+    st = general_conv(pass, dtype, in, fil, out, p, nullptr, tiled, s);
   }
   if (st != PDNN_OK || pass != PDNN_INPUT_BACKPROP || fusion == nullptr) return st;
   if (fusion->relu_bitmask != nullptr) return launch_relu_grad_bits(dtype, fusion->relu_bitmask, out, n_dx, s);
@@ -229,8 +237,9 @@ int dispatch_conv(int pass, int dtype, const void* in, const void* fil, void* ou
     const int st2 = padded_conv(pass, dtype, in, fil, out, *p, epi, fusion, ws, ws_elems, s);
     if (st2 != kNeedsDirect) return st2;
   }
-  if (pass != PDNN_FORWARD) return run_direct_backprop(pass, dtype, in, fil, out, *p, fusion, s);
-  return launch_direct_conv(pass, dtype, in, fil, out, *p, epi, s);
+  const bool tiled = algorithm != PDNN_ALGO_DIRECT;
+  if (pass != PDNN_FORWARD) return run_direct_backprop(pass, dtype, in, fil, out, *p, fusion, tiled, s);
+  return general_conv(pass, dtype, in, fil, out, *p, epi, tiled, s);
 }
 
 }  // namespace

@@ -21,6 +21,7 @@
 #include "column_sums.cuh"
 #include "split_ring.cuh"
 #include "tc_gemm.cuh"
+#include "simt_gemm.cuh"
 #include "umma.cuh"
 
 #include <algorithm>
@@ -4457,6 +4458,8 @@ int simt_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, voi
                 float beta, cudaStream_t s, bool out_f32) {
   const int sms = device_sm_count();
   if (sms <= 0) return fail(PDNN_ALLOCATION_PROBLEM, "no CUDA device");
+  int st = PDNN_OK;
+  if (simt_matmul_tiled(dtype, tl, tr, lhs, rhs, out, batches, m, k, n, beta, s, out_f32, &st)) return st;
   const size_t total = (size_t)batches * m * n;
   const unsigned grid = grid_for(total, 256, sms);
   if (dtype == PDNN_F32)
