@@ -115,7 +115,7 @@ int device_sm_count();   // SM count of the current device; -1 if it is not an s
 // infer read-only loads) and plain loads, which stay behind the wait.  (The compiler moves no plain load ahead of a
 // store, so kernels that want several in flight request them before they write.)  Grids of fewer than four waves only: beside a kernel of that length
 // the gap is nothing, and long ones chained this way cost the kernels around them.  All launches ordinary /
-// grids below four waves / all overlapped, us: MobileNet-v2 forward at 64 images (80 launches) 824 / 785 / 782,
+// grids below four waves / all overlapped, us (with one large CTA to an SM in every GEMM): MobileNet-v2 forward at 64 images (80 launches) 824 / 785 / 782,
 // 7x45x61 100 -> 150 3x3 with gradients 152 / 135 / 135, two max pools with gradients 121 / 114 / 114, one
 // image through ResNet-50 325 / 318 / 318, VGG-16 training step in fp32 6899 / 6897 / 7190.
 __device__ __forceinline__ void overlap_wait() {

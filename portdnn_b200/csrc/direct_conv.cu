@@ -1,7 +1,7 @@
 // General direct convolution on CUDA cores: one thread per output element, fp32 accumulation.
 // It takes every shape conv2d::launch accepts in NHWC (any channel/feature count, any window and
-// stride, grouped forward, HWCF or FHWC filters) and is what Algorithm::Direct runs; the
-// tensor-core kernels hand it the shapes they cannot tile.
+// stride, grouped forward, HWCF or FHWC filters) and is what Algorithm::Direct runs; of the shapes that the tensor-core
+// kernels cannot tile it has the small and the grouped ones (the others: simt_gemm.cu).
 //
 // Definitions follow portDNN's direct kernels: src/conv2d/direct/kernels_nhwc.h:62-130 (forward),
 // :206-278 (input backprop), :356-420 (filter backprop).

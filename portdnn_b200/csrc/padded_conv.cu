@@ -5,7 +5,7 @@
 // are in order are read, and results written, in place.
 //
 // Bound by the convolution itself, then by the launches around it.  7 x 45x61, 100 -> 150 channels, 3x3, bf16,
-// all three passes: 15580 us on the direct kernel, 137 us here.
+// all three passes: 15580 us on the direct kernel, 77 us here.
 #include "padded_conv.cuh"
 #include "tc_gemm.cuh"
 
@@ -169,8 +169,8 @@ size_t scratch_bytes(int pass, int dtype, const Plan& plan) {
          round_up((size_t)plan.q.features * 2, 256) + round_up(inner * 2, 256) + 256;
 }
 
-// Where the direct kernel, one launch that walks each output's terms one after another, is still the better
-// one.  Measured (bf16, us, direct / padded copies):
+// Where the general kernels, one launch that needs no copies, are still the better ones.  Measured (bf16, us, a thread to an output
+// / copies padded to multiples of 8, which were up to a third slower than those of padded_count):
 //   forward                          |  1 image    | 4 images    | 64 images   | 256 images
 //    7x7   12 -> 12  1x1             |  4.7 / 10.1 |  4.7 / 10.0 |  4.7 / 10.1 |   6.2 / 10.2
 //   14x14  12 -> 12  1x1             | 10.5 / 10.4 |  4.7 / 10.0 |  6.2 / 10.2 |  14.4 / 12.0

@@ -673,10 +673,9 @@ __device__ __forceinline__ bool epilogue_tile_tma_fast(const GemmArgs& a, const 
 //
 // A CTA runs up to two independent pipelines ("groups") side by side, each with its own TMA
 // producer warp, MMA issuer warp, four epilogue warps, ring of stages, accumulators in TMEM and
-// staging slices; group g takes every second tile of the CTA.  One thread can issue a
-// tcgen05.mma only every ~130 cycles once the barrier wait, the commit and the loop around four
-// MMAs are counted, which is two to three times the time the tensor pipe needs for a 128 x 64 or
-// 128 x 128 MMA; two issuers keep the pipe busy, and two epilogue teams halve the time a tile's
+// staging slices; group g takes every second tile of the CTA.  One issuer gives the pipe a tcgen05.mma every
+// 60 to 73 cycles, waits and commits included, where the pipe takes one of 128 x 64 every 48 and one of
+// 128 x 128 every 64; two issuers keep the pipe busy, and two epilogue teams halve the time a tile's
 // accumulator waits to be drained.  The resident B tiles, the bias copy and the TMEM allocation
 // are shared.  The fp32 (3xTF32) variant runs one group plus the eight hi/lo split warps.
 //
