@@ -6,7 +6,7 @@
 // Those kernels load two words for each multiply-add and walk a sum in one thread.  Here a block of 256 threads
 // takes a tile of BM x BN outputs, four rows by four columns to a thread, and the operands pass through shared
 // memory sixteen terms at a time, the next sixteen being on their way in registers meanwhile: 8 words of shared memory for
-// 16 multiply-adds, two to an instruction, which leaves the multiply-adds as the bound.  Where the tiles are fewer than the device takes, up to
+// 16 multiply-adds, two to an instruction.  Where the tiles are fewer than the device takes, up to
 // eight blocks of a cluster share the terms of a tile and add up their sums through distributed shared memory, in the
 // order of the terms; a filter gradient that is one long sum is also cut into slices, added up by a second launch.
 #include "simt_gemm.cuh"
@@ -66,7 +66,8 @@ __device__ __forceinline__ void fma_two(float2& c, float2 a, float2 b) {
       : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
 }
 
-// Bound by the multiply-adds in large layers, by the latency of a step's loads in small ones.  Times of both
+// Bound by shared memory in large layers (28x45x61 101 -> 150 3x3 fp32: 85 % of its wavefronts, multiply-add pipe 52 %), by the latency
+// of a step's loads in small ones.  Times of both
 // this and a thread to an output: thread_to_an_output and simt_matmul_tiled.
 template <typename T, int A, bool B_RUNS, int BN>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const SimtArgs g) {
@@ -152,8 +153,9 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const
   };
 
   const int chunks = (g.inner + kTerms - 1) / kTerms, steps = runs_r * runs_s * chunks;
-  const int parts = g.splits * g.slices, per = (steps + parts - 1) / parts;
-  const int begin = min(steps, (slice * g.splits + rank) * per), end = min(steps, begin + per);
+  const long long parts = (long long)g.splits * g.slices;
+  auto part_at = [&](int part) { return (int)(steps * (long long)part / parts); };
+  const int begin = part_at(slice * g.splits + rank), end = part_at(slice * g.splits + rank + 1);
 
   // the elements of A and B that this thread brings
   const int ak = kARuns ? t % kTerms : t / BM, am = kARuns ? t / kTerms : t % BM;
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const
   // A tap outside the image has no term, whatever the other operand is there, but the tiles multiply it by zero: a
   // sum that is not a number is formed again from the terms that there are.
   auto terms_inside = [&](int row, int n) -> float {
-    const int from = min(steps, slice * g.splits * per), to = min(steps, from + g.splits * per);
+    const int from = part_at(slice * g.splits), to = part_at((slice + 1) * g.splits);
     float v = 0.f;
     if constexpr (A == kRows) {
 #pragma unroll 1
@@ -397,8 +399,9 @@ Tiling choose(long long m, long long counted, int n, long long inner, long long 
   const long long tiles = ((counted + bm - 1) / bm) * t.n_tiles * outer, steps = runs * ((inner + kTerms - 1) / kTerms);
   const long long room = (long long)kBlocksPerSm * sms;
   t.splits = 1, t.slices = 1;
-  while (t.splits < kMaxSplits && 2 * tiles * t.splits <= room && steps >= 8ll * t.splits) t.splits *= 2;
-  if (slices && t.splits == kMaxSplits) {
+  // (a filter gradient's pixels have always been added up in eight parts at least: fewer are longer sums, and larger errors)
+  while (t.splits < kMaxSplits && (slices || (2 * tiles * t.splits <= room && steps >= 8ll * t.splits))) t.splits *= 2;
+  if (slices) {
     const long long fit = room / (tiles * t.splits), most = steps / 64;
     t.slices = (int)(fit < most ? fit : most);
     if (t.slices < 2) t.slices = 1;
@@ -420,35 +423,35 @@ Tiling conv_tiling(int pass, const PdnnConv2DParams& p, bool any_order, int sms)
   return choose(taps * p.channels, taps * p.channels, p.features, p.batch * px_out, 1, 1, true, sms);
 }
 
-int sm_count() {
-  const int sms = device_sm_count();
-  return sms > 0 ? sms : 148;
-}
-
-}  // namespace
-
 // Where a thread to an output is still the better one (direct_conv.cu): its time is the length of a sum until the work fills the
 // device, that of the tiles the latency of their loads.  us, thread to an output / tiles here:
 //   images, size, channels, window      | forward     | input gradient | filter gradient
 //   f32   1 x 7x7    13 -> 13   1x1     | 4.7 / 5.4   |  3.1 / 5.8     |   4.5 / 8.4
 //   f32   1 x 7x7    13 -> 13   3x3     |  25 / 9.2   |   13 / 9.9     |   4.7 / 10.9
 //   f32   1 x 14x14  37 -> 51   1x1     | 9.0 / 8.7   |  6.6 / 9.7     |  12.6 / 12.1
-//   f32   1 x 14x14  37 -> 51   3x3     |  65 / 10    |   41 / 9.0     |    22 / 12.4
-//   f32   4 x 28x28  21 -> 30   3x3     |  44 / 10.5  |   29 / 11.1    |   183 / 18
-//   f32  64 x 56x56  13 -> 15   1x1     |  63 / 33    |   58 / 34      | 10760 / 102
-//   f32   8 x 20x30 133 -> 77   3x3     | 495 / 72    |  577 / 85      |  2055 / 81
-//   f32   4 x 14x14 301 -> 251  3x3     | 812 / 63    |  726 / 70      |  1902 / 53
-//   f16   2 x 9x19   37 -> 51   1x1     | 4.9 / 7.5   |  5.8 / 10.9    |  21.2 / 13.8
+//   f32   1 x 14x14  37 -> 51   3x3     |  65 / 10    |   41 / 9.0     |    22 / 7.3
+//   f32   4 x 28x28  21 -> 30   3x3     |  44 / 10.5  |   29 / 11.1    |   183 / 19
+//   f32  64 x 56x56  13 -> 15   1x1     |  63 / 33    |   58 / 34      | 10760 / 109
+//   f32   8 x 20x30 133 -> 77   3x3     | 495 / 72    |  577 / 85      |  2055 / 83
+//   f32   4 x 14x14 301 -> 251  3x3     | 812 / 63    |  726 / 70      |  1902 / 65
+//   f16   2 x 9x19   37 -> 51   1x1     | 4.9 / 7.5   |  5.8 / 10.9    |  21.2 / 9.8
 //   f16   1 x 14x14  20 -> 30   3x3     | 15.3 / 8.9  | 19.3 / 8.5     |  13.3 / 20.8
-//   f16   4 x 14x14  37 -> 51   1x1     | 5.1 / 7.4   |  6.0 / 11      |    46 / 15.5
+//   f16   4 x 14x14  37 -> 51   1x1     | 5.1 / 7.4   |  6.0 / 11      |    46 / 16.6
 // The forward pass moves over by the terms of a sum or by the work of one image: an image has the same result alone and in any batch.
-static bool thread_to_an_output(int pass, const PdnnConv2DParams& p) {
+bool thread_to_an_output(int pass, const PdnnConv2DParams& p) {
   const double taps = (double)p.window_rows * p.window_cols, pixels = (double)p.out_rows * p.out_cols;
   const double per_image = pixels * taps * p.channels * p.features;
   if (pass == PDNN_FORWARD) return taps * p.channels < 64 && per_image < 5e5;
   if (pass == PDNN_INPUT_BACKPROP) return taps * p.features < 100.0 * p.stride_rows * p.stride_cols && per_image * p.batch < 1e7;
-  return pixels * p.batch < 256 && per_image * p.batch < 2e6;
+  return pixels * p.batch < 160 && per_image * p.batch < 2e6;
 }
+
+int sm_count() {
+  const int sms = device_sm_count();
+  return sms > 0 ? sms : 148;
+}
+
+}  // namespace
 
 bool simt_conv_applicable(int pass, const PdnnConv2DParams& p) {
   if (p.groups != 1 || p.input_format != 0 || (p.filter_format != 0 && p.filter_format != 2)) return false;
