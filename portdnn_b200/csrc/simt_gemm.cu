@@ -428,14 +428,14 @@ Tiling conv_tiling(int pass, const PdnnConv2DParams& p, bool any_order, int sms)
 //   images, size, channels, window      | forward     | input gradient | filter gradient
 //   f32   1 x 7x7    13 -> 13   1x1     | 4.7 / 5.4   |  3.1 / 5.8     |   4.5 / 8.4
 //   f32   1 x 7x7    13 -> 13   3x3     |  25 / 9.2   |   13 / 9.9     |   4.7 / 10.9
-//   f32   1 x 14x14  37 -> 51   1x1     | 9.0 / 8.7   |  6.6 / 9.7     |  12.6 / 12.1
+//   f32   1 x 14x14  37 -> 51   1x1     | 9.0 / 8.7   |  6.6 / 9.7     |  12.6 / 6.8
 //   f32   1 x 14x14  37 -> 51   3x3     |  65 / 10    |   41 / 9.0     |    22 / 7.3
 //   f32   4 x 28x28  21 -> 30   3x3     |  44 / 10.5  |   29 / 11.1    |   183 / 19
 //   f32  64 x 56x56  13 -> 15   1x1     |  63 / 33    |   58 / 34      | 10760 / 109
 //   f32   8 x 20x30 133 -> 77   3x3     | 495 / 72    |  577 / 85      |  2055 / 83
 //   f32   4 x 14x14 301 -> 251  3x3     | 812 / 63    |  726 / 70      |  1902 / 65
 //   f16   2 x 9x19   37 -> 51   1x1     | 4.9 / 7.5   |  5.8 / 10.9    |  21.2 / 9.8
-//   f16   1 x 14x14  20 -> 30   3x3     | 15.3 / 8.9  | 19.3 / 8.5     |  13.3 / 20.8
+//   f16   1 x 14x14  20 -> 30   3x3     | 15.3 / 8.9  | 19.3 / 8.5     |  13.3 / 9.9
 //   f16   4 x 14x14  37 -> 51   1x1     | 5.1 / 7.4   |  6.0 / 11      |    46 / 16.6
 // The forward pass moves over by the terms of a sum or by the work of one image: an image has the same result alone and in any batch.
 bool thread_to_an_output(int pass, const PdnnConv2DParams& p) {
@@ -464,7 +464,9 @@ bool simt_conv_applicable(int pass, const PdnnConv2DParams& p) {
   const long long back = ((long long)p.window_rows + p.pad_rows + 1) * p.out_cols + p.window_cols + p.pad_cols + 1;
   if (x + reach * p.channels > kMostElements || y + back * p.features > kMostElements) return false;
   if (p.stride_rows > 64 || p.stride_cols > 64) return false;
-  return !thread_to_an_output(pass, p);
+  const Tiling t = conv_tiling(pass, p, true, sm_count());
+  const double blocks = (double)t.m_tiles * t.n_tiles * t.slices * kMaxSplits * (pass == PDNN_INPUT_BACKPROP ? p.stride_rows * p.stride_cols : 1);
+  return blocks < 2147483632.0 && !thread_to_an_output(pass, p);
 }
 
 int simt_conv(int pass, int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
@@ -503,7 +505,6 @@ int simt_conv(int pass, int dtype, const void* in, const void* fil, void* out, c
   }
   g.m_tiles = t.m_tiles, g.n_tiles = t.n_tiles, g.splits = t.splits, g.slices = t.slices;
   const long long blocks = (long long)outer * t.slices * t.n_tiles * t.m_tiles * t.splits;
-  if (blocks > 0x7FFFFFF0ll) return fail(PDNN_INDEX_EXCEEDED, "conv2d: grid too large");
   int st;
   if (pass == PDNN_FILTER_BACKPROP) st = launch_typed<kPixels, false>(dtype, t.bn, g, (unsigned)blocks, s);
   else if (g.bk == 1 && g.bn != 1) st = launch_typed<kRows, true>(dtype, t.bn, g, (unsigned)blocks, s);
