@@ -2313,28 +2313,28 @@ bool plan_solo(GemmArgs& g, bool mask_tma) {
   const long long tiles = g.a_mn ? (long long)g.n_tiles * g.tiles_w * ((g.num_taps + tap_pack - 1) / tap_pack) * g.splits
                                  : (long long)g.n_tiles * g.tiles_w * g.tiles_h * g.tiles_n;
   if (tiles > 2ll * device_sm_count()) return false;
-  GemmArgs t = g;
-  t.solo = 1;
-  t.groups = t.acc_bufs = 1;
-  t.acc_stride = std::max(32, next_pow2(t.bn));
-  t.tmem_cols = t.acc_stride;
-  t.bias_tile_only = 1;
-  t.bias_smem_bytes = (t.epi_fast && t.bias != nullptr) ? ceil_div(t.bn, 64) * 128 : 0;
-  t.res_taps = t.num_taps;
-  t.b_res = 0;
-  t.b_res_bytes = 0;
-  const int blocks = ceil_div(t.bn, t.cpb), stage = kABytes + t.bn * 128, fixed = 1024 + kBarBlockBytes + t.bias_smem_bytes + t.mask_smem_bytes;
-  const int steps = t.a_mn ? t.slabs_per_split : t.num_taps * t.cblocks;
-  auto stages = [&] { return std::min(kMaxStages, (kSoloSmem - fixed - t.mask_slots * 4 * 4096) / stage); };
-  t.mask_slots = (mask_tma && t.mask_bits == nullptr) ? std::min(2, blocks) : 0;
-  if (t.mask_slots == 2 && stages() < 3) t.mask_slots = 1;
-  t.stages = stages();
+  const int bias_smem_bytes = (g.epi_fast && g.bias != nullptr) ? ceil_div(g.bn, 64) * 128 : 0;
+  const int blocks = ceil_div(g.bn, g.cpb), stage = kABytes + g.bn * 128, fixed = 1024 + kBarBlockBytes + bias_smem_bytes + g.mask_smem_bytes;
+  const int steps = g.a_mn ? g.slabs_per_split : g.num_taps * g.cblocks;
+  int mask_slots = (mask_tma && g.mask_bits == nullptr) ? std::min(2, blocks) : 0;
+  auto stages = [&] { return std::min(kMaxStages, (kSoloSmem - fixed - mask_slots * 4 * 4096) / stage); };
+  if (mask_slots == 2 && stages() < 3) mask_slots = 1;
   // (two stages will do: wide tiles, and tiles of 128 columns beside a mask slot; ResNet-50 backward at 24 images 1249 us with
   // three for those of 128, 1237 so; 7x45x61 100 -> 150 3x3 with gradients, tiles of 192, 117 and 115)
-  if (t.stages < std::min(2, steps)) return false;
-  t.nsw = blocks > 2 ? 4 : blocks;
-  while (t.nsw > 1 && t.nsw * 4 * 4096 > t.stages * stage) t.nsw /= 2;
-  g = t;
+  if (stages() < std::min(2, steps)) return false;
+  g.solo = 1;
+  g.groups = g.acc_bufs = 1;
+  g.acc_stride = std::max(32, next_pow2(g.bn));
+  g.tmem_cols = g.acc_stride;
+  g.bias_tile_only = 1;
+  g.bias_smem_bytes = bias_smem_bytes;
+  g.res_taps = g.num_taps;
+  g.b_res = 0;
+  g.b_res_bytes = 0;
+  g.mask_slots = mask_slots;
+  g.stages = stages();
+  g.nsw = blocks > 2 ? 4 : blocks;
+  while (g.nsw > 1 && g.nsw * 4 * 4096 > g.stages * stage) g.nsw /= 2;
   return true;
 }
 
