@@ -210,9 +210,16 @@ int run_conv(int pass, int dtype, const void* in, const void* fil, void* out, co
     if (epi != nullptr && epi->relu_bitmask != nullptr)
       return fail(PDNN_INVALID_PARAMETER, "conv2d: a ReLU bitmask needs NHWC tensors");
     const bool read_out = epi != nullptr && epi->beta != 0.f;
+    // the filter that the layer reads is a copy, which the transpose right ahead of it writes
+    PdnnConvEpilogue e = {};
+    PdnnBackpropFusion f = {};
+    if (epi != nullptr) e = *epi;
+    if (fusion != nullptr) f = *fusion;
+    e.constant_filter = f.constant_filter = 0;
     return conv2d_nchw(pass, dtype, in, fil, out, *p, read_out, s,
                        [&](const void* a, const void* b, void* c, const PdnnConv2DParams& q) {
-                         return dispatch_conv(pass, dtype, a, b, c, &q, PDNN_ALGO_TILED, epi, fusion, nullptr, 0, s);
+                         return dispatch_conv(pass, dtype, a, b, c, &q, PDNN_ALGO_TILED, epi != nullptr ? &e : nullptr,
+                                              fusion != nullptr ? &f : nullptr, nullptr, 0, s);
                        });
   }
   return dispatch_conv(pass, dtype, in, fil, out, p, algorithm, epi, fusion, ws, ws_elems, s);
