@@ -1051,12 +1051,12 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     }
   } else if (role == 1) {
     // ------------------------------- MMA issuer ---------------------------------------------
+    // (Every role waits for the preceding kernel ahead of its first wait with a time limit, also where it touches no tensor: the
+    // limit is for this kernel's own arrivals.)
+    grid_dependency_wait();
     // The successor may be placed once every CTA of this grid has got here: nothing of the grid is still waiting for an SM
     // then, and its columns of tensor memory are taken.
-    if (grp == 0) {
-      grid_dependency_wait();
-      grid_launch_dependents();
-    }
+    if (grp == 0) grid_launch_dependents();
     {
       // The whole warp runs the loops on warp-uniform values; warp_mma_* / warp_commit elect the one
       // lane that issues each instruction.
@@ -1332,6 +1332,7 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
     bool ok = true;
     TileWalker walker;
     walker.init(a, first_tile, tile_step);
+    grid_dependency_wait();  // (ahead of the first wait with a time limit)
 #pragma unroll 1
     for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, walker.advance()) {
       const TileCoord t = walker.coord(a);
@@ -2025,6 +2026,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) umma_gemm_cluster_kernel(c
     const uint32_t a_kadv = a.a_kadv >> 4, b_kadv = a.b_kadv >> 4, idesc = a.idesc;
     int s = 0;
     uint32_t ph = 0, accumulate = 0u;
+    grid_dependency_wait();  // (ahead of the first wait with a time limit, here and below)
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       if (!mbar_wait(full_bar(s), ph, abort_flag, g_error_record, a.wait_limit_ns, 0xE00u + (unsigned)s)) break;
@@ -2048,6 +2050,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) umma_gemm_cluster_kernel(c
   // rows of bn floats and 16 bytes more, so that neither the row-wise stores nor the packets below conflict
   const uint32_t row_bytes = (uint32_t)a.bn * 4u + 16u;
   if (warp >= 2) {
+    grid_dependency_wait();  // (the stores below, too, and what they add or mask with)
     if (mbar_wait(acc_bar, 0u, abort_flag, g_error_record, a.wait_limit_ns, 0xF00u)) {
       // every copy into the ring has landed and every MMA has read it
       tc_fence_after_sync();
@@ -2065,7 +2068,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1) umma_gemm_cluster_kernel(c
     }
     tc_fence_before_sync();
   }
-  if (warp != 0) grid_dependency_wait();  // the stores below, and what they add or mask with
   // a thread's packets all lie in the same columns: kClusterThreads is a multiple of the packets of a row
   const int packets = a.bn >> 3, pk = (int)threadIdx.x % packets, col = t.nf0 + pk * 8;
   uint4 bias = make_uint4(0u, 0u, 0u, 0u);
