@@ -13,6 +13,9 @@ namespace pdnn {
 namespace {
 
 constexpr int kBlock = 256;
+// Blocks to an SM of the kernels whose grids are one wave: the launch bound that the compiler keeps and the size of the grid.
+constexpr int kMomentBlocks = 3, kApplyBlocks = 4;
+constexpr int gradient_blocks(int packet) { return packet == 8 ? 3 : 4; }  // (80 and 63 registers)
 
 template <typename F>
 int dispatch(int dtype, F&& f) {
@@ -215,7 +218,7 @@ __global__ void __launch_bounds__(kBlock) softmax_grad_kernel(const T* __restric
 // The elementwise steps on packets of V channels (C % V == 0, 16-byte aligned tensors): n counts
 // packets.  The per-channel operands are read as packets too (they stay in L1).
 template <typename T, int V>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, kApplyBlocks)
     batchnorm_apply_vec_kernel(const T* x, const T* beta, const T* gamma,
                                const T* mean, const T* var, T* __restrict__ out, size_t n,
                                int C, float eps) {
@@ -273,7 +276,7 @@ __global__ void __launch_bounds__(kBlock)
 // below, the division by the deviation used to come after the multiplication by gamma; the last factor is now
 // rounded first, as it always was where they do not.)
 template <typename T, int V>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, gradient_blocks(V))
     batchnorm_grad_training_vec_kernel(const T* x, const T* dy, const float4* terms, T* __restrict__ out, size_t n, int C) {
   overlap_wait();
   const size_t cvecs = (size_t)(C / V);
@@ -600,7 +603,7 @@ __device__ __forceinline__ void load_four(const T* p, float (&v)[kMomentChannels
 // partial[slice][value of the set][c].  APPLY: the forward output is written on the way,
 // out = (x - mean) / sqrt(var + eps) * gamma + beta with the given mean and variance.
 template <typename T, bool DY, bool APPLY>
-__global__ void __launch_bounds__(kBlock, 3)
+__global__ void __launch_bounds__(kBlock, kMomentBlocks)
     batchnorm_moments_kernel(const T* x, const T* dy, const T* beta,
                              const T* gamma, const T* mean, const T* var,
                              T* __restrict__ out, float* __restrict__ partial, size_t rows, int C, size_t rows_per_slice, float eps) {
@@ -878,7 +881,7 @@ struct StoreGradStats {
 // f16 16.1 / 12.8 and 36.3 / 32.8, 128x56x56x64 41.9 / 37.3 and 75.2 / 70.5).
 int moment_slices(size_t rows, int C, int sms, size_t* rows_per_slice) {
   const size_t ctiles = (size_t)(C + 32 * kMomentChannels - 1) / (32 * kMomentChannels);
-  size_t want = ((size_t)sms * 3 + ctiles - 1) / ctiles;
+  size_t want = ((size_t)sms * kMomentBlocks + ctiles - 1) / ctiles;
   size_t per = (rows + want - 1) / want;
   per = (per + 8 * kBatch - 1) / (8 * kBatch) * (8 * kBatch);
   if (per < 64) per = 64;
@@ -1026,7 +1029,7 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
       return check_launch("batchnorm forward (training)");
     }
     if (vec)
-      launch_overlapped(batchnorm_apply_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms, 4), kBlock, s,
+      launch_overlapped(batchnorm_apply_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms, kApplyBlocks), kBlock, s,
                         static_cast<const T*>(input), static_cast<const T*>(beta), static_cast<const T*>(gamma),
                         static_cast<const T*>(mean), static_cast<const T*>(variance), static_cast<T*>(output), n / VN, C,
                         p.epsilon);
@@ -1095,7 +1098,7 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
       launch_overlapped(batchnorm_merge_kernel<T, true, StoreGradStats<T>>, (C + kMergeChannels - 1) / kMergeChannels,
                         kMergeChannels * kMergeLanes, s, sc.partial, x, dy, slices, C, rows, per_slice,
                         StoreGradStats<T>{sc.terms, g, static_cast<T*>(beta_grad), static_cast<T*>(gamma_grad), (float)rows, p.epsilon});
-      launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms, VN == 8 ? 3 : 4), kBlock, s, x,
+      launch_overlapped(batchnorm_grad_training_vec_kernel<T, VN>, channel_stable_grid(n / VN, C / VN, sms, gradient_blocks(VN)), kBlock, s, x,
                         dy, static_cast<const float4*>(sc.terms), static_cast<T*>(output), n / VN, C);
       count_launch(2);
       cudaFreeAsync(sc.base, s);
