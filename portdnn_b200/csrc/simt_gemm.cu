@@ -48,6 +48,7 @@ struct SimtArgs {
   int a_rows, a_cols, a_channels, dir;
   int step_rows, step_cols, pad_rows, pad_cols, window_rows, window_cols;
   int conv, m_tiles, n_tiles, splits, slices;
+  int misses;  // some tap of some pixel lies outside the tensor that is read
   int act, staged;  // staged: the epilogue rounds to the tensors' type between its steps, as the direct kernel does
   float alpha, beta;
   int out_f32;
@@ -174,13 +175,18 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const
   }
 
   // the step that is fetched next
-  int run = begin / max(chunks, 1), k0 = (begin - run * chunks) * kTerms;
-  int ri = runs_s > 0 ? run / runs_s : 0, si = run - ri * runs_s;
-  bool new_run = true;
+  int run, k0, ri, si;
+  bool new_run;
   int at[kARuns ? kA : 1];
   int b_tap = 0;
+  auto first_step = [&] {
+    run = begin / max(chunks, 1), k0 = (begin - run * chunks) * kTerms;
+    ri = runs_s > 0 ? run / runs_s : 0, si = run - ri * runs_s;
+    new_run = true;
+  };
   const int b_first = bk * g.bk + (n0 + bn) * g.bn, b_step = kStepB * (B_RUNS ? g.bn : g.bk);
   float ra[kA], rb[kB];
+  unsigned inside = 0;  // which of ra are elements of the tensor
   auto fetch = [&](int buf) {
     if (new_run) {
       if constexpr (A == kRows) {
@@ -192,14 +198,21 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const
     }
     if constexpr (A == kRows) {
       const bool k_ok = k0 + ak < g.inner;
+      inside = 0;
 #pragma unroll
-      for (int i = 0; i < kA; ++i) ra[i] = k_ok && at[i] >= 0 ? to_f32(pa[at[i] + k0 + ak]) : 0.f;
+      for (int i = 0; i < kA; ++i) {
+        const bool ok = k_ok && at[i] >= 0;
+        ra[i] = ok ? to_f32(pa[at[i] + k0 + ak]) : 0.f;
+        inside |= (unsigned)ok << i;
+      }
     } else if constexpr (A == kPixels) {
+      inside = 0;
 #pragma unroll
       for (int i = 0; i < kA; ++i) {
         const int4 e = table[buf * kTerms + ak + i * kStepA];
         const bool ok = row_ok && (unsigned)(e.y + tap_h) < (unsigned)g.a_rows && (unsigned)(e.z + tap_w) < (unsigned)g.a_cols;
         ra[i] = ok ? to_f32(pa[e.x + tap_at]) : 0.f;
+        inside |= (unsigned)ok << i;
       }
     } else {
 #pragma unroll
@@ -245,6 +258,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const
       look_up(begin + 1);
       __syncthreads();
     }
+    first_step();
     fetch(begin & 1);
     put(0);
     __syncthreads();
@@ -267,32 +281,54 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const
     }
   }
 
-  // A tap outside the image has no term, whatever the other operand is there, but the tiles multiply it by zero: a
-  // sum that is not a number is formed again from the terms that there are.
-  auto terms_inside = [&](int row, int n) -> float {
-    const int from = part_at(slice * g.splits), to = part_at((slice + 1) * g.splits);
-    float v = 0.f;
-    if constexpr (A == kRows) {
+  // A tap outside the image has no term, whatever the other operand is there, but the tiles multiply it by zero: a block with a
+  // sum that is not a number forms its sums again from the terms that there are.  us, all numbers finite / one NaN in dy or the
+  // filter, fp32, forward, input gradient, filter gradient: 24x60x61 66 -> 97 3x3 532 / 845, 599 / 892, 630 / 1176; when the thread that
+  // stores a sum walked its terms alone, the NaN took 3564, 2886, 34876.
+  if constexpr (A != kColumns) {
+    if (g.misses) {
+      bool bad = false;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bad = bad || acc[i][j].x != acc[i][j].x || acc[i][j].y != acc[i][j].y;
+      if (__syncthreads_or(bad)) {
+        first_step();
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int st = from; st < to; ++st) {
-        const int rn = st / chunks, first = (st - rn * chunks) * kTerms, ti = rn / runs_s, tj = rn - ti * runs_s;
-        const int a0 = run_at(table[row], ti, tj);
-        if (a0 < 0) continue;
-        const int b0 = ((first_r + ti * tap_r) * g.window_cols + first_s + tj * tap_s) * g.bs + n * g.bn;
+        for (int step = begin; step < end; ++step) {
+          look_up(step);
+          __syncthreads();  // (everyone has read the step before)
+          fetch(step & 1);
+          put(0);
+#pragma unroll
+          for (int i = 0; i < kA; ++i) {  // where the elements are, in the second buffer
+            const float there = (inside >> i) & 1u ? 1.f : 0.f;
+            if (kARuns) as(1, ak)[am + i * kStepA] = there;
+            else as(1, ak + i * kStepA)[am] = there;
+          }
+          __syncthreads();
 #pragma unroll 1
-        for (int k = first; k < min(first + kTerms, g.inner); ++k) v = fmaf(to_f32(pa[a0 + k]), to_f32(pb[b0 + k * g.bk]), v);
-      }
-    } else if constexpr (A == kPixels) {
-      const int m = m0 + row, c = m % g.a_channels, tap = m / g.a_channels, h = tap / g.window_cols, w = tap - h * g.window_cols;
-#pragma unroll 1
-      for (int p = from * kTerms; p < min(to * kTerms, g.inner); ++p) {
-        const int4 e = pixel(p);
-        if ((unsigned)(e.y + h) >= (unsigned)g.a_rows || (unsigned)(e.z + w) >= (unsigned)g.a_cols) continue;
-        v = fmaf(to_f32(pa[e.x + (h * g.a_cols + w) * g.a_channels + c]), to_f32(pb[p * g.bk + n * g.bn]), v);
+          for (int k = 0; k < kTerms; ++k) {
+            const float4 av = *reinterpret_cast<const float4*>(as(0, k) + tm * 4), bv = *reinterpret_cast<const float4*>(bs(0, k) + tn * 4);
+            const float4 there = *reinterpret_cast<const float4*>(as(1, k) + tm * 4);
+            const float b[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (there.x != 0.f) acc[0][j].x = fmaf(av.x, b[j], acc[0][j].x);
+              if (there.y != 0.f) acc[0][j].y = fmaf(av.y, b[j], acc[0][j].y);
+              if (there.z != 0.f) acc[1][j].x = fmaf(av.z, b[j], acc[1][j].x);
+              if (there.w != 0.f) acc[1][j].y = fmaf(av.w, b[j], acc[1][j].y);
+            }
+          }
+        }
+        __syncthreads();
       }
     }
-    return v;
-  };
+  }
   const float bias = g.staged && g.bias != nullptr && n0 + t % BN < g.n ? load<T>(g.bias, n0 + t % BN) : 0.f;
 
   // the sums of the cluster's blocks, in the order of their terms, each block a share of the rows
@@ -325,7 +361,6 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) simt_gemm_kernel(const
       const int row = row0 + u * kRowStep, m = m0 + row;
       if (row >= last || m >= M) break;
       float v = sums[u];
-      if (g.conv && v != v) v = terms_inside(row, n);
       long long o = n * g.on;
       if (g.partial != nullptr) {
         g.partial[(long long)slice * M * g.n + m * g.om + o] = v;
@@ -446,6 +481,12 @@ bool thread_to_an_output(int pass, const PdnnConv2DParams& p) {
   return pixels * p.batch < 160 && per_image * p.batch < 2e6;
 }
 
+// Whether a tap of an output (of a pixel of the input, in an input gradient) can lie outside along one axis.
+bool taps_miss(int pass, int in, int out, int window, int stride, int pad) {
+  if (pass == PDNN_INPUT_BACKPROP) return pad < window - 1 || ((long long)in - 1 + pad) / stride > out - 1;
+  return pad > 0 || ((long long)out - 1) * stride - pad + window > in;
+}
+
 int sm_count() {
   const int sms = device_sm_count();
   return sms > 0 ? sms : 148;
@@ -498,6 +539,8 @@ int simt_conv(int pass, int dtype, const void* in, const void* fil, void* out, c
     g.bs = 0, g.bk = p.features, g.bn = 1;
     g.om = fhwc ? 1 : p.features, g.on = fhwc ? taps * p.channels : 1;
   }
+  g.misses = taps_miss(pass, p.in_rows, p.out_rows, p.window_rows, p.stride_rows, p.pad_rows) ||
+             taps_miss(pass, p.in_cols, p.out_cols, p.window_cols, p.stride_cols, p.pad_cols);
   const size_t n_out = (size_t)taps * p.channels * p.features, need = (size_t)t.slices * n_out * sizeof(float);
   if (t.slices > 1 && cudaMallocAsync(reinterpret_cast<void**>(&g.partial), need, s) != cudaSuccess) {
     cudaGetLastError();
