@@ -126,9 +126,10 @@ __global__ void __launch_bounds__(kBlock)
 // A count off a multiple of 8, padded.  A multiple of 8 would do, but rows that start inside a 32-byte sector cost the tiles' loads
 // one more sector and often a second line each (bf16, us, 7x45x61 3x3, input gradient: 128 -> 152 features 27.0, 160 16.5,
 // 192 13.1; forward pass, 104 -> 128 channels 14.5, 112 11.7, 128 10.1).  So whole lines of 64 where they
-// are hardly more to copy, else whole sectors of 16.
-int padded_count(int n) {
+// are hardly more to copy, else whole sectors of 16; `narrow`: the multiple of 8.
+int padded_count(int n, bool narrow) {
   if (n % 8 == 0) return n;
+  if (narrow) return (int)round_up((size_t)n, 8);
   const int lines = (int)round_up((size_t)n, 64);
   return 10ll * lines <= 13ll * n ? lines : (int)round_up((size_t)n, 16);
 }
@@ -142,14 +143,14 @@ struct Plan {
 
 // The tensor-core kernels have to take the padded layer; `plan.q` keeps the channels of a few-channel
 // layer, which is packed on its own there.
-bool make_plan(int pass, int dtype, const PdnnConv2DParams& p, Plan* plan) {
+bool plan_with(int pass, int dtype, const PdnnConv2DParams& p, bool narrow, Plan* plan) {
   if (dtype == PDNN_F32 || p.groups != 1 || p.input_format != 0) return false;
   if (p.filter_format != 0 && p.filter_format != 2) return false;
   PdnnConv2DParams q = p;
   const void* aligned = reinterpret_cast<const void*>(uintptr_t(256));
-  q.features = padded_count(p.features);
+  q.features = padded_count(p.features, narrow);
   if (!tc_conv_supported(pass, dtype, aligned, aligned, aligned, q)) {
-    q.channels = padded_count(p.channels);
+    q.channels = padded_count(p.channels, narrow);
     if (!tc_conv_supported(pass, dtype, aligned, aligned, aligned, q)) return false;
   }
   const size_t px_in = (size_t)p.batch * p.in_rows * p.in_cols, px_out = (size_t)p.batch * p.out_rows * p.out_cols;
@@ -160,6 +161,11 @@ bool make_plan(int pass, int dtype, const PdnnConv2DParams& p, Plan* plan) {
   plan->same_c = q.channels == p.channels, plan->same_k = q.features == p.features;
   const size_t most = 0xF0000000u;  // packet indices are 32 bits wide
   return plan->x < most && plan->w < most && plan->y < most;
+}
+
+// Multiples of 8 where wider copies have too many elements.
+bool make_plan(int pass, int dtype, const PdnnConv2DParams& p, Plan* plan) {
+  return plan_with(pass, dtype, p, false, plan) || plan_with(pass, dtype, p, true, plan);
 }
 
 // The copies, the kernels' own workspace and the padded result, each on a boundary of 256 bytes.
@@ -217,15 +223,26 @@ int padded_conv(int pass, int dtype, const void* in, const void* fil, void* out,
                 const PdnnConvEpilogue* epi, const PdnnBackpropFusion* fusion, void* ws, size_t ws_elems, cudaStream_t s) {
   Plan plan;
   if (!make_plan(pass, dtype, p, &plan)) return kNeedsDirect;
-  const PdnnConv2DParams& q = plan.q;
   const int sms = device_sm_count();
-  const size_t need = scratch_bytes(pass, dtype, plan);
+  size_t need = scratch_bytes(pass, dtype, plan);
+  // Scratch that holds copies to multiples of 8 only is used for those, whether the caller brought it or no more is to be had.
+  Plan less;
+  const size_t need_less = plan_with(pass, dtype, p, true, &less) ? scratch_bytes(pass, dtype, less) : need;
+  auto make_do = [&] {
+    if (need_less >= need) return false;
+    plan = less, need = need_less;
+    return true;
+  };
   char* base = static_cast<char*>(ws);
+  if (base != nullptr && ws_elems * 2 < need && ws_elems * 2 >= need_less) make_do();
   const bool own = base == nullptr || ws_elems * 2 < need;
-  if (own && cudaMallocAsync(reinterpret_cast<void**>(&base), need, s) != cudaSuccess) {
+  auto allocate = [&] {
+    if (cudaMallocAsync(reinterpret_cast<void**>(&base), need, s) == cudaSuccess) return true;
     cudaGetLastError();
-    return kNeedsDirect;  // (the direct kernel reads the tensors where they are)
-  }
+    return false;
+  };
+  if (own && !allocate() && !(make_do() && allocate())) return kNeedsDirect;  // (the direct kernel reads the tensors where they are)
+  const PdnnConv2DParams& q = plan.q;
   char* at = reinterpret_cast<char*>(round_up(reinterpret_cast<uintptr_t>(base), 256));
   auto take = [&](size_t bytes) {
     char* r = at;
