@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(256) widen_to_f32_kernel(const T* __restrict__
 
 // What no tensor-core kernel takes: fp32 tiles on the CUDA cores where they gain, else a thread to an output.
 int general_conv(int pass, int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
-                 const PdnnConvEpilogue* epi, bool tiled, cudaStream_t s) {
-  if (tiled && simt_conv_applicable(pass, p)) return simt_conv(pass, dtype, in, fil, out, p, epi, s);
+                 const PdnnConvEpilogue* epi, bool tiled, void* ws, size_t ws_elems, cudaStream_t s) {
+  if (tiled && simt_conv_applicable(pass, p)) return simt_conv(pass, dtype, in, fil, out, p, epi, ws, ws_elems, s);
   return launch_direct_conv(pass, dtype, in, fil, out, p, epi, s);
 }
 
@@ -138,7 +138,7 @@ int general_conv(int pass, int dtype, const void* in, const void* fil, void* out
 // does not take): the ReLU-gradient mask as a pointwise pass in place, an fp32 filter gradient
 // through a temporary in the tensors' own type.
 int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
-                        const PdnnBackpropFusion* fusion, bool tiled, cudaStream_t s) {
+                        const PdnnBackpropFusion* fusion, bool tiled, void* ws, size_t ws_elems, cudaStream_t s) {
   const size_t es = dtype_size(dtype);
   if (pass == PDNN_FILTER_BACKPROP && fusion != nullptr && fusion->accumulate && !(fusion->output_f32 && dtype != PDNN_F32)) {
     // dW += gradient in the tensors' own type: the gradient into a temporary, then one blend
@@ -148,7 +148,7 @@ int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, vo
       cudaGetLastError();
       return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for the filter gradient", n * es);
     }
-    int st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, s);
+    int st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, ws, ws_elems, s);
     if (st == PDNN_OK) st = launch_scale_blend(dtype, tmp, 1.f, out, 1.f, out, n, s);
     cudaFreeAsync(tmp, s);
     return st;
@@ -160,7 +160,7 @@ int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, vo
       cudaGetLastError();
       return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for the filter gradient", n * es);
     }
-    int st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, s);
+    int st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, ws, ws_elems, s);
     if (st == PDNN_OK) {
       const unsigned grid = grid_for(n, 256, device_sm_count());
       if (dtype == PDNN_F16) widen_to_f32_kernel<__half><<<grid, 256, 0, s>>>(static_cast<const __half*>(tmp), static_cast<float*>(out), n, fusion->accumulate != 0);
@@ -178,11 +178,11 @@ int run_direct_backprop(int pass, int dtype, const void* in, const void* fil, vo
       cudaGetLastError();
       return fail(PDNN_ALLOCATION_PROBLEM, "conv2d: cannot allocate %zu bytes for the input gradient", n_dx * es);
     }
-    st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, s);
+    st = general_conv(pass, dtype, in, fil, tmp, p, nullptr, tiled, ws, ws_elems, s);
     if (st == PDNN_OK) st = launch_scale_blend(dtype, tmp, 1.f, out, 1.f, out, n_dx, s);
     cudaFreeAsync(tmp, s);
   } else {
-    st = general_conv(pass, dtype, in, fil, out, p, nullptr, tiled, s);
+    st = general_conv(pass, dtype, in, fil, out, p, nullptr, tiled, ws, ws_elems, s);
   }
   if (st != PDNN_OK || pass != PDNN_INPUT_BACKPROP || fusion == nullptr) return st;
   if (fusion->relu_bitmask != nullptr) return launch_relu_grad_bits(dtype, fusion->relu_bitmask, out, n_dx, s);
@@ -245,8 +245,8 @@ int dispatch_conv(int pass, int dtype, const void* in, const void* fil, void* ou
     if (st2 != kNeedsDirect) return st2;
   }
   const bool tiled = algorithm != PDNN_ALGO_DIRECT;
-  if (pass != PDNN_FORWARD) return run_direct_backprop(pass, dtype, in, fil, out, *p, fusion, tiled, s);
-  return general_conv(pass, dtype, in, fil, out, *p, epi, tiled, s);
+  if (pass != PDNN_FORWARD) return run_direct_backprop(pass, dtype, in, fil, out, *p, fusion, tiled, ws, ws_elems, s);
+  return general_conv(pass, dtype, in, fil, out, *p, epi, tiled, ws, ws_elems, s);
 }
 
 }  // namespace
@@ -312,6 +312,7 @@ int pdnn_conv2d_workspace_size(int pass, int dtype, const PdnnConv2DParams* para
   // packed and padded operands - goes to scratch that the call allocates where the caller brings none.
   size_t elems = tc_conv_workspace_elems(pass, dtype, *params);
   if (elems == 0) elems = padded_conv_workspace_elems(pass, dtype, *params);
+  if (elems == 0 && !tc_conv_shape_supported(pass, dtype, *params)) elems = simt_conv_workspace_elems(pass, dtype, *params);
   // Winograd: 16 * (C*K + tiles*C + tiles*K), include/portdnn/conv2d/workspace_size.h:53-73.  It is
   // reported as recommended, not required: without it the layer still runs (on the implicit GEMM).
   if ((algorithm == PDNN_ALGO_WINOGRAD || algorithm == PDNN_ALGO_WINOGRAD_LARGE) &&

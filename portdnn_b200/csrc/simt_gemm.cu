@@ -458,6 +458,10 @@ Tiling conv_tiling(int pass, const PdnnConv2DParams& p, bool any_order, int sms)
   return choose(taps * p.channels, taps * p.channels, p.features, p.batch * px_out, 1, 1, true, sms);
 }
 
+size_t slices_bytes(const Tiling& t, const PdnnConv2DParams& p) {
+  return (size_t)t.slices * p.window_rows * p.window_cols * p.channels * p.features * sizeof(float);
+}
+
 // Where a thread to an output is still the better one (direct_conv.cu): its time is the length of a sum until the work fills the
 // device, that of the tiles the latency of their loads.  us, thread to an output / tiles here:
 //   images, size, channels, window      | forward     | input gradient | filter gradient
@@ -510,8 +514,15 @@ bool simt_conv_applicable(int pass, const PdnnConv2DParams& p) {
   return blocks < 2147483632.0 && !thread_to_an_output(pass, p);
 }
 
+size_t simt_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p) {
+  if (pass != PDNN_FILTER_BACKPROP || !simt_conv_applicable(pass, p)) return 0;
+  const Tiling t = conv_tiling(pass, p, true, sm_count());
+  if (t.slices == 1) return 0;
+  return slices_bytes(t, p) / dtype_size(dtype);
+}
+
 int simt_conv(int pass, int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
-              const PdnnConvEpilogue* epi, cudaStream_t s) {
+              const PdnnConvEpilogue* epi, void* ws, size_t ws_elems, cudaStream_t s) {
   const int sms = sm_count(), taps = p.window_rows * p.window_cols;
   Tiling t = conv_tiling(pass, p, pass != PDNN_FORWARD || (epi != nullptr && epi->any_order), sms);
   const bool fhwc = p.filter_format == 2;
@@ -541,10 +552,16 @@ int simt_conv(int pass, int dtype, const void* in, const void* fil, void* out, c
   }
   g.misses = taps_miss(pass, p.in_rows, p.out_rows, p.window_rows, p.stride_rows, p.pad_rows) ||
              taps_miss(pass, p.in_cols, p.out_cols, p.window_cols, p.stride_cols, p.pad_cols);
-  const size_t n_out = (size_t)taps * p.channels * p.features, need = (size_t)t.slices * n_out * sizeof(float);
-  if (t.slices > 1 && cudaMallocAsync(reinterpret_cast<void**>(&g.partial), need, s) != cudaSuccess) {
-    cudaGetLastError();
-    g.partial = nullptr, t.slices = 1;
+  const size_t n_out = (size_t)taps * p.channels * p.features;
+  bool own = false;
+  if (t.slices > 1) {
+    const size_t need = slices_bytes(t, p);
+    own = ws == nullptr || !aligned16(ws) || ws_elems * dtype_size(dtype) < need;
+    g.partial = static_cast<float*>(ws);
+    if (own && cudaMallocAsync(reinterpret_cast<void**>(&g.partial), need, s) != cudaSuccess) {
+      cudaGetLastError();
+      g.partial = nullptr, own = false, t.slices = 1;
+    }
   }
   g.m_tiles = t.m_tiles, g.n_tiles = t.n_tiles, g.splits = t.splits, g.slices = t.slices;
   const long long blocks = (long long)outer * t.slices * t.n_tiles * t.m_tiles * t.splits;
@@ -558,7 +575,7 @@ int simt_conv(int pass, int dtype, const void* in, const void* fil, void* out, c
     else launch_column_sums(g.partial, t.slices, n_out, sms, s, StoreSum<__nv_bfloat16>{static_cast<__nv_bfloat16*>(out), false});
     st = check_launch("conv2d filter gradient");
   }
-  if (g.partial != nullptr) cudaFreeAsync(g.partial, s);
+  if (own) cudaFreeAsync(g.partial, s);
   return st;
 }
 

@@ -4213,11 +4213,15 @@ __global__ void __launch_bounds__(256) simt_matmul_kernel(const T* __restrict__ 
 
 bool tc_conv_supported(int pass, int dtype, const void* in, const void* fil, const void* out,
                        const PdnnConv2DParams& p) {
-  if (encode_fn() == nullptr) return false;
+  if (encode_fn() == nullptr || !tc_conv_shape_supported(pass, dtype, p)) return false;
   if (pass == PDNN_FORWARD && small_c_applicable(dtype, p)) return aligned16(out);
   if (pass == PDNN_FILTER_BACKPROP && small_c_applicable(dtype, p)) return aligned16(fil);
+  return aligned16(in) && aligned16(fil) && aligned16(out);
+}
+
+bool tc_conv_shape_supported(int pass, int dtype, const PdnnConv2DParams& p) {
+  if (pass != PDNN_INPUT_BACKPROP && small_c_applicable(dtype, p)) return true;
   if (!conv_common_ok(dtype, p)) return false;
-  if (!aligned16(in) || !aligned16(fil) || !aligned16(out)) return false;
   for (int ph = 0; ph < p.stride_rows; ++ph)
     for (int pw = 0; pw < p.stride_cols; ++pw)
       if (p.in_rows - ph <= 0 || p.in_cols - pw <= 0) return false;

@@ -12,6 +12,9 @@ namespace pdnn {
 bool tc_conv_supported(int pass, int dtype, const void* in, const void* fil, const void* out,
                        const PdnnConv2DParams& p);
 
+// The part of it that the layer's shape decides.
+bool tc_conv_shape_supported(int pass, int dtype, const PdnnConv2DParams& p);
+
 // Scratch elements (of dtype) the pass can use: the filter backprop's partial sums, the packed copies of a layer
 // of few channels, the packed filter of a grouped layer.
 size_t tc_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p);
