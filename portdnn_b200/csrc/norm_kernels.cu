@@ -109,7 +109,13 @@ __global__ void __launch_bounds__(kBlock) softmax_forward_vec_kernel(const T* x,
 // Few pixels of many channels: a block of four warps per pixel, a packet to a thread, so that a quarter of the exponentials and
 // divisions stand one after another in a thread.  The sums of the packets are added up in the order of
 // softmax_forward_vec_kernel, whose lane has packets lane, lane + 32, ...: a pixel's result does not depend on how many there are.
+// us, a warp to a pixel / here, 250, 700, 1024, 2000 pixels: f16 1000 channels 2.95 1.65, 3.00 2.05, 3.03 2.38, 3.77 3.72; 264 channels 2.13 1.61,
+// 2.16 1.76, 2.18 2.33, 2.55 2.61; f32 500 channels 2.10 1.48, 2.15 1.71, 2.19 2.23, 2.65 2.73; 132 channels 1.71 1.44, 1.74 1.56, 1.76 1.88,
+// 1.98 2.36.  So up to six blocks to an SM, and up to a whole wave of them where a warp has more than 64 packets of 16 bits.
 constexpr int kSoftmaxRow = 128;
+bool softmax_by_rows(size_t rows, int packets, bool wide, int sms) {
+  return rows <= (size_t)sms * (wide && packets > 64 ? 2048 / kSoftmaxRow : 6);
+}
 template <typename T, int V>
 __global__ void __launch_bounds__(kSoftmaxRow) softmax_forward_row_kernel(const T* x, T* __restrict__ y, int C) {
   overlap_wait();
@@ -970,7 +976,7 @@ int launch_softmax(int direction, int dtype, const void* input, const void* grad
     if (direction == 0 && vec && p.channels <= 32 * VN)
       launch_overlapped(softmax_forward_vec_kernel<T, VN, 1>, grid, kBlock, s, static_cast<const T*>(input),
                         static_cast<T*>(output), rows, p.channels);
-    else if (direction == 0 && vec && p.channels <= kSoftmaxRow * VN && rows <= (size_t)sms * (2048 / kSoftmaxRow))  // (one wave)
+    else if (direction == 0 && vec && p.channels <= kSoftmaxRow * VN && softmax_by_rows(rows, p.channels / VN, VN == 8, sms))
       launch_overlapped(softmax_forward_row_kernel<T, VN>, (unsigned)rows, kSoftmaxRow, s, static_cast<const T*>(input),
                         static_cast<T*>(output), p.channels);
     else if (direction == 0 && vec && p.channels <= 128 * VN)

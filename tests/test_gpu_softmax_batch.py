@@ -4,6 +4,7 @@ import torch
 
 import portdnn_b200 as pd
 from gpu_util import TORCH_DTYPES
+from launched import launched
 
 pytestmark = pytest.mark.gpu
 
@@ -18,3 +19,14 @@ def test_alone_and_beside_others(packets, dtype):
     few = pd.softmax(x[:500].reshape(-1), 500, 1, 1, c).view(500, c)
     assert torch.equal(few, many[:500])
     assert torch.equal(pd.softmax(x[7].contiguous(), 1, 1, 1, c), many[7])
+
+
+@pytest.mark.parametrize("dtype,channels,rows,by_rows", [
+    ("f16", 1000, 148 * 16, True), ("f16", 1000, 148 * 16 + 1, False), ("f16", 512, 148 * 6, True), ("f16", 512, 148 * 6 + 1, False),
+    ("f32", 500, 148 * 6, True), ("f32", 500, 148 * 6 + 1, False), ("f32", 128, 8, False)])
+def test_where_four_warps_take_a_pixel(dtype, channels, rows, by_rows):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the numbers of pixels are those of 148 SMs")
+    x = torch.randn(rows * channels, device="cuda").to(TORCH_DTYPES[dtype])
+    kernels = launched(lambda: pd.softmax(x, rows, 1, 1, channels))
+    assert len(kernels) == 1 and ("softmax_forward_row_kernel" in kernels[0].name) == by_rows
