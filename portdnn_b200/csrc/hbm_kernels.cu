@@ -420,6 +420,18 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
+// How many of `all` rows a thread walks down a column of a stride-2 gradient: enough threads to fill the device a few times over,
+// otherwise walks as long as possible.  Few columns: shorter walks still, each of which costs a thread 0.3 us a row (us, 4 rows / 1: pools,
+// one image 112x112x64 f16 8.6 / 5.7, four 60x80x96 9.0 / 6.8), as long as all threads are on the device together,
+// 512 to an SM (depthwise, us, walks within one wave / a row less each, beyond it: 24x45x62x96 f16 5.1 / 7.0, 10x17x24x688 4.2 / 5.1).
+int rows_of_a_walk(int all, size_t columns, int sms) {
+  auto threads = [&](int rows) { return columns * ((all + rows - 1) / rows); };
+  int rows = all;
+  while (rows > 4 && threads(rows) < (size_t)sms * 2048) rows = (rows + 1) / 2;
+  while (rows > 1 && threads((rows + 1) / 2) <= (size_t)sms * 512) rows = (rows + 1) / 2;
+  return rows;
+}
+
 // The gather for 3x3 windows with stride 2, walking the windows instead of the input pixels.  With
 // m = (h + pad) / 2 the input rows 2m - pad and 2m + 1 - pad lie in windows {m - 1, m} (as their
 // rows 2 and 0) and {m} (row 1); columns likewise.  A thread owns a packet of channels at one
@@ -2003,11 +2015,7 @@ int pooling_max_grad_impl(int op, int dtype, const void* x, const void* y, const
                            (p.in_rows - 1 + p.pad_rows) / 2 + 1, (p.in_cols - 1 + p.pad_cols) / 2 + 1, 0, 0,
                            reads_from_the_end(in_items * VN * sizeof(T))};
           const size_t columns = (size_t)p.batch * g.K * (p.channels / VN);
-          g.rows = g.M;
-          while (g.rows > 4 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 2048) g.rows = (g.rows + 1) / 2;
-          // few columns: shorter walks still, each of which costs a thread 0.3 us a row (us, 4 rows / 1: one image 112x112x64 f16
-          // 8.6 / 5.7, four 60x80x96 9.0 / 6.8, both kernels)
-          while (g.rows > 1 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 512) g.rows = (g.rows + 1) / 2;
+          g.rows = rows_of_a_walk(g.M, columns, sms);
           g.strips = (g.M + g.rows - 1) / g.rows;
           const size_t n_items = columns * g.strips;
           // Below three quarters of a wave the overlap is worth more, above it the read-only loads (us, overlapped /
@@ -2247,11 +2255,8 @@ int launch_depthwise(int pass, int dtype, const void* in, const void* fil, void*
         p.stride_cols == 2) {
       IbpS2Geometry g{p.in_rows, p.in_cols, p.out_rows, p.out_cols, p.channels, p.pad_rows, p.pad_cols, p.batch,
                       (p.in_rows - 1 + p.pad_rows) / 2 + 1, (p.in_cols - 1 + p.pad_cols) / 2 + 1, 0, 0};
-      // enough threads to fill the device a few times over, otherwise strips as long as possible
       const size_t columns = (size_t)p.batch * g.K * (p.channels / VN);
-      g.rows = g.M;
-      while (g.rows > 4 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 2048) g.rows = (g.rows + 1) / 2;
-      while (g.rows > 1 && columns * ((g.M + g.rows - 1) / g.rows) < (size_t)sms * 512) g.rows = (g.rows + 1) / 2;  // (as for the pools)
+      g.rows = rows_of_a_walk(g.M, columns, sms);
       g.strips = (g.M + g.rows - 1) / g.rows;
       const size_t n_items = columns * g.strips;
       if (n_items < 0xFFFF0000ull) {

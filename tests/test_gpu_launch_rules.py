@@ -1,0 +1,36 @@
+"""Which kernel or grid a call takes on either side of a rule's line, read from the kernel nodes of a captured graph.  The lines
+themselves were measured; the figures stand beside the rules."""
+import pytest
+import torch
+
+import portdnn_b200 as pd
+from gpu_util import TORCH_DTYPES
+from launched import launched
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _sms():
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+
+
+def _rand(n, dtype):
+    return torch.randn(n, device="cuda").to(TORCH_DTYPES[dtype])
+
+
+@pytest.mark.parametrize("n,h,w,c,dtype", [(24, 45, 62, 96, "f16"), (10, 17, 24, 688, "f16"), (39, 31, 28, 64, "f32"), (30, 60, 59, 40, "bf16")])
+def test_short_walks_stay_within_one_wave(n, h, w, c, dtype):
+    """Stride-2 gradients, depthwise and of 3x3 pools: threads by the length of their walks, 512 to an SM at most where the
+    walks are shorter than four rows."""
+    p = pd.depthwise_params(n, h, w, c, 1, 3, 2)
+    dy, f = _rand(n * p.out_rows * p.out_cols * c, dtype), _rand(9 * c, dtype)
+    kernels = launched(lambda: pd.depthwise_conv2d(pd.INPUT_BACKPROP, dy, f, p))
+    assert len(kernels) == 1 and "depthwise_ibp_s2_kernel" in kernels[0].name
+    assert 148 * 256 < kernels[0].blocks * kernels[0].threads <= 148 * 512 + 256
+    q = pd.pool_params(n, h, w, c, 3, 2, True)
+    x = _rand(n * h * w * c, dtype)
+    y = pd.pooling(pd.POOL_MAX, 0, x, q)
+    kernels = [k for k in launched(lambda: pd.pooling_max_grad(pd.POOL_MAX, x, y, dy, q)) if "pool_max_grad_s2" in k.name]
+    assert len(kernels) == 1 and 148 * 256 < kernels[0].blocks * kernels[0].threads <= 148 * 512 + 256
