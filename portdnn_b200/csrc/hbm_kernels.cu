@@ -1237,8 +1237,9 @@ __device__ __forceinline__ float binary_value(float a, float b, int op) {
 }
 
 // MODE 0: forward, 1: gradient, 2: a binary operator on tensors of one shape.  OP: the operator where it is one that networks run
-// between their convolutions, else -1 and the operator is any_op: with the choice in the loop a packet cost more instructions
-// than memory time.  Four packets in flight (two of either operand), 16 blocks to an SM, or 32 where the tensors
+// between their convolutions, else -1 and the operator is any_op: with the choice in the loop a packet costs more instructions
+// than memory time, and a body with the choice in every one of its packets is slow to fetch (bf16 tanh gradient, 416 elements
+// 0.89 us in one body of two packets, 1.52 in two bodies of two and of one; 3 million 2.82 and 4.96).  Known operators: four packets in flight (two of either operand), 16 blocks to an SM, or 32 where the tensors
 // stream through L2 (256x56x56x256: 130 and 127 us).  f16, us, choice in the loop and two packets / here: ReLU6 64x14x14x576
 // 4.8 / 4.0, 64x28x28x256 6.6 / 5.6; ReLU gradient 5.5 / 4.1, 8.6 / 6.2; the sum of two tensors, through
 // binaryop_kernel's coordinates before, 6.4 / 4.1, 10.2 / 6.4.
@@ -1246,7 +1247,7 @@ template <typename T, int V, int MODE, int OP>
 __global__ void __launch_bounds__(kBlock)
     pointwise_kernel(int any_op, const T* a, const T* b, T* __restrict__ out, size_t n_packets) {
   overlap_wait();
-  constexpr int U = MODE == 0 ? 4 : 2;
+  constexpr int U = MODE == 0 && OP >= 0 ? 4 : 2;
   const int op = OP >= 0 ? OP : any_op;
   const size_t step = (size_t)gridDim.x * kBlock;
   auto put = [&](size_t i, const float (&av)[V], const float (&bv)[V]) {
@@ -1257,6 +1258,24 @@ __global__ void __launch_bounds__(kBlock)
     store_vec<T, V>(out + i * V, res);
   };
   size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x;
+  if constexpr (OP < 0 && MODE != 2) {
+    for (; i < n_packets; i += U * step) {
+      const int count = i + step < n_packets ? U : 1;
+      float av[U][V], bv[U][V];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (u >= count) break;
+        load_vec<T, V>(a + (i + u * step) * V, av[u]);
+        if (MODE != 0) load_vec<T, V>(b + (i + u * step) * V, bv[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (u >= count) break;
+        put(i + u * step, av[u], bv[u]);
+      }
+    }
+    return;
+  }
   for (; i + (U - 1) * step < n_packets; i += U * step) {
     float av[U][V], bv[U][V];
 #pragma unroll
@@ -2310,7 +2329,7 @@ int launch_pointwise(int op, int dtype, const void* in, void* out, size_t n, cud
     else if (op == PDNN_ACT_RELU6)
       launch_overlapped(pointwise_kernel<T, VN, 0, PDNN_ACT_RELU6>, grid, kBlock, s, op, a, none, to, n / VN);
     else
-      launch_overlapped(pointwise_kernel<T, VN, 0, -1>, grid, kBlock, s, op, a, none, to, n / VN);
+      launch_overlapped(pointwise_kernel<T, VN, 0, -1>, grid_for(n / VN, kBlock, sms), kBlock, s, op, a, none, to, n / VN);
     return check_launch("pointwise");
   });
 }
@@ -2332,7 +2351,7 @@ int launch_pointwise_grad(int op, int dtype, const void* fwd, const void* err, v
     else if (op == PDNN_ACT_RELU)
       launch_overlapped(pointwise_kernel<T, VN, 1, PDNN_ACT_RELU>, grid, kBlock, s, op, a, b, to, n / VN);
     else
-      launch_overlapped(pointwise_kernel<T, VN, 1, -1>, grid, kBlock, s, op, a, b, to, n / VN);
+      launch_overlapped(pointwise_kernel<T, VN, 1, -1>, grid_for(n / VN, kBlock, sms), kBlock, s, op, a, b, to, n / VN);
     return check_launch("pointwise gradient");
   });
 }
