@@ -887,10 +887,13 @@ struct StoreGradStats {
 
 // Slices of the moments kernel, a multiple of 32 rows each (whole batches of every row lane): one wave of three blocks per SM,
 // all of which then end together, and half as many sets to merge as with two (us, forward / gradient, two waves / one: 64x28x28x256
-// f16 16.1 / 12.8 and 36.3 / 32.8, 128x56x56x64 41.9 / 37.3 and 75.2 / 70.5).
-int moment_slices(size_t rows, int C, int sms, size_t* rows_per_slice) {
+// f16 16.1 / 12.8 and 36.3 / 32.8, 128x56x56x64 41.9 / 37.3 and 75.2 / 70.5).  No block more than that: one of a second wave
+// takes as long as the first (64x28x28x2048 f16, 28 slices of 16 tiles for 444 places 119.5 and 209.6, 27 slices 84.4 and 172.9).
+// `waves` 2: the forward pass in fp32 on tensors well beyond the L2 cache (30x56x56x640 90.3 in one, 84.6 in two; 110x24x24x752 73.8 / 69.7;
+// 64x28x28x640, 128 MB, 48.5 / 50.4).
+int moment_slices(size_t rows, int C, int sms, int waves, size_t* rows_per_slice) {
   const size_t ctiles = (size_t)(C + 32 * kMomentChannels - 1) / (32 * kMomentChannels);
-  size_t want = ((size_t)sms * kMomentBlocks + ctiles - 1) / ctiles;
+  const size_t want = std::max<size_t>((size_t)sms * kMomentBlocks * waves / ctiles, 1);
   size_t per = (rows + want - 1) / want;
   per = (per + 8 * kBatch - 1) / (8 * kBatch) * (8 * kBatch);
   if (per < 64) per = 64;
@@ -1020,7 +1023,7 @@ int launch_batchnorm_forward(int dtype, const void* input, const void* beta, con
     if (vec && p.is_training) {
       // output, batch moments and running statistics in two kernels
       size_t per = 0;
-      const int slices = moment_slices(rows, C, sms, &per);
+      const int slices = moment_slices(rows, C, sms, sizeof(T) == 4 && 2 * n * sizeof(T) > 5 * kStreamedBytes ? 2 : 1, &per);
       Scratch sc;
       const int st = get_scratch(&sc, Moments<false>::N / 2 * slices, C, s);
       if (st != PDNN_OK) return st;
@@ -1092,7 +1095,7 @@ int launch_batchnorm_gradient(int dtype, const void* input, const void* gradient
                      (p.is_training || aligned16(pop_variance));
     const bool one_pass = vec && p.is_training;
     size_t per_slice = 0;
-    const int slices = one_pass ? moment_slices(rows, C, sms, &per_slice) : slices_for(rows, C, sms, vec ? 32 * VN : 32);
+    const int slices = one_pass ? moment_slices(rows, C, sms, 1, &per_slice) : slices_for(rows, C, sms, vec ? 32 * VN : 32);
     if (!one_pass) per_slice = (rows + slices - 1) / slices;
     Scratch sc;
     int st = get_scratch(&sc, one_pass ? Moments<true>::N / 2 * slices : slices, C, s);
