@@ -34,3 +34,25 @@ def test_short_walks_stay_within_one_wave(n, h, w, c, dtype):
     y = pd.pooling(pd.POOL_MAX, 0, x, q)
     kernels = [k for k in launched(lambda: pd.pooling_max_grad(pd.POOL_MAX, x, y, dy, q)) if "pool_max_grad_s2" in k.name]
     assert len(kernels) == 1 and 148 * 256 < kernels[0].blocks * kernels[0].threads <= 148 * 512 + 256
+
+
+@pytest.mark.parametrize("n,h,c,dtype,most", [(64, 28, 2048, "f16", 444), (64, 28, 904, "f16", 444), (64, 28, 1664, "bf16", 444), (128, 14, 640, "f32", 444),
+                                              (16, 56, 1024, "f32", 888)])
+def test_statistics_take_whole_waves(n, h, c, dtype, most):
+    """Three blocks to an SM, in one wave or, fp32 tensors well beyond the L2 cache, two; no block more."""
+    p, size = pd.batchnorm_params(n, h, h, c, True), n * h * h * c
+    x, dy, v = _rand(size, dtype), _rand(size, dtype), _rand(c, dtype).abs()
+    for call, limit in ((lambda: pd.batchnorm_forward(x, v, v, v, v, p), most), (lambda: pd.batchnorm_gradient(x, dy, v, p), 444)):
+        kernels = [k for k in launched(call) if "batchnorm_moments_kernel" in k.name]
+        assert len(kernels) == 1 and limit * 3 // 4 < kernels[0].blocks <= limit
+
+
+@pytest.mark.parametrize("c", [904, 936, 1000, 1016, 888])
+def test_threads_of_a_gradient_keep_their_channels(c):
+    """16-bit training gradients: the threads are a multiple of the packets of a pixel, also where a wave has no room for more
+    than four of their units."""
+    n, h = 118, 8
+    p, size = pd.batchnorm_params(n, h, h, c, True), n * h * h * c
+    x, dy, g = _rand(size, "bf16"), _rand(size, "bf16"), _rand(c, "bf16")
+    kernels = [k for k in launched(lambda: pd.batchnorm_gradient(x, dy, g, p)) if "grad_training_vec" in k.name]
+    assert len(kernels) == 1 and kernels[0].blocks * kernels[0].threads % (c // 8) == 0
