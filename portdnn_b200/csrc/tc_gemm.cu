@@ -2299,7 +2299,8 @@ void set_operand_layout(GemmArgs& g, int dtype, int b_mn) {
 
 // Chooses the store path of the epilogue and sizes the pipeline; call once the output fields of
 // `g` are set.  out_dims / out_strides describe the output as a 4-D tensor whose dimension 0 is
-// the column (feature) axis and whose other dimensions are the ones the row-tile box spans.
+// the column (feature) axis and whose other dimensions are the ones the row-tile box spans; filter_row: elements
+// of a row of the filter in memory (64 where there is none).
 //
 // plan_solo: GEMMs of at most two tiles to an SM, 16-bit operands.  What bounds them is not their few steps but what stands
 // around them: a CTA of the persistent form takes an SM's shared memory, so it starts where the preceding
@@ -2309,15 +2310,30 @@ void set_operand_layout(GemmArgs& g, int dtype, int b_mn) {
 // us at 24 images, f16, persistent / solo: 28x28 512 -> 128 forward 8.5 / 6.7, its filter gradient 8.1 / 6.4; 7x7 512 -> 2048 7.3 / 6.6
 // forward, 9.4 / 8.4 and 8.5 / 7.1 backward; 14x14 256 -> 256 3x3 12.0 / 12.3 (168 tiles), 12.6 / 13.0, 10.9 / 10.3.  ResNet-50
 // backward 1437 -> 1300, with the shorter loops.  More than two tiles to an SM are worked off by persistent CTAs.
+//
+// Between one tile to an SM and two it depends (35677 random layers of 149 to 296 tiles, 1x1 to 5x5, 16 to 1536 channels and features,
+// persistent / solo, mean and range of nine tenths):
+//  * The persistent form would keep the filter in shared memory: 1.20 to 1.28 where the filter's rows are whole lines of 64 elements;
+//    otherwise a solo CTA's copies of it cost more, 1.17 (0.91 - 1.59) at one step, 1.06 (0.72 - 1.34) at four, 0.91 (0.71 - 1.13) at nine.
+//  * It would not: up to 1.42 tiles to an SM 0.95 (0.77 - 1.08), the tiles of two pipelines being spread over all SMs, beyond that
+//    1.02 (0.91 - 1.11); reductions of up to 6 steps, of up to 10 in filter gradients, 1.02 to 1.06 everywhere.
+// With all solo the mean of the 35677 was 2.4 % behind the better of the two, 1.2 % so.  Up to one tile to an SM solo is ahead by 0 to 50 %.
+bool solo_is_better(const GemmArgs& g, long long tiles, int steps, int filter_row) {
+  const int sms = device_sm_count();
+  if (tiles <= sms || tiles > 2ll * sms) return tiles <= sms;
+  if (!g.a_mn && g.b_batch_mul == 0 && g.n_tiles <= 16 && steps * g.bn * 128 <= 96 * 1024) return filter_row % 64 == 0 || steps < 5;
+  return steps <= (g.a_mn ? 10 : 6) || 100 * tiles > 142ll * sms;
+}
+
 constexpr int kSoloSmem = 113 * 1024, kSoloSmemMin = 108 * 1024;  // (the minimum: see launch_gemm)
-bool plan_solo(GemmArgs& g, bool mask_tma) {
+bool plan_solo(GemmArgs& g, bool mask_tma, int filter_row) {
   const int tap_pack = std::max(g.tap_pack, 1);
   const long long tiles = g.a_mn ? (long long)g.n_tiles * g.tiles_w * ((g.num_taps + tap_pack - 1) / tap_pack) * g.splits
                                  : (long long)g.n_tiles * g.tiles_w * g.tiles_h * g.tiles_n;
-  if (tiles > 2ll * device_sm_count()) return false;
+  const int steps = g.a_mn ? g.slabs_per_split : g.num_taps * g.cblocks;
+  if (!solo_is_better(g, tiles, steps, filter_row)) return false;
   const int bias_smem_bytes = (g.epi_fast && g.bias != nullptr) ? ceil_div(g.bn, 64) * 128 : 0;
   const int blocks = ceil_div(g.bn, g.cpb), stage = kABytes + g.bn * 128, fixed = 1024 + kBarBlockBytes + bias_smem_bytes + g.mask_smem_bytes;
-  const int steps = g.a_mn ? g.slabs_per_split : g.num_taps * g.cblocks;
   int mask_slots = (mask_tma && g.mask_bits == nullptr) ? std::min(2, blocks) : 0;
   auto stages = [&] { return std::min(kMaxStages, (kSoloSmem - fixed - mask_slots * 4 * 4096) / stage); };
   if (mask_slots == 2 && stages() < 3) mask_slots = 1;
@@ -2340,7 +2356,7 @@ bool plan_solo(GemmArgs& g, bool mask_tma) {
   return true;
 }
 
-bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], const uint64_t out_strides[3], bool allow_solo = true) {
+bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], const uint64_t out_strides[3], int filter_row, bool allow_solo = true) {
   g.cpb = 128 / (int)dtype_size(g.out_dtype);
   g.tma_store = 0;
   if (g.beta == 0.f && g.bn % g.cpb == 0 && aligned16(g.out)) {
@@ -2383,7 +2399,7 @@ bool setup_store(GemmArgs& g, int compute_dtype, const uint64_t out_dims[4], con
   const bool mask_tma = g.epi_fast && g.relu_mask != nullptr;
   g.mask_smem_bytes = mask_tma ? 128 : 0;  // the mask slots' barriers; the slots count as staging
   g.solo = 0;
-  if (allow_solo && !split && g.tma_store && !g.pair && !g.cta_pair && !g.halo && g.group_k == 0 && plan_solo(g, mask_tma)) return true;
+  if (allow_solo && !split && g.tma_store && !g.pair && !g.cta_pair && !g.halo && g.group_k == 0 && plan_solo(g, mask_tma, filter_row)) return true;
   if (g.pair && !g.cta_pair && (split || g.groups != 2 || !g.tma_store)) return false;  // the caller plans again without pairing
   if (g.epi_fast && g.bias != nullptr) {
     const int padded = ceil_div(g.n_tiles * g.bn, 64) * 64;
@@ -2991,7 +3007,7 @@ int finish_forward(GemmArgs& g, int dtype, void* y, const PdnnConv2DParams& p, c
   if (cluster != 0) return cluster_epilogue_ok(g) ? launch_gemm_cluster(g, cluster, s) : kPlanAgain;
   const uint64_t od[4] = {(uint64_t)p.features, (uint64_t)p.out_cols, (uint64_t)p.out_rows, (uint64_t)p.batch};
   const uint64_t os[3] = {(uint64_t)ld * es, (uint64_t)p.out_cols * ld * es, (uint64_t)p.out_rows * p.out_cols * ld * es};
-  if (!setup_store(g, dtype, od, os, plan_out == nullptr)) return (g.halo || g.pair) ? kPlanAgain : PDNN_INVALID_PARAMETER;
+  if (!setup_store(g, dtype, od, os, p.filter_format == 0 ? p.features : p.channels, plan_out == nullptr)) return (g.halo || g.pair) ? kPlanAgain : PDNN_INVALID_PARAMETER;
   if (plan_out != nullptr) {
     *plan_out = g;
     return PDNN_OK;
@@ -3737,11 +3753,11 @@ int conv_input_backprop(int dtype, const void* dy, const void* w, void* dx, cons
         // the general epilogue's beta.
         g.accumulate = accumulate ? 1 : 0;
         const bool solo = p.stride_rows == 1 && p.stride_cols == 1;  // (several classes go side by side in one launch)
-        bool planned = setup_store(g, dtype, od, os, solo);
+        bool planned = setup_store(g, dtype, od, os, p.filter_format == 0 ? p.features : p.channels, solo);
         if (planned && accumulate && !g.epi_fast) {
           g.accumulate = 0;
           g.beta = 1.f;
-          planned = setup_store(g, dtype, od, os, solo);
+          planned = setup_store(g, dtype, od, os, p.filter_format == 0 ? p.features : p.channels, solo);
         }
         if (!planned) {
           if (g.halo || g.pair) return conv_input_backprop(dtype, dy, w, dx, p, relu_mask, mask_bits, accumulate, constant_filter, s, false, try_cluster);  // plan again without the halo / pairing
@@ -4018,7 +4034,7 @@ int conv_filter_backprop_small_c(int dtype, const void* x, const void* dy, void*
     const uint64_t od[4] = {(uint64_t)p.features, (uint64_t)q.rows, (uint64_t)p.window_rows, (uint64_t)f.splits};
     const uint64_t os[3] = {(uint64_t)p.features * 4, (uint64_t)q.rows * p.features * 4,
                             (uint64_t)p.window_rows * q.rows * p.features * 4};
-    if (!setup_store(g, dtype, od, os)) {
+    if (!setup_store(g, dtype, od, os, 64)) {
       release();
       return -1;
     }
@@ -4164,7 +4180,7 @@ int conv_filter_backprop(int dtype, const void* x, const void* dy, void* dw, con
     const uint64_t eo = dtype_size(g.out_dtype);
     const uint64_t od[4] = {(uint64_t)p.features, (uint64_t)p.channels, (uint64_t)nt, (uint64_t)(reduce ? 1 : f.splits)};
     const uint64_t os[3] = {(uint64_t)p.features * eo, (uint64_t)p.channels * p.features * eo, (uint64_t)n_out * eo};
-    if (!setup_store(g, dtype, od, os)) {
+    if (!setup_store(g, dtype, od, os, 64)) {
       if (own) cudaFreeAsync(partial, s);
       return PDNN_INVALID_PARAMETER;
     }
@@ -4454,7 +4470,7 @@ int tc_matmul(int dtype, int tl, int tr, const void* lhs, const void* rhs, void*
     const uint64_t eo = dtype_size(g.out_dtype);
     const uint64_t od[4] = {(uint64_t)n, (uint64_t)m, 1, (uint64_t)batches};
     const uint64_t os[3] = {(uint64_t)n * eo, (uint64_t)m * n * eo, (uint64_t)m * n * eo};
-    if (!setup_store(g, dtype, od, os)) return PDNN_INVALID_PARAMETER;
+    if (!setup_store(g, dtype, od, os, tr ? k : n)) return PDNN_INVALID_PARAMETER;
   }
   return launch_gemm(g, dtype, s);
 }

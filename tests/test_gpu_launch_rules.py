@@ -56,3 +56,25 @@ def test_threads_of_a_gradient_keep_their_channels(c):
     x, dy, g = _rand(size, "bf16"), _rand(size, "bf16"), _rand(c, "bf16")
     kernels = [k for k in launched(lambda: pd.batchnorm_gradient(x, dy, g, p)) if "grad_training_vec" in k.name]
     assert len(kernels) == 1 and kernels[0].blocks * kernels[0].threads % (c // 8) == 0
+
+
+# n, h, c, k, window, pass; one tile to a CTA or persistent CTAs of two pipelines
+@pytest.mark.parametrize("layer,which,solo", [
+    ((24, 14, 256, 256, 3), pd.FORWARD, False),         # 168 tiles of 36 steps
+    ((24, 14, 256, 256, 3), pd.INPUT_BACKPROP, False),
+    ((24, 14, 256, 128, 1), pd.FORWARD, True),          # at most one tile to an SM
+    ((36, 28, 64, 64, 1), pd.FORWARD, True),            # 221 tiles, the filter in whole lines
+    ((36, 28, 64, 72, 1), pd.FORWARD, True),            # one step: whatever the filter's rows are
+    ((36, 28, 512, 24, 1), pd.FORWARD, False),          # eight steps, rows of 48 bytes
+    ((60, 24, 32, 16, 3), pd.FORWARD, False),
+    ((10, 54, 1024, 64, 1), pd.FORWARD, True),          # 228 tiles: beyond 1.42 to an SM
+])
+def test_small_ctas(layer, which, solo):
+    p = pd.conv_params(layer[0], layer[1], layer[1], *layer[2:], 1)
+    n_in, n_fil, _ = pd.api.conv_sizes(which, p)
+    x, f = _rand(n_in, "bf16"), _rand(n_fil, "bf16")
+    kernels = [k for k in launched(lambda: pd.conv2d(which, x, f, p)) if "umma_gemm_kernel" in k.name]
+    assert len(kernels) == 1
+    # the persistent form has two pipelines, 384 threads, and one CTA to an SM
+    assert (kernels[0].threads == 192 and kernels[0].shared_bytes < 114 * 1024) == solo
+    assert solo or kernels[0].blocks <= 148
