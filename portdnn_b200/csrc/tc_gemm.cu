@@ -2300,7 +2300,7 @@ void set_operand_layout(GemmArgs& g, int dtype, int b_mn) {
 // Chooses the store path of the epilogue and sizes the pipeline; call once the output fields of
 // `g` are set.  out_dims / out_strides describe the output as a 4-D tensor whose dimension 0 is
 // the column (feature) axis and whose other dimensions are the ones the row-tile box spans; filter_row: elements
-// of a row of the filter in memory (64 where there is none).
+// of a row of the filter in memory.
 //
 // plan_solo: GEMMs of at most two tiles to an SM, 16-bit operands.  What bounds them is not their few steps but what stands
 // around them: a CTA of the persistent form takes an SM's shared memory, so it starts where the preceding
@@ -2311,18 +2311,26 @@ void set_operand_layout(GemmArgs& g, int dtype, int b_mn) {
 // forward, 9.4 / 8.4 and 8.5 / 7.1 backward; 14x14 256 -> 256 3x3 12.0 / 12.3 (168 tiles), 12.6 / 13.0, 10.9 / 10.3.  ResNet-50
 // backward 1437 -> 1300, with the shorter loops.  More than two tiles to an SM are worked off by persistent CTAs.
 //
-// Between one tile to an SM and two it depends (35677 random layers of 149 to 296 tiles, 1x1 to 5x5, 16 to 1536 channels and features,
-// persistent / solo, mean and range of nine tenths):
-//  * The persistent form would keep the filter in shared memory: 1.20 to 1.28 where the filter's rows are whole lines of 64 elements;
-//    otherwise a solo CTA's copies of it cost more, 1.17 (0.91 - 1.59) at one step, 1.06 (0.72 - 1.34) at four, 0.91 (0.71 - 1.13) at nine.
-//  * It would not: up to 1.42 tiles to an SM 0.95 (0.77 - 1.08), the tiles of two pipelines being spread over all SMs, beyond that
-//    1.02 (0.91 - 1.11); reductions of up to 6 steps, of up to 10 in filter gradients, 1.02 to 1.06 everywhere.
-// With all solo the mean of the 35677 was 2.4 % behind the better of the two, 1.2 % so.  Up to one tile to an SM solo is ahead by 0 to 50 %.
+// Between one tile to an SM and two it depends (35677 random layers of 149 to 296 tiles, 1x1 to 5x5, 8 to 1536 channels and features,
+// each in a chain of its own; persistent / solo, mean and range of nine tenths):
+//  * Filter rows of whole lines of 64 elements: 1.20 to 1.28 where the persistent form would keep the filter in shared memory, 1.02 (0.93 -
+//    1.10) where it would not.  Beside other layers the next launch's CTAs start in the place of the first that end: ResNet-50 with the
+//    layers of up to 1.42 tiles to an SM persistent / all solo, forward at 24 and 32 images 554 / 531 and 620 / 596 us,
+//    backward 1317 / 1303 and 1489 / 1466.  So solo.
+//  * Other rows, the filter kept: a solo CTA's copies of it cost more, the shorter the pieces that a row's start leaves.  Multiples of
+//    8, and rows shorter than a line: 1.17 (0.91 - 1.59) at one step, 1.06 (0.72 - 1.34) at four, 0.91 (0.71 - 1.13) at nine; of
+//    16: 1.06 at eight, 0.98 at nine; of 32: 1.04 at nine.  Not kept: 0.94 (0.77 - 1.08) up to 1.42 tiles to an SM, the tiles of two pipelines being spread over all
+//    SMs, 1.01 (0.88 - 1.12) beyond, and 1.02 to 1.06 for reductions of up to 6 steps.
+//  * Filter gradients: 0.96 (0.82 - 1.05) up to 1.42 tiles to an SM and from 11 steps on, else 1.02.
+// Up to one tile to an SM solo is ahead by 0 to 50 %.
 bool solo_is_better(const GemmArgs& g, long long tiles, int steps, int filter_row) {
   const int sms = device_sm_count();
   if (tiles <= sms || tiles > 2ll * sms) return tiles <= sms;
-  if (!g.a_mn && g.b_batch_mul == 0 && g.n_tiles <= 16 && steps * g.bn * 128 <= 96 * 1024) return filter_row % 64 == 0 || steps < 5;
-  return steps <= (g.a_mn ? 10 : 6) || 100 * tiles > 142ll * sms;
+  const bool spread = 100 * tiles <= 142ll * sms;
+  if (g.a_mn) return steps <= 10 || !spread;
+  if (filter_row % 64 == 0) return true;
+  const bool kept = g.b_batch_mul == 0 && g.n_tiles <= 16 && steps * g.bn * 128 <= 96 * 1024;
+  return kept ? filter_row % 32 == 0 || steps < (filter_row % 16 == 0 && filter_row > 64 ? 9 : 5) : steps <= 6 || !spread;
 }
 
 constexpr int kSoloSmem = 113 * 1024, kSoloSmemMin = 108 * 1024;  // (the minimum: see launch_gemm)

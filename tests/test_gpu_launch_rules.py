@@ -60,8 +60,10 @@ def test_threads_of_a_gradient_keep_their_channels(c):
 
 # n, h, c, k, window, pass; one tile to a CTA or persistent CTAs of two pipelines
 @pytest.mark.parametrize("layer,which,solo", [
-    ((24, 14, 256, 256, 3), pd.FORWARD, False),         # 168 tiles of 36 steps
-    ((24, 14, 256, 256, 3), pd.INPUT_BACKPROP, False),
+    ((24, 14, 256, 256, 3), pd.FORWARD, True),          # 168 tiles of 36 steps, the filter in whole lines
+    ((24, 14, 256, 200, 3), pd.FORWARD, False),         # rows of 400 bytes
+    ((24, 14, 264, 256, 3), pd.INPUT_BACKPROP, True),
+    ((24, 14, 256, 264, 3), pd.INPUT_BACKPROP, False),
     ((24, 14, 256, 128, 1), pd.FORWARD, True),          # at most one tile to an SM
     ((36, 28, 64, 64, 1), pd.FORWARD, True),            # 221 tiles, the filter in whole lines
     ((36, 28, 64, 72, 1), pd.FORWARD, True),            # one step: whatever the filter's rows are
