@@ -585,13 +585,15 @@ bool simt_matmul_tiled(int dtype, int tl, int tr, const void* lhs, const void* r
   const Tiling t = choose(m, m, n, k, 1, batches, false, sm_count());
   const long long tiles = (long long)batches * t.n_tiles * t.m_tiles, blocks = tiles * t.splits;
   if (blocks > 0x7FFFFFF0ll) return false;
-  // What each side takes, in us: a thread to an output walks its terms (45 ns each) or the device is full (2.5 multiply-adds per ps);
-  // here a step takes 0.3 us or the tiles, remainders and all, fill it (10 per ps).  Measured, thread to an output / here: f16
+  // What each side takes, in us: a thread to an output walks its terms (25 ns each, 45 with lhs transposed, whose terms lie apart) or
+  // the device is full (2.5 multiply-adds per ps); here a step takes 0.45 us or the tiles, remainders and all, fill it (10 per
+  // ps).  Over 11417 random products the choice is 1.5 % behind the faster side on average and slower than a thread to an output
+  // by more than 1 % in one of a hundred.  Measured, thread to an output / here: f16
   // 2 x 1008 x 543 51 / 12.4, 2 x 543 x 1008 (rhs transposed) 32 / 11.2, 500 x 2000 x 1001 380 / 122, 1001 x 2000 transposed 1502 / 127;
   // f32 128 x 1024 x 333 33 / 11.8, 16 of 3000 x 37 x 51 37 / 25; and f32 2000 of 16 x 17 x 15 7.3 / 31, 16 of 400 x 13 x 13 3.6 / 7.5,
   // f16 10 x 100 x 11 7.2 / 11, f32 4000000 x 3 x 3 73 / 548.
   const double steps = (k + kTerms - 1) / kTerms, macs = (double)batches * m * n * k;
-  const double walk = 3 + 0.045 * k + macs / 2.5e6, here = 6 + 0.3 * steps / t.splits + (double)tiles * kOutputs * steps * kTerms / 1e7;
+  const double walk = 3 + (tl ? 0.045 : 0.025) * k + macs / 2.5e6, here = 6 + 0.45 * steps / t.splits + (double)tiles * kOutputs * steps * kTerms / 1e7;
   if (walk <= here) return false;
   SimtArgs g = {};
   g.a = lhs, g.b = rhs, g.out = out;
