@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256) widen_to_f32_kernel(const T* __restrict__
 // What no tensor-core kernel takes: fp32 tiles on the CUDA cores where they gain, else a thread to an output.
 int general_conv(int pass, int dtype, const void* in, const void* fil, void* out, const PdnnConv2DParams& p,
                  const PdnnConvEpilogue* epi, bool tiled, void* ws, size_t ws_elems, cudaStream_t s) {
-  if (tiled && simt_conv_applicable(pass, p)) return simt_conv(pass, dtype, in, fil, out, p, epi, ws, ws_elems, s);
+  if (tiled && simt_conv_applicable(pass, dtype, p)) return simt_conv(pass, dtype, in, fil, out, p, epi, ws, ws_elems, s);
   return launch_direct_conv(pass, dtype, in, fil, out, p, epi, s);
 }
 

@@ -175,33 +175,28 @@ size_t scratch_bytes(int pass, int dtype, const Plan& plan) {
          round_up((size_t)plan.q.features * 2, 256) + round_up(inner * 2, 256) + 256;
 }
 
-// Where the general kernels, one launch that needs no copies, are still the better ones.  Measured (bf16, us, a thread to an output
-// / copies padded to multiples of 8, which were up to a third slower than those of padded_count):
-//   forward                          |  1 image    | 4 images    | 64 images   | 256 images
-//    7x7   12 -> 12  1x1             |  4.7 / 10.1 |  4.7 / 10.0 |  4.7 / 10.1 |   6.2 / 10.2
-//   14x14  12 -> 12  1x1             | 10.5 / 10.4 |  4.7 / 10.0 |  6.2 / 10.2 |  14.4 / 12.0
-//   28x28  12 -> 20  1x1             |  4.7 / 10.0 |  4.6 / 10.0 | 22.6 / 15.5 |  71.7 / 21.1
-//    7x7  100 -> 20  1x1             | 10.3 / 10.1 | 10.3 / 10.1 | 12.3 / 10.2 |  24.6 / 12.9
-//    3x3   20 -> 30  3x3             | 12.3 / 10.2 | 12.3 / 12.2 | 14.4 / 12.5 |  14.4 / 13.0
-//   28x28  20 -> 30  3x3             | 16.5 / 11.6 | 20.8 / 12.0 | 224  / 21.7 | 874   / 48.6
-//   images, size, channels, window   | input backprop | filter backprop
-//   1 x 7x7    20 -> 30   3x3        |  21 / 20       |    7 / 20
-//   1 x 14x14  20 -> 30   3x3        |  21 / 17       |   15 / 17
-//   1 x 28x28  20 -> 30   3x3        |  21 / 17       |   50 / 19
-//   4 x 28x28  20 -> 30   3x3        |  23 / 17       |  189 / 23
-//   1 x 7x7    100 -> 150 3x3        | 107 / 21       |   33 / 17
-//   8 x 28x28  100 -> 150 1x1        | 128 / 18       |  517 / 28
-//   7 x 45x45  100 -> 150 3x3        | 2523 / 40      | 7574 / 60
-// The forward pass moves over by the terms of a sum or by the work of one image, not of the batch: the two kernels
-// add up in different orders, and an image has the same result alone and in any batch.  The input backprop moves
-// over by the terms or by the work of the layer, the filter gradient (one block per input channel, tap and 32
-// features) by the work alone.
-bool direct_is_better(int pass, const PdnnConv2DParams& p) {
-  const double taps = (double)p.window_rows * p.window_cols;
-  const double per_image = (double)p.out_rows * p.out_cols * taps * p.channels * p.features, macs = per_image * p.batch;
-  if (pass == PDNN_FORWARD) return per_image < 1e5 && taps * p.channels < 64;
-  if (pass == PDNN_FILTER_BACKPROP) return macs < 1.5e6;
-  return macs < 8e6 && taps * p.features < 256;
+// Where the general kernels, one launch that needs no copies, are still the better ones (a thread to an output or fp32 tiles, as
+// simt_gemm.cu chooses).  Measured on 14652 random layers, copies and tensor cores / general, means:
+//   terms of a sum                  |  multiply-adds of the layer
+//                                   | 1e5    1e5..3e5   3e5..1e6   1e6..3e6   3e6..1e7   1e7..3e7
+//   forward, taps * channels     32 | 2.02   2.08       2.00       1.53       1.07       0.93
+//                                64 | 1.33   1.35       1.35       1.19       1.06       0.86
+//                               128 | 0.69   0.69       0.68       0.75       0.78       0.82
+//   input gradient, taps *       32 | 2.73   2.24       1.95       1.44       0.83       0.81
+//   features / strides           64 | 1.20   1.08       1.11       1.08       0.92       0.88
+//                               128 | 0.77   0.87       0.84       0.80       0.80       0.80
+//   filter gradient, pixels      32 | 2.37   1.79       1.17       0.64       0.59
+//                                64 | 1.40   1.23       0.70       0.70       0.83
+//                               128 | 0.91   0.76       0.77       0.71       1.00
+// On average the choice is 1.4, 3.2 and 0.8 % behind the faster of the two.  The forward pass moves over by the terms of a
+// sum or by the work of one image, not of the batch: the kernels add up in different orders, and an image has the same result
+// alone and in any batch.
+bool general_is_better(int pass, const PdnnConv2DParams& p) {
+  const double taps = (double)p.window_rows * p.window_cols, pixels = (double)p.out_rows * p.out_cols;
+  const double per_image = pixels * taps * p.channels * p.features, macs = per_image * p.batch;
+  if (pass == PDNN_FORWARD) return taps * p.channels < 64 && per_image < 3e5;
+  if (pass == PDNN_FILTER_BACKPROP) return pixels * p.batch < 64 && macs < 5e5;
+  return taps * p.features < 64.0 * p.stride_rows * p.stride_cols && macs < 5e6;
 }
 
 }  // namespace
@@ -209,7 +204,7 @@ bool direct_is_better(int pass, const PdnnConv2DParams& p) {
 bool padded_conv_applicable(int pass, int dtype, const PdnnConv2DParams& p, const PdnnConvEpilogue* epi) {
   if (pass == PDNN_FORWARD && epi != nullptr && epi->beta != 0.f) return false;  // (reads what the output holds)
   Plan plan;
-  return !direct_is_better(pass, p) && make_plan(pass, dtype, p, &plan);
+  return !general_is_better(pass, p) && make_plan(pass, dtype, p, &plan);
 }
 
 size_t padded_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p) {

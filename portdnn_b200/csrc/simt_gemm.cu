@@ -463,26 +463,32 @@ size_t slices_bytes(const Tiling& t, const PdnnConv2DParams& p) {
 }
 
 // Where a thread to an output is still the better one (direct_conv.cu): its time is the length of a sum until the work fills the
-// device, that of the tiles the latency of their loads.  us, thread to an output / tiles here:
-//   images, size, channels, window      | forward     | input gradient | filter gradient
-//   f32   1 x 7x7    13 -> 13   1x1     | 4.7 / 5.4   |  3.1 / 5.8     |   4.5 / 8.4
-//   f32   1 x 7x7    13 -> 13   3x3     |  25 / 9.2   |   13 / 9.9     |   4.7 / 10.9
-//   f32   1 x 14x14  37 -> 51   1x1     | 9.0 / 8.7   |  6.6 / 9.7     |  12.6 / 6.8
-//   f32   1 x 14x14  37 -> 51   3x3     |  65 / 10    |   41 / 9.0     |    22 / 7.3
-//   f32   4 x 28x28  21 -> 30   3x3     |  44 / 10.5  |   29 / 11.1    |   183 / 19
-//   f32  64 x 56x56  13 -> 15   1x1     |  63 / 33    |   58 / 34      | 10760 / 109
-//   f32   8 x 20x30 133 -> 77   3x3     | 495 / 72    |  577 / 85      |  2055 / 83
-//   f32   4 x 14x14 301 -> 251  3x3     | 812 / 63    |  726 / 70      |  1902 / 65
-//   f16   2 x 9x19   37 -> 51   1x1     | 4.9 / 7.5   |  5.8 / 10.9    |  21.2 / 9.8
-//   f16   1 x 14x14  20 -> 30   3x3     | 15.3 / 8.9  | 19.3 / 8.5     |  13.3 / 9.9
-//   f16   4 x 14x14  37 -> 51   1x1     | 5.1 / 7.4   |  6.0 / 11      |    46 / 16.6
-// The forward pass moves over by the terms of a sum or by the work of one image: an image has the same result alone and in any batch.
-bool thread_to_an_output(int pass, const PdnnConv2DParams& p) {
+// device, that of the tiles the latency of their loads.  Measured on 22861 random layers, tiles / thread to an output, means:
+//   terms of a sum                 |   f32, multiply-adds of the layer      |   16 bits
+//                                  | 1e5    1e6..3e6   3e6..1e7   1e7..3e7  | 1e5    1e6..3e6   3e6..1e7   1e7..3e7
+//   forward, taps * channels    16 | 1.94   1.10       0.77       0.52      | 2.21   1.56       0.76       0.49
+//                               64 | 0.96   1.00       0.89       0.55      | 1.83   1.80       1.35       0.67
+//                              160 | 0.52   0.48       0.47       0.45      | 1.19   1.03       1.02       0.75
+//                              700 | 0.18   0.17       0.17       0.23      | 0.45   0.42       0.41       0.46
+//   input gradient, taps *      16 | 1.77   0.95       0.56       0.41      | 2.24   1.14       0.72       0.56
+//   features / strides          64 | 0.91   0.97       0.74       0.48      | 1.57   1.27       1.02       0.56
+//                              160 | 0.51   0.56       0.50       0.40      | 0.82   0.92       0.84       0.59
+//   filter gradient, pixels     32 | 1.70   0.69                            | 1.93   0.62       0.43
+//                              100 | 0.89   0.47       0.25       0.20      | 1.01   0.53       0.28       0.19
+// On average the choice is 3.2, 4.5 and 0.6 % (16 bits 3.9, 2.7 and 0.5 %) behind the faster of the two.  Fewer than four columns leave most
+// of a tile idle: 1.8 to 4.4 (sums of up to 64 terms, 1e6 multiply-adds and more), whatever the work.  The forward pass moves over by the terms of a
+// sum or by the work of one image: an image has the same result alone and in any batch.
+bool thread_to_an_output(int pass, int dtype, const PdnnConv2DParams& p) {
   const double taps = (double)p.window_rows * p.window_cols, pixels = (double)p.out_rows * p.out_cols;
-  const double per_image = pixels * taps * p.channels * p.features;
-  if (pass == PDNN_FORWARD) return taps * p.channels < 64 && per_image < 5e5;
-  if (pass == PDNN_INPUT_BACKPROP) return taps * p.features < 100.0 * p.stride_rows * p.stride_cols && per_image * p.batch < 1e7;
-  return pixels * p.batch < 160 && per_image * p.batch < 2e6;
+  const double per_image = pixels * taps * p.channels * p.features, macs = per_image * p.batch;
+  const bool half = dtype != PDNN_F32;
+  if (pass != PDNN_FILTER_BACKPROP) {
+    const bool forward = pass == PDNN_FORWARD;
+    const double terms = forward ? taps * p.channels : taps * p.features / ((double)p.stride_rows * p.stride_cols);
+    if ((forward ? p.features : p.channels) < 4 && terms < (half ? 128 : 64)) return true;
+    return forward ? terms < (half ? 128 : 48) && per_image < (half ? 1e6 : 5e5) : terms < (half ? 100 : 48) && macs < (half ? 5e6 : 3e6);
+  }
+  return pixels * p.batch < 80 && macs < 5e5;
 }
 
 // Whether a tap of an output (of a pixel of the input, in an input gradient) can lie outside along one axis.
@@ -498,7 +504,7 @@ int sm_count() {
 
 }  // namespace
 
-bool simt_conv_applicable(int pass, const PdnnConv2DParams& p) {
+bool simt_conv_applicable(int pass, int dtype, const PdnnConv2DParams& p) {
   if (p.groups != 1 || p.input_format != 0 || (p.filter_format != 0 && p.filter_format != 2)) return false;
   const long long taps = (long long)p.window_rows * p.window_cols;
   const long long x = (long long)p.batch * p.in_rows * p.in_cols * p.channels, y = (long long)p.batch * p.out_rows * p.out_cols * p.features;
@@ -511,11 +517,11 @@ bool simt_conv_applicable(int pass, const PdnnConv2DParams& p) {
   if (p.stride_rows > 64 || p.stride_cols > 64) return false;
   const Tiling t = conv_tiling(pass, p, true, sm_count());
   const double blocks = (double)t.m_tiles * t.n_tiles * t.slices * kMaxSplits * (pass == PDNN_INPUT_BACKPROP ? p.stride_rows * p.stride_cols : 1);
-  return blocks < 2147483632.0 && !thread_to_an_output(pass, p);
+  return blocks < 2147483632.0 && !thread_to_an_output(pass, dtype, p);
 }
 
 size_t simt_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p) {
-  if (pass != PDNN_FILTER_BACKPROP || !simt_conv_applicable(pass, p)) return 0;
+  if (pass != PDNN_FILTER_BACKPROP || !simt_conv_applicable(pass, dtype, p)) return 0;
   const Tiling t = conv_tiling(pass, p, true, sm_count());
   if (t.slices == 1) return 0;
   return slices_bytes(t, p) / dtype_size(dtype);

@@ -7,7 +7,7 @@
 namespace pdnn {
 
 // Whether simt_conv takes the layer: NHWC tensors, one group, element indices of 32 bits, and a layer that gains by it.
-bool simt_conv_applicable(int pass, const PdnnConv2DParams& p);
+bool simt_conv_applicable(int pass, int dtype, const PdnnConv2DParams& p);
 
 // Scratch elements (of dtype) that the pass can use: the slices of a long filter gradient.
 size_t simt_conv_workspace_elems(int pass, int dtype, const PdnnConv2DParams& p);

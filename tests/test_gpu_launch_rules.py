@@ -80,3 +80,30 @@ def test_small_ctas(layer, which, solo):
     # the persistent form has two pipelines, 384 threads, and one CTA to an SM
     assert (kernels[0].threads == 192 and kernels[0].shared_bytes < 114 * 1024) == solo
     assert solo or kernels[0].blocks <= 148
+
+
+@pytest.mark.parametrize("layer,which,dtype,kernel", [
+    ((24, 28, 2, 2, 7), pd.FORWARD, "f32", "simt_gemm_kernel"),             # sums of 98 terms
+    ((24, 28, 5, 2, 3), pd.FORWARD, "f32", "direct_forward_kernel"),        # two columns, 45 terms
+    ((24, 28, 5, 6, 3), pd.FORWARD, "f32", "direct_forward_kernel"),        # 45 terms, 212 thousand multiply-adds an image
+    ((24, 60, 5, 6, 3), pd.FORWARD, "f32", "simt_gemm_kernel"),             # a million
+    ((1, 30, 9, 45, 1), pd.INPUT_BACKPROP, "f32", "direct_input_backprop_kernel"),
+    ((1, 30, 9, 49, 1), pd.INPUT_BACKPROP, "f32", "simt_gemm_kernel"),
+    ((5, 4, 270, 14, 2), pd.INPUT_BACKPROP, "f16", "direct_input_backprop_kernel"),
+    ((5, 4, 270, 18, 2), pd.INPUT_BACKPROP, "f16", "umma_gemm"),            # copies
+    ((1, 7, 13, 20, 1), pd.FILTER_BACKPROP, "f16", "direct_filter_backprop_kernel"),
+    ((2, 7, 13, 20, 1), pd.FILTER_BACKPROP, "f16", "umma_gemm"),
+])
+def test_odd_layers(layer, which, dtype, kernel):
+    p = pd.conv_params(layer[0], layer[1], layer[1], *layer[2:], 1)
+    n_in, n_fil, _ = pd.api.conv_sizes(which, p)
+    x, f = _rand(n_in, dtype), _rand(n_fil, dtype)
+    assert any(kernel in k.name for k in launched(lambda: pd.conv2d(which, x, f, p)))
+
+
+# products that a thread to an output had been faster at than the tiles that took them, and one that tiles are faster at
+@pytest.mark.parametrize("m,k,n,dtype,tiles", [(844, 101, 38, "bf16", False), (267, 144, 13, "f32", False), (74, 110, 1028, "f16", False), (1000, 2000, 501, "f16", True)])
+def test_odd_products(m, k, n, dtype, tiles):
+    a, b = _rand(m * k, dtype), _rand(k * n, dtype)
+    kernels = launched(lambda: pd.matmul(a, b, 1, m, k, n))
+    assert len(kernels) == 1 and ("simt_gemm_kernel" in kernels[0].name) == tiles
