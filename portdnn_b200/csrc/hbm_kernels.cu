@@ -2237,10 +2237,11 @@ int launch_depthwise(int pass, int dtype, const void* in, const void* fil, void*
       return st;
     }
     if constexpr (!std::is_same<T, float>::value) {
-      // fp16 has the strips below for small layers: up to 4 MB of tensors they are ahead by up to 12 % at stride 1 (one image,
-      // 56x56x144: 2.86 and 3.11 us), above it the tiles, at up to 160 channels by 0 to 30 %, with more by 5 to 44.
+      // fp16 has the strips below for small layers.  Strips / tiles, means over 12641 random layers: stride 1, tensors of 1 to 2 MB 0.96,
+      // 2 to 6 MB 1.02 (a tenth below 0.91), 6 to 8 MB 1.09, 8 to 12 MB 1.16, above 1.10; stride 2, below 8 MB 0.98, above 1.13.  With 8
+      // channels, whose pixels are four words of a tile's rows, 0.84 to 0.94 at nearly all sizes.
       const size_t bytes = 2 * (size_t)p.batch * p.channels * ((size_t)p.in_rows * p.in_cols + (size_t)p.out_rows * p.out_cols);
-      const bool tiles = std::is_same<T, __nv_bfloat16>::value || bytes >= (4u << 20);
+      const bool tiles = std::is_same<T, __nv_bfloat16>::value || (p.channels > 8 && bytes >= ((size_t)(p.stride_rows == 1 ? 6 : 8) << 20));
       if (tiles && pass == PDNN_FORWARD && launch_depthwise_forward_tiles(dtype, in, fil, out, p, false, s))
         return check_launch("depthwise conv2d (3x3 tiles)");
       if (tiles && pass == PDNN_INPUT_BACKPROP && p.window_rows == 3 && p.window_cols == 3 && p.stride_rows == 1 && p.stride_cols == 1 &&

@@ -3901,7 +3901,9 @@ __global__ void __launch_bounds__(256)
 // of A and 64 of dy, for every pair of filter rows again.  With 8 channels to a pixel two filter rows fill a tile
 // (tap_pack 2); with 4 channels - 64-byte rows, where an even column stride keeps them on 16 bytes - four do: 320 rows
 // for four instead of 384, half the MMAs, half the bytes to pack.  224x224x3, 7x7/2 to 64 features, f16, packing and second stage
-// included: 256 images 375 -> 285 us, 24 images 47 -> 39.
+// included: 256 images 375 -> 285 us, 24 images 47 -> 39.  With 1 or 2 rows left over (5x5, 6x6) there are 2 tiles for 3, not half as many,
+// and small layers are left with half the CTAs: 8 channels / 4, means over 7273 random layers, 3x3, 4x4, 7x7 and 8x8: up to 10000 output
+// pixels 0.90, 10000 to 30000 1.00, 100000 1.05, more 1.10 to 1.29; 5x5 and 6x6: 0.91, 0.98, 0.97, 1.00 to 1.07.
 struct SmallCFbpPlan {
   FbpPlan f;
   SmallCPlan sp;
@@ -3915,6 +3917,7 @@ SmallCFbpPlan plan_small_c_fbp(int dtype, const PdnnConv2DParams& p, int sms) {
   const int epr = dtype == PDNN_F32 ? 32 : 64;
   q.sp = plan_small_c(dtype, p);
   q.narrow = dtype != PDNN_F32 && p.channels <= 4 && p.stride_cols % 2 == 0 && p.window_rows >= 3 &&
+             (double)p.batch * p.out_rows * p.out_cols >= ((p.window_rows & 3) % 3 == 0 ? 2e4 : 3e5) &&
              (size_t)p.batch * q.sp.Hp * (q.sp.Wp + 1) < 0x7FFFFFFFull;
   if (q.narrow) {
     q.sp.Wp = (q.sp.Wp + 1) / 2 * 2;  // rows stay 16-byte aligned

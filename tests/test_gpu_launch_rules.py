@@ -107,3 +107,20 @@ def test_odd_products(m, k, n, dtype, tiles):
     a, b = _rand(m * k, dtype), _rand(k * n, dtype)
     kernels = launched(lambda: pd.matmul(a, b, 1, m, k, n))
     assert len(kernels) == 1 and ("simt_gemm_kernel" in kernels[0].name) == tiles
+
+
+@pytest.mark.parametrize("n,h,c,stride,tiles", [(16, 28, 96, 1, False), (48, 28, 96, 1, True), (24, 56, 32, 2, False), (64, 56, 32, 2, True), (64, 112, 8, 1, False),
+                                                (64, 112, 16, 1, True)])
+def test_depthwise_half(n, h, c, stride, tiles):
+    p = pd.depthwise_params(n, h, h, c, 1, 3, stride)
+    x, f = _rand(n * h * h * c, "f16"), _rand(9 * c, "f16")
+    kernels = launched(lambda: pd.depthwise_conv2d(pd.FORWARD, x, f, p))
+    assert len(kernels) == 1 and ("depthwise_forward_tile_kernel" in kernels[0].name) == tiles
+
+
+@pytest.mark.parametrize("n,h,window,narrow", [(2, 38, 3, False), (24, 64, 3, True), (24, 64, 7, True), (24, 64, 5, False), (100, 112, 5, True)])
+def test_stem_filter_gradients(n, h, window, narrow):
+    p = pd.conv_params(n, h, h, 3, 64, window, 2)
+    x, dy = _rand(n * h * h * 3, "f16"), _rand(n * p.out_rows * p.out_cols * 64, "f16")
+    kernels = launched(lambda: pd.conv2d(pd.FILTER_BACKPROP, x, dy, p))
+    assert any("pack_small_c_input_narrow" in k.name for k in kernels) == narrow
