@@ -368,15 +368,15 @@ __global__ void __launch_bounds__(kTileThreads + 32, 1)
                 V acc = L::zero();
 #pragma unroll
                 for (int t = 0; t < 9; ++t) {
-                    constexpr bool by_column = std::is_same<L, HalfSums>::value;
-                    const int r = by_column ? t % 3 : t / 3, c = by_column ? t / 3 : t % 3;
-                    // a tap outside the image is no term of the sum: the zero there and an infinite weight would be one
-                    if (!decltype(every_tap)::value) {
-                      const int ih = (h0 + k) * ST - g.pad_rows + r, iw = (w0 + j) * ST - g.pad_cols + c;
-                      if (ih < 0 || ih >= g.in_rows || iw < 0 || iw >= g.in_cols) continue;
-                    }
-                    L::fma(acc, win[(j * ST + c) % 3][k * ST + r], f[r * 3 + c]);
+                  constexpr bool by_column = std::is_same<L, HalfSums>::value;
+                  const int r = by_column ? t % 3 : t / 3, c = by_column ? t / 3 : t % 3;
+                  // a tap outside the image is no term of the sum: the zero there and an infinite weight would be one
+                  if (!decltype(every_tap)::value) {
+                    const int ih = (h0 + k) * ST - g.pad_rows + r, iw = (w0 + j) * ST - g.pad_cols + c;
+                    if (ih < 0 || ih >= g.in_rows || iw < 0 || iw >= g.in_cols) continue;
                   }
+                  L::fma(acc, win[(j * ST + c) % 3][k * ST + r], f[r * 3 + c]);
+                }
                 if (k == 0 || second) yp[k * y_row + j * pixel_words] = L::pack(acc);
               }
             }

@@ -1013,18 +1013,18 @@ __device__ __forceinline__ void umma_gemm_body(const GemmArgs& a, const int cta,
                 warp_tma_load_4d(sa + (uint32_t)j * a_box_bytes, &a.a_map[ej.a_map], fb, there ? 0 : 0x40000000, kw + ej.dw, kh + ej.dh, kn);
               }
             } else {
-            warp_tma_load_4d(sa, amap, fb, t.w0, kw + e.dw, kh + e.dh, kn);
-            if (packed) warp_tma_load_4d(sa + (uint32_t)half * a_box_bytes, amap2, fb, c2nd, kw + e2.dw, kh + e2.dh, kn);
-            else warp_tma_load_4d(sa + a_box_bytes, amap, fb, t.w0 + epr, kw + e.dw, kh + e.dh, kn);
-            if constexpr (SPLIT) {  // four boxes of 32 fp32 words
-              if (packed) {
-                warp_tma_load_4d(sa + a_box_bytes, amap, fb, t.w0 + epr, kw + e.dw, kh + e.dh, kn);
-                warp_tma_load_4d(sa + 3u * a_box_bytes, amap2, fb, c2nd + epr, kw + e2.dw, kh + e2.dh, kn);
-              } else {
-                warp_tma_load_4d(sa + 2u * a_box_bytes, amap, fb, t.w0 + 2 * epr, kw + e.dw, kh + e.dh, kn);
-                warp_tma_load_4d(sa + 3u * a_box_bytes, amap, fb, t.w0 + 3 * epr, kw + e.dw, kh + e.dh, kn);
+              warp_tma_load_4d(sa, amap, fb, t.w0, kw + e.dw, kh + e.dh, kn);
+              if (packed) warp_tma_load_4d(sa + (uint32_t)half * a_box_bytes, amap2, fb, c2nd, kw + e2.dw, kh + e2.dh, kn);
+              else warp_tma_load_4d(sa + a_box_bytes, amap, fb, t.w0 + epr, kw + e.dw, kh + e.dh, kn);
+              if constexpr (SPLIT) {  // four boxes of 32 fp32 words
+                if (packed) {
+                  warp_tma_load_4d(sa + a_box_bytes, amap, fb, t.w0 + epr, kw + e.dw, kh + e.dh, kn);
+                  warp_tma_load_4d(sa + 3u * a_box_bytes, amap2, fb, c2nd + epr, kw + e2.dw, kh + e2.dh, kn);
+                } else {
+                  warp_tma_load_4d(sa + 2u * a_box_bytes, amap, fb, t.w0 + 2 * epr, kw + e.dw, kh + e.dh, kn);
+                  warp_tma_load_4d(sa + 3u * a_box_bytes, amap, fb, t.w0 + 3 * epr, kw + e.dw, kh + e.dh, kn);
+                }
               }
-            }
             }
             if (b_mode == B_MN_4) {
               warp_tma_load_4d(sb, &a.b_map, fb, t.nf0, kw, kh, kn);
