@@ -188,13 +188,13 @@ size_t scratch_bytes(int pass, int dtype, const Plan& plan) {
 //   filter gradient, pixels      32 | 2.37   1.79       1.17       0.64       0.59
 //                                64 | 1.40   1.23       0.70       0.70       0.83
 //                               128 | 0.91   0.76       0.77       0.71       1.00
-// On average the choice is 1.4, 3.2 and 0.8 % behind the faster of the two.  The forward pass moves over by the terms of a
+// On average the choice is 2.7, 3.2 and 0.8 % behind the faster of the two.  The forward pass moves over by the terms of a
 // sum or by the work of one image, not of the batch: the kernels add up in different orders, and an image has the same result
-// alone and in any batch.
+// alone and in any batch.  (With 3e5 for an image 1.4 %, but 35 images of 13x18, 27 -> 192 1x1/2, 11.4 us for 6.4.)
 bool general_is_better(int pass, const PdnnConv2DParams& p) {
   const double taps = (double)p.window_rows * p.window_cols, pixels = (double)p.out_rows * p.out_cols;
   const double per_image = pixels * taps * p.channels * p.features, macs = per_image * p.batch;
-  if (pass == PDNN_FORWARD) return taps * p.channels < 64 && per_image < 3e5;
+  if (pass == PDNN_FORWARD) return taps * p.channels < 64 && per_image < 1e5;
   if (pass == PDNN_FILTER_BACKPROP) return pixels * p.batch < 64 && macs < 5e5;
   return taps * p.features < 64.0 * p.stride_rows * p.stride_cols && macs < 5e6;
 }
