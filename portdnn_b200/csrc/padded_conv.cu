@@ -126,12 +126,14 @@ __global__ void __launch_bounds__(kBlock)
 // A count off a multiple of 8, padded.  A multiple of 8 would do, but rows that start inside a 32-byte sector cost the tiles' loads
 // one more sector and often a second line each (bf16, us, 7x45x61 3x3, input gradient: 128 -> 152 features 27.0, 160 16.5,
 // 192 13.1; forward pass, 104 -> 128 channels 14.5, 112 11.7, 128 10.1).  So whole lines of 64 where they
-// are hardly more to copy, else whole sectors of 16; `narrow`: the multiple of 8.
-int padded_count(int n, bool narrow) {
+// are hardly more to copy, else whole sectors of 16; `narrow`: the multiple of 8.  A window of one pixel reads each row once, so that
+// what is copied counts for more (lines / multiples of 8, means over 8535 random layers, tensors 12 to 20 % wider: 1x1 forward
+// 1.02, filter gradient 1.04, a third wider 1.04 and 1.06; 3x3 0.82).
+int padded_count(int n, bool narrow, bool one_pixel) {
   if (n % 8 == 0) return n;
   if (narrow) return (int)round_up((size_t)n, 8);
   const int lines = (int)round_up((size_t)n, 64);
-  return 10ll * lines <= 13ll * n ? lines : (int)round_up((size_t)n, 16);
+  return 10ll * lines <= (one_pixel ? 11ll : 13ll) * n ? lines : (int)round_up((size_t)n, 16);
 }
 
 struct Plan {
@@ -148,9 +150,10 @@ bool plan_with(int pass, int dtype, const PdnnConv2DParams& p, bool narrow, Plan
   if (p.filter_format != 0 && p.filter_format != 2) return false;
   PdnnConv2DParams q = p;
   const void* aligned = reinterpret_cast<const void*>(uintptr_t(256));
-  q.features = padded_count(p.features, narrow);
+  const bool one_pixel = p.window_rows * p.window_cols == 1;
+  q.features = padded_count(p.features, narrow, one_pixel);
   if (!tc_conv_supported(pass, dtype, aligned, aligned, aligned, q)) {
-    q.channels = padded_count(p.channels, narrow);
+    q.channels = padded_count(p.channels, narrow, one_pixel);
     if (!tc_conv_supported(pass, dtype, aligned, aligned, aligned, q)) return false;
   }
   const size_t px_in = (size_t)p.batch * p.in_rows * p.in_cols, px_out = (size_t)p.batch * p.out_rows * p.out_cols;

@@ -124,3 +124,14 @@ def test_stem_filter_gradients(n, h, window, narrow):
     x, dy = _rand(n * h * h * 3, "f16"), _rand(n * p.out_rows * p.out_cols * 64, "f16")
     kernels = launched(lambda: pd.conv2d(pd.FILTER_BACKPROP, x, dy, p))
     assert any("pack_small_c_input_narrow" in k.name for k in kernels) == narrow
+
+
+@pytest.mark.parametrize("c,k,window,wide", [(100, 150, 3, (128, 192)), (100, 150, 1, (112, 160)), (59, 121, 1, (64, 128)), (50, 49, 3, (64, 64)), (50, 49, 1, (64, 64)),
+                                             (49, 130, 3, (64, 144)), (57, 114, 1, (64, 128))])
+def test_widths_of_padded_copies(c, k, window, wide):
+    """Whole lines of 64 where they are at most 1.3 times as much, 1.1 for windows of one pixel; else whole sectors of 16."""
+    p, q = pd.conv_params(4, 30, 30, c, k, window, 1), pd.conv_params(4, 30, 30, *wide, window, 1)
+    _, elems = pd.conv2d_workspace_size(pd.FORWARD, pd.F16, p, pd.ALGO_IM2COL)
+    _, inner = pd.conv2d_workspace_size(pd.FORWARD, pd.F16, q, pd.ALGO_IM2COL)
+    sizes = (2 * 3600 * q.channels, 2 * 3600 * q.features, 2 * window * window * q.channels * q.features, 2 * q.features, 2 * inner)
+    assert 2 * elems == sum(-(-n // 256) * 256 for n in sizes) + 256
