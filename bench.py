@@ -310,9 +310,9 @@ def hbm_operators(torch, pd, workloads, peak_gbs, full=False):
             pb = pd.batchnorm_params(256, 56, 56, 256, training)
             tag = "training" if training else "frozen"
             add("batchnorm forward %s f16" % tag, lambda: pd.batchnorm_forward(x, beta, gamma, mean, var, pb, out=y),
-                (8 if training else 4) * n)
+                4 * n)  # (each tensor once, as in all rows; the gradients read both inputs twice)
             add("batchnorm gradient %s f16" % tag,
-                lambda: pd.batchnorm_gradient(x, dyb, gamma, pb, pop_mean=mean, pop_variance=var, out=y), (10 if training else 8) * n)
+                lambda: pd.batchnorm_gradient(x, dyb, gamma, pb, pop_mean=mean, pop_variance=var, out=y), 6 * n)
         xs = torch.randn(64 * 56 * 56 * 256, device=dev).half()
         ys = torch.empty_like(xs)
         add("softmax forward 64x56x56x256 f16", lambda: pd.softmax(xs, 64, 56, 56, 256, out=ys), 4 * xs.numel())
