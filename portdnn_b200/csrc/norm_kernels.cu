@@ -557,8 +557,8 @@ __global__ void __launch_bounds__(kBlock)
 
 // ---- batch statistics in one pass -------------------------------------------------------------------
 // Per-channel moments of the rows, without a first pass for the mean.  A thread subtracts a value of its own,
-// the mean of its first kBatch rows, from the rows it reads, so that what it adds up is of the size of the
-// deviations however far the channel lies from zero; sets of rows are then merged pairwise (Chan, Golub and
+// the mean of its first kBatch rows (in the gradient, from kSettled rows on, the mean of those), from the rows it reads, so that
+// what it adds up is of the size of the deviations however far the channel lies from zero; sets of rows are then merged pairwise (Chan, Golub and
 // LeVeque: the sums of two sets around their own means, plus the product of the means' differences weighted
 // n_a n_b / (n_a + n_b)), the difference of two means being that of the subtracted values plus that of what is
 // left.  So a large mean enters no sum: in fp32 the variance is off by 6e-8 of itself at a mean of 1000 deviations

@@ -224,22 +224,22 @@ int padded_conv(int pass, int dtype, const void* in, const void* fil, void* out,
   const int sms = device_sm_count();
   size_t need = scratch_bytes(pass, dtype, plan);
   // Scratch that holds copies to multiples of 8 only is used for those, whether the caller brought it or no more is to be had.
-  Plan less;
-  const size_t need_less = plan_with(pass, dtype, p, true, &less) ? scratch_bytes(pass, dtype, less) : need;
-  auto make_do = [&] {
-    if (need_less >= need) return false;
+  auto make_do = [&](size_t at_most) {
+    Plan less;
+    const size_t need_less = plan_with(pass, dtype, p, true, &less) ? scratch_bytes(pass, dtype, less) : need;
+    if (need_less >= need || need_less > at_most) return false;
     plan = less, need = need_less;
     return true;
   };
   char* base = static_cast<char*>(ws);
-  if (base != nullptr && ws_elems * 2 < need && ws_elems * 2 >= need_less) make_do();
+  if (base != nullptr && ws_elems * 2 < need) make_do(ws_elems * 2);
   const bool own = base == nullptr || ws_elems * 2 < need;
   auto allocate = [&] {
     if (cudaMallocAsync(reinterpret_cast<void**>(&base), need, s) == cudaSuccess) return true;
     cudaGetLastError();
     return false;
   };
-  if (own && !allocate() && !(make_do() && allocate())) return kNeedsDirect;  // (the direct kernel reads the tensors where they are)
+  if (own && !allocate() && !(make_do(need) && allocate())) return kNeedsDirect;  // (the direct kernel reads the tensors where they are)
   const PdnnConv2DParams& q = plan.q;
   char* at = reinterpret_cast<char*>(round_up(reinterpret_cast<uintptr_t>(base), 256));
   auto take = [&](size_t bytes) {
