@@ -1247,7 +1247,8 @@ template <typename T, int V, int MODE, int OP>
 __global__ void __launch_bounds__(kBlock)
     pointwise_kernel(int any_op, const T* a, const T* b, T* __restrict__ out, size_t n_packets) {
   overlap_wait();
-  constexpr int U = MODE == 0 && OP >= 0 ? 4 : 2;
+  constexpr bool kOneBody = OP < 0 && MODE != 2 && V > 1;
+  constexpr int U = MODE == 0 && !kOneBody ? 4 : 2;
   const int op = OP >= 0 ? OP : any_op;
   const size_t step = (size_t)gridDim.x * kBlock;
   auto put = [&](size_t i, const float (&av)[V], const float (&bv)[V]) {
@@ -1258,7 +1259,7 @@ __global__ void __launch_bounds__(kBlock)
     store_vec<T, V>(out + i * V, res);
   };
   size_t i = (size_t)blockIdx.x * kBlock + threadIdx.x;
-  if constexpr (OP < 0 && MODE != 2) {
+  if constexpr (kOneBody) {
     for (; i < n_packets; i += U * step) {
       const int count = i + step < n_packets ? U : 1;
       float av[U][V], bv[U][V];

@@ -473,9 +473,10 @@ size_t slices_bytes(const Tiling& t, const PdnnConv2DParams& p) {
 //   input gradient, taps *      16 | 1.77   0.95       0.56       0.41      | 2.24   1.14       0.72       0.56
 //   features / strides          64 | 0.91   0.97       0.74       0.48      | 1.57   1.27       1.02       0.56
 //                              160 | 0.51   0.56       0.50       0.40      | 0.82   0.92       0.84       0.59
+//     (fp32 at stride 1, up to 3e6: 1.13 at 64 to 100; a thread looks at every tap, at stride 2 too, whose terms are a quarter)
 //   filter gradient, pixels     32 | 1.70   0.69                            | 1.93   0.62       0.43
 //                              100 | 0.89   0.47       0.25       0.20      | 1.01   0.53       0.28       0.19
-// On average the choice is 3.2, 4.5 and 0.6 % (16 bits 3.9, 2.7 and 0.5 %) behind the faster of the two.  Fewer than four columns leave most
+// On average the choice is 3.2, 2.7 and 0.6 % (16 bits 3.9, 2.3 and 0.5 %) behind the faster of the two.  Fewer than four columns leave most
 // of a tile idle: 1.8 to 4.4 (sums of up to 64 terms, 1e6 multiply-adds and more), whatever the work.  The forward pass moves over by the terms of a
 // sum or by the work of one image: an image has the same result alone and in any batch.
 bool thread_to_an_output(int pass, int dtype, const PdnnConv2DParams& p) {
@@ -484,9 +485,10 @@ bool thread_to_an_output(int pass, int dtype, const PdnnConv2DParams& p) {
   const bool half = dtype != PDNN_F32;
   if (pass != PDNN_FILTER_BACKPROP) {
     const bool forward = pass == PDNN_FORWARD;
-    const double terms = forward ? taps * p.channels : taps * p.features / ((double)p.stride_rows * p.stride_cols);
+    const double terms = taps * (forward ? p.channels : p.features);
     if ((forward ? p.features : p.channels) < 4 && terms < (half ? 128 : 64)) return true;
-    return forward ? terms < (half ? 128 : 48) && per_image < (half ? 1e6 : 5e5) : terms < (half ? 100 : 48) && macs < (half ? 5e6 : 3e6);
+    if (forward) return terms < (half ? 128 : 48) && per_image < (half ? 1e6 : 5e5);
+    return half ? terms * 2 < 115.0 * (p.stride_rows + p.stride_cols) && macs < 5e6 : terms < 90 && macs < 3e6;
   }
   return pixels * p.batch < 80 && macs < 5e5;
 }
@@ -591,15 +593,17 @@ bool simt_matmul_tiled(int dtype, int tl, int tr, const void* lhs, const void* r
   const Tiling t = choose(m, m, n, k, 1, batches, false, sm_count());
   const long long tiles = (long long)batches * t.n_tiles * t.m_tiles, blocks = tiles * t.splits;
   if (blocks > 0x7FFFFFF0ll) return false;
-  // What each side takes, in us: a thread to an output walks its terms (25 ns each, 45 with lhs transposed, whose terms lie apart) or
-  // the device is full (2.5 multiply-adds per ps); here a step takes 0.45 us or the tiles, remainders and all, fill it (10 per
-  // ps).  Over 11417 random products the choice is 1.5 % behind the faster side on average and slower than a thread to an output
-  // by more than 1 % in one of a hundred.  Measured, thread to an output / here: f16
+  // What each side takes, in us: a thread to an output walks its terms (26 ns each in fp32, 44 in 16 bits, 52 where the terms of lhs, or of
+  // 32 and more rows of rhs, lie apart) or the device is full (2.5 multiply-adds per ps, 1.5 with rows of rhs apart); here a
+  // step takes 0.75 us or the tiles, remainders and all, fill it (10 per ps).  Over 11417 random products the choice is 0.9 % behind the
+  // faster side on average, and slower than a thread to an output by more than 11 % in one of a hundred.  Measured, thread to an output / here: f16
   // 2 x 1008 x 543 51 / 12.4, 2 x 543 x 1008 (rhs transposed) 32 / 11.2, 500 x 2000 x 1001 380 / 122, 1001 x 2000 transposed 1502 / 127;
   // f32 128 x 1024 x 333 33 / 11.8, 16 of 3000 x 37 x 51 37 / 25; and f32 2000 of 16 x 17 x 15 7.3 / 31, 16 of 400 x 13 x 13 3.6 / 7.5,
   // f16 10 x 100 x 11 7.2 / 11, f32 4000000 x 3 x 3 73 / 548.
   const double steps = (k + kTerms - 1) / kTerms, macs = (double)batches * m * n * k;
-  const double walk = 3 + (tl ? 0.045 : 0.025) * k + macs / 2.5e6, here = 6 + 0.45 * steps / t.splits + (double)tiles * kOutputs * steps * kTerms / 1e7;
+  const bool apart = tr && n >= 32;
+  const double term = tl || apart ? 0.052 : tr ? 0.03 : dtype == PDNN_F32 ? 0.026 : 0.044;
+  const double walk = 3 + term * k + macs / (apart ? 1.5e6 : 2.5e6), here = 5 + 0.75 * steps / t.splits + (double)tiles * kOutputs * steps * kTerms / 1e7;
   if (walk <= here) return false;
   SimtArgs g = {};
   g.a = lhs, g.b = rhs, g.out = out;

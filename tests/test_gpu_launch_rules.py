@@ -87,8 +87,8 @@ def test_small_ctas(layer, which, solo):
     ((24, 28, 5, 2, 3), pd.FORWARD, "f32", "direct_forward_kernel"),        # two columns, 45 terms
     ((24, 28, 5, 6, 3), pd.FORWARD, "f32", "direct_forward_kernel"),        # 45 terms, 212 thousand multiply-adds an image
     ((24, 60, 5, 6, 3), pd.FORWARD, "f32", "simt_gemm_kernel"),             # a million
-    ((1, 30, 9, 45, 1), pd.INPUT_BACKPROP, "f32", "direct_input_backprop_kernel"),
-    ((1, 30, 9, 49, 1), pd.INPUT_BACKPROP, "f32", "simt_gemm_kernel"),
+    ((1, 30, 9, 89, 1), pd.INPUT_BACKPROP, "f32", "direct_input_backprop_kernel"),
+    ((1, 30, 9, 91, 1), pd.INPUT_BACKPROP, "f32", "simt_gemm_kernel"),
     ((5, 4, 270, 14, 2), pd.INPUT_BACKPROP, "f16", "direct_input_backprop_kernel"),
     ((5, 4, 270, 18, 2), pd.INPUT_BACKPROP, "f16", "umma_gemm"),            # copies
     ((1, 7, 13, 20, 1), pd.FILTER_BACKPROP, "f16", "direct_filter_backprop_kernel"),
