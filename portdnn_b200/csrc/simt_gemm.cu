@@ -399,7 +399,9 @@ int launch(const SimtArgs& g, unsigned blocks, cudaStream_t s) {
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = (unsigned long long)blocks * kThreads < 4ull * 2048ull * (unsigned long long)device_sm_count() ? 2 : 1;  // as launch_overlapped()
+  // (not with slices, whose second launch is a few blocks: 60x26x25 55 -> 61 1x1/2 filter gradient, replayed from a graph with the caller's
+  // scratch, 19.4 us overlapped, 15.7 not; called 19.8 and 18.4)
+  cfg.numAttrs = g.partial == nullptr && (unsigned long long)blocks * kThreads < 4ull * 2048ull * (unsigned long long)device_sm_count() ? 2 : 1;  // as launch_overlapped()
   cudaLaunchKernelEx(&cfg, simt_gemm_kernel<T, A, B_RUNS, BN>, g);
   return check_launch("fp32 tiles");
 }
