@@ -3921,7 +3921,7 @@ SmallCFbpPlan plan_small_c_fbp(int dtype, const PdnnConv2DParams& p, int sms) {
   const int epr = dtype == PDNN_F32 ? 32 : 64;
   q.sp = plan_small_c(dtype, p);
   q.narrow = dtype != PDNN_F32 && p.channels <= 4 && p.stride_cols % 2 == 0 && p.window_rows >= 3 &&
-             (double)p.batch * p.out_rows * p.out_cols >= ((p.window_rows & 3) % 3 == 0 ? 2e4 : 3e5) &&
+             (double)p.batch * p.out_rows * p.out_cols >= ((p.window_rows & 3) % 3 == 0 ? 2e4 : 1e5) &&
              (size_t)p.batch * q.sp.Hp * (q.sp.Wp + 1) < 0x7FFFFFFFull;
   if (q.narrow) {
     q.sp.Wp = (q.sp.Wp + 1) / 2 * 2;  // rows stay 16-byte aligned
