@@ -10,11 +10,11 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", ["f16", "f32"])
-@pytest.mark.parametrize("case", ["pool3_s1", "pool3_s2", "pool2", "depthwise_s1", "depthwise_s2", "conv1x1", "conv1x1_wide"])
+@pytest.mark.parametrize("case", ["pool3_s1", "pool3_s2", "pool2", "depthwise_s1", "depthwise_s2", "conv1x1", "conv1x1_pair"])
 def test_a_batch_is_its_images(case, dtype):
     dt, g = TORCH_DTYPES[dtype], torch.Generator(device="cuda").manual_seed(3)
     conv = case.startswith("conv")
-    h, w, c, k = (31, 45, 512, 128) if case == "conv1x1_wide" else (61, 45, 136, 72) if conv else (61, 45, 136, 136)
+    h, w, c, k = (31, 45, 512, 128) if case == "conv1x1_pair" else (61, 45, 136, 72) if conv else (61, 45, 136, 136)
     n = (80 << 20) // (h * w * c * dt.itemsize) + 1
     x = torch.randn(n, h, w, c, device="cuda", generator=g).to(dt)
     stride = 2 if case.endswith("s2") or case == "pool2" else 1

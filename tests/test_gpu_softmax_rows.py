@@ -1,4 +1,4 @@
-"""Softmax of few pixels, four warps to a pixel (test_gpu_softmax_batch.py has the lines), beside the one-warp form with more pixels; packets that
+"""Softmax of few pixels: four warps to a pixel, up to one wave of blocks, beside the one-warp form with more pixels; packets that
 fill the block and packets that do not; rows whose maximum lies anywhere, equal values, infinities."""
 import pytest
 import torch
